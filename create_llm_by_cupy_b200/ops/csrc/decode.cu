@@ -1,0 +1,303 @@
+// One-token attention against a KV cache (causal GQA decode).
+//
+// What bounds it: the K and V rows of the valid prefix are read once; at small batch the time is latency - how
+// many loads are in flight - not bandwidth. So:
+//   * one cluster of CTAs per (sequence, KV head), every CTA and every warp of it taking its own 32-key tiles
+//     (a prefix of n keys is n / 32 independent chains instead of four);
+//   * all query heads of the group share each K / V row that was loaded (up to 4 heads per CTA), with 16-byte
+//     loads, a whole half tile in flight per lane;
+//   * the partial softmax states (maximum, sum, weighted values) meet in shared memory, first over the warps of
+//     a CTA, then over the CTAs of the cluster through distributed shared memory: no workspace, no second launch.
+// The previous kernel had one CTA of four warps per QUERY head, each warp walking its keys one by one through a
+// five-step shuffle and an exponential. Device time before -> now: B = 1, 16 / 4 heads of 128, 1801 keys 352 -> 13 us;
+// B = 8, 32 / 8 heads of 128, 3001 keys (98 MB of cache) 742 -> 62 us; B = 1, 12 / 4 heads of 64, 101 keys 20 -> 7 us.
+#include <cooperative_groups.h>
+
+#include "common.cuh"
+
+namespace b200 {
+namespace cg = cooperative_groups;
+
+constexpr int DA_MAX_WARPS = 8;
+constexpr int DA_TILE = 32;          // keys per warp and step: one per lane in the softmax phase
+
+struct DecodeParams {
+  const bf16* q;        // [B, QH, D]
+  const bf16* kc;       // [B, KVH, Tmax, D]
+  const bf16* vc;
+  bf16* out;            // [B, QH, D]
+  const int* lens;      // [B]
+  int QH, KVH, Tmax, groups;    // groups: CTA groups per KV head (RT query heads each)
+  float scale;
+};
+
+__device__ __forceinline__ void unpack16B(const uint4& u, float (&f)[8]) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = __uint_as_float(w[i] << 16);
+    f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+
+// Sums v[r] over the LPK lanes that share a key. With RT = 4 (2) the first two (one) exchange steps also split the
+// heads over the lanes, so the sum costs 5 shuffles instead of 16 at LPK = 16. Returns the sum of head `head`.
+template <int RT, int LPK>
+__device__ __forceinline__ float group_sum(float (&v)[RT], int lane, int& head) {
+  float x;
+  int o = LPK / 2;
+  head = 0;
+  if constexpr (RT == 4) {
+    const bool b1 = (lane & o) != 0;
+    float k0 = b1 ? v[2] : v[0], k1 = b1 ? v[3] : v[1];
+    const float s0 = b1 ? v[0] : v[2], s1 = b1 ? v[1] : v[3];
+    k0 += __shfl_xor_sync(0xffffffffu, s0, o);
+    k1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    o >>= 1;
+    const bool b0 = (lane & o) != 0;
+    x = (b0 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b0 ? k0 : k1, o);
+    o >>= 1;
+    head = (b1 ? 2 : 0) + (b0 ? 1 : 0);
+  } else if constexpr (RT == 2) {
+    const bool b0 = (lane & o) != 0;
+    x = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], o);
+    o >>= 1;
+    head = b0 ? 1 : 0;
+  } else {
+    x = v[0];
+  }
+  for (; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+template <int RT>
+struct alignas(RT * 4) HeadRow {     // one key's scores / weights, one vector load
+  float v[RT];
+};
+
+// 160 registers: three CTAs of four warps, or one of eight, fit an SM.
+// grid (cluster size, KVH * groups, B), cluster (cluster size, 1, 1), block 32 * warps (any number up to 8).
+template <int D, int RT>
+__global__ void __maxnreg__(160)
+decode_attn_kernel(const DecodeParams p) {
+  constexpr int LPK = D / 8;                 // lanes per key, 16 bytes each
+  constexpr int KPS = 32 / LPK;              // keys per load step
+  constexpr int STEPS = DA_TILE / KPS;       // 16 / 8 / 4 for D = 128 / 64 / 32
+  constexpr int HALF = STEPS >= 16 ? 8 : STEPS;    // loads in flight per lane
+  __shared__ HeadRow<RT> s_p[DA_MAX_WARPS][DA_TILE];
+  __shared__ float s_m[DA_MAX_WARPS][RT], s_l[DA_MAX_WARPS][RT];
+  __shared__ float s_o[DA_MAX_WARPS][RT][D];
+  __shared__ float c_m[RT], c_l[RT], c_o[RT][D];        // this CTA's state, read by the cluster
+
+  cg::cluster_group cluster = cg::this_cluster();
+  const int cs = int(gridDim.x), rank = int(blockIdx.x);
+  const int nw = int(blockDim.x) >> 5, warp = int(threadIdx.x) >> 5, lane = int(threadIdx.x) & 31;
+  const int b = blockIdx.z, kvh = int(blockIdx.y) / p.groups, g = int(blockIdx.y) % p.groups;
+  const int R = p.QH / p.KVH;
+  const int h0 = kvh * R + g * RT, nh = min(RT, R - g * RT);
+  const int len = min(p.lens[b], p.Tmax);
+  const int kl = lane / LPK, dl = lane % LPK;           // key slot and 8-element column of this lane
+
+  float qv[RT][8], acc[RT][8], m[RT], l[RT];
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+    uint4 u = make_uint4(0u, 0u, 0u, 0u);
+    if (r < nh) u = *reinterpret_cast<const uint4*>(p.q + (size_t(b) * p.QH + h0 + r) * D + dl * 8);
+    unpack16B(u, qv[r]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) { qv[r][e] *= p.scale; acc[r][e] = 0.f; }
+    m[r] = -INFINITY;
+    l[r] = 0.f;
+  }
+  const bf16* kb = p.kc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D + dl * 8;
+  const bf16* vb = p.vc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D + dl * 8;
+
+  // tile t goes to CTA t % cs, warp (t / cs) % nw: neighbouring tiles on different SMs
+  for (int t = rank + warp * cs; t * DA_TILE < len; t += nw * cs) {
+    const int key0 = t * DA_TILE;
+    uint4 buf[HALF];
+#pragma unroll
+    for (int half = 0; half < STEPS; half += HALF) {
+#pragma unroll
+      for (int s = 0; s < HALF; ++s) {
+        const int key = key0 + (half + s) * KPS + kl;
+        buf[s] = make_uint4(0u, 0u, 0u, 0u);
+        if (key < len) buf[s] = __ldg(reinterpret_cast<const uint4*>(kb + size_t(key) * D));
+      }
+#pragma unroll
+      for (int s = 0; s < HALF; ++s) {
+        float kf[8], v[RT];
+        unpack16B(buf[s], kf);
+#pragma unroll
+        for (int r = 0; r < RT; ++r) {
+          float a = qv[r][0] * kf[0];
+#pragma unroll
+          for (int e = 1; e < 8; ++e) a += qv[r][e] * kf[e];
+          v[r] = a;
+        }
+        int head;
+        const float x = group_sum<RT, LPK>(v, lane, head);
+        if ((lane & (LPK / RT - 1)) == 0) s_p[warp][(half + s) * KPS + kl].v[head] = x;
+      }
+    }
+    // the first values travel while the softmax of the tile is formed
+#pragma unroll
+    for (int s = 0; s < HALF; ++s) {
+      const int key = key0 + s * KPS + kl;
+      buf[s] = make_uint4(0u, 0u, 0u, 0u);
+      if (key < len) buf[s] = __ldg(reinterpret_cast<const uint4*>(vb + size_t(key) * D));
+    }
+    __syncwarp();
+    const bool valid = key0 + lane < len;
+    HeadRow<RT> row = s_p[warp][lane];
+    float corr[RT];
+#pragma unroll
+    for (int r = 0; r < RT; ++r) {
+      const float sc = valid ? row.v[r] : -INFINITY;
+      float mx = sc;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      const float mn = fmaxf(m[r], mx);
+      const float ref = mn == -INFINITY ? 0.f : mn;
+      corr[r] = __expf(m[r] - ref);                     // 0 on the first tile
+      const float pe = valid ? __expf(sc - ref) : 0.f;
+      l[r] = l[r] * corr[r] + pe;                       // lane-local; summed over lanes at the end
+      m[r] = mn;
+      row.v[r] = pe;
+    }
+    s_p[warp][lane] = row;                              // own row: read by this lane only until the barrier
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) acc[r][e] *= corr[r];
+#pragma unroll
+    for (int half = 0; half < STEPS; half += HALF) {
+      if (half > 0) {
+#pragma unroll
+        for (int s = 0; s < HALF; ++s) {
+          const int key = key0 + (half + s) * KPS + kl;
+          buf[s] = make_uint4(0u, 0u, 0u, 0u);
+          if (key < len) buf[s] = __ldg(reinterpret_cast<const uint4*>(vb + size_t(key) * D));
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < HALF; ++s) {
+        float vf[8];
+        unpack16B(buf[s], vf);
+        const HeadRow<RT> w = s_p[warp][(half + s) * KPS + kl];
+#pragma unroll
+        for (int r = 0; r < RT; ++r)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) acc[r][e] += w.v[r] * vf[e];
+      }
+    }
+    __syncwarp();                                       // the next tile overwrites s_p
+  }
+
+  // over the key slots of the warp, then the warps of the CTA
+#pragma unroll
+  for (int r = 0; r < RT; ++r) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], o);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+#pragma unroll
+      for (int o = LPK; o < 32; o <<= 1) acc[r][e] += __shfl_xor_sync(0xffffffffu, acc[r][e], o);
+      if (kl == 0) s_o[warp][r][dl * 8 + e] = acc[r][e];
+    }
+    if (lane == 0) { s_m[warp][r] = m[r]; s_l[warp][r] = l[r]; }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < RT * D; i += blockDim.x) {
+    const int r = i / D, d = i % D;
+    float mx = -INFINITY;
+    for (int w = 0; w < nw; ++w) mx = fmaxf(mx, s_m[w][r]);
+    const float ref = mx == -INFINITY ? 0.f : mx;
+    float ls = 0.f, o = 0.f;
+    for (int w = 0; w < nw; ++w) {
+      const float f = __expf(s_m[w][r] - ref);
+      ls += s_l[w][r] * f;
+      o += s_o[w][r][d] * f;
+    }
+    c_o[r][d] = o;
+    if (d == 0) { c_m[r] = mx; c_l[r] = ls; }
+  }
+  // over the CTAs of the cluster: every CTA finishes its share of the outputs
+  cluster.sync();
+  for (int i = rank * int(blockDim.x) + int(threadIdx.x); i < RT * D; i += cs * int(blockDim.x)) {
+    const int r = i / D, d = i % D;
+    if (r >= nh) break;
+    float mx = -INFINITY;
+    for (int c = 0; c < cs; ++c) mx = fmaxf(mx, *cluster.map_shared_rank(&c_m[r], c));
+    const float ref = mx == -INFINITY ? 0.f : mx;
+    float ls = 0.f, o = 0.f;
+    for (int c = 0; c < cs; ++c) {
+      const float f = __expf(*cluster.map_shared_rank(&c_m[r], c) - ref);
+      ls += *cluster.map_shared_rank(&c_l[r], c) * f;
+      o += *cluster.map_shared_rank(&c_o[r][d], c) * f;
+    }
+    // ls == 0: no valid key, or one whose weight is not a number (then it stays one)
+    p.out[(size_t(b) * p.QH + h0 + r) * D + d] = __float2bfloat16(ls == 0.f ? 0.f : o / ls);
+  }
+  cluster.sync();                                       // peers still read this CTA's state until here
+}
+
+template <int D, int RT>
+static int launch_decode(DecodeParams p, int B, cudaStream_t st) {
+  p.groups = (p.QH / p.KVH + RT - 1) / RT;
+  const long pairs = long(B) * p.KVH * p.groups;
+  const int tiles = (p.Tmax + DA_TILE - 1) / DA_TILE;
+  // 8 CTAs per (sequence, KV head) until there are two per SM without it; fewer where the cache is shorter than
+  // 8 tiles. Up to 8 warps per CTA while at most one CTA per SM exists, else 4 (they share the SM's registers).
+  int cs = 1;
+  while (cs < 8 && cs < tiles && pairs * cs < 4L * num_sms()) cs *= 2;
+  int warps = (tiles + cs - 1) / cs;
+  const int cap = pairs * cs <= num_sms() ? DA_MAX_WARPS : 4;
+  if (warps > cap) warps = cap;
+  if (warps < 1) warps = 1;
+  if (p.KVH * p.groups > 65535 || B > 65535) return static_cast<int>(cudaErrorInvalidValue);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cs, p.KVH * p.groups, B);
+  cfg.blockDim = dim3(32 * warps);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cs;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, decode_attn_kernel<D, RT>, p));
+}
+
+template <int D>
+static int launch_decode_heads(const DecodeParams& p, int B, cudaStream_t st) {
+  const int R = p.QH / p.KVH;
+  if (R == 1) return launch_decode<D, 1>(p, B, st);
+  if (R == 2) return launch_decode<D, 2>(p, B, st);
+  return launch_decode<D, 4>(p, B, st);
+}
+
+}  // namespace b200
+
+using namespace b200;
+
+// out[b, h] = softmax(q[b, h] K^T * scale) V over the first lens[b] (at most Tmax) keys of the caches
+// [B, KVH, Tmax, D]; zeros where lens[b] <= 0.
+B200_API int b200_decode_attn(const void* q, const void* kcache, const void* vcache, void* out, const void* lens,
+                              int B, int QH, int KVH, int Tmax, int D, float scale, cudaStream_t st) {
+  if (B <= 0) return 0;
+  if (QH <= 0 || KVH <= 0 || QH % KVH != 0) return static_cast<int>(cudaErrorInvalidValue);
+  const uintptr_t all = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) |
+                        reinterpret_cast<uintptr_t>(vcache);
+  if ((all & 15) != 0) return static_cast<int>(cudaErrorInvalidValue);
+  DecodeParams p = {static_cast<const bf16*>(q), static_cast<const bf16*>(kcache), static_cast<const bf16*>(vcache),
+                    static_cast<bf16*>(out), static_cast<const int*>(lens), QH, KVH, Tmax, 1, scale};
+  switch (D) {
+    case 32: return launch_decode_heads<32>(p, B, st);
+    case 64: return launch_decode_heads<64>(p, B, st);
+    case 128: return launch_decode_heads<128>(p, B, st);
+    default: return static_cast<int>(cudaErrorInvalidValue);
+  }
+}

@@ -730,80 +730,6 @@ __global__ void __launch_bounds__(FA_THREADS, 1) flash_bwd_dq_kernel(const Flash
   store_acc_rows<D>(dq, aQ + warp * 16 * D * 2, sQ + warp * 16 * D * 2, dqb, p.dq_ts, m0 + warp * 16, T, lane, 1.f, 1.f);
 }
 
-// ================================================================= decode (one new token, KV cache)
-// q [B, QH, D]; cache K/V [B, KVH, Tmax, D] (K already rotated); len[b] keys are valid.
-// One warp per (b, head): keys strided over lanes is wasteful for D-wide dot products, so every
-// lane owns D/32.. elements of the head dim and the warp walks the keys; 4 warps split the keys.
-template <int D>
-__global__ void __launch_bounds__(128) decode_attn_kernel(const bf16* __restrict__ q, const bf16* __restrict__ kc,
-                                                          const bf16* __restrict__ vc, bf16* __restrict__ out,
-                                                          const int* __restrict__ lens, int QH, int KVH, int Tmax,
-                                                          float scale) {
-  constexpr int EPL = (D + 31) / 32;        // elements per lane
-  __shared__ float s_m[4], s_l[4];
-  __shared__ float s_o[4][D];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.x, b = blockIdx.y;
-  const int kvh = h / (QH / KVH);
-  const int len = min(lens[b], Tmax);
-  float qv[EPL];
-#pragma unroll
-  for (int e = 0; e < EPL; ++e) {
-    const int d = lane + e * 32;
-    qv[e] = (d < D) ? __bfloat162float(q[(size_t(b) * QH + h) * D + d]) * scale : 0.f;
-  }
-  const bf16* kb = kc + (size_t(b) * KVH + kvh) * Tmax * D;
-  const bf16* vb = vc + (size_t(b) * KVH + kvh) * Tmax * D;
-  float m = -INFINITY, l = 0.f, acc[EPL];
-#pragma unroll
-  for (int e = 0; e < EPL; ++e) acc[e] = 0.f;
-  for (int t = warp; t < len; t += 4) {
-    float dot = 0.f;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      const int d = lane + e * 32;
-      if (d < D) dot += qv[e] * __bfloat162float(kb[size_t(t) * D + d]);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
-    const float mn = fmaxf(m, dot);
-    const float c = __expf(m - mn), pe = __expf(dot - mn);
-    l = l * c + pe;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      const int d = lane + e * 32;
-      if (d < D) acc[e] = acc[e] * c + pe * __bfloat162float(vb[size_t(t) * D + d]);
-    }
-    m = mn;
-  }
-  if (lane == 0) { s_m[warp] = m; s_l[warp] = l; }
-#pragma unroll
-  for (int e = 0; e < EPL; ++e) {
-    const int d = lane + e * 32;
-    if (d < D) s_o[warp][d] = acc[e];
-  }
-  __syncthreads();
-  if (warp == 0) {
-    float M = fmaxf(fmaxf(s_m[0], s_m[1]), fmaxf(s_m[2], s_m[3]));
-    float L = 0.f;
-    float w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      w[i] = (s_m[i] == -INFINITY) ? 0.f : __expf(s_m[i] - M);
-      L += s_l[i] * w[i];
-    }
-    const float inv = L > 0.f ? 1.f / L : 0.f;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      const int d = lane + e * 32;
-      if (d < D) {
-        const float v = s_o[0][d] * w[0] + s_o[1][d] * w[1] + s_o[2][d] * w[2] + s_o[3][d] * w[3];
-        out[(size_t(b) * QH + h) * D + d] = __float2bfloat16(v * inv);
-      }
-    }
-  }
-}
-
 template <typename K>
 static int set_smem(K kern, int bytes) {
   return static_cast<int>(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -926,24 +852,6 @@ B200_API int b200_flash_bwd(const void* q, const void* k, const void* v, const v
     case 128: return launch_bwd<128>(p, rope, st);
     default: return static_cast<int>(cudaErrorInvalidValue);
   }
-}
-
-B200_API int b200_decode_attn(const void* q, const void* kcache, const void* vcache, void* out, const void* lens,
-                              int B, int QH, int KVH, int Tmax, int D, float scale, cudaStream_t st) {
-  if (B <= 0) return 0;
-  dim3 grid(QH, B);
-#define B200_DEC(DD)                                                                                             \
-  decode_attn_kernel<DD><<<grid, 128, 0, st>>>(static_cast<const bf16*>(q), static_cast<const bf16*>(kcache),    \
-                                               static_cast<const bf16*>(vcache), static_cast<bf16*>(out),        \
-                                               static_cast<const int*>(lens), QH, KVH, Tmax, scale)
-  switch (D) {
-    case 32: B200_DEC(32); break;
-    case 64: B200_DEC(64); break;
-    case 128: B200_DEC(128); break;
-    default: return static_cast<int>(cudaErrorInvalidValue);
-  }
-#undef B200_DEC
-  return static_cast<int>(cudaGetLastError());
 }
 
 // delta[b, h, t] = sum_d dO * O (fp32), the row term of the softmax gradient. strides: o (3), dout (3).

@@ -655,6 +655,8 @@ def decode_attn(q, kcache, vcache, lens, scale=None):
         return torch.einsum("bht,bhtd->bhd", p, vx).to(q.dtype)
     _bf16(q, kcache, vcache)
     assert q.is_contiguous() and kcache.is_contiguous() and vcache.is_contiguous() and lens.dtype == torch.int32
+    # the kernel loads 16 bytes at a time: a view that starts between two such words is copied first
+    q, kcache, vcache = (t if t.data_ptr() % 16 == 0 else t.clone() for t in (q, kcache, vcache))
     out = torch.empty_like(q)
     native.check(_lib().b200_decode_attn(native.ptr(q), native.ptr(kcache), native.ptr(vcache), native.ptr(out),
                                          native.ptr(lens), B, QH, KVH, Tmax, D, _f(scale), native.stream_ptr()),

@@ -1,0 +1,41 @@
+"""Kernels of the decoding path against plain fp32 restatements, at the edges of their tiles."""
+import pytest
+import torch
+
+from create_llm_by_cupy_b200.ops import functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def bf(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("QH,KVH,Tmax,lens", [
+    (2, 2, 1, [1]),                                 # one key, R = 1
+    (6, 2, 33, [31, 32, 33]),                       # edges of a 32-key tile, 3 of 4 head slots used
+    (4, 2, 300, [1, 255, 256, 257, 300]),           # edges of a pass of 8 CTAs, R = 2
+    (16, 2, 2100, [2048, 2100, 5]),                 # 8 query heads per KV head: two CTA groups; several passes
+    (32, 8, 130, [129] * 20),                       # many (sequence, head) pairs: four-warp CTAs
+])
+def test_decode_attention_edges(D, QH, KVH, Tmax, lens):
+    B = len(lens)
+    q, kc, vc = bf(B, QH, D, seed=1), bf(B, KVH, Tmax, D, seed=2), bf(B, KVH, Tmax, D, seed=3)
+    ln = torch.tensor(lens, dtype=torch.int32)
+    for b, n in enumerate(lens):                    # what lies beyond a prefix is never read
+        kc[b, :, n:], vc[b, :, n:] = float("nan"), float("nan")
+    out = F.decode_attn(q.cuda(), kc.cuda(), vc.cuda(), ln.cuda()).float().cpu()
+    ref = F.decode_attn(q.float(), kc.nan_to_num().float(), vc.nan_to_num().float(), ln)
+    # half a bf16 ulp of the result, and fp32 sums over at most 2100 weighted values (|v| < 6)
+    assert ((out - ref).abs() <= 2.0 ** -8 * ref.abs() + 6 * 2100 * 2.0 ** -23).all()
+
+
+def test_decode_attention_empty_long_and_unaligned():
+    q, kc, vc = (bf(*s, seed=i).cuda() for i, s in enumerate([(3, 4, 64), (3, 2, 40, 64), (3, 2, 40, 64)]))
+    out = F.decode_attn(q, kc, vc, torch.tensor([0, -3, 99], dtype=torch.int32, device="cuda"))
+    assert (out[:2] == 0).all()                     # no key; a length past the cache means the whole cache
+    full = F.decode_attn(q, kc, vc, torch.full((3,), 40, dtype=torch.int32, device="cuda"))
+    assert torch.equal(out[2], full[2])
+    shifted = [torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t) for t in (q, kc, vc)]
+    assert torch.equal(F.decode_attn(*shifted, torch.full((3,), 40, dtype=torch.int32, device="cuda")), full)
