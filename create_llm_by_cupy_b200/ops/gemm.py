@@ -13,6 +13,19 @@ from . import native
 
 GEMM_OUT_F32 = 1
 GEMM_ADD_C = 2
+# Few rows: the skinny kernel (weights streamed once, K split over a cluster) instead of 128-row tensor-core tiles.
+# Up to 8 rows it always wins (768 x 768: 3.6 against 6.8 us, 2048 x 11008: 11 / 18, 4096 x 22016: 34 / 43). Beyond
+# that every 64-column CTA reads the activations again, while the tensor-core tiles are bound by their serial walk
+# over K on N / 128 SMs, so the line lies at rows x columns: 16 rows, 4096 x 22016 41 / 33.5 us but 2048 x 11008 13.4 /
+# 17.7; 32 rows, 2048 x 11008 18 / 14 but 11008 x 4096 36 / 52; 64 rows, 768 x 4096 8.1 / 8.0, 2048 x 3072 10.1 / 13.9.
+SKINNY_ROWS = 64
+SKINNY_AREA = 1 << 18
+
+
+def _skinny(M: int, N: int) -> bool:
+    return M <= 8 or (M <= SKINNY_ROWS and (16 if M <= 16 else 32 if M <= 32 else 64) * N < SKINNY_AREA)
+
+
 GEMM_WHOLE_TILES = 8      # CTA-pair kernel: do not split the tiles of a part-filled last round
 
 # Code-path switches (module attributes; tests and the benchmark's baseline arm set them).
@@ -104,6 +117,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         flags |= GEMM_ADD_C
     native.status_tensor()
     impl = impl or GEMM_IMPL
+    if (impl == "2cta" and _skinny(M, N) and not trans_a and not force_fallback and bn == 0 and max_ctas == 0
+            and lda % 8 == 0 and ldb % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0):
+        rc = native.lib().b200_gemm_skinny(
+            native.ptr(a), native.ptr(b), native.ptr(out), native.ptr(add), M, N, K, lda, ldb, ldd, ldc,
+            int(not trans_b), flags & GEMM_OUT_F32, ctypes.c_float(alpha), native.stream_ptr())
+        native.check(rc, "b200_gemm_skinny")
+        native.bump()
+        return out
     if (impl == "2cta" and not force_fallback and bn == 0 and max_ctas == 0 and M >= 256 and N >= 256
             and lda % 8 == 0 and ldb % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0):
         _apply_dynamic()

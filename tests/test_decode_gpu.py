@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from create_llm_by_cupy_b200.ops import functional as F
+from create_llm_by_cupy_b200.ops.gemm import gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -39,3 +40,31 @@ def test_decode_attention_empty_long_and_unaligned():
     assert torch.equal(out[2], full[2])
     shifted = [torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t) for t in (q, kc, vc)]
     assert torch.equal(F.decode_attn(*shifted, torch.full((3,), 40, dtype=torch.int32, device="cuda")), full)
+
+
+@pytest.mark.parametrize("trans_b", [False, True])
+@pytest.mark.parametrize("M,N,K", [
+    (1, 1, 1), (1, 8, 8),                 # smallest
+    (7, 63, 65), (8, 64, 64), (9, 65, 63),  # around one tile of columns, one stage of K, 8 rows
+    (16, 200, 1000), (17, 768, 768),      # ragged K slices of a cluster; 3 row groups
+    (33, 1290, 520), (64, 4104, 2050),    # the widest row count
+    (3, 40000, 136),                      # more column tiles than resident CTAs: no K split
+])
+def test_skinny_gemm_edges(M, N, K, trans_b):
+    pad = lambda n: (n + 7) // 8 * 8      # aligned pitches, ragged extents
+    a = bf(M, pad(K), seed=1).cuda()[:, :K]
+    b = (bf(N, pad(K), seed=2).cuda()[:, :K] if trans_b else bf(K, pad(N), seed=2).cuda()[:, :N])
+    ref = a.double() @ (b.double().t() if trans_b else b.double())
+    bound = a.double().abs() @ (b.double().abs().t() if trans_b else b.double().abs()) * (K * 2.0 ** -23) + 1e-30
+    y = gemm(a, b, trans_b=trans_b, out_dtype=torch.float32, alpha=0.5)
+    assert ((y.double() - 0.5 * ref).abs() <= bound).all()              # fp32 sums
+    c = bf(M, N, seed=3).cuda()
+    want = ref + c.double()
+    z = gemm(a, b, trans_b=trans_b, add=c, out=c)                       # in place, bf16 result
+    assert ((z.double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all()
+
+
+def test_skinny_gemm_reads_nothing_past_its_operands():
+    a, b = torch.full((5, 72), float("nan")).bfloat16().cuda(), torch.full((72, 136), float("nan")).bfloat16().cuda()
+    a[:3, :68], b[:68, :131] = 1.0, 1.0
+    assert (gemm(a[:3, :68], b[:68, :131]) == 68).all()
