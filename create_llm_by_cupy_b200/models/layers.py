@@ -244,6 +244,9 @@ class GroupedQueryAttention:
         B = x.shape[0]
         kqv = F.gemm(x, self.params[0])
         tabs = self._rope(kcache.shape[2], x.device)
+        if F.decode_append_fusable(kqv, kcache, vcache, lens, pos, self.QH, self.KVH):
+            o = F.decode_attn_append(kqv, kcache, vcache, lens, pos, self.QH, self.KVH, tabs[0], tabs[1], self.scale)
+            return F.gemm(o.view(B, self.H), self.params[1], add=residual)
         F.rope_inplace(kqv, tabs[0], tabs[1], 1, self.KVH, self.D, col0=0, pos0=pos)
         F.rope_inplace(kqv, tabs[0], tabs[1], 1, self.QH, self.D, col0=self.KV, pos0=pos)
         k = kqv[:, :self.KV].view(B, self.KVH, self.D)

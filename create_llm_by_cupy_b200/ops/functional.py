@@ -665,6 +665,36 @@ def decode_attn(q, kcache, vcache, lens, scale=None):
     return out
 
 
+def decode_append_fusable(kqv, kcache, vcache, lens, pos: int, QH: int, KVH: int) -> bool:
+    """True when ``decode_attn_append`` runs for the packed projection ``kqv`` [B, (KVH + QH + KVH) * D] and the
+    caches [B, KVH, Tmax, D]."""
+    if not kqv.is_cuda or kcache.dim() != 4:
+        return False
+    B, D = kqv.shape[0], kcache.shape[3]
+    return (D in (32, 64, 128) and QH % KVH == 0 and kqv.shape[1] == (QH + 2 * KVH) * D and kqv.is_contiguous()
+            and kqv.dtype == kcache.dtype == vcache.dtype == torch.bfloat16 and lens.dtype == torch.int32
+            and kcache.shape[:2] == (B, KVH) and kcache.shape == vcache.shape and 0 <= pos < kcache.shape[2]
+            and kcache.is_contiguous() and vcache.is_contiguous()
+            and (kqv.data_ptr() | kcache.data_ptr() | vcache.data_ptr()) % 16 == 0)
+
+
+def decode_attn_append(kqv, kcache, vcache, lens, pos: int, QH: int, KVH: int, cos, sin, scale: float):
+    """Attention of the token at position ``pos`` from its packed projection: rotates K and Q (tables [> pos, D/2]),
+    appends K and V to the caches and attends over the first ``lens[b]`` keys, in one kernel. Returns [B, QH, D].
+    Only where ``decode_append_fusable`` holds."""
+    B, _, Tmax, D = kcache.shape
+    assert cos.dtype == sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+    assert cos.shape[0] > pos and cos.shape[1] == D // 2 and sin.shape == cos.shape
+    out = torch.empty((B, QH, D), dtype=kqv.dtype, device=kqv.device)
+    row = pos * D * 2                                   # bytes of `pos` table rows of D / 2 fp32
+    native.check(_lib().b200_decode_attn_append(
+        native.ptr(kqv), native.ptr(kcache), native.ptr(vcache), native.ptr(out), native.ptr(lens),
+        native.c_void_p(cos.data_ptr() + row), native.c_void_p(sin.data_ptr() + row), B, QH, KVH, Tmax, D,
+        kqv.shape[1], pos, _f(scale), native.stream_ptr()), "decode_attn_append")
+    native.bump()
+    return out
+
+
 # --------------------------------------------------------------------------- cross-entropy rows
 def ce_stats(logits, targets, rmax, rsum, tlogit, col0: int, first: bool):
     """Fold one fp32 logits chunk [M, C] (vocab ids col0..col0+C) into the running row statistics."""

@@ -68,3 +68,36 @@ def test_skinny_gemm_reads_nothing_past_its_operands():
     a, b = torch.full((5, 72), float("nan")).bfloat16().cuda(), torch.full((72, 136), float("nan")).bfloat16().cuda()
     a[:3, :68], b[:68, :131] = 1.0, 1.0
     assert (gemm(a[:3, :68], b[:68, :131]) == 68).all()
+
+
+@pytest.mark.parametrize("QH,KVH,D,Tmax,pos", [(3, 3, 32, 1, 0), (8, 2, 64, 70, 0), (8, 1, 64, 70, 69), (6, 3, 128, 600, 287),
+                                              (12, 4, 64, 600, 288), (32, 8, 128, 300, 256)])
+def test_decode_step_fused_append_matches_separate_kernels(QH, KVH, D, Tmax, pos):
+    """The one-kernel form against rotation, cache copies and attention as separate kernels."""
+    for B in (1, 3, 17):
+        kqv = bf(B, (QH + 2 * KVH) * D, seed=1).cuda()
+        kc, vc = bf(B, KVH, Tmax, D, seed=2).cuda(), bf(B, KVH, Tmax, D, seed=3).cuda()
+        lens = torch.tensor([(pos + 1, pos, Tmax)[i % 3] for i in range(B)], dtype=torch.int32).cuda()   # pos outside / inside
+        cos, sin = F.rope_table(Tmax, D, 10000.0, "cuda")
+        kc1, vc1, row = kc.clone(), vc.clone(), kqv.clone()
+        assert F.decode_append_fusable(kqv, kc, vc, lens, pos, QH, KVH)
+        o = F.decode_attn_append(kqv, kc, vc, lens, pos, QH, KVH, cos, sin, D ** -0.5)
+        assert torch.equal(kqv, row)
+        F.rope_inplace(row, cos, sin, 1, KVH + QH, D, col0=0, pos0=pos)
+        kc1[:, :, pos] = row[:, :KVH * D].view(B, KVH, D)
+        vc1[:, :, pos] = row[:, (KVH + QH) * D:].view(B, KVH, D)
+        assert torch.equal(vc, vc1)
+        # a rotated element may round the other way where the compiler fuses the other product
+        assert ((kc.float() - kc1.float()).abs() <= 2.0 ** -7 * kc1.float().abs()).all()
+        o1 = F.decode_attn(row[:, KVH * D:(KVH + QH) * D].reshape(B, QH, D).contiguous(), kc1, vc1, lens)
+        # one bf16 ulp of q or k moves a score by at most 2^-8 sum |q k| / sqrt(D) (< 0.05 here), values stay below 6
+        assert (o.float() - o1.float()).abs().max() <= 0.05 and (o == o1).float().mean() > 0.9
+
+
+def test_decode_append_form_is_left_where_it_does_not_apply():
+    kqv, kc, vc = bf(2, 512, seed=1).cuda(), bf(2, 2, 40, 64, seed=2).cuda(), bf(2, 2, 40, 64, seed=3).cuda()
+    lens = torch.ones(2, dtype=torch.int32, device="cuda")
+    ok = lambda **kw: F.decode_append_fusable(**{**dict(kqv=kqv, kcache=kc, vcache=vc, lens=lens, pos=3, QH=4, KVH=2), **kw})
+    assert ok()
+    assert not ok(pos=40) and not ok(pos=-1) and not ok(kcache=kc.transpose(1, 2)) and not ok(kqv=kqv[:, ::2])
+    assert not ok(kcache=kc.float()) and not ok(kcache=kc[:1]) and not ok(lens=lens.long()) and not ok(kqv=kqv.cpu())
