@@ -626,6 +626,40 @@ __global__ void add_bf16_kernel(const bf16* __restrict__ a, const bf16* __restri
       out[i] = __float2bfloat16(__bfloat162float(a[i]) + __bfloat162float(b[i]));
 }
 
+// Row-major matrices whose rows do not start on 16-byte boundaries cannot be read by TMA or by 16-byte loads. This
+// copies such a matrix into (or out of) one whose pitch is a multiple of 8: `nseg` column segments, segment s at
+// column s * sseg of the source and s * dseg of the destination, C columns each, the destination's columns [C, W) of a
+// segment set to zero. A thread moves 8 columns; the side that allows it is accessed with 16 bytes, the other one with
+// eight 2-byte accesses that share their L1 lines. Bound by those accesses: 1024 x 5460 (22 MB of traffic) in 9 us.
+__global__ void __launch_bounds__(256)
+repitch_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int R, int nseg, int C, int W, int sseg,
+               int dseg, long long ls, long long ld) {
+  const int chunks = (W + 7) >> 3;
+  const size_t total = size_t(R) * nseg * chunks;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
+    const int c = int(i % chunks) * 8;
+    const size_t rs = i / chunks;
+    const int seg = int(rs % nseg);
+    const size_t row = rs / nseg;
+    const uint16_t* sp = src + row * ls + size_t(seg) * sseg + c;
+    uint16_t* dp = dst + row * ld + size_t(seg) * dseg + c;
+    alignas(16) uint16_t v[8];
+    if (c + 8 <= C && (reinterpret_cast<uintptr_t>(sp) & 15) == 0) {
+      *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(sp);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = c + e < C ? sp[e] : uint16_t(0);
+    }
+    if (c + 8 <= W && (reinterpret_cast<uintptr_t>(dp) & 15) == 0) {
+      *reinterpret_cast<uint4*>(dp) = *reinterpret_cast<const uint4*>(v);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (c + e < W) dp[e] = v[e];
+    }
+  }
+}
+
 static inline int grid_for(size_t work_items, int block) {
   size_t g = (work_items + block - 1) / block;
   const size_t cap = size_t(num_sms()) * 16;
@@ -704,6 +738,16 @@ B200_API int b200_rmsnorm_bwd(const void* dy, const void* x, const void* gamma, 
   B200_CHECK(cudaGetLastError());
   rmsnorm_dgamma_reduce_kernel<<<(H + 31) / 32, 256, 0, st>>>(pp, static_cast<bf16*>(dgamma), rows, H,
                                                                  accumulate_dgamma);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// 2-byte elements; pitches and segment strides in elements. C <= W; src and dst may not overlap.
+B200_API int b200_repitch(const void* src, void* dst, int R, int nseg, int C, int W, int sseg, int dseg, long long ls,
+                          long long ld, cudaStream_t st) {
+  if (R <= 0 || nseg <= 0 || W <= 0) return 0;
+  if (C < 0 || C > W) return static_cast<int>(cudaErrorInvalidValue);
+  repitch_kernel<<<grid_for(size_t(R) * nseg * ((W + 7) / 8), 256), 256, 0, st>>>(
+      static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, nseg, C, W, sseg, dseg, ls, ld);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -1154,19 +1154,21 @@ B200_API int b200_gemm_bf16_2cta_ce_dlogits(const void* A, const void* B, void* 
 // tile through TMA and writes DGV = [d gate | d value] with
 //   d gate = d act * value * s * (1 + gate (1 - s)),  d value = d act * gate * s,  s = sigmoid(gate).
 // I a multiple of 8; every base 16-byte aligned, every pitch a multiple of 8 elements. GV and DGV may not alias.
+// w_rows <= I: rows that W_out has in memory; d(act) of the columns beyond them is zero (an activation padded to
+// a width that is a multiple of 8).
 B200_API int b200_gemm_bf16_2cta_swiglu_bwd(const void* DOUT, const void* WOUT, const void* GV, void* DGV, int M, int I,
-                                            int K, int lda, int ldb, int ldgv, int lddgv, int flags,
+                                            int K, int lda, int ldb, int ldgv, int lddgv, int w_rows,
                                             cudaStream_t stream) {
   if (M <= 0 || I <= 0) return 0;
   const uintptr_t all = reinterpret_cast<uintptr_t>(DOUT) | reinterpret_cast<uintptr_t>(WOUT) |
                         reinterpret_cast<uintptr_t>(GV) | reinterpret_cast<uintptr_t>(DGV);
-  if (K <= 0 || (I % 8) != 0 || GV == nullptr || DGV == nullptr || GV == DGV || (all & 15) != 0 || (lda % 8) != 0 ||
+  if (K <= 0 || (I % 8) != 0 || w_rows <= 0 || w_rows > I || GV == nullptr || DGV == nullptr || GV == DGV || (all & 15) != 0 || (lda % 8) != 0 ||
       (ldb % 8) != 0 || (ldgv % 8) != 0 || (lddgv % 8) != 0)
     return static_cast<int>(cudaErrorInvalidValue);
   Gemm2Params p = base_params(DGV, nullptr, M, I, K, lddgv, 0, G2_WHOLE_TILES | G2_TMA_OUT, 1.0f);
   p.sw_I = I;
   const CUtensorMap* tA = get_tensor_map_2d(DOUT, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = get_tensor_map_2d(WOUT, I, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
+  const CUtensorMap* tB = get_tensor_map_2d(WOUT, w_rows, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
   const CUtensorMap* tG = get_tensor_map_2d(GV, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
   const CUtensorMap* tV = get_tensor_map_2d(static_cast<const bf16*>(GV) + I, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
   const CUtensorMap* tDG = get_tensor_map_2d(DGV, M, I, lddgv, 128, 64, 2, SWIZZLE_128B_);

@@ -15,8 +15,8 @@ import torch
 from . import native
 from .gemm import (gemm, gemm_ce_dlogits, gemm_ce_fusable, gemm_ce_stats, gemm_delta, gemm_delta_fusable,  # noqa: F401
                    gemm_rope, gemm_rope_fusable,
-                   gemm_swiglu, gemm_swiglu_bwd, gemm_swiglu_bwd_fusable, gemm_swiglu_fusable, wgrad_event,
-                   wgrad_gemm, wgrad_join)
+                   gemm_swiglu, gemm_swiglu_bwd, gemm_swiglu_bwd_fusable, gemm_swiglu_fusable, pad_gate_value,
+                   wgrad_event, wgrad_gemm, wgrad_gemm_gate_value, wgrad_join)
 
 _f = ctypes.c_float
 
@@ -101,6 +101,12 @@ CE_EPILOGUE = True
 # delta = rowsum(dO * O) of the attention backward inside the epilogue of the output projection's dgrad GEMM
 # (``gemm.gemm_delta``) instead of a pass of its own.
 DELTA_EPILOGUE = True
+
+
+def gemm_impl_is_pair() -> bool:
+    """The CTA-pair GEMM (with its epilogues) is the selected implementation."""
+    from . import gemm as _g
+    return _g.GEMM_IMPL == "2cta"
 
 
 def _lib():

@@ -70,6 +70,46 @@ def _rowmajor_2d(t: torch.Tensor) -> tuple[torch.Tensor, int]:
     return t, (t.stride(0) if t.size(0) > 1 else max(t.size(1), t.stride(0)))
 
 
+# Operands whose rows do not start on 16-byte boundaries (an FFN width of int(8 H / 3), say) are copied into a pitch
+# that is a multiple of 8 and multiplied on the tensor cores: up to three more launches, about 7 us. The CUDA-core kernel
+# takes such operands as they are, at 0.27 us per 16 of K and 4.7e12 multiply-adds per second: 128 x 128 x 65 3.1 against
+# 9.2 us with the copies, 256 x 256 x 33 3.0 / 11.4, but 2048 x 5460 x 1024 2430 / 50. It stays below both limits.
+PAD_WORK = 1 << 25
+PAD_K = 1024
+# An output with such a pitch goes through an aligned one (and a copy) from this M * N on; below it the epilogue
+# stores element by element (2048 x 2730: 119 us, 24 + 9 with the copy).
+PAD_OUT_AREA = 1 << 16
+
+
+def repitch(src: torch.Tensor, dst: torch.Tensor, cols: int, width: int, nseg: int = 1, sseg: int = 0, dseg: int = 0):
+    """Copy ``cols`` columns of each of ``nseg`` column segments of ``src`` [R, ...] to ``dst`` [R, ...] (bf16; segment s at
+    columns ``s * sseg`` / ``s * dseg``), zeros in the columns up to ``width`` of a segment of ``dst``."""
+    assert src.is_cuda and src.element_size() == dst.element_size() == 2 and src.stride(1) == dst.stride(1) == 1
+    native.status_tensor()
+    native.check(native.lib().b200_repitch(
+        native.ptr(src), native.ptr(dst), src.shape[0], nseg, cols, width, sseg, dseg, ctypes.c_longlong(src.stride(0)),
+        ctypes.c_longlong(dst.stride(0)), native.stream_ptr()), "repitch")
+    native.bump()
+    return dst
+
+
+def _padded(t: torch.Tensor, ld: int) -> tuple[torch.Tensor, int]:
+    """(``t``, pitch) in rows that start on 16-byte boundaries (a copy when they do not already)."""
+    if ld % 8 == 0 and t.data_ptr() % 16 == 0:
+        return t, ld
+    rows, cols = t.shape
+    buf = torch.empty((rows, (cols + 7) // 8 * 8), dtype=t.dtype, device=t.device)
+    return repitch(t, buf, cols, buf.shape[1])[:, :cols], buf.shape[1]
+
+
+def _copy_rows(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
+    """``dst.copy_(src)`` for 2-D matrices of one dtype (bf16 or fp32) and any pitch."""
+    if src.dtype == torch.float32:
+        src, dst = src.view(torch.bfloat16), dst.view(torch.bfloat16)
+    repitch(src, dst, src.shape[1], src.shape[1])
+    return dst
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bool = False,
          out: torch.Tensor | None = None, add: torch.Tensor | None = None,
          out_dtype: torch.dtype | None = None, alpha: float = 1.0, bn: int = 0,
@@ -117,6 +157,19 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         flags |= GEMM_ADD_C
     native.status_tensor()
     impl = impl or GEMM_IMPL
+    if impl == "2cta" and not force_fallback and bn == 0 and max_ctas == 0:
+        if (lda % 8 or ldb % 8 or (a.data_ptr() | b.data_ptr()) % 16) and M * N > 0 and (
+                M * N * K >= PAD_WORK or K >= PAD_K):
+            (a, lda), (b, ldb) = _padded(a, lda), _padded(b, ldb)
+        es = out.element_size()
+        if (M >= 256 and N >= 256 and M * N >= PAD_OUT_AREA and lda % 8 == 0 and ldb % 8 == 0
+                and (a.data_ptr() | b.data_ptr()) % 16 == 0 and (ldd * es % 16 or out.data_ptr() % 16)):
+            tmp = torch.empty((M, (N + 7) // 8 * 8), dtype=out_dtype, device=a.device)[:, :N]
+            if add is not None:
+                _copy_rows(add, tmp)
+            gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=tmp, add=None if add is None else tmp, alpha=alpha)
+            _copy_rows(tmp, out)
+            return out
     if (impl == "2cta" and _skinny(M, N) and not trans_a and not force_fallback and bn == 0 and max_ctas == 0
             and lda % 8 == 0 and ldb % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0):
         rc = native.lib().b200_gemm_skinny(
@@ -243,10 +296,11 @@ def gemm_swiglu(x: torch.Tensor, w_gate_val: torch.Tensor, keep_gv: bool = True)
 
 
 def gemm_swiglu_bwd_fusable(dout: torch.Tensor, w_out: torch.Tensor, gv: torch.Tensor) -> bool:
-    """True when ``gemm_swiglu_bwd`` runs as one kernel (``dout`` [M, H], ``w_out`` [I, H], ``gv`` [M, 2 I], bf16)."""
+    """True when ``gemm_swiglu_bwd`` runs as one kernel (``dout`` [M, H], ``w_out`` [I, H], ``gv`` [M, 2 I], bf16; I of
+    ``gv`` may be the width of ``w_out`` rounded up to a multiple of 8)."""
     if not (dout.is_cuda and GEMM_IMPL == "2cta" and _tma_ok(dout, w_out, gv)):
         return False
-    I = w_out.shape[0]
+    I = (w_out.shape[0] + 7) // 8 * 8
     return dout.shape[0] >= 256 and I >= 256 and I % 8 == 0 and gv.shape == (dout.shape[0], 2 * I)
 
 
@@ -255,14 +309,14 @@ def gemm_swiglu_bwd(dout: torch.Tensor, w_out: torch.Tensor, gv: torch.Tensor) -
     projection ``gv``: the gradient of the activation, ``dout @ w_out^T``, exists only in tensor memory; the GEMM's
     epilogue reads the gate / value tiles and writes the two gradients. Only where ``gemm_swiglu_bwd_fusable``."""
     M, K = dout.shape
-    I = w_out.shape[0]
+    I = gv.shape[1] // 2
     assert gemm_swiglu_bwd_fusable(dout, w_out, gv)
     dgv = torch.empty_like(gv)
     native.status_tensor()
     _apply_dynamic()
     rc = native.lib().b200_gemm_bf16_2cta_swiglu_bwd(
         native.ptr(dout), native.ptr(w_out), native.ptr(gv), native.ptr(dgv), M, I, K, dout.stride(0), w_out.stride(0),
-        gv.stride(0), dgv.stride(0), 0, native.stream_ptr())
+        gv.stride(0), dgv.stride(0), w_out.shape[0], native.stream_ptr())
     native.check(rc, "b200_gemm_bf16_2cta_swiglu_bwd")
     native.bump()
     return dgv
@@ -426,6 +480,33 @@ def wgrad_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None
         res = gemm(a, b, trans_a=True, out=out)
     a.record_stream(ws)
     b.record_stream(ws)
+    return res
+
+
+def pad_gate_value(w: torch.Tensor, I: int) -> torch.Tensor:
+    """``[gate | value]`` [R, 2 I] with both halves padded by zero columns to a multiple of 8: [R, 2 Ip]."""
+    Ip = (I + 7) // 8 * 8
+    out = torch.empty((w.shape[0], 2 * Ip), dtype=w.dtype, device=w.device)
+    return repitch(w, out, I, Ip, 2, I, Ip)
+
+
+def wgrad_gemm_gate_value(x: torch.Tensor, dgv: torch.Tensor, I: int, out: torch.Tensor | None = None) -> torch.Tensor:
+    """``x^T @ dgv`` without the padding columns of ``dgv`` [M, 2 Ip] (see ``pad_gate_value``): [K, 2 I], on the
+    weight-gradient stream like ``wgrad_gemm``."""
+    def compute():
+        full = gemm(x, dgv, trans_a=True)
+        dst = torch.empty((x.shape[1], 2 * I), dtype=x.dtype, device=x.device) if out is None else out
+        return repitch(full, dst, I, I, 2, dgv.shape[1] // 2, I)
+
+    if not WGRAD_OVERLAP:
+        return compute()
+    ws = _wgrad_stream(x.device)
+    ws.wait_stream(torch.cuda.current_stream(x.device))
+    _wgrad_pending[x.device.index] = True
+    with torch.cuda.stream(ws):
+        res = compute()
+    x.record_stream(ws)
+    dgv.record_stream(ws)
     return res
 
 

@@ -1,0 +1,75 @@
+"""GEMM operands and FFN widths whose rows do not start on 16-byte boundaries."""
+import pytest
+import torch
+
+from create_llm_by_cupy_b200.models.layers import SwiGLU
+from create_llm_by_cupy_b200.ops import functional as F
+from create_llm_by_cupy_b200.ops import gemm as G
+
+pytestmark = pytest.mark.gpu
+
+
+def bf(*shape, seed, std=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * std).to(torch.bfloat16).cuda()
+
+
+@pytest.mark.parametrize("R,nseg,C,W,extra", [(1, 1, 1, 1, 0), (3, 1, 8, 8, 1), (5, 2, 7, 8, 0), (300, 2, 1365, 1368, 0),
+                                              (17, 1, 100, 104, 3), (2, 3, 16, 16, 5)])
+def test_repitch(R, nseg, C, W, extra):
+    src = bf(R, nseg * C + extra, seed=1)
+    dst = torch.full((R, nseg * W), float("nan"), dtype=torch.bfloat16, device="cuda")
+    G.repitch(src, dst, C, W, nseg, C, W)
+    d3 = dst.view(R, nseg, W)
+    assert torch.equal(d3[:, :, :C], src[:, :nseg * C].reshape(R, nseg, C)) and (d3[:, :, C:] == 0).all()
+    back = torch.full_like(src, 7.0)
+    G.repitch(dst, back, C, C, nseg, W, C)
+    assert torch.equal(back[:, :nseg * C], src[:, :nseg * C]) and (back[:, nseg * C:] == 7.0).all()
+
+
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(5, 3, 7), (63, 65, 1031), (100, 301, 1203), (257, 259, 633), (300, 1365, 130)])
+def test_gemm_with_odd_pitches(M, N, K, trans_a, trans_b, out_dtype):
+    a, b = bf(*((K, M) if trans_a else (M, K)), seed=1), bf(*((N, K) if trans_b else (K, N)), seed=2)
+    c = bf(M, N, seed=3).to(out_dtype)
+    ref = (a.double().t() if trans_a else a.double()) @ (b.double().t() if trans_b else b.double())
+    bound = (a.double().abs().t() if trans_a else a.double().abs()) @ (b.double().abs().t() if trans_b else b.double().abs())
+    bound = bound * (K * 2.0 ** -23) + 2.0 ** -22
+    ulp = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -23
+    for add in (None, c):
+        want = ref if add is None else ref + c.double()
+        y = G.gemm(a, b, trans_a=trans_a, trans_b=trans_b, add=add, out_dtype=out_dtype)
+        assert y.is_contiguous() and ((y.double() - want).abs() <= bound + ulp * want.abs()).all()
+    z = torch.full((M * N + 1,), 3.0, dtype=out_dtype, device="cuda")          # nothing is written past a misaligned output
+    G.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=z[1:].view(M, N))
+    assert z[0] == 3.0 and torch.equal(z[1:].view(M, N), G.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out_dtype=out_dtype))
+
+
+@pytest.mark.parametrize("M,H,I", [(256, 128, 257), (300, 512, 1365), (1000, 1024, 2730), (255, 512, 1365)])
+def test_swiglu_layer_with_odd_width(M, H, I):
+    layer = SwiGLU(H, 2, device="cuda", ffn_size=I, generator=torch.Generator().manual_seed(0))
+    x, res, dout = bf(M, H, seed=1), bf(M, H, seed=2), bf(M, H, seed=3)
+    cpu = SwiGLU(H, 2, dtype=torch.float32, ffn_size=I)
+    cpu.params = [p.float().cpu() for p in layer.params]
+    want = cpu.forward(x.float().cpu(), residual=res.float().cpu())
+    wdx = cpu.backward(dout.float().cpu())
+    for keep in (True, False):                     # gate kept from the forward, or recomputed in the backward
+        layer.cache_gate = keep
+        out = layer.forward(x, residual=res)
+        into = [torch.full_like(p, float("nan")) for p in layer.params]
+        dx = layer.backward(dout, grad_out=into if keep else None)
+        F.wgrad_join(dx.device)
+        for got, ref in zip((out, dx, *layer.grads), (want, wdx, *cpu.grads)):
+            # three bf16 tensors lie between the inputs and a gradient: 2^-9 each, four times that for the norm
+            assert got.is_contiguous() and got.shape == ref.shape
+            assert (got.float().cpu() - ref).norm() <= 12 * 2.0 ** -9 * ref.norm()
+        if keep:
+            assert all(g.data_ptr() == i.data_ptr() for g, i in zip(layer.grads, into))
+    assert layer.forward(x, train_flg=False).shape == (M, H)
+
+
+def test_gemm_one_row_without_a_pitch():
+    row = bf(1029, seed=1)[None].expand(1, -1).as_strided((1, 1029), (0, 1))      # row stride 0
+    b = bf(1029, 37, seed=2)
+    want = row.double() @ b.double()
+    assert ((G.gemm(row, b).double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
