@@ -301,6 +301,8 @@ class SwiGLU:
         where that form exists (one kernel, the projection is only written when the backward will read it),
         else the GEMM followed by the activation kernel."""
         if F.SWIGLU_EPILOGUE and getattr(self, "pending_gather", None) is None:
+            if not keep_gv and F.gemm_skinny_swiglu_fusable(x, self.params[0]):
+                return None, F.gemm_skinny_swiglu(x, self.params[0])
             if F.gemm_swiglu_fusable(x, self.params[0]):
                 return F.gemm_swiglu(x, self.params[0], keep_gv=keep_gv)
             if self._padded_width(x):

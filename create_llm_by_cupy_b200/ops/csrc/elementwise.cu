@@ -682,6 +682,10 @@ B200_API int b200_rmsnorm_fwd(const void* x, const void* gamma, void* y, void* r
     rmsnorm_fwd_scalar_kernel<<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
   } else if (H <= 256) {
     rmsnorm_fwd_kernel<1><<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+  } else if (H <= 1024 && M <= num_sms()) {
+    // a row per CTA while there is an SM for each: one chunk per thread instead of a chain of up to four per lane
+    // (one row of 768: 3.3 -> 2.5 us)
+    rmsnorm_fwd_cta_kernel<1, 1><<<M, 256, 0, st>>>(xp, gp, yp, rp, M, H, eps);
   } else if (H <= 1024) {
     rmsnorm_fwd_kernel<4><<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
   } else if (H <= 8192) {

@@ -31,6 +31,7 @@ struct SkinnyParams {
   void* D;
   int M, N, K, lda, ldb, ldd, ldc;
   int out_f32, kslice;                     // kslice: k range of one CTA, a multiple of SK_TK
+  int I;                                   // GLU: B = [gate | value], N = 2 I, D [M, I] = silu(gate) * value
   float alpha;
 };
 
@@ -66,16 +67,20 @@ __device__ __forceinline__ uint32_t sw_addr(uint32_t base, int row, int chunk) {
 
 // One stage: the 64 x 64 weight tile and the [8 MT, 64] token tile at k0. Bytes past K, N or M arrive as zeros
 // (cp.async with a short source size; the address of a skipped chunk is the matrix base).
-template <int MT, bool K_ROWS>
+template <int MT, bool K_ROWS, bool GLU>
 __device__ __forceinline__ void skinny_load(const SkinnyParams& p, uint32_t stage, int n0, int k0, int k_end) {
   const int tid = threadIdx.x;
 #pragma unroll
   for (int i = 0; i < SK_W_BYTES / 16 / SK_THREADS; ++i) {
     const int idx = tid + i * SK_THREADS, row = idx >> 3, chunk = idx & 7;
     const int k = K_ROWS ? k0 + row : k0 + chunk * 8;
-    const int n = K_ROWS ? n0 + chunk * 8 : n0 + row;
+    int n = K_ROWS ? n0 + chunk * 8 : n0 + row;
     int left;                                             // elements of this chunk inside the matrix
-    if (K_ROWS) left = k < k_end ? p.N - n : 0;
+    if (GLU) {                                            // 32 gate columns beside the 32 value columns of the same index
+      n = n0 + (chunk & 3) * 8;
+      left = k < k_end ? p.I - n : 0;
+      n += chunk < 4 ? 0 : p.I;
+    } else if (K_ROWS) left = k < k_end ? p.N - n : 0;
     else left = n < p.N ? k_end - k : 0;
     left = left < 0 ? 0 : (left > 8 ? 8 : left);
     const bf16* src = left > 0 ? (K_ROWS ? p.B + size_t(k) * p.ldb + n : p.B + size_t(n) * p.ldb + k) : p.B;
@@ -91,14 +96,15 @@ __device__ __forceinline__ void skinny_load(const SkinnyParams& p, uint32_t stag
 }
 
 // grid (k slices, column tiles), cluster (k slices, 1, 1)
-template <int MT, bool K_ROWS>
+template <int MT, bool K_ROWS, bool GLU>
 __global__ void __launch_bounds__(SK_THREADS)
 gemm_skinny_kernel(const SkinnyParams p) {
   using S = SkinnySmem<MT>;
   extern __shared__ __align__(128) uint8_t smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int ks = int(gridDim.x), rank = int(blockIdx.x);
-  const int n0 = int(blockIdx.y) * SK_TN;
+  constexpr int kOut = GLU ? SK_TN / 2 : SK_TN;  // output columns of a CTA
+  const int n0 = int(blockIdx.y) * kOut;
   const int k_begin = rank * p.kslice, k_end = min(p.K, k_begin + p.kslice);
   const int steps = k_end > k_begin ? (k_end - k_begin + SK_TK - 1) / SK_TK : 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -112,7 +118,7 @@ gemm_skinny_kernel(const SkinnyParams p) {
 
 #pragma unroll
   for (int s = 0; s < S::kStages - 1; ++s) {
-    if (s < steps) skinny_load<MT, K_ROWS>(p, base + s * S::kStageBytes, n0, k_begin + s * SK_TK, k_end);
+    if (s < steps) skinny_load<MT, K_ROWS, GLU>(p, base + s * S::kStageBytes, n0, k_begin + s * SK_TK, k_end);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   const int mi = lane >> 3, mr = lane & 7;       // ldmatrix: matrix and row that this lane addresses
@@ -121,7 +127,7 @@ gemm_skinny_kernel(const SkinnyParams p) {
     __syncthreads();                             // stage s has landed; everyone has left stage s - 1
     const int nx = s + S::kStages - 1;
     if (nx < steps)
-      skinny_load<MT, K_ROWS>(p, base + (nx % S::kStages) * S::kStageBytes, n0, k_begin + nx * SK_TK, k_end);
+      skinny_load<MT, K_ROWS, GLU>(p, base + (nx % S::kStages) * S::kStageBytes, n0, k_begin + nx * SK_TK, k_end);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const uint32_t sw = base + (s % S::kStages) * S::kStageBytes, sa = sw + SK_W_BYTES;
     uint32_t w[SK_TK / 16][4];
@@ -154,11 +160,17 @@ gemm_skinny_kernel(const SkinnyParams p) {
       sum[(t * 8 + (lane & 3) * 2 + (e & 1)) * SK_TN + warp * 16 + (lane >> 2) + (e >> 1) * 8] = acc[t][e];
   cluster.sync();
   const int rows = min(p.M, MT * 8);
-  for (int i = rank * SK_THREADS + int(threadIdx.x); i < rows * SK_TN; i += ks * SK_THREADS) {
-    const int row = i / SK_TN, col = n0 + i % SK_TN;
-    if (col >= p.N) continue;
+  for (int i = rank * SK_THREADS + int(threadIdx.x); i < rows * kOut; i += ks * SK_THREADS) {
+    const int row = i / kOut, col = n0 + i % kOut, at = row * SK_TN + i % kOut;
+    if (col >= (GLU ? p.I : p.N)) continue;
     float v = 0.f;
-    for (int c = 0; c < ks; ++c) v += cluster.map_shared_rank(sum, c)[i];
+    for (int c = 0; c < ks; ++c) v += cluster.map_shared_rank(sum, c)[at];
+    if constexpr (GLU) {
+      float u = 0.f;
+      for (int c = 0; c < ks; ++c) u += cluster.map_shared_rank(sum, c)[at + kOut];
+      static_cast<bf16*>(p.D)[size_t(row) * p.ldd + col] = __float2bfloat16(v / (1.f + __expf(-v)) * u);
+      continue;
+    }
     v *= p.alpha;
     if (p.out_f32) {
       if (p.C) v += static_cast<const float*>(p.C)[size_t(row) * p.ldc + col];
@@ -171,12 +183,12 @@ gemm_skinny_kernel(const SkinnyParams p) {
   cluster.sync();                                // peers read this CTA's sums until here
 }
 
-template <int MT, bool K_ROWS>
+template <int MT, bool K_ROWS, bool GLU>
 static int launch_skinny(SkinnyParams p, cudaStream_t st) {
   using S = SkinnySmem<MT>;
-  auto kern = gemm_skinny_kernel<MT, K_ROWS>;
+  auto kern = gemm_skinny_kernel<MT, K_ROWS, GLU>;
   if (S::kTotal > 48 * 1024) B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-  const int tiles = (p.N + SK_TN - 1) / SK_TN, ksteps = (p.K + SK_TK - 1) / SK_TK;
+  const int tiles = GLU ? (2 * p.I + SK_TN - 1) / SK_TN : (p.N + SK_TN - 1) / SK_TN, ksteps = (p.K + SK_TK - 1) / SK_TK;
   if (tiles > 65535) return static_cast<int>(cudaErrorInvalidValue);
   // k slices: as many as keep the GPU's resident CTAs (about 4 per SM) filled once, at most 8 (a portable cluster)
   // and at least 2 stages each
@@ -198,12 +210,12 @@ static int launch_skinny(SkinnyParams p, cudaStream_t st) {
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, p));
 }
 
-template <bool K_ROWS>
+template <bool K_ROWS, bool GLU>
 static int launch_skinny_rows(const SkinnyParams& p, cudaStream_t st) {
-  if (p.M <= 8) return launch_skinny<1, K_ROWS>(p, st);
-  if (p.M <= 16) return launch_skinny<2, K_ROWS>(p, st);
-  if (p.M <= 32) return launch_skinny<4, K_ROWS>(p, st);
-  return launch_skinny<8, K_ROWS>(p, st);
+  if (p.M <= 8) return launch_skinny<1, K_ROWS, GLU>(p, st);
+  if (p.M <= 16) return launch_skinny<2, K_ROWS, GLU>(p, st);
+  if (p.M <= 32) return launch_skinny<4, K_ROWS, GLU>(p, st);
+  return launch_skinny<8, K_ROWS, GLU>(p, st);
 }
 
 }  // namespace b200
@@ -220,6 +232,20 @@ B200_API int b200_gemm_skinny(const void* A, const void* B, void* D, const void*
       (lda % 8) != 0 || (ldb % 8) != 0)
     return static_cast<int>(cudaErrorInvalidValue);
   SkinnyParams p = {static_cast<const bf16*>(A), static_cast<const bf16*>(B), C, D, M, N, K, lda, ldb, ldd, ldc,
-                    out_f32, 0, alpha};
-  return b_k_rows ? launch_skinny_rows<true>(p, stream) : launch_skinny_rows<false>(p, stream);
+                    out_f32, 0, 0, alpha};
+  return b_k_rows ? launch_skinny_rows<true, false>(p, stream) : launch_skinny_rows<false, false>(p, stream);
+}
+
+// ACT[M, I] = silu(A W_gate) * (A W_value) for B = [W_gate | W_value] ([K, 2 I] row-major), M <= 64, I a multiple of 8:
+// the activation in the epilogue of the few-rows GEMM (one launch and one round trip of the projection less per block of
+// a decoded token).
+B200_API int b200_gemm_skinny_swiglu(const void* A, const void* B, void* ACT, int M, int I, int K, int lda, int ldb,
+                                     int ldact, cudaStream_t stream) {
+  if (M <= 0 || I <= 0) return 0;
+  if (K <= 0 || M > 64 || (I % 8) != 0 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) != 0 ||
+      (lda % 8) != 0 || (ldb % 8) != 0)
+    return static_cast<int>(cudaErrorInvalidValue);
+  SkinnyParams p = {static_cast<const bf16*>(A), static_cast<const bf16*>(B), nullptr, ACT, M, 2 * I, K, lda, ldb, ldact,
+                    0, 0, 0, I, 1.f};
+  return launch_skinny_rows<true, true>(p, stream);
 }

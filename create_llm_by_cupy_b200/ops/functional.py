@@ -13,7 +13,7 @@ import math
 import torch
 
 from . import native
-from .gemm import (gemm, gemm_ce_dlogits, gemm_ce_fusable, gemm_ce_stats, gemm_delta, gemm_delta_fusable,  # noqa: F401
+from .gemm import (gemm, gemm_skinny_swiglu, gemm_skinny_swiglu_fusable, gemm_ce_dlogits, gemm_ce_fusable, gemm_ce_stats, gemm_delta, gemm_delta_fusable,  # noqa: F401
                    gemm_rope, gemm_rope_fusable,
                    gemm_swiglu, gemm_swiglu_bwd, gemm_swiglu_bwd_fusable, gemm_swiglu_fusable, pad_gate_value,
                    wgrad_event, wgrad_gemm, wgrad_gemm_gate_value, wgrad_join)

@@ -295,6 +295,27 @@ def gemm_swiglu(x: torch.Tensor, w_gate_val: torch.Tensor, keep_gv: bool = True)
     return gv, act
 
 
+def gemm_skinny_swiglu_fusable(x: torch.Tensor, w_gate_val: torch.Tensor) -> bool:
+    """True when ``gemm_skinny_swiglu(x, w_gate_val)`` runs: few rows (``x`` [M, K], ``w_gate_val`` [K, 2 I], bf16)."""
+    return (x.is_cuda and GEMM_IMPL == "2cta" and x.dim() == 2 and w_gate_val.shape[1] % 16 == 0
+            and 0 < x.shape[0] and _skinny(x.shape[0], w_gate_val.shape[1]) and _tma_ok(x, w_gate_val))
+
+
+def gemm_skinny_swiglu(x: torch.Tensor, w_gate_val: torch.Tensor) -> torch.Tensor:
+    """``silu(x @ W_gate) * (x @ W_value)`` [M, I] for few rows, in one kernel that stores only the activation. Only where
+    ``gemm_skinny_swiglu_fusable`` holds."""
+    M, K = x.shape
+    I = w_gate_val.shape[1] // 2
+    assert gemm_skinny_swiglu_fusable(x, w_gate_val)
+    act = torch.empty((M, I), dtype=torch.bfloat16, device=x.device)
+    native.status_tensor()
+    native.check(native.lib().b200_gemm_skinny_swiglu(
+        native.ptr(x), native.ptr(w_gate_val), native.ptr(act), M, I, K, x.stride(0), w_gate_val.stride(0), I,
+        native.stream_ptr()), "b200_gemm_skinny_swiglu")
+    native.bump()
+    return act
+
+
 def gemm_swiglu_bwd_fusable(dout: torch.Tensor, w_out: torch.Tensor, gv: torch.Tensor) -> bool:
     """True when ``gemm_swiglu_bwd`` runs as one kernel (``dout`` [M, H], ``w_out`` [I, H], ``gv`` [M, 2 I], bf16; I of
     ``gv`` may be the width of ``w_out`` rounded up to a multiple of 8)."""

@@ -101,3 +101,25 @@ def test_decode_append_form_is_left_where_it_does_not_apply():
     assert ok()
     assert not ok(pos=40) and not ok(pos=-1) and not ok(kcache=kc.transpose(1, 2)) and not ok(kqv=kqv[:, ::2])
     assert not ok(kcache=kc.float()) and not ok(kcache=kc[:1]) and not ok(lens=lens.long()) and not ok(kqv=kqv.cpu())
+
+
+@pytest.mark.parametrize("M,I,K", [(1, 8, 8), (3, 40, 72), (8, 2048, 768), (9, 5504, 2048), (17, 264, 130), (64, 1000, 512)])
+def test_skinny_swiglu_edges(M, I, K):
+    x, w = bf(M, (K + 7) // 8 * 8, seed=1).cuda()[:, :K], (bf(K, 2 * I, seed=2).float() * K ** -0.5).bfloat16().cuda()
+    assert F.gemm_skinny_swiglu_fusable(x, w)
+    g, v = (x.double() @ w.double()).chunk(2, 1)
+    want = torch.nn.functional.silu(g) * v
+    # the activation's slope is at most 1.1 |v| in the gate and |g| in the value, both fp32 sums over K terms below 30
+    tol = 2.0 ** -8 * want.abs() + (1.1 * v.abs() + g.abs() + 1e-3) * 30 * K * 2.0 ** -23 + 1e-5 * want.abs()
+    assert ((F.gemm_skinny_swiglu(x, w).double() - want).abs() <= tol).all()
+
+
+@pytest.mark.parametrize("H", [264, 768, 1024])
+@pytest.mark.parametrize("M", [1, 5, 148, 149])
+def test_rmsnorm_few_rows(M, H):
+    x, gamma = bf(M, H, seed=1).cuda(), bf(H, seed=2).cuda()
+    y, rstd = F.rmsnorm_fwd(x, gamma)
+    r = torch.rsqrt(x.double().square().mean(-1) + 1e-6)
+    want = x.double() * r[:, None] * gamma.double()
+    assert ((rstd.double() - r).abs() <= 1e-6 * r).all()
+    assert ((y.double() - want).abs() <= (2.0 ** -8 + 1e-6) * want.abs()).all()
