@@ -5,12 +5,18 @@
 //   * one cluster of CTAs per (sequence, KV head), every CTA and every warp of it taking its own 32-key tiles
 //     (a prefix of n keys is n / 32 independent chains instead of four);
 //   * all query heads of the group share each K / V row that was loaded (up to 4 heads per CTA), with 16-byte
-//     loads, a whole half tile in flight per lane;
+//     loads, half a tile in flight per lane;
+//   * the scores of a tile are mma.sync products (rows = heads, columns = keys, fp32 sums): a lane's 16-byte pieces of
+//     q and of the keys are fragments as they stand, because a dot product does not care in which order the head
+//     dimension is walked as long as both sides walk it alike. No exchange between lanes is left before the softmax
+//     (summing a key's product over lanes cost 5 shuffles in a chain per pair of keys). The weights stay fp32 and
+//     multiply V on the FMA units;
 //   * the partial softmax states (maximum, sum, weighted values) meet in shared memory, first over the warps of
 //     a CTA, then over the CTAs of the cluster through distributed shared memory: no workspace, no second launch.
 // The previous kernel had one CTA of four warps per QUERY head, each warp walking its keys one by one through a
-// five-step shuffle and an exponential. Device time before -> now: B = 1, 16 / 4 heads of 128, 1801 keys 352 -> 13 us;
-// B = 8, 32 / 8 heads of 128, 3001 keys (98 MB of cache) 742 -> 62 us; B = 1, 12 / 4 heads of 64, 101 keys 20 -> 7 us.
+// five-step shuffle and an exponential. Device time before -> now: B = 1, 16 / 4 heads of 128, 1801 keys 352 -> 11 us;
+// B = 8, 32 / 8 heads of 128, 3001 keys (98 MB of cache) 742 -> 28 us (59 with the scores
+// on the FMA units, and at 160 registers a second, part-filled round of CTAs); B = 1, 12 / 4 heads of 64, 101 keys 20 -> 7 us.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -18,8 +24,8 @@
 namespace b200 {
 namespace cg = cooperative_groups;
 
-constexpr int DA_MAX_WARPS = 8;
-constexpr int DA_TILE = 32;          // keys per warp and step: one per lane in the softmax phase
+constexpr int DA_MAX_WARPS = 16;
+constexpr int DA_TILE = 32;          // keys per warp and step
 
 struct DecodeParams {
   const bf16* q;        // [B, QH, D]
@@ -48,34 +54,10 @@ __device__ __forceinline__ void unpack16B(const uint4& u, float (&f)[8]) {
   }
 }
 
-// Sums v[r] over the LPK lanes that share a key. With RT = 4 (2) the first two (one) exchange steps also split the
-// heads over the lanes, so the sum costs 5 shuffles instead of 16 at LPK = 16. Returns the sum of head `head`.
-template <int RT, int LPK>
-__device__ __forceinline__ float group_sum(float (&v)[RT], int lane, int& head) {
-  float x;
-  int o = LPK / 2;
-  head = 0;
-  if constexpr (RT == 4) {
-    const bool b1 = (lane & o) != 0;
-    float k0 = b1 ? v[2] : v[0], k1 = b1 ? v[3] : v[1];
-    const float s0 = b1 ? v[0] : v[2], s1 = b1 ? v[1] : v[3];
-    k0 += __shfl_xor_sync(0xffffffffu, s0, o);
-    k1 += __shfl_xor_sync(0xffffffffu, s1, o);
-    o >>= 1;
-    const bool b0 = (lane & o) != 0;
-    x = (b0 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b0 ? k0 : k1, o);
-    o >>= 1;
-    head = (b1 ? 2 : 0) + (b0 ? 1 : 0);
-  } else if constexpr (RT == 2) {
-    const bool b0 = (lane & o) != 0;
-    x = (b0 ? v[1] : v[0]) + __shfl_xor_sync(0xffffffffu, b0 ? v[0] : v[1], o);
-    o >>= 1;
-    head = b0 ? 1 : 0;
-  } else {
-    x = v[0];
-  }
-  for (; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
+__device__ __forceinline__ void mma_scores(float (&d)[4], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
 }
 
 __device__ __forceinline__ uint4 pack16B(const float (&f)[8]) {
@@ -110,10 +92,10 @@ struct alignas(RT * 4) HeadRow {     // one key's scores / weights, one vector l
   float v[RT];
 };
 
-// 160 registers: three CTAs of four warps, or one of eight, fit an SM.
-// grid (cluster size, KVH * groups, B), cluster (cluster size, 1, 1), block 32 * warps (any number up to 8).
+// 128 registers: four CTAs of four warps, or one of sixteen, fit an SM.
+// grid (cluster size, KVH * groups, B), cluster (cluster size, 1, 1), block 32 * warps (any number up to 16).
 template <int D, int RT, bool APPEND>
-__global__ void __maxnreg__(160)
+__global__ void __maxnreg__(128)
 decode_attn_kernel(const DecodeParams p) {
   constexpr int LPK = D / 8;                 // lanes per key, 16 bytes each
   constexpr int KPS = 32 / LPK;              // keys per load step
@@ -149,28 +131,31 @@ decode_attn_kernel(const DecodeParams p) {
     __syncthreads();
   }
 
-  float qv[RT][8], acc[RT][8], m[RT], l[RT];
+  const int hl = lane >> 2, tl = lane & 3;              // fragment coordinates: head (or key) row, quad
+  constexpr int QC = D / 32;                            // 16-byte pieces of a row per lane: chunks tl, tl + 4, ...
+  uint32_t qa[QC][4];
 #pragma unroll
-  for (int r = 0; r < RT; ++r) {
+  for (int i = 0; i < QC; ++i) {
     uint4 u = make_uint4(0u, 0u, 0u, 0u);
-    if (r < nh) {
-      if constexpr (APPEND) u = rotated_chunk<D>(new_row + (p.KVH + h0 + r) * D, dl, p.cosr, p.sinr);
-      else u = *reinterpret_cast<const uint4*>(p.q + (size_t(b) * p.QH + h0 + r) * D + dl * 8);
+    if (hl < nh) {
+      if constexpr (APPEND) u = rotated_chunk<D>(new_row + (p.KVH + h0 + hl) * D, tl + 4 * i, p.cosr, p.sinr);
+      else u = reinterpret_cast<const uint4*>(p.q + (size_t(b) * p.QH + h0 + hl) * D)[tl + 4 * i];
     }
-    unpack16B(u, qv[r]);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) { qv[r][e] *= p.scale; acc[r][e] = 0.f; }
-    m[r] = -INFINITY;
-    l[r] = 0.f;
+    qa[i][0] = u.x; qa[i][1] = u.y; qa[i][2] = u.z; qa[i][3] = u.w;
   }
-  const bf16* kb = p.kc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D + dl * 8;
-  const bf16* vb = p.vc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D + dl * 8;
+  float acc[RT][8], m = -INFINITY, l = 0.f;             // m, l: of head hl
+#pragma unroll
+  for (int r = 0; r < RT; ++r)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[r][e] = 0.f;
+  const bf16* kb = p.kc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
+  const bf16* vb = p.vc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
 
-  auto row16 = [&](const bf16* rows, int which, int key) {
+  auto piece = [&](const bf16* rows, int which, int key, int chunk) {      // 16 bytes of a key's row
     uint4 u = make_uint4(0u, 0u, 0u, 0u);
     if (key < len) {
-      if (APPEND && key == p.pos) u = s_new[which][dl];
-      else u = *reinterpret_cast<const uint4*>(rows + size_t(key) * D);
+      if (APPEND && key == p.pos) u = s_new[which][chunk];
+      else u = reinterpret_cast<const uint4*>(rows + size_t(key) * D)[chunk];
     }
     return u;
   };
@@ -178,73 +163,69 @@ decode_attn_kernel(const DecodeParams p) {
   // tile t goes to CTA t % cs, warp (t / cs) % nw: neighbouring tiles on different SMs
   for (int t = rank + warp * cs; t * DA_TILE < len; t += nw * cs) {
     const int key0 = t * DA_TILE;
-    uint4 buf[HALF];
+    float sc[4][4];                                     // keys 8 nb + 2 tl, + 1 of head hl in [nb][0], [nb][1]
+    uint4 vbuf[HALF];
 #pragma unroll
-    for (int half = 0; half < STEPS; half += HALF) {
+    for (int nb0 = 0; nb0 < 4; nb0 += 2) {
+      uint4 kbuf[2][QC];
 #pragma unroll
-      for (int s = 0; s < HALF; ++s) {
-        const int key = key0 + (half + s) * KPS + kl;
-        buf[s] = row16(kb, 0, key);
-      }
+      for (int n = 0; n < 2; ++n)
 #pragma unroll
-      for (int s = 0; s < HALF; ++s) {
-        float kf[8], v[RT];
-        unpack16B(buf[s], kf);
+        for (int i = 0; i < QC; ++i) kbuf[n][i] = piece(kb, 0, key0 + (nb0 + n) * 8 + hl, tl + 4 * i);
 #pragma unroll
-        for (int r = 0; r < RT; ++r) {
-          float a = qv[r][0] * kf[0];
+      for (int n = 0; n < 2; ++n) {
 #pragma unroll
-          for (int e = 1; e < 8; ++e) a += qv[r][e] * kf[e];
-          v[r] = a;
+        for (int e = 0; e < 4; ++e) sc[nb0 + n][e] = 0.f;
+#pragma unroll
+        for (int i = 0; i < QC; ++i) {
+          mma_scores(sc[nb0 + n], qa[i][0], qa[i][1], kbuf[n][i].x, kbuf[n][i].y);
+          mma_scores(sc[nb0 + n], qa[i][2], qa[i][3], kbuf[n][i].z, kbuf[n][i].w);
         }
-        int head;
-        const float x = group_sum<RT, LPK>(v, lane, head);
-        if ((lane & (LPK / RT - 1)) == 0) s_p[warp][(half + s) * KPS + kl].v[head] = x;
       }
     }
     // the first values travel while the softmax of the tile is formed
 #pragma unroll
-    for (int s = 0; s < HALF; ++s) {
-      const int key = key0 + s * KPS + kl;
-      buf[s] = row16(vb, 1, key);
-    }
+    for (int s = 0; s < HALF; ++s) vbuf[s] = piece(vb, 1, key0 + s * KPS + kl, dl);
+    float mx = -INFINITY;
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        sc[nb][e] = key0 + nb * 8 + tl * 2 + e < len ? sc[nb][e] * p.scale : -INFINITY;
+        mx = fmaxf(mx, sc[nb][e]);
+      }
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float mn = fmaxf(m, mx), ref = mn == -INFINITY ? 0.f : mn;
+    const float corr = __expf(m - ref);                 // 0 on the first tile
+    m = mn;
+    l *= corr;
+#pragma unroll
+    for (int nb = 0; nb < 4; ++nb)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int k = nb * 8 + tl * 2 + e;
+        const float pe = key0 + k < len ? __expf(sc[nb][e] - ref) : 0.f;
+        l += pe;                                        // this lane's keys; summed over the quad at the end
+        if (hl < RT) s_p[warp][k].v[hl] = pe;
+      }
     __syncwarp();
-    const bool valid = key0 + lane < len;
-    HeadRow<RT> row = s_p[warp][lane];
-    float corr[RT];
 #pragma unroll
     for (int r = 0; r < RT; ++r) {
-      const float sc = valid ? row.v[r] : -INFINITY;
-      float mx = sc;
+      const float cr = __shfl_sync(0xffffffffu, corr, r * 4);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float mn = fmaxf(m[r], mx);
-      const float ref = mn == -INFINITY ? 0.f : mn;
-      corr[r] = __expf(m[r] - ref);                     // 0 on the first tile
-      const float pe = valid ? __expf(sc - ref) : 0.f;
-      l[r] = l[r] * corr[r] + pe;                       // lane-local; summed over lanes at the end
-      m[r] = mn;
-      row.v[r] = pe;
+      for (int e = 0; e < 8; ++e) acc[r][e] *= cr;
     }
-    s_p[warp][lane] = row;                              // own row: read by this lane only until the barrier
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < RT; ++r)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[r][e] *= corr[r];
 #pragma unroll
     for (int half = 0; half < STEPS; half += HALF) {
       if (half > 0) {
 #pragma unroll
-        for (int s = 0; s < HALF; ++s) {
-          const int key = key0 + (half + s) * KPS + kl;
-          buf[s] = row16(vb, 1, key);
-        }
+        for (int s = 0; s < HALF; ++s) vbuf[s] = piece(vb, 1, key0 + (half + s) * KPS + kl, dl);
       }
 #pragma unroll
       for (int s = 0; s < HALF; ++s) {
         float vf[8];
-        unpack16B(buf[s], vf);
+        unpack16B(vbuf[s], vf);
         const HeadRow<RT> w = s_p[warp][(half + s) * KPS + kl];
 #pragma unroll
         for (int r = 0; r < RT; ++r)
@@ -256,17 +237,17 @@ decode_attn_kernel(const DecodeParams p) {
   }
 
   // over the key slots of the warp, then the warps of the CTA
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  if (tl == 0 && hl < RT) { s_m[warp][hl] = m; s_l[warp][hl] = l; }
 #pragma unroll
   for (int r = 0; r < RT; ++r) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], o);
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
 #pragma unroll
       for (int o = LPK; o < 32; o <<= 1) acc[r][e] += __shfl_xor_sync(0xffffffffu, acc[r][e], o);
       if (kl == 0) s_o[warp][r][dl * 8 + e] = acc[r][e];
     }
-    if (lane == 0) { s_m[warp][r] = m[r]; s_l[warp][r] = l[r]; }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < RT * D; i += blockDim.x) {
@@ -309,7 +290,7 @@ static int launch_decode(DecodeParams p, int B, cudaStream_t st) {
   const long pairs = long(B) * p.KVH * p.groups;
   const int tiles = (p.Tmax + DA_TILE - 1) / DA_TILE;
   // 8 CTAs per (sequence, KV head) until there are two per SM without it; fewer where the cache is shorter than
-  // 8 tiles. Up to 8 warps per CTA while at most one CTA per SM exists, else 4 (they share the SM's registers).
+  // 8 tiles. Up to 16 warps per CTA while at most one CTA per SM exists, else 4 (they share the SM's registers).
   int cs = 1;
   while (cs < 8 && cs < tiles && pairs * cs < 4L * num_sms()) cs *= 2;
   int warps = (tiles + cs - 1) / cs;
