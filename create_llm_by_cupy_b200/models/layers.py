@@ -64,7 +64,7 @@ class RMSNorm:
         self.cache = None
 
     def forward(self, x: torch.Tensor, train_flg: bool = True) -> torch.Tensor:
-        y, rstd = F.rmsnorm_fwd(x, self.params[0], self.eps)
+        y, rstd = F.rmsnorm_fwd(x, self.params[0], self.eps, keep_rstd=train_flg)
         self.cache = (x, rstd) if train_flg else None
         return y
 
@@ -115,11 +115,12 @@ class GroupedQueryAttention:
 
     # -- helpers ---------------------------------------------------------------------------
     def _split(self, kqv: torch.Tensor, B: int, T: int):
-        v3 = kqv.view(B, T, -1)
-        k = v3[:, :, :self.KV].unflatten(2, (self.KVH, self.D))
-        q = v3[:, :, self.KV:self.KV + self.H].unflatten(2, (self.QH, self.D))
-        v = v3[:, :, self.KV + self.H:].unflatten(2, (self.KVH, self.D))
-        return q, k, v
+        kqv = kqv.view(B, T, -1)
+        sb, st, sc = kqv.stride()
+        o, strides = kqv.storage_offset(), (sb, st, self.D * sc, sc)
+        return (kqv.as_strided((B, T, self.QH, self.D), strides, o + self.KV * sc),
+                kqv.as_strided((B, T, self.KVH, self.D), strides, o),
+                kqv.as_strided((B, T, self.KVH, self.D), strides, o + (self.KV + self.H) * sc))
 
     def _rope(self, T, device):
         return F.rope_table(max(T, self.T), self.D, self.rope_base, device)
@@ -242,8 +243,12 @@ class GroupedQueryAttention:
     def decode_step(self, x, pos: int, kcache, vcache, lens, residual=None):
         """x: [B, H] normed hidden state of the token at position ``pos`` (same for the batch)."""
         B = x.shape[0]
-        kqv = F.gemm(x, self.params[0])
         tabs = self._rope(kcache.shape[2], x.device)
+        out = F.decode_attn_block(x, self.params[0], self.params[1], kcache, vcache, lens, pos, self.QH, self.KVH,
+                                  tabs[0], tabs[1], self.scale, residual)
+        if out is not None:
+            return out
+        kqv = F.gemm(x, self.params[0])
         if F.decode_append_fusable(kqv, kcache, vcache, lens, pos, self.QH, self.KVH):
             o = F.decode_attn_append(kqv, kcache, vcache, lens, pos, self.QH, self.KVH, tabs[0], tabs[1], self.scale)
             return F.gemm(o.view(B, self.H), self.params[1], add=residual)
@@ -316,6 +321,11 @@ class SwiGLU:
 
     def forward(self, x: torch.Tensor, residual=None, train_flg: bool = True) -> torch.Tensor:
         keep = train_flg and self.cache_gate
+        if not train_flg and F.SWIGLU_EPILOGUE and getattr(self, "pending_gather", None) is None:
+            out = F.mlp_few_rows(x, self.params[0], self.params[1], residual)
+            if out is not None:
+                self.cache = None
+                return out
         gv, act = self._gate_act(x, keep)
         if self.drop is not None and train_flg:
             out = self.drop.forward(F.gemm(act, self.params[1]), True)

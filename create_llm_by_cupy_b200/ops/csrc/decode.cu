@@ -15,8 +15,8 @@
 //     a CTA, then over the CTAs of the cluster through distributed shared memory: no workspace, no second launch.
 // The previous kernel had one CTA of four warps per QUERY head, each warp walking its keys one by one through a
 // five-step shuffle and an exponential. Device time before -> now: B = 1, 16 / 4 heads of 128, 1801 keys 352 -> 11 us;
-// B = 8, 32 / 8 heads of 128, 3001 keys (98 MB of cache) 742 -> 28 us (59 with the scores
-// on the FMA units, and at 160 registers a second, part-filled round of CTAs); B = 1, 12 / 4 heads of 64, 101 keys 20 -> 7 us.
+// B = 8, 32 / 8 heads of 128, 3001 keys (98 MB of cache, 15 us at the copy rate) 742 -> 28 us (59 with the scores on the
+// FMA units and a second, part-filled round of CTAs at 160 registers); B = 1, 12 / 4 heads of 64, 101 keys 20 -> 7 us.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -377,4 +377,35 @@ B200_API int b200_decode_attn_append(const void* kqv, void* kcache, void* vcache
   p.sinr = static_cast<const float*>(sinr);
   p.ld = ld; p.pos = pos;
   return launch_decode_dim(p, B, D, st);
+}
+
+// gemm_skinny.cu
+B200_API int b200_gemm_skinny(const void* A, const void* B, void* D, const void* C, int M, int N, int K, int lda, int ldb,
+                              int ldd, int ldc, int b_k_rows, int out_f32, float alpha, cudaStream_t stream);
+B200_API int b200_gemm_skinny_swiglu(const void* A, const void* B, void* ACT, int M, int I, int K, int lda, int ldb,
+                                     int ldact, cudaStream_t stream);
+
+// The attention half of a block for one token per sequence, three launches from one call (at a few microseconds of
+// device time each, a call into this library from Python costs as much as a launch):
+//   kqv = x W_kqv;  o = rotate, append to the caches, attend;  out = o W_o (+ residual)
+// x [B, H] (pitch ldx), W_kqv [H, (QH + 2 KVH) D], W_o [QH D, H] contiguous, kqv / o: caller's scratch.
+B200_API int b200_decode_attn_block(const void* x, const void* w_kqv, const void* w_o, const void* residual, void* out,
+                                    void* kqv, void* o, void* kcache, void* vcache, const void* lens, const void* cosr,
+                                    const void* sinr, int B, int H, int QH, int KVH, int Tmax, int D, int ldx, int ldr,
+                                    int pos, float scale, cudaStream_t st) {
+  const int N = (QH + 2 * KVH) * D, HO = QH * D;
+  int rc = b200_gemm_skinny(x, w_kqv, kqv, nullptr, B, N, H, ldx, N, N, 0, 1, 0, 1.f, st);
+  if (rc == 0)
+    rc = b200_decode_attn_append(kqv, kcache, vcache, o, lens, cosr, sinr, B, QH, KVH, Tmax, D, N, pos, scale, st);
+  if (rc == 0) rc = b200_gemm_skinny(o, w_o, out, residual, B, H, HO, HO, H, H, ldr, 1, 0, 1.f, st);
+  return rc;
+}
+
+// The MLP half for few rows, two launches from one call: out = (silu(x W_gate) * (x W_value)) W_out (+ residual);
+// W_gate_val [H, 2 I] and W_out [I, H] contiguous, act: caller's scratch [M, I].
+B200_API int b200_mlp_few_rows(const void* x, const void* w_gate_val, const void* w_out, const void* residual, void* out,
+                               void* act, int M, int H, int I, int ldx, int ldr, cudaStream_t st) {
+  const int rc = b200_gemm_skinny_swiglu(x, w_gate_val, act, M, I, H, ldx, 2 * I, I, st);
+  if (rc != 0) return rc;
+  return b200_gemm_skinny(act, w_out, out, residual, M, H, I, I, H, H, ldr, 1, 0, 1.f, st);
 }

@@ -37,7 +37,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // ------------------------------------------------------------------ RMSNorm forward
-// One warp per row; the row stays in registers between the reduction and the scaling pass when
+// rstd may be null (inference). One warp per row; the row stays in registers between the reduction and the scaling pass when
 // it fits (H <= 32 * 8 * NV), otherwise it is read a second time (served by L1/L2).
 template <int NV>
 __global__ void __launch_bounds__(128)
@@ -71,7 +71,7 @@ rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma, b
   }
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / float(H) + eps);
-  if (lane == 0) rstd[row] = r;
+  if (lane == 0 && rstd) rstd[row] = r;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = lane + i * 32;
@@ -146,7 +146,7 @@ rmsnorm_fwd_cta_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamm
 #pragma unroll
       for (int w = 0; w < 8; ++w) t += sss[it & 1][r][w];
       const float rs = rsqrtf(t * inv_h + eps);
-      if (tid == 0) rstd[row] = rs;
+      if (tid == 0 && rstd) rstd[row] = rs;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
         const int c = tid + i * 256;
@@ -175,7 +175,7 @@ __global__ void rmsnorm_fwd_scalar_kernel(const bf16* __restrict__ x, const bf16
   }
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / float(H) + eps);
-  if (lane == 0) rstd[row] = r;
+  if (lane == 0 && rstd) rstd[row] = r;
   for (int c = lane; c < H; c += 32)
     y[size_t(row) * H + c] = __float2bfloat16(__bfloat162float(xr[c]) * r * __bfloat162float(gamma[c]));
 }

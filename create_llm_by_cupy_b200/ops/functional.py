@@ -121,10 +121,11 @@ def _bf16(*ts):
 
 
 # --------------------------------------------------------------------------- RMSNorm
-def rmsnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6):
-    """y = x * rsqrt(mean(x^2) + eps) * gamma over the last dim. Returns (y, rstd[M] fp32)."""
+def rmsnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6, keep_rstd: bool = True):
+    """y = x * rsqrt(mean(x^2) + eps) * gamma over the last dim. Returns (y, rstd[M] fp32; None on CUDA when not
+    ``keep_rstd``, which only the backward needs)."""
     H = x.shape[-1]
-    x2 = x.reshape(-1, H)
+    x2 = x if x.dim() == 2 else x.reshape(-1, H)
     M = x2.shape[0]
     if not x.is_cuda:
         xf = x2.float()
@@ -134,11 +135,11 @@ def rmsnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6):
     _bf16(x, gamma)
     x2 = x2.contiguous()
     y = torch.empty_like(x2)
-    rstd = torch.empty(M, dtype=torch.float32, device=x.device)
+    rstd = torch.empty(M, dtype=torch.float32, device=x.device) if keep_rstd else None
     native.check(_lib().b200_rmsnorm_fwd(native.ptr(x2), native.ptr(gamma), native.ptr(y), native.ptr(rstd),
                                          M, H, _f(eps), native.stream_ptr()), "rmsnorm_fwd")
     native.bump()
-    return y.view(x.shape), rstd
+    return (y if x.dim() == 2 else y.view(x.shape)), rstd
 
 
 def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma: torch.Tensor, rstd: torch.Tensor,
@@ -391,8 +392,9 @@ def dropout_bwd(dout: torch.Tensor, mask: torch.Tensor, p: float) -> torch.Tenso
 # --------------------------------------------------------------------------- flash attention
 def _strides3(t: torch.Tensor) -> list[int]:
     """(batch, token, head) element strides of a [B, T, heads, D] view."""
-    assert t.dim() == 4 and t.stride(3) == 1
-    return [t.stride(0), t.stride(1), t.stride(2)]
+    s = t.stride()
+    assert len(s) == 4 and s[3] == 1
+    return [s[0], s[1], s[2]]
 
 
 def _attn_reference(q, k, v, valid_len, scale, cos, sin):
@@ -698,6 +700,64 @@ def decode_attn_append(kqv, kcache, vcache, lens, pos: int, QH: int, KVH: int, c
         native.c_void_p(cos.data_ptr() + row), native.c_void_p(sin.data_ptr() + row), B, QH, KVH, Tmax, D,
         kqv.shape[1], pos, _f(scale), native.stream_ptr()), "decode_attn_append")
     native.bump()
+    return out
+
+
+def _few_rows_ok(x, weights, residual, out_cols: int) -> bool:
+    """Shapes and layouts of the one-call forms below: few bf16 rows ``x``, contiguous weights, a residual like the output."""
+    from . import gemm as _g
+    M = x.shape[0]
+    if not (x.is_cuda and _g.GEMM_IMPL == "2cta" and M > 0 and _g._tma_ok(x, *weights)):
+        return False
+    if not all(w.is_contiguous() and _g._skinny(M, w.shape[1]) for w in weights):
+        return False
+    return residual is None or (residual.dtype == torch.bfloat16 and residual.shape == (M, out_cols)
+                                and residual.stride(1) == 1)
+
+
+def decode_attn_block(x, w_kqv, w_o, kcache, vcache, lens, pos: int, QH: int, KVH: int, cos, sin, scale: float,
+                      residual=None):
+    """K|Q|V projection, rotation, cache append, attention and output projection (+ residual) of one token per sequence
+    from one native call (the same three kernels as ``gemm``, ``decode_attn_append``, ``gemm``). Returns [B, H], or None
+    where one of those forms does not apply."""
+    if not (x.is_cuda and kcache.dim() == 4 and _few_rows_ok(x, (w_kqv, w_o), residual, w_o.shape[1])):
+        return None
+    B, H = x.shape
+    _, _, Tmax, D = kcache.shape
+    N = w_kqv.shape[1]
+    scratch = torch.empty((B, N + QH * D), dtype=torch.bfloat16, device=x.device).view(-1)
+    kqv = scratch[:B * N].view(B, N)
+    if (w_kqv.shape[0] != H or w_o.shape != (QH * D, H)
+            or not decode_append_fusable(kqv, kcache, vcache, lens, pos, QH, KVH)):
+        return None
+    assert cos.dtype == sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
+    assert cos.shape[0] > pos and cos.shape[1] == D // 2 and sin.shape == cos.shape
+    out = torch.empty((B, H), dtype=torch.bfloat16, device=x.device)
+    row, base = pos * D * 2, scratch.data_ptr()
+    native.check(_lib().b200_decode_attn_block(
+        native.ptr(x), native.ptr(w_kqv), native.ptr(w_o), native.ptr(residual), native.ptr(out), native.c_void_p(base),
+        native.c_void_p(base + 2 * B * N), native.ptr(kcache), native.ptr(vcache), native.ptr(lens),
+        native.c_void_p(cos.data_ptr() + row), native.c_void_p(sin.data_ptr() + row), B, H, QH, KVH, Tmax, D, x.stride(0),
+        residual.stride(0) if residual is not None else 0, pos, _f(scale), native.stream_ptr()), "decode_attn_block")
+    native.bump(3)
+    return out
+
+
+def mlp_few_rows(x, w_gate_val, w_out, residual=None):
+    """SwiGLU MLP of few rows from one native call (``gemm_skinny_swiglu`` and ``gemm``), or None where those forms do not
+    apply."""
+    if not _few_rows_ok(x, (w_gate_val, w_out), residual, w_out.shape[1]):
+        return None
+    M, H = x.shape
+    I = w_out.shape[0]
+    if w_gate_val.shape != (H, 2 * I) or w_out.shape[1] != H or I % 8 != 0:
+        return None
+    act = torch.empty((M, I), dtype=torch.bfloat16, device=x.device)
+    out = torch.empty((M, H), dtype=torch.bfloat16, device=x.device)
+    native.check(_lib().b200_mlp_few_rows(
+        native.ptr(x), native.ptr(w_gate_val), native.ptr(w_out), native.ptr(residual), native.ptr(out), native.ptr(act),
+        M, H, I, x.stride(0), residual.stride(0) if residual is not None else 0, native.stream_ptr()), "mlp_few_rows")
+    native.bump(2)
     return out
 
 

@@ -65,9 +65,12 @@ def _apply_dynamic():
 def _rowmajor_2d(t: torch.Tensor) -> tuple[torch.Tensor, int]:
     """Return (tensor, pitch) for a 2-D view whose last dim is contiguous; copy if it is not."""
     assert t.dim() == 2
-    if t.stride(1) != 1 or (t.size(0) > 1 and t.stride(0) < t.size(1)):
+    rows, cols = t.shape
+    s0, s1 = t.stride()
+    if s1 != 1 or (rows > 1 and s0 < cols):
         t = t.contiguous()
-    return t, (t.stride(0) if t.size(0) > 1 else max(t.size(1), t.stride(0)))
+        s0 = t.stride(0)
+    return t, (s0 if rows > 1 else max(cols, s0))
 
 
 # Operands whose rows do not start on 16-byte boundaries (an FFN width of int(8 H / 3), say) are copied into a pitch
@@ -493,12 +496,29 @@ def wgrad_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None
     caller must call ``wgrad_join()`` before the result is consumed on the main stream."""
     if not (WGRAD_OVERLAP and a.is_cuda):
         return gemm(a, b, trans_a=True, out=out)
-    cur = torch.cuda.current_stream(a.device)
+    return _on_wgrad_stream(lambda: gemm(a, b, trans_a=True, out=out), a, b)
+
+
+def _on_wgrad_stream(compute, a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
+    """``compute()``, which reads ``a`` and ``b``, on the side stream behind everything issued on the current one."""
     ws = _wgrad_stream(a.device)
-    ws.wait_stream(cur)
     _wgrad_pending[a.device.index] = True
-    with torch.cuda.stream(ws):
-        res = gemm(a, b, trans_a=True, out=out)
+    if a.device.index == torch._C._cuda_getDevice():
+        # what ``ws.wait_stream`` and ``with torch.cuda.stream(ws)`` do, without their device checks and stream
+        # objects (about 25 us of host time per weight gradient)
+        prev = torch._C._cuda_getCurrentStream(a.device.index)
+        ev = torch.cuda.Event()
+        ev.record(torch.cuda.Stream(stream_id=prev[0], device_index=prev[1], device_type=prev[2]))
+        ws.wait_event(ev)
+        torch._C._cuda_setStream(stream_id=ws.stream_id, device_index=ws.device_index, device_type=ws.device_type)
+        try:
+            res = compute()
+        finally:
+            torch._C._cuda_setStream(stream_id=prev[0], device_index=prev[1], device_type=prev[2])
+    else:
+        ws.wait_stream(torch.cuda.current_stream(a.device))
+        with torch.cuda.stream(ws):
+            res = compute()
     a.record_stream(ws)
     b.record_stream(ws)
     return res
@@ -519,16 +539,7 @@ def wgrad_gemm_gate_value(x: torch.Tensor, dgv: torch.Tensor, I: int, out: torch
         dst = torch.empty((x.shape[1], 2 * I), dtype=x.dtype, device=x.device) if out is None else out
         return repitch(full, dst, I, I, 2, dgv.shape[1] // 2, I)
 
-    if not WGRAD_OVERLAP:
-        return compute()
-    ws = _wgrad_stream(x.device)
-    ws.wait_stream(torch.cuda.current_stream(x.device))
-    _wgrad_pending[x.device.index] = True
-    with torch.cuda.stream(ws):
-        res = compute()
-    x.record_stream(ws)
-    dgv.record_stream(ws)
-    return res
+    return _on_wgrad_stream(compute, x, dgv) if WGRAD_OVERLAP else compute()
 
 
 def wgrad_event(device):

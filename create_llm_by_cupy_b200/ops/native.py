@@ -81,8 +81,19 @@ def source_digest() -> str:
     return _build.source_digest()
 
 
+def _current_index() -> int:
+    """Index of the current device. ``torch.cuda.current_device()`` re-checks the initialisation, and a
+    ``torch.cuda.current_stream()`` object goes through four Python layers; on launches of a few microseconds those
+    two were most of the host's time (18 -> 8 us per launch of a decoded token)."""
+    return torch._C._cuda_getDevice() if _status else torch.cuda.current_device()
+
+
 def status_tensor(device=None) -> torch.Tensor:
     """Per-device 4-int status block that kernels write when a bounded wait runs out."""
+    if device is None:
+        t = _status.get(_current_index())
+        if t is not None:
+            return t
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     if dev.index is None:
         dev = torch.device("cuda", torch.cuda.current_device())
@@ -117,7 +128,7 @@ def check(rc: int, what: str) -> None:
 
 
 def stream_ptr() -> c_void_p:
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return c_void_p(torch._C._cuda_getCurrentRawStream(_current_index()))
 
 
 def ptr(t: torch.Tensor | None) -> c_void_p:

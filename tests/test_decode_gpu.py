@@ -123,3 +123,21 @@ def test_rmsnorm_few_rows(M, H):
     want = x.double() * r[:, None] * gamma.double()
     assert ((rstd.double() - r).abs() <= 1e-6 * r).all()
     assert ((y.double() - want).abs() <= (2.0 ** -8 + 1e-6) * want.abs()).all()
+
+
+@pytest.mark.parametrize("B,H,QH,KVH,I", [(1, 64, 2, 1, 8), (3, 256, 4, 2, 264), (16, 768, 12, 4, 2048), (7, 512, 4, 4, 1365)])
+def test_one_call_forms_match_the_separate_calls(B, H, QH, KVH, I, monkeypatch):
+    from create_llm_by_cupy_b200.models.layers import GroupedQueryAttention, SwiGLU
+    g = torch.Generator().manual_seed(0)
+    gqa, mlp = GroupedQueryAttention(H, 40, QH, KVH, 2, device="cuda", generator=g), SwiGLU(H, 2, device="cuda", generator=g, ffn_size=I)
+    x, res = bf(B, H, seed=1).cuda(), bf(B, 2 * H, seed=2).cuda()[:, :H]              # a residual with a pitch
+    kc, vc = bf(B, KVH, 40, H // QH, seed=3).cuda(), bf(B, KVH, 40, H // QH, seed=4).cuda()
+    lens = torch.full((B,), 18, dtype=torch.int32, device="cuda")
+    for r in (None, res):
+        k1, v1, k2, v2 = kc.clone(), vc.clone(), kc.clone(), vc.clone()
+        o1, m1 = gqa.decode_step(x, 17, k1, v1, lens, residual=r), mlp.forward(x, residual=r, train_flg=False)
+        with monkeypatch.context() as mp:
+            mp.setattr(F, "decode_attn_block", lambda *a, **k: None)
+            mp.setattr(F, "mlp_few_rows", lambda *a, **k: None)
+            o2, m2 = gqa.decode_step(x, 17, k2, v2, lens, residual=r), mlp.forward(x, residual=r, train_flg=False)
+        assert torch.equal(o1, o2) and torch.equal(m1, m2) and torch.equal(k1, k2) and torch.equal(v1, v2)
