@@ -65,8 +65,11 @@ enum Gemm2Flags : int { G2_OUT_F32 = 1, G2_ADD_C = 2, G2_TMA_OUT = 4, G2_WHOLE_T
 //                  leaves d(gate), d(value) (the backward of silu(gate) * value), d(activation) is never stored
 //   EPI_DELTA      D = A B^T is d(attention output) [tokens, heads x head_dim]; the epilogue also fetches the forward's
 //                  output tile by TMA and leaves delta[b, head, t] = sum_d dO O, which the attention backward needs
+//   EPI_SPLIT      a work item is one of `splits` K ranges of a tile; its fp32 sums go to a workspace
+//                  [splits][rows padded to whole tiles][N] that a second kernel adds up
 enum Gemm2Epi : int {
-  EPI_PLAIN = 0, EPI_ROPE = 1, EPI_SWIGLU = 2, EPI_CE_STATS = 3, EPI_CE_DLOGITS = 4, EPI_SWIGLU_BWD = 5, EPI_DELTA = 6
+  EPI_PLAIN = 0, EPI_ROPE = 1, EPI_SWIGLU = 2, EPI_CE_STATS = 3, EPI_CE_DLOGITS = 4, EPI_SWIGLU_BWD = 5, EPI_DELTA = 6,
+  EPI_SPLIT = 7
 };
 
 struct Gemm2Params {
@@ -106,6 +109,7 @@ struct Gemm2Params {
   // the map in the tmC slot; dl_out [batch][dl_heads][dl_T] fp32.
   float* dl_out;
   int dl_T, dl_heads, dl_dim;
+  int splits;                // EPI_SPLIT: item t is K range t % splits of tile t / splits
 };
 
 // A work item: tile coordinates, first column and width.
@@ -274,6 +278,10 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   const int num_tiles = p.n_items;          // work items (whole tiles and half tiles)
   const int num_kb = (p.K + G2_BK - 1) / G2_BK;
   const bool dyn = p.sched != nullptr;      // null: tile t + k * num_pairs goes to pair t (fixed assignment)
+  constexpr bool kSplit = EPI == EPI_SPLIT;
+  auto item = [&](int t) { return g2_item(kSplit ? t / p.splits : t, p.t_full, num_m, num_n); };
+  auto kb_first = [&](int t) { return kSplit ? (t % p.splits) * num_kb / p.splits : 0; };
+  auto kb_last = [&](int t) { return kSplit ? (t % p.splits + 1) * num_kb / p.splits : num_kb; };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -327,11 +335,11 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         // the draw is in flight while this tile's first loads are issued
         if (!dyn) t_next = t + num_pairs;
         else if (rank == 0) t_next = num_pairs + atomicAdd(&p.sched[0], 1);
-        const G2Item wi = g2_item(t, p.t_full, num_m, num_n);
+        const G2Item wi = item(t);
         const int m0 = wi.mb * 2 * G2_BM + int(rank) * G2_BM;
         const int n0 = EPI == EPI_SWIGLU ? wi.nb * (G2_BN / 2) + int(rank) * p.sw_I : wi.n0 + int(rank) * (wi.bn / 2);
         const uint32_t stage_tx = 2 * (G2_A_BYTES + (wi.bn / 2) * G2_BK * 2);
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = kb_first(t), kb_end = kb_last(t); kb < kb_end; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
           uint8_t* sA = smem + stage * G2_STAGE_BYTES;
           uint8_t* sB = sA + G2_A_BYTES;
@@ -389,7 +397,8 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * G2_BN;
         const uint32_t idesc = t < p.t_full ? idesc_full : idesc_half;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int kb0 = kb_first(t);
+        for (int kb = kb0, kb_end = kb_last(t); kb < kb_end; ++kb) {
           if (!mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sA = smem_u32(smem + stage * G2_STAGE_BYTES);
@@ -400,7 +409,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                                         : umma_smem_desc(sA + kk * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? umma_smem_desc(sB + kk * 2048, 8192, 1024)
                                         : umma_smem_desc(sB + kk * 32, 16, 1024);
-            umma_bf16_ss_pair(tmem_d, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_bf16_ss_pair(tmem_d, adesc, bdesc, idesc, kb != kb0 || kk != 0 ? 1u : 0u);
           }
           umma_commit_pair(&empty[stage]);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
@@ -678,8 +687,8 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       for (int t = pair; ok && t >= 0 && t < num_tiles;
            t = dyn ? rd.next(sched_full, sched_empty, tile_ring, abort_flag, true, lane == 0, rank != 0)
                    : t + num_pairs) {
-        const G2Item wi = g2_item(t, p.t_full, num_m, num_n);
-        const int row0 = wi.mb * 2 * G2_BM + int(rank) * G2_BM;
+        const G2Item wi = item(t);
+        const int row0 = wi.mb * 2 * G2_BM + int(rank) * G2_BM + (kSplit ? t % p.splits * num_m * 2 * G2_BM : 0);
         const int n0 = wi.n0;
         const int ngroups = wi.bn / gcols;
         const bool rope_on = kRope && !out_f32 && n0 < p.rope_cols;
@@ -959,11 +968,11 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     const int rem = whole % all_pairs;
     if (rem > 0 && 2 * rem <= all_pairs) halved = rem;
   }
-  const int num_tiles = whole + halved;
+  const int num_tiles = EPI == EPI_SPLIT ? whole * p.splits : whole + halved;
   int pairs = all_pairs;
   if (num_tiles < pairs) pairs = num_tiles;
   Gemm2Params q = p;
-  q.t_full = whole - halved;
+  q.t_full = EPI == EPI_SPLIT ? num_tiles : whole - halved;
   q.n_items = num_tiles;
   q.sched = nullptr;
   if (g_dynamic_tiles && num_tiles > pairs) {
@@ -972,6 +981,54 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
   }
   kern<<<2 * pairs, G2_THREADS, G2_SMEM, stream>>>(*tA, *tB, *tBh, *tD, *tC, tE ? *tE : *tA, q);
   return static_cast<int>(cudaGetLastError());
+}
+
+// out = sum over the splits of ws[split][row][col] (+ C), fixed order. 16-byte accesses where every row allows them.
+__global__ void __launch_bounds__(256)
+splitk_sum_kernel(const float* __restrict__ ws, void* D, const void* C, int M, int N, int splits, int ldws, size_t plane,
+                  int ldd, int ldc, int out_f32, int vec) {
+  const int per_row = (N + 3) >> 2;
+  const size_t total = size_t(M) * per_row;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
+    const int row = int(i / per_row), col = int(i % per_row) * 4;
+    const float* w = ws + size_t(row) * ldws + col;                     // ldws is a multiple of 4: never past a row's end
+    float4 a = *reinterpret_cast<const float4*>(w);
+    for (int s = 1; s < splits; ++s) {
+      const float4 b = *reinterpret_cast<const float4*>(w + s * plane);
+      a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    }
+    float v[4] = {a.x, a.y, a.z, a.w};
+    const size_t at = size_t(row) * ldd + col, ct = size_t(row) * ldc + col;
+    if (vec && col + 4 <= N) {
+      if (out_f32) {
+        if (C) {
+          const float4 c = *reinterpret_cast<const float4*>(static_cast<const float*>(C) + ct);
+          v[0] += c.x; v[1] += c.y; v[2] += c.z; v[3] += c.w;
+        }
+        *reinterpret_cast<float4*>(static_cast<float*>(D) + at) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+        if (C) {
+          const uint2 c = *reinterpret_cast<const uint2*>(static_cast<const bf16*>(C) + ct);
+          const float2 c0 = __bfloat1622float2(*reinterpret_cast<const bf162*>(&c.x));
+          const float2 c1 = __bfloat1622float2(*reinterpret_cast<const bf162*>(&c.y));
+          v[0] += c0.x; v[1] += c0.y; v[2] += c1.x; v[3] += c1.y;
+        }
+        uint2 o;
+        *reinterpret_cast<bf162*>(&o.x) = __floats2bfloat162_rn(v[0], v[1]);
+        *reinterpret_cast<bf162*>(&o.y) = __floats2bfloat162_rn(v[2], v[3]);
+        *reinterpret_cast<uint2*>(static_cast<bf16*>(D) + at) = o;
+      }
+    } else {
+      for (int e = 0; e < 4 && col + e < N; ++e) {
+        if (out_f32) {
+          static_cast<float*>(D)[at + e] = v[e] + (C ? static_cast<const float*>(C)[ct + e] : 0.f);
+        } else {
+          const float c = C ? __bfloat162float(static_cast<const bf16*>(C)[ct + e]) : 0.f;
+          static_cast<bf16*>(D)[at + e] = __float2bfloat16(v[e] + c);
+        }
+      }
+    }
+  }
 }
 
 static Gemm2Params base_params(void* D, const void* C, int M, int N, int K, int ldd, int ldc, int flags, float alpha) {
@@ -1071,6 +1128,45 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
   if (a_mn_major) return launch_tc2<true, false>(tA, tB, tBh, tD, tC, p, stream);
   if (b_mn_major) return launch_tc2<false, true>(tA, tB, tBh, tD, tC, p, stream);
   return launch_tc2<false, false>(tA, tB, tBh, tD, tC, p, stream);
+}
+
+// The same product where the output has too few 256 x 256 tiles for the CTA pairs and K is long: `splits` K ranges per
+// tile (tiles * splits at most the number of pairs, splits at most K / 64), fp32 sums in ws ([splits][M rounded up to
+// 256][N rounded up to 4] floats, 16-byte aligned), then one kernel that adds them (+ C). Deterministic.
+// 768 x 1280 over K = 8192 is 15 tiles: 15 pairs walk 128 k-blocks each while 59 idle; with 4 splits 60 pairs walk 32.
+B200_API int b200_gemm_bf16_2cta_split(const void* A, const void* B, void* D, const void* C, int M, int N, int K, int lda,
+                                       int ldb, int ldd, int ldc, int a_mn_major, int b_mn_major, int flags, float alpha,
+                                       void* ws, int splits, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  const uintptr_t all = reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(ws);
+  const int num_m = (M + 2 * G2_BM - 1) / (2 * G2_BM), tiles = num_m * ((N + G2_BN - 1) / G2_BN);
+  if (K <= 0 || ws == nullptr || (all & 15) != 0 || (lda % 8) != 0 || (ldb % 8) != 0 || splits < 2 ||
+      splits > (K + G2_BK - 1) / G2_BK || tiles * splits > num_sms() / 2)
+    return static_cast<int>(cudaErrorInvalidValue);
+  const int ldws = (N + 3) / 4 * 4, rows = num_m * 2 * G2_BM;
+  Gemm2Params p = base_params(ws, nullptr, M, N, K, ldws, 0, G2_OUT_F32 | G2_WHOLE_TILES | G2_TMA_OUT, alpha);
+  p.splits = splits;
+  const CUtensorMap* tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
+                                     : get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
+  const CUtensorMap* tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
+                                     : get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
+  const CUtensorMap* tD = get_tensor_map_2d(ws, uint64_t(splits) * rows, N, ldws, 128, 32, 4, SWIZZLE_128B_);
+  if (!tA || !tB || !tD) return static_cast<int>(cudaErrorInvalidValue);
+  int rc;
+  if (a_mn_major && b_mn_major) rc = launch_tc2<true, true, EPI_SPLIT>(tA, tB, tB, tD, tD, p, stream);
+  else if (a_mn_major) rc = launch_tc2<true, false, EPI_SPLIT>(tA, tB, tB, tD, tD, p, stream);
+  else if (b_mn_major) rc = launch_tc2<false, true, EPI_SPLIT>(tA, tB, tB, tD, tD, p, stream);
+  else rc = launch_tc2<false, false, EPI_SPLIT>(tA, tB, tB, tD, tD, p, stream);
+  if (rc != 0) return rc;
+  const int f32 = (flags & G2_OUT_F32) ? 1 : 0, mask = f32 ? 15 : 7;
+  const int vec = ldd % 4 == 0 && (reinterpret_cast<uintptr_t>(D) & mask) == 0 &&
+                  (C == nullptr || (ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & mask) == 0));
+  const size_t chunks = size_t(M) * ((N + 3) / 4);
+  const size_t blocks = (chunks + 255) / 256, cap = size_t(num_sms()) * 8;
+  splitk_sum_kernel<<<int(blocks < cap ? blocks : cap), 256, 0, stream>>>(
+      static_cast<const float*>(ws), D, (flags & G2_ADD_C) ? C : nullptr, M, N, splits, ldws, size_t(rows) * ldws, ldd, ldc,
+      f32, vec);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // act[M, I] = silu(A W_gate) * (A W_value) for B = [W_gate | W_value] ([K, 2 I] row-major), A [M, K] row-major,

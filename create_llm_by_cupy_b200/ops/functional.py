@@ -8,6 +8,7 @@ multi-process tests and the CPU smoke configuration run; it is never used for CU
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 
 import torch
@@ -142,12 +143,17 @@ def rmsnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6, keep_rs
     return (y if x.dim() == 2 else y.view(x.shape)), rstd
 
 
+@functools.lru_cache(maxsize=1024)
+def _norm_partial_rows(M: int, device: int) -> int:
+    return native.lib().b200_rmsnorm_bwd_partial_rows(M)
+
+
 def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma: torch.Tensor, rstd: torch.Tensor,
                 add: torch.Tensor | None = None):
     """Returns (dx (+ add), dgamma). ``x`` is the layer INPUT; ``add`` is the residual gradient."""
     H = x.shape[-1]
-    x2 = x.reshape(-1, H)
-    dy2 = dy.reshape(-1, H)
+    x2 = x if x.dim() == 2 else x.reshape(-1, H)
+    dy2 = dy if dy.dim() == 2 and dy.shape[1] == H else dy.reshape(-1, H)
     M = x2.shape[0]
     if not x.is_cuda:
         xf, dyf, g = x2.float(), dy2.float(), gamma.float()
@@ -165,7 +171,7 @@ def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma: torch.Tensor, rstd: to
     dx = torch.empty_like(x2)
     dgamma = torch.empty_like(gamma)
     lib = _lib()
-    rows = lib.b200_rmsnorm_bwd_partial_rows(M)
+    rows = _norm_partial_rows(M, x.get_device())
     partial = torch.empty((rows, H), dtype=torch.float32, device=x.device)
     native.check(lib.b200_rmsnorm_bwd(native.ptr(dy2), native.ptr(x2), native.ptr(gamma), native.ptr(rstd),
                                       native.ptr(add2), native.ptr(dx), native.ptr(dgamma), native.ptr(partial),

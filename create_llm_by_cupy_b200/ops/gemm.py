@@ -6,10 +6,13 @@ Replaces the ``cp.matmul`` (cuBLAS) call sites of the reference
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
 from . import native
+
+c_void_p, c_float = ctypes.c_void_p, ctypes.c_float
 
 GEMM_OUT_F32 = 1
 GEMM_ADD_C = 2
@@ -113,6 +116,36 @@ def _copy_rows(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
     return dst
 
 
+# 1: GEMMs with too few 256 x 256 tiles for the CTA pairs and a long K run as several K ranges per tile.
+GEMM_SPLIT_K = 1
+
+
+@functools.lru_cache(maxsize=4096)
+def split_count(M: int, N: int, K: int, pairs: int) -> int:
+    """K ranges per 256 x 256 tile (1: no split), by the time each number takes: 0.29 us per 64-deep block of K that one
+    pair walks and, for a split, the second kernel with 2 us of launch and the fp32 sums read at about 4 TB/s. A split
+    has to win 4 us, what its workspace and second launch cost the host. Measured, one range against the rule's:
+    768 x 1280 over K = 8192 44.3 / 22.4 us, 768 x 768 over 8192 44.4 / 17.6, 256 x 4096 over 11008 57.0 / 29.4. Left whole:
+    777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4)."""
+    tiles = -(-M // 256) * -(-N // 256)
+    kb = -(-K // 64)
+    def cost(n):
+        return 0.29 * kb if n == 1 else 0.29 * -(-kb // n) + 2.0 + 1e-6 * n * M * N
+
+    best = min(range(1, max(1, min(pairs // tiles, kb // 4, 16)) + 1), key=cost)
+    return best if cost(best) < cost(1) - 4.0 else 1
+
+
+_pairs: dict = {}
+
+
+def _cta_pairs(index: int) -> int:
+    n = _pairs.get(index)
+    if n is None:
+        n = _pairs[index] = torch.cuda.get_device_properties(index).multi_processor_count // 2
+    return n
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bool = False,
          out: torch.Tensor | None = None, add: torch.Tensor | None = None,
          out_dtype: torch.dtype | None = None, alpha: float = 1.0, bn: int = 0,
@@ -160,43 +193,52 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         flags |= GEMM_ADD_C
     native.status_tensor()
     impl = impl or GEMM_IMPL
+    lib = native.lib()
     if impl == "2cta" and not force_fallback and bn == 0 and max_ctas == 0:
-        if (lda % 8 or ldb % 8 or (a.data_ptr() | b.data_ptr()) % 16) and M * N > 0 and (
-                M * N * K >= PAD_WORK or K >= PAD_K):
+        pa, pb = a.data_ptr(), b.data_ptr()
+        ok = (lda | ldb) % 8 == 0 and (pa | pb) % 16 == 0
+        if not ok and M * N > 0 and (M * N * K >= PAD_WORK or K >= PAD_K):
             (a, lda), (b, ldb) = _padded(a, lda), _padded(b, ldb)
-        es = out.element_size()
-        if (M >= 256 and N >= 256 and M * N >= PAD_OUT_AREA and lda % 8 == 0 and ldb % 8 == 0
-                and (a.data_ptr() | b.data_ptr()) % 16 == 0 and (ldd * es % 16 or out.data_ptr() % 16)):
-            tmp = torch.empty((M, (N + 7) // 8 * 8), dtype=out_dtype, device=a.device)[:, :N]
-            if add is not None:
-                _copy_rows(add, tmp)
-            gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=tmp, add=None if add is None else tmp, alpha=alpha)
-            _copy_rows(tmp, out)
+            pa, pb, ok = a.data_ptr(), b.data_ptr(), True
+        if ok and M <= SKINNY_ROWS and not trans_a and _skinny(M, N):
+            rc = lib.b200_gemm_skinny(
+                c_void_p(pa), c_void_p(pb), native.ptr(out), native.ptr(add), M, N, K, lda, ldb, ldd, ldc,
+                int(not trans_b), flags & GEMM_OUT_F32, c_float(alpha), native.stream_ptr())
+            native.check(rc, "b200_gemm_skinny")
+            native.bump()
             return out
-    if (impl == "2cta" and _skinny(M, N) and not trans_a and not force_fallback and bn == 0 and max_ctas == 0
-            and lda % 8 == 0 and ldb % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0):
-        rc = native.lib().b200_gemm_skinny(
-            native.ptr(a), native.ptr(b), native.ptr(out), native.ptr(add), M, N, K, lda, ldb, ldd, ldc,
-            int(not trans_b), flags & GEMM_OUT_F32, ctypes.c_float(alpha), native.stream_ptr())
-        native.check(rc, "b200_gemm_skinny")
-        native.bump()
-        return out
-    if (impl == "2cta" and not force_fallback and bn == 0 and max_ctas == 0 and M >= 256 and N >= 256
-            and lda % 8 == 0 and ldb % 8 == 0 and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0):
-        _apply_dynamic()
-        # Half tiles shorten the tail of a GEMM that has the GPU to itself. While weight-gradient GEMMs
-        # are in flight on the side stream the tail is filled by the other kernel's CTAs, and narrower
-        # tiles only cost efficiency (measured on the 1.3 B step: 1.1 ms faster alone, 1.2 ms slower beside).
-        if _wgrad_pending.get(a.device.index, False):
-            flags |= GEMM_WHOLE_TILES
-        rc = native.lib().b200_gemm_bf16_2cta(
-            native.ptr(a), native.ptr(b), native.ptr(out), native.ptr(add),
-            M, N, K, lda, ldb, ldd, ldc, int(trans_a), int(not trans_b), flags,
-            ctypes.c_float(alpha), native.stream_ptr())
-        native.check(rc, "b200_gemm_bf16_2cta")
-        native.bump()
-        return out
-    rc = native.lib().b200_gemm_bf16(
+        if ok and M >= 256 and N >= 256:
+            po = out.data_ptr()
+            if (po % 16 or ldd * (4 if flags & GEMM_OUT_F32 else 2) % 16) and M * N >= PAD_OUT_AREA:
+                tmp = torch.empty((M, (N + 7) // 8 * 8), dtype=out_dtype, device=a.device)[:, :N]
+                if add is not None:
+                    _copy_rows(add, tmp)
+                gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=tmp, add=None if add is None else tmp, alpha=alpha)
+                _copy_rows(tmp, out)
+                return out
+            dev = a.get_device()
+            splits = split_count(M, N, K, _cta_pairs(dev)) if GEMM_SPLIT_K else 1
+            if splits > 1:
+                ws = torch.empty(splits * (-(-M // 256) * 256) * (-(-N // 4) * 4), dtype=torch.float32, device=a.device)
+                rc = lib.b200_gemm_bf16_2cta_split(
+                    c_void_p(pa), c_void_p(pb), c_void_p(po), native.ptr(add), M, N, K, lda, ldb, ldd, ldc, int(trans_a),
+                    int(not trans_b), flags, c_float(alpha), native.ptr(ws), splits, native.stream_ptr())
+                native.check(rc, "b200_gemm_bf16_2cta_split")
+                native.bump(2)
+                return out
+            _apply_dynamic()
+            # Half tiles shorten the tail of a GEMM that has the GPU to itself. While weight-gradient GEMMs
+            # are in flight on the side stream the tail is filled by the other kernel's CTAs, and narrower
+            # tiles only cost efficiency (measured on the 1.3 B step: 1.1 ms faster alone, 1.2 ms slower beside).
+            if _wgrad_pending.get(dev, False):
+                flags |= GEMM_WHOLE_TILES
+            rc = lib.b200_gemm_bf16_2cta(
+                c_void_p(pa), c_void_p(pb), c_void_p(po), native.ptr(add), M, N, K, lda, ldb, ldd, ldc, int(trans_a),
+                int(not trans_b), flags, c_float(alpha), native.stream_ptr())
+            native.check(rc, "b200_gemm_bf16_2cta")
+            native.bump()
+            return out
+    rc = lib.b200_gemm_bf16(
         native.ptr(a), native.ptr(b), native.ptr(out), native.ptr(add),
         M, N, K, lda, ldb, ldd, ldc, int(trans_a), int(not trans_b), flags,
         ctypes.c_float(alpha), bn, max_ctas, int(force_fallback), native.stream_ptr())

@@ -1,0 +1,40 @@
+"""Split-K form of the CTA-pair GEMM against the fp64 product."""
+import pytest
+import torch
+
+from create_llm_by_cupy_b200.ops import gemm as G
+
+pytestmark = pytest.mark.gpu
+
+
+def bf(*shape, seed):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(torch.bfloat16).cuda()
+
+
+@pytest.mark.parametrize("trans_a,trans_b", [(True, False), (False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(256, 256, 4096), (257, 300, 2056), (512, 264, 8192), (768, 1280, 8192), (777, 768, 4104),
+                                   (300, 2000, 5504)])
+def test_split_k(M, N, K, trans_a, trans_b):
+    p8 = lambda n: (n + 7) // 8 * 8
+    assert G.split_count(M, N, K, 74) > 1
+    a = bf(K, p8(M), seed=1)[:, :M] if trans_a else bf(M, p8(K), seed=1)[:, :K]
+    b = bf(N, p8(K), seed=2)[:, :K] if trans_b else bf(K, p8(N), seed=2)[:, :N]
+    ad, bd = (a.double().t() if trans_a else a.double()), (b.double().t() if trans_b else b.double())
+    ref, bound = ad @ bd, ad.abs() @ bd.abs() * (K * 2.0 ** -23)
+    y = G.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out_dtype=torch.float32, alpha=0.5)
+    assert ((y.double() - 0.5 * ref).abs() <= bound).all()
+    assert torch.equal(y, G.gemm(a, b, trans_a=trans_a, trans_b=trans_b, out_dtype=torch.float32, alpha=0.5))
+    for dt, ulp in ((torch.bfloat16, 2.0 ** -8), (torch.float32, 2.0 ** -23)):
+        c = bf(M, N, seed=3).to(dt)
+        want = ref + c.double()
+        z = G.gemm(a, b, trans_a=trans_a, trans_b=trans_b, add=c, out=c)
+        assert ((z.double() - want).abs() <= bound + ulp * want.abs()).all()
+
+
+def test_split_rule():
+    assert G.split_count(8192, 2048, 2048, 74) == 1          # enough tiles
+    assert G.split_count(768, 768, 768, 74) == 1             # K too short to pay for the second kernel
+    for M, N, K in [(256, 256, 1 << 20), (2048, 2048, 8192), (768, 1280, 8192), (1, 1, 64), (100000, 1, 4096)]:
+        s = G.split_count(M, N, K, 74)
+        tiles = -(-M // 256) * -(-N // 256)
+        assert 1 <= s <= 16 and (s == 1 or (tiles * s <= 74 and s <= -(-K // 64)))
