@@ -7,6 +7,8 @@
 // Differences by design: gradients may arrive as bf16 or fp32, the clip coefficient and the
 // skip-on-non-finite decision are taken on the device from the statistics buffer (no host
 // round trip between the norm and the update), and everything is 128-bit vectorised.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace b200 {
@@ -115,7 +117,7 @@ adamw_kernel(const TG* __restrict__ grad, float* __restrict__ m, float* __restri
 
 // stats[0] += sum over finite g of g^2 ; stats[1] = 1 if any g is NaN/Inf.
 template <typename TG>
-__global__ void __launch_bounds__(256)
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
 grad_stats_kernel(const TG* __restrict__ g, size_t n, float* __restrict__ stats) {
   float ss = 0.f;
   int bad = 0;
@@ -176,13 +178,29 @@ grad_stats_kernel(const TG* __restrict__ g, size_t n, float* __restrict__ stats)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) { sss[warp] = ss; sbad[warp] = bad; }
   __syncthreads();
+  // One atomic per cluster of 8 CTAs: the fp32 total collects at most 148 terms in whatever order they arrive
+  // instead of 1184 (its distance from the 64-bit sum at 44 M gradients was up to 1e-6, and varied from run to run as
+  // much; now 2e-7, for 6 us more).
+  __shared__ float c_ss;
+  __shared__ int c_bad;
   if (threadIdx.x == 0) {
     float t = 0.f;
     int b = 0;
     for (int w = 0; w < int(blockDim.x >> 5); ++w) { t += sss[w]; b |= sbad[w]; }
+    c_ss = t;
+    c_bad = b;
+  }
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+    float t = 0.f;
+    int b = 0;
+    for (int r = 0; r < 8; ++r) { t += *cluster.map_shared_rank(&c_ss, r); b |= *cluster.map_shared_rank(&c_bad, r); }
     atomicAdd(&stats[0], t);
     if (b) stats[1] = 1.f;
   }
+  cluster.sync();                      // the first CTA has read the others' sums
 }
 
 // acc (fp32) += g (bf16|fp32) * scale   — gradient-shard accumulation across micro-batches.
@@ -337,10 +355,10 @@ static int adamw_launch(const void* grad, int grad_fp32, void* m, void* v, void*
   const float* hyper = static_cast<const float*>(hyper_dev);
   AdamArgs a{lr, beta1, beta2, eps, weight_decay, m_corr, v_corr, grad_scale, max_grad_norm};
   // a limited grid is what runs beside the next forward's GEMMs (pipelined optimizer): streaming accesses and the same
-  // shared-memory carve-out as their CTAs
-  const size_t ctas = (size_t(n) + 1023) / 1024;
-  const bool stream = g_adam_max_blocks > 0 && ctas > size_t(g_adam_max_blocks);
-  const int grid = stream ? g_adam_max_blocks : int(ctas < (size_t(1) << 30) ? ctas : size_t(1) << 30);
+  // shared-memory carve-out as their CTAs, for the smallest unit too
+  const bool stream = g_adam_max_blocks > 0;
+  const size_t ctas = (size_t(n) + 1023) / 1024, cap = stream ? size_t(g_adam_max_blocks) : size_t(1) << 30;
+  const int grid = int(ctas < cap ? ctas : cap);
   const uintptr_t all = reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(m) |
                         reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(master) |
                         (reinterpret_cast<uintptr_t>(param) << 1);
@@ -386,7 +404,7 @@ B200_API int b200_adamw_dev(const void* grad, int grad_fp32, void* m, void* v, v
 // Adds into stats[0..1]; the caller zeroes stats once per step.
 B200_API int b200_grad_stats(const void* g, int fp32, long long n, void* stats, cudaStream_t st) {
   if (n <= 0) return 0;
-  const int grid = grid_cap(size_t(n), 256 * 8);
+  const int grid = (grid_cap(size_t(n), 256 * 8) + 7) / 8 * 8;      // whole clusters
   if (fp32) grad_stats_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(g), size_t(n),
                                                            static_cast<float*>(stats));
   else grad_stats_kernel<bf16><<<grid, 256, 0, st>>>(static_cast<const bf16*>(g), size_t(n),
