@@ -285,6 +285,7 @@ def gemm_rope(a: torch.Tensor, b: torch.Tensor, cos: torch.Tensor, sin: torch.Te
     Only where ``gemm_rope_fusable`` holds."""
     M, K = a.shape
     N = b.shape[1]
+    _same_inner("gemm_rope", K, b.shape[0])
     assert gemm_rope_fusable(a, b, head_dim, rope_cols)
     assert cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
     assert cos.shape[0] >= T and cos.shape[1] == head_dim // 2
@@ -308,6 +309,12 @@ def _tma_ok(*ts) -> bool:
                and t.data_ptr() % 16 == 0 for t in ts)
 
 
+def _same_inner(what: str, K: int, Kb: int) -> None:
+    """The kernels take one inner dimension for both operands: a shorter one would be read past its end."""
+    if K != Kb:
+        raise ValueError(f"{what}: inner dims differ ({K} vs {Kb})")
+
+
 def _whole_tiles_flag(device) -> int:
     return GEMM_WHOLE_TILES if _wgrad_pending.get(device.index, False) else 0
 
@@ -327,6 +334,7 @@ def gemm_swiglu(x: torch.Tensor, w_gate_val: torch.Tensor, keep_gv: bool = True)
     Only where ``gemm_swiglu_fusable`` holds."""
     M, K = x.shape
     I = w_gate_val.shape[1] // 2
+    _same_inner("gemm_swiglu", K, w_gate_val.shape[0])
     assert gemm_swiglu_fusable(x, w_gate_val)
     act = torch.empty((M, I), dtype=torch.bfloat16, device=x.device)
     gv = torch.empty((M, 2 * I), dtype=torch.bfloat16, device=x.device) if keep_gv else None
@@ -351,6 +359,7 @@ def gemm_skinny_swiglu(x: torch.Tensor, w_gate_val: torch.Tensor) -> torch.Tenso
     ``gemm_skinny_swiglu_fusable`` holds."""
     M, K = x.shape
     I = w_gate_val.shape[1] // 2
+    _same_inner("gemm_skinny_swiglu", K, w_gate_val.shape[0])
     assert gemm_skinny_swiglu_fusable(x, w_gate_val)
     act = torch.empty((M, I), dtype=torch.bfloat16, device=x.device)
     native.status_tensor()
@@ -376,6 +385,7 @@ def gemm_swiglu_bwd(dout: torch.Tensor, w_out: torch.Tensor, gv: torch.Tensor) -
     epilogue reads the gate / value tiles and writes the two gradients. Only where ``gemm_swiglu_bwd_fusable``."""
     M, K = dout.shape
     I = gv.shape[1] // 2
+    _same_inner("gemm_swiglu_bwd", K, w_out.shape[1])
     assert gemm_swiglu_bwd_fusable(dout, w_out, gv)
     dgv = torch.empty_like(gv)
     native.status_tensor()
@@ -404,6 +414,7 @@ def gemm_delta(dout: torch.Tensor, w_o: torch.Tensor, o: torch.Tensor, T: int, h
     epilogue reads the forward's output ``o`` tile by tile. Only where ``gemm_delta_fusable`` holds."""
     M, K = dout.shape
     N = w_o.shape[0]
+    _same_inner("gemm_delta", K, w_o.shape[1])
     assert gemm_delta_fusable(dout, w_o, o, T, head_dim)
     do = torch.empty((M, N), dtype=torch.bfloat16, device=dout.device)
     delta = torch.empty((M // T, N // head_dim, T), dtype=torch.float32, device=dout.device)
@@ -430,6 +441,7 @@ def gemm_ce_stats(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, tlogi
     (size of the whole vocabulary, 0: unknown) lets the bounds-checking build report targets beyond it."""
     M, K = x.shape
     V = w.shape[0]
+    _same_inner("gemm_ce_stats", K, w.shape[1])
     assert gemm_ce_fusable(x, w) and targets.dtype == torch.int32 and targets.numel() == M
     nt = (V + 255) // 256
     pmax = torch.empty((nt, M), dtype=torch.float32, device=x.device)
@@ -450,6 +462,7 @@ def gemm_ce_dlogits(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, lse
     w.r.t. the logits of vocabulary rows ``col0 .. col0 + V_chunk``, formed in the GEMM epilogue."""
     M, K = x.shape
     C = w.shape[0]
+    _same_inner("gemm_ce_dlogits", K, w.shape[1])
     assert gemm_ce_fusable(x, w) and C % 8 == 0
     out = torch.empty((M, C), dtype=torch.bfloat16, device=x.device)
     native.status_tensor()

@@ -1,0 +1,63 @@
+"""Checks and choices of the GEMM front end that come before any launch. Tensors that call themselves CUDA tensors, and a
+library that only records its calls, take the place of the device."""
+import pytest
+import torch
+
+from create_llm_by_cupy_b200.models.layers import SwiGLU
+from create_llm_by_cupy_b200.ops import gemm as G
+from create_llm_by_cupy_b200.ops import native
+
+
+class FakeCuda(torch.Tensor):
+    is_cuda = property(lambda self: True)
+
+
+def fake(*shape, dtype=torch.bfloat16):
+    return torch.zeros(*shape, dtype=dtype).as_subclass(FakeCuda)
+
+
+class Recorder:
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        return lambda *args: self.calls.append((name, args)) or 0
+
+    def names(self):
+        return [name for name, _ in self.calls]
+
+
+@pytest.fixture
+def lib(monkeypatch):
+    rec = Recorder()
+    monkeypatch.setattr(native, "lib", lambda: rec)
+    monkeypatch.setattr(native, "status_tensor", lambda device=None: None)
+    monkeypatch.setattr(native, "stream_ptr", lambda: native.c_void_p(0))
+    return rec
+
+
+@pytest.mark.parametrize("K", [64, 192])                      # shorter and longer than the weight's 128
+def test_fused_forms_refuse_differing_inner_dimensions(lib, K):
+    w = fake(128, 512)                                        # [K, 2 I]
+    wt = fake(512, 128)                                       # [N, K]
+    few, many = fake(4, K), fake(256, K)
+    targets, lse, coef = fake(256, dtype=torch.int32), fake(256, dtype=torch.float32), fake(256, dtype=torch.float32)
+    cos = fake(256, 32, dtype=torch.float32)
+    for call in (lambda: G.gemm(many, w), lambda: G.gemm_skinny_swiglu(few, w), lambda: G.gemm_swiglu(many, w),
+                 lambda: G.gemm_rope(many, w, cos, cos, 256, 64, 128),
+                 lambda: G.gemm_swiglu_bwd(many, wt, fake(256, 1024)), lambda: G.gemm_delta(many, wt, fake(256, 512), 256, 64),
+                 lambda: G.gemm_ce_stats(many, wt, targets, lse), lambda: G.gemm_ce_dlogits(many, wt, targets, lse, coef)):
+        with pytest.raises(ValueError, match="inner dims differ"):
+            call()
+    assert lib.calls == []
+
+
+@pytest.mark.parametrize("rows", [4, 256])
+@pytest.mark.parametrize("train", [True, False])
+def test_swiglu_layer_refuses_an_input_of_another_width(lib, rows, train):
+    layer = SwiGLU(128, 2, ffn_size=256)
+    layer.params = [p.as_subclass(FakeCuda) for p in layer.params]
+    layer.cache_gate = False
+    with pytest.raises(ValueError, match="inner dims differ"):
+        layer.forward(fake(rows, 192), train_flg=train)
+    assert lib.calls == []
