@@ -48,14 +48,22 @@ int* status_ptr();
 
 enum SwizzleMode { SWIZZLE_NONE_ = 0, SWIZZLE_128B_ = 3 };
 
-// Returns a pointer to a cached 2D tensor map for a row-major matrix of `rows` x `cols` elements
-// of `elem_bytes` bytes with a row pitch of `ld` elements. The box is box_cols x box_rows.
-// Returns nullptr (and prints why) when the matrix breaks a TMA rule (16-byte base / pitch).
-const CUtensorMap* get_tensor_map_2d(const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                                     uint32_t box_rows, uint32_t box_cols, int elem_bytes, int swizzle);
+// A tensor map by value (the cache it came from may drop its entry at any time); converts to a pointer to itself, null
+// when it could not be made.
+struct TensorMap {
+  CUtensorMap map;
+  bool valid = false;
+  operator const CUtensorMap*() const { return valid ? &map : nullptr; }
+};
 
-const CUtensorMap* get_tensor_map_bthd(const void* base, uint64_t B, uint64_t T, uint64_t heads, uint64_t D,
-                                       uint64_t bs, uint64_t ts, uint64_t hs, uint32_t box_t, uint32_t box_d);
+// 2D tensor map for a row-major matrix of `rows` x `cols` elements of `elem_bytes` bytes with a row pitch of `ld`
+// elements. The box is box_cols x box_rows. Not valid (and prints why) when the matrix breaks a TMA rule (16-byte base /
+// pitch).
+TensorMap get_tensor_map_2d(const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_rows,
+                            uint32_t box_cols, int elem_bytes, int swizzle);
+
+TensorMap get_tensor_map_bthd(const void* base, uint64_t B, uint64_t T, uint64_t heads, uint64_t D, uint64_t bs,
+                              uint64_t ts, uint64_t hs, uint32_t box_t, uint32_t box_d);
 
 int num_sms();
 

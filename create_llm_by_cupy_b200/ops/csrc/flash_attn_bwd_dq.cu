@@ -180,9 +180,9 @@ int flash_bwd_dq_from_ds(const void* ds, const void* k, void* dq, const void* va
   if (D != 128 && D != 64) return static_cast<int>(cudaErrorInvalidValue);
   const int nt = (T + 127) / 128;
   const unsigned long long Tp = (unsigned long long)nt * 128;
-  const CUtensorMap* tds =
+  TensorMap tds =
       get_tensor_map_bthd(ds, B, Tp, QH, Tp, (unsigned long long)QH * Tp * Tp, Tp, Tp * Tp, DQG_KEYS, 64);
-  const CUtensorMap* tk = get_tensor_map_bthd(k, B, T, KVH, D, ks[0], ks[1], ks[2], DQG_KEYS, 64);
+  TensorMap tk = get_tensor_map_bthd(k, B, T, KVH, D, ks[0], ks[1], ks[2], DQG_KEYS, 64);
   if (!tds || !tk) return static_cast<int>(cudaErrorInvalidValue);
   DqGemmParams p;
   p.dq = static_cast<bf16*>(dq);

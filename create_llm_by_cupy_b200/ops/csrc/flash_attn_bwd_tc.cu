@@ -1224,12 +1224,12 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   if (D == 64 && ds_ws == nullptr) return static_cast<int>(cudaErrorInvalidValue);
   for (int i = 0; i < 21; ++i)
     if (s[i] % 8 != 0) return static_cast<int>(cudaErrorInvalidValue);
-  const CUtensorMap* tq128 = get_tensor_map_bthd(q, B, T, QH, D, s[0], s[1], s[2], 128, 64);
-  const CUtensorMap* tdo128 = get_tensor_map_bthd(dout, B, T, QH, D, s[9], s[10], s[11], 128, 64);
-  const CUtensorMap* tq64 = get_tensor_map_bthd(q, B, T, QH, D, s[0], s[1], s[2], 64, 64);
-  const CUtensorMap* tdo64 = get_tensor_map_bthd(dout, B, T, QH, D, s[9], s[10], s[11], 64, 64);
-  const CUtensorMap* tk = get_tensor_map_bthd(k, B, T, KVH, D, s[3], s[4], s[5], 128, 64);
-  const CUtensorMap* tv = get_tensor_map_bthd(v, B, T, KVH, D, s[6], s[7], s[8], 128, 64);
+  TensorMap tq128 = get_tensor_map_bthd(q, B, T, QH, D, s[0], s[1], s[2], 128, 64);
+  TensorMap tdo128 = get_tensor_map_bthd(dout, B, T, QH, D, s[9], s[10], s[11], 128, 64);
+  TensorMap tq64 = get_tensor_map_bthd(q, B, T, QH, D, s[0], s[1], s[2], 64, 64);
+  TensorMap tdo64 = get_tensor_map_bthd(dout, B, T, QH, D, s[9], s[10], s[11], 64, 64);
+  TensorMap tk = get_tensor_map_bthd(k, B, T, KVH, D, s[3], s[4], s[5], 128, 64);
+  TensorMap tv = get_tensor_map_bthd(v, B, T, KVH, D, s[6], s[7], s[8], 128, 64);
   if (!tq128 || !tdo128 || !tq64 || !tdo64 || !tk || !tv) return static_cast<int>(cudaErrorInvalidValue);
   FlashBwdTcParams p;
   p.dq = static_cast<bf16*>(dq); p.dk = static_cast<bf16*>(dk); p.dv = static_cast<bf16*>(dv);
@@ -1269,7 +1269,7 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   p.unrot_sin = unrot_cos != nullptr ? static_cast<const float*>(unrot_sin) : nullptr;
   p.unrot_ld = unrot_ld;
   if (p.unrot_cos != nullptr && (p.unrot_sin == nullptr || unrot_ld < T)) return static_cast<int>(cudaErrorInvalidValue);
-  const CUtensorMap* tds = tk;           // placeholder when no workspace is given (never dereferenced then)
+  TensorMap tds = tk;           // placeholder when no workspace is given (never dereferenced then)
   if (ds_ws != nullptr) {
     const unsigned long long Tp = (unsigned long long)nt * 128;
     tds = get_tensor_map_bthd(ds_ws, B, Tp, QH, Tp, (unsigned long long)QH * Tp * Tp, Tp, Tp * Tp, 128, 64);

@@ -389,10 +389,10 @@ B200_API int b200_flash_fwd_tc3(const void* q, const void* k, const void* v, voi
   for (int i = 0; i < 12; ++i)
     if (strides[i] % 8 != 0) return static_cast<int>(cudaErrorInvalidValue);
   if ((reinterpret_cast<uintptr_t>(o) & 15) != 0) return static_cast<int>(cudaErrorInvalidValue);
-  const CUtensorMap* tq = get_tensor_map_bthd(q, B, T, QH, D, strides[0], strides[1], strides[2], 128, 64);
-  const CUtensorMap* tk = get_tensor_map_bthd(k, B, T, KVH, D, strides[3], strides[4], strides[5], 128, 64);
-  const CUtensorMap* tv = get_tensor_map_bthd(v, B, T, KVH, D, strides[6], strides[7], strides[8], 128, 64);
-  const CUtensorMap* to = get_tensor_map_bthd(o, B, T, QH, D, strides[9], strides[10], strides[11], 128, 64);
+  TensorMap tq = get_tensor_map_bthd(q, B, T, QH, D, strides[0], strides[1], strides[2], 128, 64);
+  TensorMap tk = get_tensor_map_bthd(k, B, T, KVH, D, strides[3], strides[4], strides[5], 128, 64);
+  TensorMap tv = get_tensor_map_bthd(v, B, T, KVH, D, strides[6], strides[7], strides[8], 128, 64);
+  TensorMap to = get_tensor_map_bthd(o, B, T, QH, D, strides[9], strides[10], strides[11], 128, 64);
   if (!tq || !tk || !tv || !to) return static_cast<int>(cudaErrorInvalidValue);
   Flash3Params p;
   p.lse = static_cast<float*>(lse);

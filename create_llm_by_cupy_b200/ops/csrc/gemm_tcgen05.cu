@@ -569,9 +569,9 @@ B200_API int b200_gemm_bf16(const void* A, const void* B, void* D, const void* C
   }
 
   // K-major operand: matrix [MN, K], box 64 (K) x tile rows. MN-major: matrix [K, MN], box 64 x 64.
-  const CUtensorMap* tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(A, M, K, lda, GEMM_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(B, N, K, ldb, bn, 64, 2, SWIZZLE_128B_);
   if (!tA || !tB) return static_cast<int>(cudaErrorInvalidValue);
 
@@ -632,9 +632,9 @@ B200_API int b200_gemm_bf16_allgather(const void* A, void* D, const void* C, int
   if ((reinterpret_cast<uintptr_t>(A) & 15) != 0 || (lda % 8) != 0 || (ldb % 8) != 0)
     return static_cast<int>(cudaErrorInvalidValue);
   const int bn = 256;
-  const CUtensorMap* tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(A, M, K, lda, GEMM_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(B, N, K, ldb, bn, 64, 2, SWIZZLE_128B_);
   if (!tA || !tB) return static_cast<int>(cudaErrorInvalidValue);
   if (a_mn_major && b_mn_major) return launch_tc<256, true, true, true>(tA, tB, p, stream, 0);

@@ -1097,22 +1097,22 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
   Gemm2Params p = base_params(D, C, M, N, K, ldd, ldc, flags, alpha);
   p.rope_cos = rope_cos; p.rope_sin = rope_sin; p.rope_T = rope_T; p.rope_cols = rope_cols; p.rope_dim = rope_dim;
   p.rope_ld = rope_ld;
-  const CUtensorMap* tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tBh = b_mn_major ? tB : get_tensor_map_2d(B, N, K, ldb, G2_BN / 4, 64, 2, SWIZZLE_128B_);
+  TensorMap tBh = b_mn_major ? tB : get_tensor_map_2d(B, N, K, ldb, G2_BN / 4, 64, 2, SWIZZLE_128B_);
   if (!tA || !tB || !tBh) return static_cast<int>(cudaErrorInvalidValue);
   // Output (and C) through TMA when their bases and pitches are 16-byte aligned; otherwise the
   // epilogue stores straight from registers.
   const int eb = (flags & G2_OUT_F32) ? 4 : 2;
   const bool add = (flags & G2_ADD_C) != 0;
-  const CUtensorMap* tD = tA;
-  const CUtensorMap* tC = tA;
+  TensorMap tD = tA;
+  TensorMap tC = tA;
   if ((reinterpret_cast<uintptr_t>(D) & 15) == 0 && (size_t(ldd) * eb) % 16 == 0 &&
       (!add || ((reinterpret_cast<uintptr_t>(C) & 15) == 0 && (size_t(ldc) * eb) % 16 == 0))) {
-    const CUtensorMap* d = get_tensor_map_2d(D, M, N, ldd, 128, 128 / eb, eb, SWIZZLE_128B_);
-    const CUtensorMap* c = add ? get_tensor_map_2d(C, M, N, ldc, 128, 128 / eb, eb, SWIZZLE_128B_) : d;
+    TensorMap d = get_tensor_map_2d(D, M, N, ldd, 128, 128 / eb, eb, SWIZZLE_128B_);
+    TensorMap c = add ? get_tensor_map_2d(C, M, N, ldc, 128, 128 / eb, eb, SWIZZLE_128B_) : d;
     if (d && c) {
       tD = d;
       tC = c;
@@ -1146,11 +1146,11 @@ B200_API int b200_gemm_bf16_2cta_split(const void* A, const void* B, void* D, co
   const int ldws = (N + 3) / 4 * 4, rows = num_m * 2 * G2_BM;
   Gemm2Params p = base_params(ws, nullptr, M, N, K, ldws, 0, G2_OUT_F32 | G2_WHOLE_TILES | G2_TMA_OUT, alpha);
   p.splits = splits;
-  const CUtensorMap* tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tA = a_mn_major ? get_tensor_map_2d(A, K, M, lda, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
+  TensorMap tB = b_mn_major ? get_tensor_map_2d(B, K, N, ldb, 64, 64, 2, SWIZZLE_128B_)
                                      : get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tD = get_tensor_map_2d(ws, uint64_t(splits) * rows, N, ldws, 128, 32, 4, SWIZZLE_128B_);
+  TensorMap tD = get_tensor_map_2d(ws, uint64_t(splits) * rows, N, ldws, 128, 32, 4, SWIZZLE_128B_);
   if (!tA || !tB || !tD) return static_cast<int>(cudaErrorInvalidValue);
   int rc;
   if (a_mn_major && b_mn_major) rc = launch_tc2<true, true, EPI_SPLIT>(tA, tB, tB, tD, tD, p, stream);
@@ -1185,11 +1185,11 @@ B200_API int b200_gemm_bf16_2cta_swiglu(const void* A, const void* B, void* GV, 
   Gemm2Params p = base_params(ACT, nullptr, M, 2 * I, K, ldact, 0, (flags & G2_WHOLE_TILES) | G2_TMA_OUT, 1.0f);
   p.sw_I = I;
   p.sw_store_gv = GV != nullptr;
-  const CUtensorMap* tA = get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = get_tensor_map_2d(B, K, 2 * I, ldb, 64, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tAct = get_tensor_map_2d(ACT, M, I, ldact, 128, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tG = tA;
-  const CUtensorMap* tV = tA;
+  TensorMap tA = get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
+  TensorMap tB = get_tensor_map_2d(B, K, 2 * I, ldb, 64, 64, 2, SWIZZLE_128B_);
+  TensorMap tAct = get_tensor_map_2d(ACT, M, I, ldact, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tG = tA;
+  TensorMap tV = tA;
   if (GV != nullptr) {
     tG = get_tensor_map_2d(GV, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
     tV = get_tensor_map_2d(static_cast<const bf16*>(GV) + I, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
@@ -1217,8 +1217,8 @@ B200_API int b200_gemm_bf16_2cta_ce_stats(const void* A, const void* B, int M, i
   p.ce_col0 = col0;
   p.ce_nt0 = nt0;
   p.ce_vocab = vocab;
-  const CUtensorMap* tA = get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
+  TensorMap tA = get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
+  TensorMap tB = get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
   if (!tA || !tB) return static_cast<int>(cudaErrorInvalidValue);
   return launch_tc2<false, false, EPI_CE_STATS>(tA, tB, tB, tA, tA, p, stream);
 }
@@ -1238,9 +1238,9 @@ B200_API int b200_gemm_bf16_2cta_ce_dlogits(const void* A, const void* B, void* 
   p.ce_lse = static_cast<const float*>(lse);
   p.ce_coef = static_cast<const float*>(coef);
   p.ce_col0 = col0;
-  const CUtensorMap* tA = get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tD = get_tensor_map_2d(D, M, N, ldd, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tA = get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
+  TensorMap tB = get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
+  TensorMap tD = get_tensor_map_2d(D, M, N, ldd, 128, 64, 2, SWIZZLE_128B_);
   if (!tA || !tB || !tD) return static_cast<int>(cudaErrorInvalidValue);
   return launch_tc2<false, false, EPI_CE_DLOGITS>(tA, tB, tB, tD, tD, p, stream);
 }
@@ -1263,12 +1263,12 @@ B200_API int b200_gemm_bf16_2cta_swiglu_bwd(const void* DOUT, const void* WOUT, 
     return static_cast<int>(cudaErrorInvalidValue);
   Gemm2Params p = base_params(DGV, nullptr, M, I, K, lddgv, 0, G2_WHOLE_TILES | G2_TMA_OUT, 1.0f);
   p.sw_I = I;
-  const CUtensorMap* tA = get_tensor_map_2d(DOUT, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = get_tensor_map_2d(WOUT, w_rows, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tG = get_tensor_map_2d(GV, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tV = get_tensor_map_2d(static_cast<const bf16*>(GV) + I, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tDG = get_tensor_map_2d(DGV, M, I, lddgv, 128, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tDV = get_tensor_map_2d(static_cast<bf16*>(DGV) + I, M, I, lddgv, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tA = get_tensor_map_2d(DOUT, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
+  TensorMap tB = get_tensor_map_2d(WOUT, w_rows, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
+  TensorMap tG = get_tensor_map_2d(GV, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tV = get_tensor_map_2d(static_cast<const bf16*>(GV) + I, M, I, ldgv, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tDG = get_tensor_map_2d(DGV, M, I, lddgv, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tDV = get_tensor_map_2d(static_cast<bf16*>(DGV) + I, M, I, lddgv, 128, 64, 2, SWIZZLE_128B_);
   if (!tA || !tB || !tG || !tV || !tDG || !tDV) return static_cast<int>(cudaErrorInvalidValue);
   return launch_tc2<false, false, EPI_SWIGLU_BWD>(tA, tB, tG, tDG, tDV, p, stream, tV);
 }
@@ -1293,11 +1293,11 @@ B200_API int b200_gemm_bf16_2cta_delta(const void* DY, const void* WO, void* DO,
   p.dl_T = T;
   p.dl_heads = N / head_dim;
   p.dl_dim = head_dim;
-  const CUtensorMap* tA = get_tensor_map_2d(DY, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tB = get_tensor_map_2d(WO, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tBh = get_tensor_map_2d(WO, N, K, ldb, G2_BN / 4, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tD = get_tensor_map_2d(DO, M, N, lddo, 128, 64, 2, SWIZZLE_128B_);
-  const CUtensorMap* tO = get_tensor_map_2d(O, M, N, ldo, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tA = get_tensor_map_2d(DY, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
+  TensorMap tB = get_tensor_map_2d(WO, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
+  TensorMap tBh = get_tensor_map_2d(WO, N, K, ldb, G2_BN / 4, 64, 2, SWIZZLE_128B_);
+  TensorMap tD = get_tensor_map_2d(DO, M, N, lddo, 128, 64, 2, SWIZZLE_128B_);
+  TensorMap tO = get_tensor_map_2d(O, M, N, ldo, 128, 64, 2, SWIZZLE_128B_);
   if (!tA || !tB || !tBh || !tD || !tO) return static_cast<int>(cudaErrorInvalidValue);
   return launch_tc2<false, false, EPI_DELTA>(tA, tB, tBh, tD, tO, p, stream);
 }
