@@ -588,11 +588,18 @@ def pad_gate_value(w: torch.Tensor, I: int) -> torch.Tensor:
 
 def wgrad_gemm_gate_value(x: torch.Tensor, dgv: torch.Tensor, I: int, out: torch.Tensor | None = None) -> torch.Tensor:
     """``x^T @ dgv`` without the padding columns of ``dgv`` [M, 2 Ip] (see ``pad_gate_value``): [K, 2 I], on the
-    weight-gradient stream like ``wgrad_gemm``."""
+    weight-gradient stream like ``wgrad_gemm``. ``out`` may be bf16 or fp32, as there."""
+    if out is not None:
+        assert out.shape == (x.shape[1], 2 * I) and out.stride(1) == 1
+        if out.dtype not in (torch.bfloat16, torch.float32):
+            raise TypeError("wgrad_gemm_gate_value: out dtype must be bf16 or fp32")
+
     def compute():
-        full = gemm(x, dgv, trans_a=True)
         dst = torch.empty((x.shape[1], 2 * I), dtype=x.dtype, device=x.device) if out is None else out
-        return repitch(full, dst, I, I, 2, dgv.shape[1] // 2, I)
+        full = gemm(x, dgv, trans_a=True, out_dtype=dst.dtype)
+        w = dst.element_size() // 2                        # fp32 moves as pairs of 2-byte words
+        repitch(*(t.view(torch.bfloat16) for t in (full, dst)), I * w, I * w, 2, dgv.shape[1] // 2 * w, I * w)
+        return dst
 
     return _on_wgrad_stream(compute, x, dgv) if WGRAD_OVERLAP else compute()
 

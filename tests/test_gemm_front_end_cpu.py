@@ -30,6 +30,10 @@ class Recorder:
 @pytest.fixture
 def lib(monkeypatch):
     rec = Recorder()
+    empty = torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: empty(*a, **k).as_subclass(FakeCuda))
+    monkeypatch.setattr(G, "_cta_pairs", lambda index: 74)
+    monkeypatch.setattr(G, "WGRAD_OVERLAP", False)
     monkeypatch.setattr(native, "lib", lambda: rec)
     monkeypatch.setattr(native, "status_tensor", lambda device=None: None)
     monkeypatch.setattr(native, "stream_ptr", lambda: native.c_void_p(0))
@@ -60,4 +64,17 @@ def test_swiglu_layer_refuses_an_input_of_another_width(lib, rows, train):
     layer.cache_gate = False
     with pytest.raises(ValueError, match="inner dims differ"):
         layer.forward(fake(rows, 192), train_flg=train)
+    assert lib.calls == []
+
+
+@pytest.mark.parametrize("out,error", [(fake(128, 514), None), (fake(128, 514, dtype=torch.float32), None),
+                                       (fake(128, 514, dtype=torch.float16), TypeError), (fake(128, 520), AssertionError),
+                                       (fake(64, 514), AssertionError), (fake(514, 128).t(), AssertionError)])
+def test_gradient_of_a_padded_width_takes_what_the_plain_gemm_takes(lib, out, error):
+    x, dgv, I = fake(256, 128), fake(256, 528), 257
+    if error is None:
+        assert G.wgrad_gemm_gate_value(x, dgv, I, out=out) is out
+        return
+    with pytest.raises(error):
+        G.wgrad_gemm_gate_value(x, dgv, I, out=out)
     assert lib.calls == []

@@ -68,6 +68,21 @@ def test_swiglu_layer_with_odd_width(M, H, I):
     assert layer.forward(x, train_flg=False).shape == (M, H)
 
 
+@pytest.mark.parametrize("pitch", [0, 3])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gate_value_gradient_into_a_given_matrix(dtype, pitch):
+    M, H, I = 300, 512, 1365
+    x, dgv = bf(M, H, seed=1), G.pad_gate_value(bf(M, 2 * I, seed=2), I)
+    d = torch.cat([dgv[:, :I], dgv[:, 1368:1368 + I]], 1).double()
+    ref, bound = x.double().t() @ d, x.double().abs().t() @ d.abs() * (M * 2.0 ** -23)     # fp32 sums
+    buf = torch.full((H, 2 * I + pitch), 7.0, dtype=dtype, device="cuda")
+    got = F.wgrad_gemm_gate_value(x, dgv, I, out=buf[:, :2 * I])
+    F.wgrad_join(x.device)
+    assert got.data_ptr() == buf.data_ptr() and got.dtype == dtype and (buf[:, 2 * I:] == 7.0).all()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+    assert ((got.double() - ref).abs() <= bound + ulp * ref.abs()).all()
+
+
 def test_gemm_one_row_without_a_pitch():
     row = bf(1029, seed=1)[None].expand(1, -1).as_strided((1, 1029), (0, 1))      # row stride 0
     b = bf(1029, 37, seed=2)
