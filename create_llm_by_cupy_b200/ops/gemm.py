@@ -72,6 +72,8 @@ def _rowmajor_2d(t: torch.Tensor) -> tuple[torch.Tensor, int]:
     s0, s1 = t.stride()
     if s1 != 1 or (rows > 1 and s0 < cols):
         t = t.contiguous()
+        if t.stride(1) != 1:             # one column: contiguous whatever that stride says, so it came back as it was
+            t = t.as_strided((rows, cols), (cols, 1))
         s0 = t.stride(0)
     return t, (s0 if rows > 1 else max(cols, s0))
 

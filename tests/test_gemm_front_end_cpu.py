@@ -78,3 +78,11 @@ def test_gradient_of_a_padded_width_takes_what_the_plain_gemm_takes(lib, out, er
     with pytest.raises(error):
         G.wgrad_gemm_gate_value(x, dgv, I, out=out)
     assert lib.calls == []
+
+
+@pytest.mark.parametrize("K", [40, 1024])
+def test_one_column_in_a_transposed_view_is_taken(lib, K):
+    w = fake(1, K)                                            # w.t(): [K, 1] with strides (1, K)
+    assert G.gemm(fake(5, K), w.t()).shape == (5, 1)
+    assert G.gemm(w.t(), fake(K, 5), trans_a=True).shape == (1, 5)
+    assert ("b200_repitch" in lib.names()) == (K >= 1024)     # the copy that refused such a view

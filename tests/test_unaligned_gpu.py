@@ -88,3 +88,12 @@ def test_gemm_one_row_without_a_pitch():
     b = bf(1029, 37, seed=2)
     want = row.double() @ b.double()
     assert ((G.gemm(row, b).double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-3).all()
+
+
+@pytest.mark.parametrize("M", [1, 5, 300])
+@pytest.mark.parametrize("K", [40, 1024, 1029])
+def test_gemm_with_one_column_in_a_transposed_view(M, K):
+    a, w = bf(M, K, seed=1), bf(1, K, seed=2)
+    want, bound = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t() * (K * 2.0 ** -23)
+    for y in (G.gemm(a, w.t()), G.gemm(w.t(), a.t(), trans_a=True).t()):           # [K, 1] with strides (1, K), as B and as A
+        assert ((y.double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all()
