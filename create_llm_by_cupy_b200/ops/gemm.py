@@ -23,10 +23,13 @@ GEMM_ADD_C = 2
 # 17.7; 32 rows, 2048 x 11008 18 / 14 but 11008 x 4096 36 / 52; 64 rows, 768 x 4096 8.1 / 8.0, 2048 x 3072 10.1 / 13.9.
 SKINNY_ROWS = 64
 SKINNY_AREA = 1 << 18
+SKINNY_COLS = 65535 * 64        # its grid has one row per 64 columns
 
 
 def _skinny(M: int, N: int) -> bool:
-    return M <= 8 or (M <= SKINNY_ROWS and (16 if M <= 16 else 32 if M <= 32 else 64) * N < SKINNY_AREA)
+    if M <= 8:
+        return N <= SKINNY_COLS
+    return M <= SKINNY_ROWS and (16 if M <= 16 else 32 if M <= 32 else 64) * N < SKINNY_AREA
 
 
 GEMM_WHOLE_TILES = 8      # CTA-pair kernel: do not split the tiles of a part-filled last round

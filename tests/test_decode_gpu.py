@@ -64,6 +64,13 @@ def test_skinny_gemm_edges(M, N, K, trans_b):
     assert ((z.double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all()
 
 
+@pytest.mark.parametrize("N", [65535 * 64, 65535 * 64 + 8])      # the most columns of the few-rows grid, and more
+def test_gemm_of_few_rows_and_very_many_columns(N):
+    a, b = bf(2, 8, seed=1).cuda(), bf(8, N, seed=2).cuda()
+    ref, bound = a.double() @ b.double(), a.double().abs() @ b.double().abs() * (8 * 2.0 ** -23)
+    assert ((gemm(a, b).double() - ref).abs() <= bound + 2.0 ** -8 * ref.abs()).all()
+
+
 def test_skinny_gemm_reads_nothing_past_its_operands():
     a, b = torch.full((5, 72), float("nan")).bfloat16().cuda(), torch.full((72, 136), float("nan")).bfloat16().cuda()
     a[:3, :68], b[:68, :131] = 1.0, 1.0

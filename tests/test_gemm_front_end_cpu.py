@@ -86,3 +86,10 @@ def test_one_column_in_a_transposed_view_is_taken(lib, K):
     assert G.gemm(fake(5, K), w.t()).shape == (5, 1)
     assert G.gemm(w.t(), fake(K, 5), trans_a=True).shape == (1, 5)
     assert ("b200_repitch" in lib.names()) == (K >= 1024)     # the copy that refused such a view
+
+
+@pytest.mark.parametrize("N,name", [(65535 * 64, "b200_gemm_skinny"), (65535 * 64 + 8, "b200_gemm_bf16")])
+def test_more_columns_than_the_few_rows_grid_has(lib, N, name):
+    G.gemm(fake(1, 8), fake(8, N))
+    assert lib.names() == [name]
+    assert G.gemm_skinny_swiglu_fusable(fake(1, 8), fake(8, (N + 15) // 16 * 16)) == (N == 65535 * 64)
