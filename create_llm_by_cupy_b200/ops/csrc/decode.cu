@@ -278,8 +278,8 @@ decode_attn_kernel(const DecodeParams p) {
       ls += *cluster.map_shared_rank(&c_l[r], c) * f;
       o += *cluster.map_shared_rank(&c_o[r][d], c) * f;
     }
-    // ls == 0: no valid key, or one whose weight is not a number (then it stays one)
-    p.out[(size_t(b) * p.QH + h0 + r) * D + d] = __float2bfloat16(ls == 0.f ? 0.f : o / ls);
+    // no valid key: zeros. ls == 0 with valid keys: every score is -infinity, and 0 / 0 is what the softmax of those is
+    p.out[(size_t(b) * p.QH + h0 + r) * D + d] = __float2bfloat16(len <= 0 ? 0.f : o / ls);
   }
   cluster.sync();                                       // peers still read this CTA's state until here
 }

@@ -42,6 +42,22 @@ def test_decode_attention_empty_long_and_unaligned():
     assert torch.equal(F.decode_attn(*shifted, torch.full((3,), 40, dtype=torch.int32, device="cuda")), full)
 
 
+@pytest.mark.parametrize("Tmax,D", [(20, 64), (700, 128)])
+def test_decode_attention_infinite_scores(Tmax, D):
+    """Keys whose score is -infinity have no weight; if all are such, or one is +infinity, the result is not a number."""
+    q, kc, vc = bf(4, 4, D, seed=1).abs(), bf(4, 2, Tmax, D, seed=2), bf(4, 2, Tmax, D, seed=3)
+    kc[0] = -float("inf")
+    kc[1, :, 7:] = -float("inf")
+    kc[2, :, :Tmax - 3] = -float("inf")
+    kc[3, :, 5] = float("inf")
+    ln = torch.full((4,), Tmax, dtype=torch.int32)
+    out = F.decode_attn(q.cuda(), kc.cuda(), vc.cuda(), ln.cuda()).float().cpu()
+    ref = F.decode_attn(q.float(), kc.float(), vc.float(), ln)
+    assert ref[[0, 3]].isnan().all() and out[[0, 3]].isnan().all()
+    # half a bf16 ulp of the result, and fp32 sums over at most 7 weighted values (|v| < 6)
+    assert ((out - ref)[1:3].abs() <= 2.0 ** -8 * ref[1:3].abs() + 6 * 7 * 2.0 ** -22).all()
+
+
 @pytest.mark.parametrize("trans_b", [False, True])
 @pytest.mark.parametrize("M,N,K", [
     (1, 1, 1), (1, 8, 8),                 # smallest
