@@ -16,9 +16,9 @@ def bf(*shape, seed):
 @pytest.mark.parametrize("QH,KVH,Tmax,lens", [
     (2, 2, 1, [1]),                                 # one key, R = 1
     (6, 2, 33, [31, 32, 33]),                       # edges of a 32-key tile, 3 of 4 head slots used
-    (4, 2, 300, [1, 255, 256, 257, 300]),           # edges of a pass of 8 CTAs, R = 2
-    (16, 2, 2100, [2048, 2100, 5]),                 # 8 query heads per KV head: two CTA groups; several passes
-    (32, 8, 130, [129] * 20),                       # many (sequence, head) pairs: four-warp CTAs
+    (4, 2, 300, [1, 255, 256, 257, 300]),           # edges of 8 tiles, one per CTA of a cluster; R = 2
+    (16, 2, 2100, [2048, 2100, 5]),                 # 8 query heads per KV head: two CTA groups; 9 warps, a tile each
+    (32, 8, 130, [129] * 20),                       # many (sequence, head) pairs: clusters of 4 CTAs of two warps
 ])
 def test_decode_attention_edges(D, QH, KVH, Tmax, lens):
     B = len(lens)
@@ -40,6 +40,55 @@ def test_decode_attention_empty_long_and_unaligned():
     assert torch.equal(out[2], full[2])
     shifted = [torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:].view(t.shape).copy_(t) for t in (q, kc, vc)]
     assert torch.equal(F.decode_attn(*shifted, torch.full((3,), 40, dtype=torch.int32, device="cuda")), full)
+
+
+# More 32-key tiles than a cluster has warps, so that warps walk several and rescale what they have summed: 8 CTAs of 4
+# warps (more than one CTA per SM) take 32 tiles per round, 8 CTAs of 16 take 128.
+ROUNDS = [(8, 32, 8, 128, [2100, 2099, 1025, 1024, 33, 1500, 2048, 700]), (1, 4, 1, 64, [9001]), (2, 2, 2, 32, [4097, 8200])]
+
+
+@pytest.mark.parametrize("trend", [2.0, -2.0])      # the largest scores come last / first
+@pytest.mark.parametrize("B,QH,KVH,D,lens", ROUNDS)
+def test_decode_attention_several_tiles_per_warp(B, QH, KVH, D, lens, trend):
+    Tmax = max(lens)
+    q, kc, vc = bf(B, QH, D, seed=1), bf(B, KVH, Tmax, D, seed=2), bf(B, KVH, Tmax, D, seed=3)
+    kc = (kc.float() * torch.exp(torch.linspace(-trend / 2, trend / 2, Tmax))[:, None]).bfloat16()
+    ln = torch.tensor(lens, dtype=torch.int32)
+    out = F.decode_attn(q.cuda(), kc.cuda(), vc.cuda(), ln.cuda()).double().cpu()
+    assert ((out - attention64(q, kc, vc, lens)).abs() <= attention_bound(out, Tmax)).all()
+
+
+def attention64(q, kc, vc, lens):
+    B, QH, D = q.shape
+    out = torch.zeros(B, QH, D, dtype=torch.float64)
+    for b, n in enumerate(lens):
+        k, v = (c[b, :, :n].double().repeat_interleave(QH // kc.shape[1], 0) for c in (kc, vc))
+        out[b] = torch.einsum("ht,htd->hd", torch.einsum("hd,htd->ht", q[b].double(), k).mul(D ** -0.5).softmax(-1), v)
+    return out
+
+
+def attention_bound(out, n):
+    """Half a bf16 ulp of the result, fp32 sums over n weighted values (|v| < 6), and weights whose exponents (fp32 sums
+    below 64 in size) are good to 64 * 2^-22."""
+    return 2.0 ** -8 * out.abs() + 6 * (n * 2.0 ** -23 + 64 * 2.0 ** -22)
+
+
+@pytest.mark.parametrize("B,QH,KVH,D,lens", ROUNDS + [(3, 6, 2, 64, [33, 32, 40]), (2, 8, 2, 128, [1, 300])])
+def test_decode_append_against_fp64(B, QH, KVH, D, lens):
+    """Tables of 0, 1 / 2 and 1 make the rotation exact, so that the rotated rows are known to the last bit."""
+    Tmax = max(lens)
+    cos, sin = (torch.randint(-2, 3, (Tmax, D // 2), generator=torch.Generator().manual_seed(s)).float() / 2 for s in (7, 8))
+    for pos in {Tmax - 1, Tmax // 2, 0}:
+        kqv, kc, vc = bf(B, (QH + 2 * KVH) * D, seed=1), bf(B, KVH, Tmax, D, seed=2), bf(B, KVH, Tmax, D, seed=3)
+        x1, x2 = kqv[:, :(KVH + QH) * D].float().view(B, -1, 2, D // 2).unbind(2)
+        c, s = cos[pos], sin[pos]
+        rot = torch.cat([x1 * c - x2 * s, x2 * c + x1 * s], -1).bfloat16()
+        kc1, vc1 = kc.clone(), vc.clone()
+        kc1[:, :, pos], vc1[:, :, pos] = rot[:, :KVH], kqv[:, (KVH + QH) * D:].view(B, KVH, D)
+        kd, vd, ln = kc.cuda(), vc.cuda(), torch.tensor(lens, dtype=torch.int32).cuda()
+        out = F.decode_attn_append(kqv.cuda(), kd, vd, ln, pos, QH, KVH, cos.cuda(), sin.cuda(), D ** -0.5).double().cpu()
+        assert torch.equal(kd.cpu(), kc1) and torch.equal(vd.cpu(), vc1)
+        assert ((out - attention64(rot[:, KVH:], kc1, vc1, lens)).abs() <= attention_bound(out, Tmax)).all()
 
 
 @pytest.mark.parametrize("Tmax,D", [(20, 64), (700, 128)])
