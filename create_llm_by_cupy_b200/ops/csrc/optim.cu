@@ -7,8 +7,6 @@
 // Differences by design: gradients may arrive as bf16 or fp32, the clip coefficient and the
 // skip-on-non-finite decision are taken on the device from the statistics buffer (no host
 // round trip between the norm and the update), and everything is 128-bit vectorised.
-#include <cooperative_groups.h>
-
 #include "common.cuh"
 
 namespace b200 {
@@ -116,13 +114,23 @@ adamw_kernel(const TG* __restrict__ grad, float* __restrict__ m, float* __restri
 }
 
 // stats[0] += sum over finite g of g^2 ; stats[1] = 1 if any g is NaN/Inf.
+// Bound by memory: every gradient read once. One CTA of 1024 threads per SM leaves 148 sums to meet in one fp32 word in
+// whatever order they arrive, and several sums per thread keep the chains short; 8 (fp32: 4) 16-byte loads per thread are
+// in flight. Back to back, with the mean distance from the 64-bit sum: 44.3 M bf16 gradients (88.6 MB) 18.5 us (4.8 TB/s),
+// 1.4e-7; 300 M 90.6 us (6.6 TB/s), 4.6e-7; 44.3 M fp32 29.8 us, 1.2e-7. The same three on 1184 CTAs of 256 threads with
+// one atomic each: 17.4 us, 4.0e-7; 87.6 us, 2.6e-6; 30.8 us, 3.7e-7. With those in clusters of 8 and one atomic per
+// cluster, for which the GPU has no room all at once: 23.3 us, 1.6e-7; 117 us, 2.2e-6; 32.9 us, 1.4e-7.
+constexpr int GS_THREADS = 1024;
 template <typename TG>
-__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(256)
+__global__ void __launch_bounds__(GS_THREADS)
 grad_stats_kernel(const TG* __restrict__ g, size_t n, float* __restrict__ stats) {
-  float ss = 0.f;
+  constexpr int LOADS = sizeof(TG) == 4 ? 4 : 8, SUMS = sizeof(TG) == 4 ? 2 : 8;
+  float sum[SUMS];
+#pragma unroll
+  for (int u = 0; u < SUMS; ++u) sum[u] = 0.f;
   int bad = 0;
-  auto take = [&](float x) {
-    if (isfinite(x)) ss += x * x;
+  auto take = [&](float x, int u) {
+    if (isfinite(x)) sum[u % SUMS] += x * x;
     else bad = 1;
   };
   // 16-byte loads over the aligned body, scalar loads for the unaligned head and the tail
@@ -134,21 +142,21 @@ grad_stats_kernel(const TG* __restrict__ g, size_t n, float* __restrict__ stats)
   const uint4* gv = reinterpret_cast<const uint4*>(g + head);
   const size_t tid = size_t(blockIdx.x) * blockDim.x + threadIdx.x, nthr = size_t(gridDim.x) * blockDim.x;
   size_t i = tid;
-  for (; i + 3 * nthr < nvec; i += 4 * nthr) {
-    uint4 t[4];
+  for (; i + (LOADS - 1) * nthr < nvec; i += LOADS * nthr) {
+    uint4 t[LOADS];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) t[u] = gv[i + u * nthr];
+    for (int u = 0; u < LOADS; ++u) t[u] = gv[i + u * nthr];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < LOADS; ++u) {
       if constexpr (sizeof(TG) == 4) {
-        take(__uint_as_float(t[u].x)); take(__uint_as_float(t[u].y));
-        take(__uint_as_float(t[u].z)); take(__uint_as_float(t[u].w));
+        take(__uint_as_float(t[u].x), u); take(__uint_as_float(t[u].y), u);
+        take(__uint_as_float(t[u].z), u); take(__uint_as_float(t[u].w), u);
       } else {
         const bf162* h = reinterpret_cast<const bf162*>(&t[u]);
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float2 f = __bfloat1622float2(h[e]);
-          take(f.x); take(f.y);
+          take(f.x, u); take(f.y, u);
         }
       }
     }
@@ -156,51 +164,38 @@ grad_stats_kernel(const TG* __restrict__ g, size_t n, float* __restrict__ stats)
   for (; i < nvec; i += nthr) {
     const uint4 t = gv[i];
     if constexpr (sizeof(TG) == 4) {
-      take(__uint_as_float(t.x)); take(__uint_as_float(t.y)); take(__uint_as_float(t.z)); take(__uint_as_float(t.w));
+      take(__uint_as_float(t.x), 0); take(__uint_as_float(t.y), 0); take(__uint_as_float(t.z), 0); take(__uint_as_float(t.w), 0);
     } else {
       const bf162* h = reinterpret_cast<const bf162*>(&t);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const float2 f = __bfloat1622float2(h[e]);
-        take(f.x); take(f.y);
+        take(f.x, 0); take(f.y, 0);
       }
     }
   }
-  for (size_t j = tid; j < head; j += nthr) take(ld_as_float<TG>(g, j));
-  for (size_t j = head + nvec * PER + tid; j < n; j += nthr) take(ld_as_float<TG>(g, j));
+  for (size_t j = tid; j < head; j += nthr) take(ld_as_float<TG>(g, j), 0);
+  for (size_t j = head + nvec * PER + tid; j < n; j += nthr) take(ld_as_float<TG>(g, j), 0);
+  float ss = sum[0];
+#pragma unroll
+  for (int u = 1; u < SUMS; ++u) ss += sum[u];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     ss += __shfl_xor_sync(0xffffffffu, ss, o);
     bad |= __shfl_xor_sync(0xffffffffu, bad, o);
   }
-  __shared__ float sss[8];
-  __shared__ int sbad[8];
+  __shared__ float sss[GS_THREADS / 32];
+  __shared__ int sbad[GS_THREADS / 32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) { sss[warp] = ss; sbad[warp] = bad; }
   __syncthreads();
-  // One atomic per cluster of 8 CTAs: the fp32 total collects at most 148 terms in whatever order they arrive
-  // instead of 1184 (its distance from the 64-bit sum at 44 M gradients was up to 1e-6, and varied from run to run as
-  // much; now 2e-7, for 6 us more).
-  __shared__ float c_ss;
-  __shared__ int c_bad;
   if (threadIdx.x == 0) {
     float t = 0.f;
     int b = 0;
-    for (int w = 0; w < int(blockDim.x >> 5); ++w) { t += sss[w]; b |= sbad[w]; }
-    c_ss = t;
-    c_bad = b;
-  }
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  cluster.sync();
-  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
-    float t = 0.f;
-    int b = 0;
-    for (int r = 0; r < 8; ++r) { t += *cluster.map_shared_rank(&c_ss, r); b |= *cluster.map_shared_rank(&c_bad, r); }
+    for (int w = 0; w < GS_THREADS / 32; ++w) { t += sss[w]; b |= sbad[w]; }
     atomicAdd(&stats[0], t);
     if (b) stats[1] = 1.f;
   }
-  cluster.sync();                      // the first CTA has read the others' sums
 }
 
 // acc (fp32) += g (bf16|fp32) * scale   — gradient-shard accumulation across micro-batches.
@@ -404,11 +399,12 @@ B200_API int b200_adamw_dev(const void* grad, int grad_fp32, void* m, void* v, v
 // Adds into stats[0..1]; the caller zeroes stats once per step.
 B200_API int b200_grad_stats(const void* g, int fp32, long long n, void* stats, cudaStream_t st) {
   if (n <= 0) return 0;
-  const int grid = (grid_cap(size_t(n), 256 * 8) + 7) / 8 * 8;      // whole clusters
-  if (fp32) grad_stats_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float*>(g), size_t(n),
-                                                           static_cast<float*>(stats));
-  else grad_stats_kernel<bf16><<<grid, 256, 0, st>>>(static_cast<const bf16*>(g), size_t(n),
-                                                     static_cast<float*>(stats));
+  const size_t want = (size_t(n) + GS_THREADS * 8 - 1) / (GS_THREADS * 8);
+  const int grid = int(want < size_t(num_sms()) ? want : size_t(num_sms()));
+  if (fp32) grad_stats_kernel<float><<<grid, GS_THREADS, 0, st>>>(static_cast<const float*>(g), size_t(n),
+                                                                  static_cast<float*>(stats));
+  else grad_stats_kernel<bf16><<<grid, GS_THREADS, 0, st>>>(static_cast<const bf16*>(g), size_t(n),
+                                                            static_cast<float*>(stats));
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -1,4 +1,4 @@
-"""Gradient statistics at the edges of their clusters, against fp64."""
+"""Gradient statistics at the edges of their CTAs, against fp64."""
 import pytest
 import torch
 
@@ -8,13 +8,13 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
-@pytest.mark.parametrize("n,shift", [(1, 0), (7, 1), (2048, 0), (2049, 0), (8 * 2048 + 1, 3), (5_000_011, 0)])
+@pytest.mark.parametrize("n,shift", [(1, 0), (7, 1), (2048, 0), (2049, 0), (8 * 2048 + 1, 3), (8192, 0), (8193, 1), (5_000_011, 0)])
 def test_grad_stats_clusters(n, shift, dtype):
     g = (torch.randn(n + shift, generator=torch.Generator().manual_seed(0)) * 1e-2).to(dtype).cuda()[shift:]
     stats = torch.tensor([2.0, 0.0], device="cuda")
     F.grad_stats(g, stats)
     want = 2.0 + g.double().square().sum()
-    # positive terms: a chain of at most 64 per thread, 5 + 8 + 8 levels above it, at most 148 additions at the end
+    # positive terms: a chain of at most 40 per thread, 8 + 5 + 32 additions above it, at most 148 at the end
     assert abs(float(stats[0]) - float(want)) <= 230 * 2.0 ** -24 * float(want) and float(stats[1]) == 0.0
     for bad in (float("nan"), float("inf")):
         b = g.clone()
