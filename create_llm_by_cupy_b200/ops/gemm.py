@@ -5,8 +5,10 @@ Replaces the ``cp.matmul`` (cuBLAS) call sites of the reference
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import functools
+import threading
 
 import torch
 
@@ -559,29 +561,46 @@ def wgrad_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None
     return _on_wgrad_stream(lambda: gemm(a, b, trans_a=True, out=out), a, b)
 
 
+# Operands of side-stream GEMMs stay referenced until the stream that issued them waits for the side stream: from then on
+# their memory may be used again in that stream's order. ``record_stream`` gives a block back only when the host has seen
+# its event complete, so a host that runs ahead takes new device memory on every pass (125M, 8 x 1024 tokens: 12.0 GB
+# reserved in place of 3.2, and cudaMalloc calls of milliseconds between the launches). It remains for a stream that issues
+# more than WGRAD_HELD of them without joining (a model's block issues four).
+WGRAD_HELD = 8
+_wgrad_held: dict = {}        # (device index, raw stream) -> deque of operand pairs
+_wgrad_lock = threading.Lock()
+
+
 def _on_wgrad_stream(compute, a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """``compute()``, which reads ``a`` and ``b``, on the side stream behind everything issued on the current one."""
     ws = _wgrad_stream(a.device)
-    _wgrad_pending[a.device.index] = True
-    if a.device.index == torch._C._cuda_getDevice():
-        # what ``ws.wait_stream`` and ``with torch.cuda.stream(ws)`` do, without their device checks and stream
-        # objects (about 25 us of host time per weight gradient)
-        prev = torch._C._cuda_getCurrentStream(a.device.index)
-        ev = torch.cuda.Event()
-        ev.record(torch.cuda.Stream(stream_id=prev[0], device_index=prev[1], device_type=prev[2]))
-        ws.wait_event(ev)
-        torch._C._cuda_setStream(stream_id=ws.stream_id, device_index=ws.device_index, device_type=ws.device_type)
-        try:
-            res = compute()
-        finally:
-            torch._C._cuda_setStream(stream_id=prev[0], device_index=prev[1], device_type=prev[2])
-    else:
+    index = a.device.index
+    _wgrad_pending[index] = True
+    issuer = torch._C._cuda_getCurrentRawStream(index)
+    try:
+        if index == torch._C._cuda_getDevice():
+            # what ``ws.wait_stream`` and ``with torch.cuda.stream(ws)`` do, without their device checks and stream
+            # objects (about 25 us of host time per weight gradient)
+            prev = torch._C._cuda_getCurrentStream(index)
+            ev = torch.cuda.Event()
+            ev.record(torch.cuda.Stream(stream_id=prev[0], device_index=prev[1], device_type=prev[2]))
+            ws.wait_event(ev)
+            torch._C._cuda_setStream(stream_id=ws.stream_id, device_index=ws.device_index, device_type=ws.device_type)
+            try:
+                return compute()
+            finally:
+                torch._C._cuda_setStream(stream_id=prev[0], device_index=prev[1], device_type=prev[2])
         ws.wait_stream(torch.cuda.current_stream(a.device))
         with torch.cuda.stream(ws):
-            res = compute()
-    a.record_stream(ws)
-    b.record_stream(ws)
-    return res
+            return compute()
+    finally:
+        # after the launch, so that whoever takes the pair out waits behind it
+        with _wgrad_lock:
+            held = _wgrad_held.setdefault((index, issuer), collections.deque())
+            held.append((a, b))
+            if len(held) > WGRAD_HELD:
+                for t in held.popleft():
+                    t.record_stream(ws)
 
 
 def pad_gate_value(w: torch.Tensor, I: int) -> torch.Tensor:
@@ -633,5 +652,9 @@ def wgrad_join(device=None) -> None:
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     ws = _wgrad_streams.get(key)
     if ws is not None:
-        torch.cuda.current_stream(dev).wait_stream(ws)
+        cur = torch.cuda.current_stream(dev)
+        with _wgrad_lock:
+            held = _wgrad_held.pop((key, cur.cuda_stream), None)
+        cur.wait_stream(ws)
+        del held                          # not before the wait
     _wgrad_pending[key] = False
