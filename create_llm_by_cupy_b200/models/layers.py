@@ -217,7 +217,7 @@ class GroupedQueryAttention:
         else:
             F.flash_attn_bwd(do.view(B, T, self.QH, self.D), q, k, v, o, lse, valid_len=valid_len,
                              scale=self.scale, rope=tabs, out=(dq, dk, dv))
-        dW_KQV = F.wgrad_gemm(x, dkqv, out=go[0])
+        dW_KQV = F.wgrad_gemm(x, dkqv, out=go[0], last=True)          # a block's backward ends with its attention
         dx = F.gemm(dkqv, self.params[0], trans_b=True)
         self.grads = [dW_KQV, dW_O]
         self.cache = None

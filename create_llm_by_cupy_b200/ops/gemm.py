@@ -143,6 +143,25 @@ def split_count(M: int, N: int, K: int, pairs: int) -> int:
     return best if cost(best) < cost(1) - 4.0 else 1
 
 
+def _splits(M: int, N: int, K: int, dev: int, side: bool | None) -> int:
+    """K ranges per tile for one call. ``split_count`` gives the GEMM the GPU to itself; beside another kernel the idle
+    pairs are not idle, and what remains of its gain depends on who waits for the result:
+      * while weight gradients are pending (``side`` None) a split pays up to three tenths of the pairs in tiles: 777 x 768
+        over 4096 (12 tiles), MLP forward + backward 82.8 / 81.5 us whole / split; 1024 x 1280 over 6832 (20) 170.6 / 163.1;
+        but 2048 x 768 over 4096 (24) 101.8 / 105.0, 2048 x 1024 over 5472 (32) 165.6 / 169.1;
+      * a weight gradient on the side stream that the issuing stream has long work to hide (``side`` False) stays whole:
+        split it delays that work (768 x 768 over 8192 beside the attention backward: attention layer 308 / 316 us, 125M
+        training pass 8582 / 8671; 2048 x 768 over 8192 beside the MLP's backward: pass 8582 / 8602);
+      * one that is waited for soon (``side`` True) is split: 768 x 1280 over 8192 at the end of the attention layer 308 /
+        290 us, pass 8582 / 8571 (at 5600 rows 6346 / 6393)."""
+    if not GEMM_SPLIT_K or side is False:
+        return 1
+    pairs = _cta_pairs(dev)
+    if side is None and _wgrad_pending.get(dev, False) and -(-M // 256) * -(-N // 256) * 10 > pairs * 3:
+        return 1
+    return split_count(M, N, K, pairs)
+
+
 _pairs: dict = {}
 
 
@@ -156,12 +175,14 @@ def _cta_pairs(index: int) -> int:
 def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bool = False,
          out: torch.Tensor | None = None, add: torch.Tensor | None = None,
          out_dtype: torch.dtype | None = None, alpha: float = 1.0, bn: int = 0,
-         max_ctas: int = 0, force_fallback: bool = False, impl: str | None = None) -> torch.Tensor:
+         max_ctas: int = 0, force_fallback: bool = False, impl: str | None = None,
+         side: bool | None = None) -> torch.Tensor:
     """``out = alpha * op(a) @ op(b) (+ add)``.
 
     ``a`` is ``[M, K]`` (``[K, M]`` with ``trans_a``); ``b`` is ``[K, N]`` (``[N, K]`` with
     ``trans_b``). Inputs are bf16 on CUDA; ``out``/``add`` are bf16 or fp32 (same dtype) and
-    ``add`` may alias ``out`` (accumulation). Accumulation is fp32 in TMEM.
+    ``add`` may alias ``out`` (accumulation). Accumulation is fp32 in TMEM. ``side`` marks a weight gradient on the
+    side stream (see ``_splits``).
     """
     M, K = (a.shape[1], a.shape[0]) if trans_a else (a.shape[0], a.shape[1])
     Kb, N = (b.shape[1], b.shape[0]) if trans_b else (b.shape[0], b.shape[1])
@@ -220,11 +241,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                 tmp = torch.empty((M, (N + 7) // 8 * 8), dtype=out_dtype, device=a.device)[:, :N]
                 if add is not None:
                     _copy_rows(add, tmp)
-                gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=tmp, add=None if add is None else tmp, alpha=alpha)
+                gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=tmp, add=None if add is None else tmp, alpha=alpha,
+                     side=side)
                 _copy_rows(tmp, out)
                 return out
             dev = a.get_device()
-            splits = split_count(M, N, K, _cta_pairs(dev)) if GEMM_SPLIT_K else 1
+            splits = _splits(M, N, K, dev, side)
             if splits > 1:
                 ws = torch.empty(splits * (-(-M // 256) * 256) * (-(-N // 4) * 4), dtype=torch.float32, device=a.device)
                 rc = lib.b200_gemm_bf16_2cta_split(
@@ -553,12 +575,13 @@ def _wgrad_stream(device):
     return st
 
 
-def wgrad_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+def wgrad_gemm(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, last: bool = False) -> torch.Tensor:
     """``a^T @ b`` for a weight gradient; runs on the side stream when overlap is enabled. The
-    caller must call ``wgrad_join()`` before the result is consumed on the main stream."""
+    caller must call ``wgrad_join()`` before the result is consumed on the main stream. ``last``: little follows on the
+    main stream before that join."""
     if not (WGRAD_OVERLAP and a.is_cuda):
         return gemm(a, b, trans_a=True, out=out)
-    return _on_wgrad_stream(lambda: gemm(a, b, trans_a=True, out=out), a, b)
+    return _on_wgrad_stream(lambda: gemm(a, b, trans_a=True, out=out, side=last), a, b)
 
 
 # Operands of side-stream GEMMs stay referenced until the stream that issued them waits for the side stream: from then on
@@ -620,7 +643,7 @@ def wgrad_gemm_gate_value(x: torch.Tensor, dgv: torch.Tensor, I: int, out: torch
 
     def compute():
         dst = torch.empty((x.shape[1], 2 * I), dtype=x.dtype, device=x.device) if out is None else out
-        full = gemm(x, dgv, trans_a=True, out_dtype=dst.dtype)
+        full = gemm(x, dgv, trans_a=True, out_dtype=dst.dtype, side=False if WGRAD_OVERLAP else None)
         w = dst.element_size() // 2                        # fp32 moves as pairs of 2-byte words
         repitch(*(t.view(torch.bfloat16) for t in (full, dst)), I * w, I * w, 2, dgv.shape[1] // 2 * w, I * w)
         return dst

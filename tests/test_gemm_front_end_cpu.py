@@ -93,3 +93,17 @@ def test_more_columns_than_the_few_rows_grid_has(lib, N, name):
     G.gemm(fake(1, 8), fake(8, N))
     assert lib.names() == [name]
     assert G.gemm_skinny_swiglu_fusable(fake(1, 8), fake(8, (N + 15) // 16 * 16)) == (N == 65535 * 64)
+
+
+@pytest.mark.parametrize("tiles,pending,side,split", [
+    ((3, 4), False, None, True), ((3, 8), False, None, True),       # alone
+    ((3, 4), True, None, True), ((2, 11), True, None, True), ((3, 8), True, None, False),     # beside weight gradients
+    ((3, 4), True, False, False), ((3, 4), True, True, True), ((3, 8), True, True, True),     # a weight gradient itself
+])
+def test_split_k_beside_other_kernels(lib, monkeypatch, tiles, pending, side, split):
+    M, N = (256 * t for t in tiles)
+    monkeypatch.setitem(G._wgrad_pending, -1, pending)              # device index of these tensors
+    G.gemm(fake(M, 8192), fake(8192, N), side=side)
+    assert lib.names()[-1] == ("b200_gemm_bf16_2cta_split" if split else "b200_gemm_bf16_2cta")
+    G.gemm(fake(M, 8192), fake(8192, N), side=side, out=fake(M, N + 1)[:, :N])                # through an aligned output
+    assert lib.names()[-2] == ("b200_gemm_bf16_2cta_split" if split else "b200_gemm_bf16_2cta")
