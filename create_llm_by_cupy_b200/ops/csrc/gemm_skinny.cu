@@ -42,6 +42,7 @@ struct SkinnySmem {
   static constexpr int kStageBytes = SK_W_BYTES + kABytes;
   static constexpr int kSum = MT * 8 * SK_TN * 4;                  // fp32 [rows][64] for the cluster's sum
   static constexpr int kTotal = kStages * kStageBytes > kSum ? kStages * kStageBytes : kSum;
+  static constexpr int kPerSm = 228 * 1024 / (kTotal + 1024);      // CTAs that fit an SM: 4 up to 8 rows, then 3
 };
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
@@ -190,10 +191,9 @@ static int launch_skinny(SkinnyParams p, cudaStream_t st) {
   if (S::kTotal > 48 * 1024) B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
   const int tiles = GLU ? (2 * p.I + SK_TN - 1) / SK_TN : (p.N + SK_TN - 1) / SK_TN, ksteps = (p.K + SK_TK - 1) / SK_TK;
   if (tiles > 65535) return static_cast<int>(cudaErrorInvalidValue);
-  // k slices: as many as keep the GPU's resident CTAs (about 4 per SM) filled once, at most 8 (a portable cluster)
-  // and at least 2 stages each
+  // k slices: as many as fill the GPU's resident CTAs once, at most 8 (a portable cluster) and at least 2 stages each
   int ks = 1;
-  while (ks < 8 && long(tiles) * ks * 2 <= 4L * num_sms() && ksteps >= 4 * ks) ks *= 2;
+  while (ks < 8 && long(tiles) * ks * 2 <= long(S::kPerSm) * num_sms() && ksteps >= 4 * ks) ks *= 2;
   p.kslice = (ksteps + ks - 1) / ks * SK_TK;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ks, tiles);
