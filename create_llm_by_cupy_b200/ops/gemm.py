@@ -19,12 +19,17 @@ c_void_p, c_float = ctypes.c_void_p, ctypes.c_float
 GEMM_OUT_F32 = 1
 GEMM_ADD_C = 2
 # Few rows: the skinny kernel (weights streamed once, K split over a cluster) instead of 128-row tensor-core tiles.
-# Up to 8 rows it always wins (768 x 768: 3.6 against 6.8 us, 2048 x 11008: 11 / 18, 4096 x 22016: 34 / 43). Beyond
-# that every 64-column CTA reads the activations again, while the tensor-core tiles are bound by their serial walk
-# over K on N / 128 SMs, so the line lies at rows x columns: 16 rows, 4096 x 22016 41 / 33.5 us but 2048 x 11008 13.4 /
-# 17.7; 32 rows, 2048 x 11008 18 / 14 but 11008 x 4096 36 / 52; 64 rows, 768 x 4096 8.1 / 8.0, 2048 x 3072 10.1 / 13.9.
+# Up to 8 rows it always wins (skinny / tiles in us: 768 x 768: 3.6 / 6.8, 2048 x 11008: 11 / 18, 4096 x 22016: 34 / 43).
+# Beyond that every 64-column CTA reads the activations again, so the line lies at rows x columns: 16 rows, K x 11008 wins
+# (K = 768 9.6 / 10.3, 2048 14.8 / 20, 4096 24.6 / 24.8) but K x 16384 does not (768 15 / 11.5, 2048 25 / 20.6); 32 rows,
+# K x 6144 wins (768 8.2 / 9.0, 2048 12.4 / 14.4, 11008 41 / 54), K x 8192 does not (768 10.3 / 9.5, 2048 16.5 / 14.5, 11008
+# 60 / 55); 64 rows, K x 3072 wins (768 10.3 / 10.3, 2048 12.4 / 15, 11008 32 / 54), K x 5120 does not (768 10.8 / 10.3,
+# 2048 16.5 / 15.6, 11008 55.6 / 54.8). K alone moves it only where it is short, and then the tiles win: K = 256, 32 rows,
+# 256 x 2048 8.2 / 6.2; 64 rows 10.3 / 6.2; from K = 512 on 6.2 / 8.0 and 8.2 / 8.2. (The SwiGLU form and the one-call forms
+# save launches as well and take a short K too.)
 SKINNY_ROWS = 64
 SKINNY_AREA = 1 << 18
+SKINNY_K = 512
 SKINNY_COLS = 65535 * 64        # its grid has one row per 64 columns
 
 
@@ -228,7 +233,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         if not ok and M * N > 0 and (M * N * K >= PAD_WORK or K >= PAD_K):
             (a, lda), (b, ldb) = _padded(a, lda), _padded(b, ldb)
             pa, pb, ok = a.data_ptr(), b.data_ptr(), True
-        if ok and M <= SKINNY_ROWS and not trans_a and _skinny(M, N):
+        if ok and M <= SKINNY_ROWS and not trans_a and (M <= 8 or K >= SKINNY_K) and _skinny(M, N):
             rc = lib.b200_gemm_skinny(
                 c_void_p(pa), c_void_p(pb), native.ptr(out), native.ptr(add), M, N, K, lda, ldb, ldd, ldc,
                 int(not trans_b), flags & GEMM_OUT_F32, c_float(alpha), native.stream_ptr())

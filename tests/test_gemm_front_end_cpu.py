@@ -107,3 +107,10 @@ def test_split_k_beside_other_kernels(lib, monkeypatch, tiles, pending, side, sp
     assert lib.names()[-1] == ("b200_gemm_bf16_2cta_split" if split else "b200_gemm_bf16_2cta")
     G.gemm(fake(M, 8192), fake(8192, N), side=side, out=fake(M, N + 1)[:, :N])                # through an aligned output
     assert lib.names()[-2] == ("b200_gemm_bf16_2cta_split" if split else "b200_gemm_bf16_2cta")
+
+
+@pytest.mark.parametrize("M,K,name", [(8, 64, "b200_gemm_skinny"), (9, 504, "b200_gemm_bf16"), (9, 512, "b200_gemm_skinny"),
+                                      (64, 511, "b200_gemm_bf16"), (64, 512, "b200_gemm_skinny"), (65, 512, "b200_gemm_bf16")])
+def test_few_rows_over_a_short_inner_dimension(lib, M, K, name):
+    G.gemm(fake(M, 512)[:, :K], fake(K, 768))
+    assert lib.names() == [name]
