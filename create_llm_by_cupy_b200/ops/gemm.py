@@ -94,9 +94,9 @@ def _rowmajor_2d(t: torch.Tensor) -> tuple[torch.Tensor, int]:
 # 9.2 us with the copies, 256 x 256 x 33 3.0 / 11.4, but 2048 x 5460 x 1024 2430 / 50. It stays below both limits.
 PAD_WORK = 1 << 25
 PAD_K = 1024
-# An output with such a pitch goes through an aligned one (and a copy) from this M * N on; below it the epilogue
-# stores element by element (2048 x 2730: 119 us, 24 + 9 with the copy).
-PAD_OUT_AREA = 1 << 16
+# An output of the CTA-pair kernel (256 x 256 and larger) with such a base or pitch goes through an aligned one and a copy:
+# the kernel's epilogue would store it element by element (over K = 1024, 256 x 257: 64 us, 18.5 with the copy; 2048 x 2730:
+# 97 / 35).
 
 
 def repitch(src: torch.Tensor, dst: torch.Tensor, cols: int, width: int, nseg: int = 1, sseg: int = 0, dseg: int = 0):
@@ -242,12 +242,12 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
             return out
         if ok and M >= 256 and N >= 256:
             po = out.data_ptr()
-            if (po % 16 or ldd * (4 if flags & GEMM_OUT_F32 else 2) % 16) and M * N >= PAD_OUT_AREA:
+            if po % 16 or ldd * (4 if flags & GEMM_OUT_F32 else 2) % 16:
                 tmp = torch.empty((M, (N + 7) // 8 * 8), dtype=out_dtype, device=a.device)[:, :N]
                 if add is not None:
                     _copy_rows(add, tmp)
                 gemm(a, b, trans_a=trans_a, trans_b=trans_b, out=tmp, add=None if add is None else tmp, alpha=alpha,
-                     side=side)
+                     impl=impl, side=side)
                 _copy_rows(tmp, out)
                 return out
             dev = a.get_device()

@@ -114,3 +114,9 @@ def test_split_k_beside_other_kernels(lib, monkeypatch, tiles, pending, side, sp
 def test_few_rows_over_a_short_inner_dimension(lib, M, K, name):
     G.gemm(fake(M, 512)[:, :K], fake(K, 768))
     assert lib.names() == [name]
+
+
+def test_an_explicit_implementation_holds_for_an_unaligned_output(lib, monkeypatch):
+    monkeypatch.setattr(G, "GEMM_IMPL", "1cta")
+    G.gemm(fake(256, 64), fake(64, 256), out=fake(256, 257)[:, :256], impl="2cta")
+    assert [n for n in lib.names() if n.startswith("b200_gemm_bf16")] == ["b200_gemm_bf16_2cta"]
