@@ -68,6 +68,30 @@ def test_swiglu_layer_with_odd_width(M, H, I):
     assert layer.forward(x, train_flg=False).shape == (M, H)
 
 
+@pytest.mark.parametrize("why", ["misaligned gradient", "epilogue switched off"])
+@pytest.mark.parametrize("M,H,I", [(256, 128, 257), (1000, 512, 1365)])
+def test_padded_width_backward_without_the_epilogue(M, H, I, why, monkeypatch):
+    """The backward of a padded forward through a gradient of the activation in memory."""
+    layer = SwiGLU(H, 2, device="cuda", ffn_size=I, generator=torch.Generator().manual_seed(0))
+    x, dout = bf(M, H, seed=1), bf(M * H + 1, seed=3)[1:].view(M, H)
+    cpu = SwiGLU(H, 2, dtype=torch.float32, ffn_size=I)
+    cpu.params = [p.float().cpu() for p in layer.params]
+    cpu.forward(x.float().cpu())
+    wdx = cpu.backward(dout.float().cpu())
+    if why == "epilogue switched off":
+        dout = dout.clone()
+    layer.forward(x)
+    assert layer.cache[1].shape == (M, 2 * ((I + 7) // 8 * 8))
+    if why == "epilogue switched off":
+        monkeypatch.setattr(F, "SWIGLU_EPILOGUE", False)
+    monkeypatch.setattr(F, "gemm_swiglu_bwd", None)                 # not called
+    dx = layer.backward(dout)
+    F.wgrad_join(dx.device)
+    for got, ref in zip((dx, *layer.grads), (wdx, *cpu.grads)):
+        # three bf16 tensors lie between the inputs and a gradient: 2^-9 each, four times that for the norm
+        assert got.shape == ref.shape and (got.float().cpu() - ref).norm() <= 12 * 2.0 ** -9 * ref.norm()
+
+
 @pytest.mark.parametrize("pitch", [0, 3])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_gate_value_gradient_into_a_given_matrix(dtype, pitch):
