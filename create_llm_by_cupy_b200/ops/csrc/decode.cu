@@ -289,8 +289,9 @@ static int launch_decode(DecodeParams p, int B, cudaStream_t st) {
   p.groups = (p.QH / p.KVH + RT - 1) / RT;
   const long pairs = long(B) * p.KVH * p.groups;
   const int tiles = (p.Tmax + DA_TILE - 1) / DA_TILE;
-  // 8 CTAs per (sequence, KV head) until there are two per SM without it; fewer where the cache is shorter than
-  // 8 tiles. Up to 16 warps per CTA while at most one CTA per SM exists, else 4 (they share the SM's registers).
+  // Up to 8 CTAs per (sequence, KV head): doubled while there are fewer than four per SM in all (as many fit, at four
+  // warps) and the cache has more tiles than CTAs. Up to 16 warps per CTA while at most one CTA per SM exists, else 4 (they
+  // share the SM's registers).
   int cs = 1;
   while (cs < 8 && cs < tiles && pairs * cs < 4L * num_sms()) cs *= 2;
   int warps = (tiles + cs - 1) / cs;

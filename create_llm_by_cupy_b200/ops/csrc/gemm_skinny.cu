@@ -4,7 +4,7 @@
 // whole GPU can stream it. A 128-row tensor-core tile per 128 columns leaves most SMs without a tile (N = 768:
 // 6 CTAs that walk all of K one after the other). Here
 //   * a CTA owns 64 columns and a slice of K; the CTAs that share a column tile form a cluster along K and add
-//     their fp32 sums through distributed shared memory, so a 768 x 768 weight is 96 CTAs and there is no
+//     their fp32 sums through distributed shared memory, so a 768 x 768 weight is 48 CTAs and there is no
 //     workspace and no second launch;
 //   * 64 x 64 weight tiles (8 KiB) arrive through a ring of cp.async stages, several CTAs per SM, so that tens of
 //     KiB per SM are in flight;

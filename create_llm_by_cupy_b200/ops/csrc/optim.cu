@@ -56,9 +56,10 @@ __device__ __forceinline__ void adam_st(float4* p, float4 v) {
   else *p = v;
 }
 
-// Bound by memory: 26 bytes per parameter with bf16 gradients (28 with fp32), every byte once. Alone on the GPU
-// (kStream false) a CTA updates 1024 parameters and ends: 44.3 M parameters take 184 us (6.3 TB/s), against 198 with
-// streaming accesses and 208 on a grid of 8 CTAs per SM that walks the shard (5.5 TB/s). Beside the next forward
+// Bound by memory: 28 bytes per parameter with bf16 gradients (30 with fp32), every byte once: the gradient and the 12 of
+// the fp32 state read, those 12 and the bf16 parameter written. Alone on the GPU (kStream false) a CTA updates 1024
+// parameters and ends: 44.3 M parameters (1.24 GB) take 184 us (6.7 TB/s), against 198 with streaming accesses (6.3) and
+// 208 on a grid of 8 CTAs per SM that walks the shard (6.0 TB/s). Beside the next forward
 // (kStream, a limited grid) the accesses stream, so that the GEMM operands stay in L2.
 template <typename TG, bool kStream>
 __global__ void __launch_bounds__(256)
