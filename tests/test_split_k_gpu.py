@@ -31,6 +31,20 @@ def test_split_k(M, N, K, trans_a, trans_b):
         assert ((z.double() - want).abs() <= bound + ulp * want.abs()).all()
 
 
+@pytest.mark.parametrize("dt,ulp", [(torch.bfloat16, 2.0 ** -8), (torch.float32, 2.0 ** -23)])
+@pytest.mark.parametrize("M,N,K,cpitch", [(257, 301, 4104, 301), (300, 303, 4104, 304), (256, 256, 4096, 259)])
+def test_split_k_element_by_element(M, N, K, cpitch, dt, ulp):
+    """Columns beyond the last group of four, and an addend whose rows do not start on 16-byte boundaries."""
+    assert G.split_count(M, N, K, 74) > 1
+    a, b = bf(M, K, seed=1), bf(K, (N + 7) // 8 * 8, seed=2)[:, :N]
+    c = bf(M, cpitch, seed=3).to(dt)[:, :N]
+    want = a.double() @ b.double() + c.double()
+    out = torch.full((M, (N + 7) // 8 * 8), 7.0, dtype=dt, device="cuda")
+    G.gemm(a, b, add=c, out=out[:, :N])
+    bound = a.double().abs() @ b.double().abs() * (K * 2.0 ** -23) + ulp * want.abs()
+    assert ((out[:, :N].double() - want).abs() <= bound).all() and (out[:, N:] == 7.0).all()
+
+
 def test_split_rule():
     assert G.split_count(8192, 2048, 2048, 74) == 1          # enough tiles
     assert G.split_count(768, 768, 768, 74) == 1             # K too short to pay for the second kernel
