@@ -26,6 +26,7 @@ namespace cg = cooperative_groups;
 
 constexpr int DA_MAX_WARPS = 16;
 constexpr int DA_TILE = 32;          // keys per warp and step
+constexpr int DA_PREFETCH = 4;       // tiles per warp that are asked for before the kernel's inputs are ready
 
 struct DecodeParams {
   const bf16* q;        // [B, QH, D]
@@ -112,8 +113,19 @@ decode_attn_kernel(const DecodeParams p) {
   const int b = blockIdx.z, kvh = int(blockIdx.y) / p.groups, g = int(blockIdx.y) % p.groups;
   const int R = p.QH / p.KVH;
   const int h0 = kvh * R + g * RT, nh = min(RT, R - g * RT);
-  const int len = min(p.lens[b], p.Tmax);
   const int kl = lane / LPK, dl = lane % LPK;           // key slot and 8-element column of this lane
+  {
+    // the first tiles of this warp travel to L2 while the projection before this kernel runs (a length that is only
+    // being written by then costs a useless or a missing prefetch, nothing else)
+    const int ahead = min(p.lens[b], p.Tmax);
+    if (lane < 2) {
+      const bf16* rows = (lane == 0 ? p.kc : p.vc) + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
+      for (int i = 0, t = rank + warp * cs; i < DA_PREFETCH && t * DA_TILE < ahead; ++i, t += nw * cs)
+        l2_prefetch(rows + size_t(t) * DA_TILE * D, uint32_t(min(DA_TILE, ahead - t * DA_TILE)) * D * 2);
+    }
+  }
+  pdl_wait();
+  const int len = min(p.lens[b], p.Tmax);
 
   __shared__ uint4 s_new[2][LPK];                       // the new token's rotated k and v
   const bf16* new_row = nullptr;
@@ -236,6 +248,7 @@ decode_attn_kernel(const DecodeParams p) {
     __syncwarp();                                       // the next tile overwrites s_p
   }
 
+  pdl_trigger();        // here, not at the top: CTAs that arrive while these fill the SMs land unevenly (see gemm_skinny.cu)
   // over the key slots of the warp, then the warps of the CTA
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
@@ -299,19 +312,8 @@ static int launch_decode(DecodeParams p, int B, cudaStream_t st) {
   if (warps > cap) warps = cap;
   if (warps < 1) warps = 1;
   if (p.KVH * p.groups > 65535 || B > 65535) return static_cast<int>(cudaErrorInvalidValue);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(cs, p.KVH * p.groups, B);
-  cfg.blockDim = dim3(32 * warps);
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = cs;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return static_cast<int>(p.kqv != nullptr ? cudaLaunchKernelEx(&cfg, decode_attn_kernel<D, RT, true>, p)
-                                           : cudaLaunchKernelEx(&cfg, decode_attn_kernel<D, RT, false>, p));
+  const auto kern = p.kqv != nullptr ? decode_attn_kernel<D, RT, true> : decode_attn_kernel<D, RT, false>;
+  return static_cast<int>(launch_pdl(kern, dim3(cs, p.KVH * p.groups, B), dim3(32 * warps), 0, st, cs, p));
 }
 
 template <int D>

@@ -41,8 +41,10 @@ __device__ __forceinline__ float warp_sum(float v) {
 // it fits (H <= 32 * 8 * NV), otherwise it is read a second time (served by L1/L2).
 template <int NV>
 __global__ void __launch_bounds__(128)
-rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma, bf16* __restrict__ y,
+rmsnorm_fwd_kernel(const bf16* x, const bf16* gamma, bf16* __restrict__ y,
                    float* __restrict__ rstd, int M, int H, float eps) {
+  pdl_wait();
+  pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 4 + warp;
   if (row >= M) return;
@@ -99,8 +101,10 @@ rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma, b
 // combined with one block-wide exchange per step.
 template <int NV, int R>
 __global__ void __launch_bounds__(256)
-rmsnorm_fwd_cta_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma, bf16* __restrict__ y,
+rmsnorm_fwd_cta_kernel(const bf16* x, const bf16* gamma, bf16* __restrict__ y,
                        float* __restrict__ rstd, int M, int H, float eps) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float sss[2][R][8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunk = H >> 3;
@@ -187,9 +191,11 @@ __global__ void rmsnorm_fwd_scalar_kernel(const bf16* __restrict__ x, const bf16
 // row of `partial` [gridDim.x, H] (coalesced), reduced by rmsnorm_dgamma_reduce_kernel.
 template <int NV>
 __global__ void __launch_bounds__(256, 2)
-rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ gamma,
-                   const float* __restrict__ rstd, const bf16* __restrict__ add, bf16* __restrict__ dx,
+rmsnorm_bwd_kernel(const bf16* dy, const bf16* x, const bf16* gamma,
+                   const float* rstd, const bf16* add, bf16* __restrict__ dx,
                    float* __restrict__ partial, int M, int H) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ float sred[];   // [warps per block][H]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
@@ -277,9 +283,11 @@ rmsnorm_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, cons
 // registers for the whole kernel, so no cross-warp combine is needed at the end.
 template <int NV, int R>
 __global__ void __launch_bounds__(256, 2)
-rmsnorm_bwd_cta_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, const bf16* __restrict__ gamma,
-                       const float* __restrict__ rstd, const bf16* __restrict__ add, bf16* __restrict__ dx,
+rmsnorm_bwd_cta_kernel(const bf16* dy, const bf16* x, const bf16* gamma,
+                       const float* rstd, const bf16* add, bf16* __restrict__ dx,
                        float* __restrict__ partial, int M, int H) {
+  pdl_wait();
+  pdl_trigger();
   __shared__ float sdot[2][R][8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunk = H >> 3;
@@ -404,8 +412,10 @@ __global__ void rmsnorm_bwd_scalar_kernel(const bf16* __restrict__ dy, const bf1
 }
 
 __global__ void __launch_bounds__(256)
-rmsnorm_dgamma_reduce_kernel(const float* __restrict__ partial, bf16* __restrict__ dgamma, int nrows, int H,
+rmsnorm_dgamma_reduce_kernel(const float* partial, bf16* __restrict__ dgamma, int nrows, int H,
                              int accumulate) {
+  pdl_wait();
+  pdl_trigger();
   // block = 32 columns x 8 row-groups: coalesced 128-byte reads, rows split over the warps
   __shared__ float red[8][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -556,8 +566,10 @@ __device__ __forceinline__ void embedding_bad_id(int* status, int kid) {
   if (status != nullptr && atomicCAS(status, 0, 4) == 0) status[1] = kid;
 }
 
-__global__ void embedding_fwd_kernel(const bf16* __restrict__ W, const int* __restrict__ idx, bf16* __restrict__ out,
+__global__ void embedding_fwd_kernel(const bf16* W, const int* idx, bf16* __restrict__ out,
                                      int M, int H, int pad_id, int V, int* status) {
+  pdl_wait();
+  pdl_trigger();
   const int chunks = H >> 3;
   const size_t total = size_t(M) * chunks;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
@@ -632,8 +644,10 @@ __global__ void add_bf16_kernel(const bf16* __restrict__ a, const bf16* __restri
 // segment set to zero. A thread moves 8 columns; the side that allows it is accessed with 16 bytes, the other one with
 // eight 2-byte accesses that share their L1 lines. Bound by those accesses: 1024 x 5460 (22 MB of traffic) in 9 us.
 __global__ void __launch_bounds__(256)
-repitch_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, int R, int nseg, int C, int W, int sseg,
+repitch_kernel(const uint16_t* src, uint16_t* __restrict__ dst, int R, int nseg, int C, int W, int sseg,
                int dseg, long long ls, long long ld) {
+  pdl_wait();
+  pdl_trigger();
   const int chunks = (W + 7) >> 3;
   const size_t total = size_t(R) * nseg * chunks;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
@@ -681,26 +695,26 @@ B200_API int b200_rmsnorm_fwd(const void* x, const void* gamma, void* y, void* r
   if (H % 8 != 0) {
     rmsnorm_fwd_scalar_kernel<<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
   } else if (H <= 256) {
-    rmsnorm_fwd_kernel<1><<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+    B200_CHECK(launch_pdl(rmsnorm_fwd_kernel<1>, dim3(grid), dim3(block), 0, st, 0, xp, gp, yp, rp, M, H, eps));
   } else if (H <= 1024 && M <= num_sms()) {
     // a row per CTA while there is an SM for each: one chunk per thread instead of a chain of up to four per lane
     // (one row of 768: 3.3 -> 2.5 us)
-    rmsnorm_fwd_cta_kernel<1, 1><<<M, 256, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+    B200_CHECK(launch_pdl((rmsnorm_fwd_cta_kernel<1, 1>), dim3(M), dim3(256), 0, st, 0, xp, gp, yp, rp, M, H, eps));
   } else if (H <= 1024) {
-    rmsnorm_fwd_kernel<4><<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+    B200_CHECK(launch_pdl(rmsnorm_fwd_kernel<4>, dim3(grid), dim3(block), 0, st, 0, xp, gp, yp, rp, M, H, eps));
   } else if (H <= 8192) {
     const int cap = num_sms() * 4;
     if (H <= 2048) {
       const int ctas = min((M + 3) / 4, cap);
-      rmsnorm_fwd_cta_kernel<1, 4><<<ctas, 256, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+      B200_CHECK(launch_pdl((rmsnorm_fwd_cta_kernel<1, 4>), dim3(ctas), dim3(256), 0, st, 0, xp, gp, yp, rp, M, H, eps));
     } else if (H <= 4096) {
       const int ctas = min((M + 1) / 2, cap);
-      rmsnorm_fwd_cta_kernel<2, 2><<<ctas, 256, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+      B200_CHECK(launch_pdl((rmsnorm_fwd_cta_kernel<2, 2>), dim3(ctas), dim3(256), 0, st, 0, xp, gp, yp, rp, M, H, eps));
     } else {
-      rmsnorm_fwd_cta_kernel<4, 1><<<min(M, cap), 256, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+      B200_CHECK(launch_pdl((rmsnorm_fwd_cta_kernel<4, 1>), dim3(min(M, cap)), dim3(256), 0, st, 0, xp, gp, yp, rp, M, H, eps));
     }
   } else {
-    rmsnorm_fwd_kernel<16><<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
+    B200_CHECK(launch_pdl(rmsnorm_fwd_kernel<16>, dim3(grid), dim3(block), 0, st, 0, xp, gp, yp, rp, M, H, eps));
   }
   return static_cast<int>(cudaGetLastError());
 }
@@ -729,19 +743,19 @@ B200_API int b200_rmsnorm_bwd(const void* dy, const void* x, const void* gamma, 
     B200_CHECK(cudaMemsetAsync(pp, 0, size_t(rows) * H * sizeof(float), st));
     rmsnorm_bwd_scalar_kernel<<<rows, 128, 0, st>>>(dyp, xp, gp, rp, ap, dxp, pp, M, H);
   } else if (H <= 256) {
-    rmsnorm_bwd_kernel<1><<<rows, 256, smem, st>>>(dyp, xp, gp, rp, ap, dxp, pp, M, H);
+    B200_CHECK(launch_pdl(rmsnorm_bwd_kernel<1>, dim3(rows), dim3(256), smem, st, 0, dyp, xp, gp, rp, ap, dxp, pp, M, H));
   } else if (H <= 1024) {
-    rmsnorm_bwd_kernel<4><<<rows, 256, smem, st>>>(dyp, xp, gp, rp, ap, dxp, pp, M, H);
+    B200_CHECK(launch_pdl(rmsnorm_bwd_kernel<4>, dim3(rows), dim3(256), smem, st, 0, dyp, xp, gp, rp, ap, dxp, pp, M, H));
   } else if (H <= 2048) {
-    rmsnorm_bwd_cta_kernel<1, 4><<<rows, 256, 0, st>>>(dyp, xp, gp, rp, ap, dxp, pp, M, H);
+    B200_CHECK(launch_pdl((rmsnorm_bwd_cta_kernel<1, 4>), dim3(rows), dim3(256), 0, st, 0, dyp, xp, gp, rp, ap, dxp, pp, M, H));
   } else if (H <= 4096) {
-    rmsnorm_bwd_cta_kernel<2, 2><<<rows, 256, 0, st>>>(dyp, xp, gp, rp, ap, dxp, pp, M, H);
+    B200_CHECK(launch_pdl((rmsnorm_bwd_cta_kernel<2, 2>), dim3(rows), dim3(256), 0, st, 0, dyp, xp, gp, rp, ap, dxp, pp, M, H));
   } else {
-    rmsnorm_bwd_cta_kernel<4, 1><<<rows, 256, 0, st>>>(dyp, xp, gp, rp, ap, dxp, pp, M, H);
+    B200_CHECK(launch_pdl((rmsnorm_bwd_cta_kernel<4, 1>), dim3(rows), dim3(256), 0, st, 0, dyp, xp, gp, rp, ap, dxp, pp, M, H));
   }
   B200_CHECK(cudaGetLastError());
-  rmsnorm_dgamma_reduce_kernel<<<(H + 31) / 32, 256, 0, st>>>(pp, static_cast<bf16*>(dgamma), rows, H,
-                                                                 accumulate_dgamma);
+  B200_CHECK(launch_pdl(rmsnorm_dgamma_reduce_kernel, dim3((H + 31) / 32), dim3(256), 0, st, 0, pp, static_cast<bf16*>(dgamma), rows, H,
+                                                                 accumulate_dgamma));
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -750,8 +764,8 @@ B200_API int b200_repitch(const void* src, void* dst, int R, int nseg, int C, in
                           long long ld, cudaStream_t st) {
   if (R <= 0 || nseg <= 0 || W <= 0) return 0;
   if (C < 0 || C > W) return static_cast<int>(cudaErrorInvalidValue);
-  repitch_kernel<<<grid_for(size_t(R) * nseg * ((W + 7) / 8), 256), 256, 0, st>>>(
-      static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, nseg, C, W, sseg, dseg, ls, ld);
+  B200_CHECK(launch_pdl(repitch_kernel, dim3(grid_for(size_t(R) * nseg * ((W + 7) / 8), 256)), dim3(256), 0, st, 0, 
+      static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), R, nseg, C, W, sseg, dseg, ls, ld));
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -809,9 +823,9 @@ B200_API int b200_embedding_fwd(const void* W, const void* idx, void* out, int M
                                 cudaStream_t st) {
   if (M <= 0) return 0;
   if (H % 8 == 0)
-    embedding_fwd_kernel<<<grid_for(size_t(M) * (H / 8), 256), 256, 0, st>>>(
+    B200_CHECK(launch_pdl(embedding_fwd_kernel, dim3(grid_for(size_t(M) * (H / 8), 256)), dim3(256), 0, st, 0, 
         static_cast<const bf16*>(W), static_cast<const int*>(idx), static_cast<bf16*>(out), M, H, pad_id, V,
-        status_ptr());
+        status_ptr()));
   else
     embedding_fwd_scalar_kernel<<<grid_for(size_t(M) * H, 256), 256, 0, st>>>(
         static_cast<const bf16*>(W), static_cast<const int*>(idx), static_cast<bf16*>(out), M, H, pad_id, V,

@@ -74,9 +74,6 @@ flash_bwd_dq_gemm_kernel(const __grid_constant__ CUtensorMap tmDS, const __grid_
   const int kvh = h / (p.QH / p.KVH);
   const int m0 = mtile * 128;
   const int T = p.T;
-  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 303) : T;
-  // 64-key steps: everything up to the end of the diagonal tile, cut at the valid length
-  const int n_tiles = min(2 * (mtile + 1), (max(vlen, 1) + DQG_KEYS - 1) / DQG_KEYS);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < DQG_STAGES; ++s) {
@@ -94,6 +91,11 @@ flash_bwd_dq_gemm_kernel(const __grid_constant__ CUtensorMap tmDS, const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                            // by every role: their bounded waits start counting behind it
+  pdl_trigger();
+  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 303) : T;
+  // 64-key steps: everything up to the end of the diagonal tile, cut at the valid length
+  const int n_tiles = min(2 * (mtile + 1), (max(vlen, 1) + DQG_KEYS - 1) / DQG_KEYS);
 
   if (warp == 0) {
     if (lane == 0) {
@@ -199,11 +201,8 @@ int flash_bwd_dq_from_ds(const void* ds, const void* k, void* dq, const void* va
                                     DqGemmSmem::kTotal));
     configured = true;
   }
-  if (D == 128)
-    flash_bwd_dq_gemm_kernel<128><<<nt * QH * B, DQG_THREADS, DqGemmSmem::kTotal, st>>>(*tds, *tk, p);
-  else
-    flash_bwd_dq_gemm_kernel<64><<<nt * QH * B, DQG_THREADS, DqGemmSmem::kTotal, st>>>(*tds, *tk, p);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_pdl(D == 128 ? flash_bwd_dq_gemm_kernel<128> : flash_bwd_dq_gemm_kernel<64>,
+                                     dim3(nt * QH * B), dim3(DQG_THREADS), DqGemmSmem::kTotal, st, 0, *tds, *tk, p));
 }
 
 }  // namespace b200

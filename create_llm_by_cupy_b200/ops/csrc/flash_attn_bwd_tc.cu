@@ -174,8 +174,6 @@ flash_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int kvh = h / (p.QH / p.KVH);
   const int m0 = mtile * 128;
   const int T = p.T;
-  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
-  const int n_tiles = min(mtile + 1, (max(vlen, 1) + 127) / 128);
 
   if (threadIdx.x == 0) {
     mbar_init(qdo_full, 1);
@@ -191,6 +189,10 @@ flash_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                            // by every role: their bounded waits start counting behind it
+  pdl_trigger();
+  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
+  const int n_tiles = min(mtile + 1, (max(vlen, 1) + 127) / 128);
   // Every 128-key tile is processed as two 64-key sub-tiles so that S and dP (64 columns each) can
   // be double-buffered, and each buffer has its own math warpgroup: warpgroup w turns the scores of
   // sub-tiles u = w, w + 2, ... into dS while the other warpgroup and the tensor core are on u + 1.
@@ -414,7 +416,6 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   }
   const int T = p.T;
   const int R = p.QH / p.KVH;
-  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
   const int tile_of_pass[2] = {pair, p.pairing ? p.n_tiles - 1 - pair : pair};
   const int n_pass = tile_of_pass[0] == tile_of_pass[1] ? 1 : 2;
 
@@ -435,6 +436,9 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                            // by every role: their bounded waits start counting behind it
+  pdl_trigger();
+  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
   // S^T and dP^T are double-buffered (64 columns each per buffer) and each buffer has its own math
   // warpgroup: warpgroup w handles iterations g = w, w + 2, ... (g counts on across the two passes)
   // while the other warpgroup and the tensor core are on g + 1. A thread owns one key row (one TMEM
@@ -834,7 +838,6 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
   }
   const int T = p.T;
   const int R = p.QH / p.KVH;
-  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
   const int tile_of_pass[2] = {pair, p.pairing ? p.n_tiles - 1 - pair : pair};
   const int n_pass = tile_of_pass[0] == tile_of_pass[1] ? 1 : 2;
 
@@ -858,6 +861,9 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                            // by every role: their bounded waits start counting behind it
+  pdl_trigger();
+  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
   constexpr uint32_t kColST = 0, kColDPT = 128, kColDV = 256, kColDK = 384;
 
   if (warp == 0) {
@@ -1282,12 +1288,11 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   p.pairing = g_dkv_pairing >= 0 ? g_dkv_pairing : ((n_key_tiles > num_sms() && n_key_tiles < 3 * num_sms()) ? 1 : 0);
   const int dkv_ctas = (p.pairing ? (nt + 1) / 2 : nt) * KVH * B;
   if (D == 128 && g_dkv_wide && dkv_wide_fits())
-    flash_bwd_dkv_wide_kernel<<<dkv_ctas, FBT_THREADS, FdkwSmem::kTotal, st>>>(*tq128, *tdo128, *tk, *tv, *tds, p);
-  else if (D == 128)
-    flash_bwd_dkv_tc_kernel<128><<<dkv_ctas, FBT_THREADS, FdkvSmem::kTotal, st>>>(*tq64, *tdo64, *tk, *tv, *tds, p);
+    B200_CHECK(launch_pdl(flash_bwd_dkv_wide_kernel, dim3(dkv_ctas), dim3(FBT_THREADS), FdkwSmem::kTotal, st, 0, *tq128, *tdo128,
+                          *tk, *tv, *tds, p));
   else
-    flash_bwd_dkv_tc_kernel<64><<<dkv_ctas, FBT_THREADS, FdkvSmem::kTotal, st>>>(*tq64, *tdo64, *tk, *tv, *tds, p);
-  B200_CHECK(cudaGetLastError());
+    B200_CHECK(launch_pdl(D == 128 ? flash_bwd_dkv_tc_kernel<128> : flash_bwd_dkv_tc_kernel<64>, dim3(dkv_ctas),
+                          dim3(FBT_THREADS), FdkvSmem::kTotal, st, 0, *tq64, *tdo64, *tk, *tv, *tds, p));
   if (ds_ws != nullptr) return flash_bwd_dq_from_ds(ds_ws, k, dq, valid_len, s + 3, s + 12, B, T, QH, KVH, D, p.bchunk,
                                                       p.unrot_cos, p.unrot_sin, p.unrot_ld, st);
   if (dkv_ctas >= 3 * num_sms()) {

@@ -139,15 +139,6 @@ flash_fwd_tc3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int h = blockIdx.y, b = blockIdx.z;
   const int kvh = h / (p.QH / p.KVH);
   const int T = p.T;
-  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 301) : T;
-  const int kv_tiles = (max(vlen, 1) + 127) / 128;
-  int nt[2];
-#pragma unroll
-  for (int w = 0; w < 2; ++w) {
-    const int mt = 2 * pt + w;
-    nt[w] = (mt * 128 < T) ? min(mt + 1, kv_tiles) : 0;
-  }
-  const int nmax = max(nt[0], nt[1]);
   constexpr uint32_t kTileBytes = 128 * kD * 2;          // live bytes of a Q / K / V tile (its slot stays 32 KiB)
 
   if (threadIdx.x == 0) {
@@ -175,6 +166,17 @@ flash_fwd_tc3_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   constexpr uint32_t kColS = 0, kColO = 256;
+  pdl_wait();                            // by every role: their bounded waits start counting behind it
+  pdl_trigger();
+  const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 301) : T;
+  const int kv_tiles = (max(vlen, 1) + 127) / 128;
+  int nt[2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    const int mt = 2 * pt + w;
+    nt[w] = (mt * 128 < T) ? min(mt + 1, kv_tiles) : 0;
+  }
+  const int nmax = max(nt[0], nt[1]);
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
@@ -409,8 +411,6 @@ B200_API int b200_flash_fwd_tc3(const void* q, const void* k, const void* v, voi
   }
   dim3 grid((T + 255) / 256, QH, B);
   if (D == 128)
-    flash_fwd_tc3_kernel<128><<<grid, F3_THREADS, F3Smem::kTotal, st>>>(*tq, *tk, *tv, *to, p);
-  else
-    flash_fwd_tc3_kernel<64><<<grid, F3_THREADS, F3Smem::kTotal, st>>>(*tq, *tk, *tv, *to, p);
-  return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(launch_pdl(flash_fwd_tc3_kernel<128>, grid, dim3(F3_THREADS), F3Smem::kTotal, st, 0, *tq, *tk, *tv, *to, p));
+  return static_cast<int>(launch_pdl(flash_fwd_tc3_kernel<64>, grid, dim3(F3_THREADS), F3Smem::kTotal, st, 0, *tq, *tk, *tv, *to, p));
 }

@@ -117,6 +117,11 @@ gemm_skinny_kernel(const SkinnyParams p) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[t][e] = 0.f;
 
+  pdl_wait();
+  // Short slices: the next kernel's CTAs settle while this one's loads are in flight. Long ones fill the GPU with several
+  // CTAs per SM; CTAs that arrive among them land unevenly and run so (a 7B block 121.5 -> 116 us with the trigger here,
+  // 113 with it behind the loop), so the next kernel is let in at the end.
+  if (steps <= 2 * S::kStages) pdl_trigger();
 #pragma unroll
   for (int s = 0; s < S::kStages - 1; ++s) {
     if (s < steps) skinny_load<MT, K_ROWS, GLU>(p, base + s * S::kStageBytes, n0, k_begin + s * SK_TK, k_end);
@@ -149,6 +154,7 @@ gemm_skinny_kernel(const SkinnyParams p) {
       mma16816(acc[t], w[3], x1[2], x1[3]);
     }
   }
+  if (steps > 2 * S::kStages) pdl_trigger();
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 
@@ -195,19 +201,7 @@ static int launch_skinny(SkinnyParams p, cudaStream_t st) {
   int ks = 1;
   while (ks < 8 && long(tiles) * ks * 2 <= long(S::kPerSm) * num_sms() && ksteps >= 4 * ks) ks *= 2;
   p.kslice = (ksteps + ks - 1) / ks * SK_TK;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(ks, tiles);
-  cfg.blockDim = dim3(SK_THREADS);
-  cfg.dynamicSmemBytes = S::kTotal;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = ks;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, p));
+  return static_cast<int>(launch_pdl(kern, dim3(ks, tiles), dim3(SK_THREADS), S::kTotal, st, ks, p));
 }
 
 template <bool K_ROWS, bool GLU>

@@ -293,6 +293,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
+  if (!AG) { pdl_wait(); pdl_trigger(); }      // by every role: their bounded waits start counting behind it
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -522,8 +523,12 @@ static int launch_tc(const CUtensorMap* tA, const CUtensorMap* tB, const GemmPar
   } else if (num_tiles < grid) {
     grid = num_tiles;
   }
-  kern<<<grid, GEMM_THREADS, S::kTotal, stream>>>(*tA, *tB, p);
-  return static_cast<int>(cudaGetLastError());
+  if constexpr (AG) {                 // waits for its peers
+    kern<<<grid, GEMM_THREADS, S::kTotal, stream>>>(*tA, *tB, p);
+    return static_cast<int>(cudaGetLastError());
+  } else {
+    return static_cast<int>(launch_pdl(kern, dim3(grid), dim3(GEMM_THREADS), S::kTotal, stream, 0, *tA, *tB, p));
+  }
 }
 
 }  // namespace b200

@@ -308,6 +308,8 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   cluster_sync_all();                                  // both CTAs' barriers exist before anyone signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                     // by every role: their bounded waits start counting behind it
+  pdl_trigger();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -979,14 +981,16 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     q.sched = next_sched_slot();
     if (q.sched == nullptr) return static_cast<int>(cudaErrorInvalidValue);
   }
-  kern<<<2 * pairs, G2_THREADS, G2_SMEM, stream>>>(*tA, *tB, *tBh, *tD, *tC, tE ? *tE : *tA, q);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_pdl(kern, dim3(2 * pairs), dim3(G2_THREADS), G2_SMEM, stream, 0, *tA, *tB, *tBh, *tD, *tC,
+                                     tE ? *tE : *tA, q));
 }
 
 // out = sum over the splits of ws[split][row][col] (+ C), fixed order. 16-byte accesses where every row allows them.
 __global__ void __launch_bounds__(256)
-splitk_sum_kernel(const float* __restrict__ ws, void* D, const void* C, int M, int N, int splits, int ldws, size_t plane,
+splitk_sum_kernel(const float* ws, void* D, const void* C, int M, int N, int splits, int ldws, size_t plane,
                   int ldd, int ldc, int out_f32, int vec) {
+  pdl_wait();
+  pdl_trigger();
   const int per_row = (N + 3) >> 2;
   const size_t total = size_t(M) * per_row;
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
@@ -1163,10 +1167,9 @@ B200_API int b200_gemm_bf16_2cta_split(const void* A, const void* B, void* D, co
                   (C == nullptr || (ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & mask) == 0));
   const size_t chunks = size_t(M) * ((N + 3) / 4);
   const size_t blocks = (chunks + 255) / 256, cap = size_t(num_sms()) * 8;
-  splitk_sum_kernel<<<int(blocks < cap ? blocks : cap), 256, 0, stream>>>(
-      static_cast<const float*>(ws), D, (flags & G2_ADD_C) ? C : nullptr, M, N, splits, ldws, size_t(rows) * ldws, ldd, ldc,
-      f32, vec);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(launch_pdl(splitk_sum_kernel, dim3(int(blocks < cap ? blocks : cap)), dim3(256), 0, stream, 0,
+                                     static_cast<const float*>(ws), D, (flags & G2_ADD_C) ? C : nullptr, M, N, splits, ldws,
+                                     size_t(rows) * ldws, ldd, ldc, f32, vec));
 }
 
 // act[M, I] = silu(A W_gate) * (A W_value) for B = [W_gate | W_value] ([K, 2 I] row-major), A [M, K] row-major,
