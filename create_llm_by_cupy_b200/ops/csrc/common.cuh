@@ -75,10 +75,10 @@ int num_sms();
 //     kernel may have written - weights included: the one before may be the optimizer - is read, and nothing is written,
 //     before it; only an L2 prefetch, which cannot go stale, may come earlier. Inputs are plain pointers, not
 //     `const __restrict__`: a load the compiler takes for invariant could be moved above the wait.
-//   * pdl_trigger() lets the next kernel start once all CTAs of this one have got there. It stands behind pdl_wait(), so
-//     that one kernel at most is waiting while another runs: with the trigger first, two or three kernels' CTAs piled up on
-//     the SMs that happened to be free (777 tokens through the 125M model: 1152 us without all this, 1049 with the trigger
-//     first, 979 like this; one token 520 / 386 / 372).
+//   * pdl_trigger() lets the next kernel start once all CTAs of this one have got there (or have ended; a kernel need not
+//     call it). It never stands before pdl_wait(), so that one kernel at most is waiting while another runs: with the
+//     trigger first, two or three kernels' CTAs piled up on the SMs that happened to be free (777 tokens through the 125M
+//     model: 1152 us without all this, 1049 with the trigger first, 979 like this; one token 520 / 386 / 372).
 // A kernel that waits for another GPU neither triggers nor is launched this way.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -190,7 +190,6 @@ flash_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();                            // by every role: their bounded waits start counting behind it
-  pdl_trigger();
   const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
   const int n_tiles = min(mtile + 1, (max(vlen, 1) + 127) / 128);
   // Every 128-key tile is processed as two 64-key sub-tiles so that S and dP (64 columns each) can
@@ -437,7 +436,6 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();                            // by every role: their bounded waits start counting behind it
-  pdl_trigger();
   const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
   // S^T and dP^T are double-buffered (64 columns each per buffer) and each buffer has its own math
   // warpgroup: warpgroup w handles iterations g = w, w + 2, ... (g counts on across the two passes)
@@ -862,7 +860,6 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();                            // by every role: their bounded waits start counting behind it
-  pdl_trigger();
   const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
   constexpr uint32_t kColST = 0, kColDPT = 128, kColDV = 256, kColDK = 384;
 
