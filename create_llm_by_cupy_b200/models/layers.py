@@ -115,12 +115,7 @@ class GroupedQueryAttention:
 
     # -- helpers ---------------------------------------------------------------------------
     def _split(self, kqv: torch.Tensor, B: int, T: int):
-        kqv = kqv.view(B, T, -1)
-        sb, st, sc = kqv.stride()
-        o, strides = kqv.storage_offset(), (sb, st, self.D * sc, sc)
-        return (kqv.as_strided((B, T, self.QH, self.D), strides, o + self.KV * sc),
-                kqv.as_strided((B, T, self.KVH, self.D), strides, o),
-                kqv.as_strided((B, T, self.KVH, self.D), strides, o + (self.KV + self.H) * sc))
+        return F.split_heads(kqv, B, T, self.QH, self.KVH, self.D)
 
     def _rope(self, T, device):
         return F.rope_table(max(T, self.T), self.D, self.rope_base, device)

@@ -2,7 +2,9 @@
 
 The library exposes a plain ``extern "C"`` surface that is loaded with ctypes, so it needs
 neither the torch headers nor a Python ABI: a full rebuild is a few nvcc invocations run in
-parallel. nvcc cross-compiles, so the build also runs on a machine without a GPU.
+parallel. nvcc cross-compiles, so the build also runs on a machine without a GPU. Beside it stands ``_b200host.so``, a
+small CPython extension (``chost/host_ops.cpp``, against torch's headers) that issues the operators of short passes; it
+takes the kernels from whichever variant of the library is loaded.
 
     python -m create_llm_by_cupy_b200.ops.build [--force] [--verbose]
 """
@@ -35,6 +37,9 @@ FAST_MATH_PREFIXES = ("flash_", "gemm_")
 BOUNDS_CHECK = os.environ.get("B200_BOUNDS_CHECK") == "1"
 LIB_NAME = "libb200llm_dbg.so" if BOUNDS_CHECK else "libb200llm.so"
 OBJ_DIR_NAME = "build_dbg" if BOUNDS_CHECK else "build"
+HOST_SRC = OUT_DIR / "chost" / "host_ops.cpp"
+HOST_LIB = OUT_DIR / "_b200host.so"
+HOST_STAMP = OUT_DIR / "build" / "host_ops.sha1"
 
 
 def flags_for(src: Path) -> list[str]:
@@ -66,6 +71,24 @@ def _digest(src: Path) -> str:
     return h.hexdigest()
 
 
+def _host_command() -> list[str]:
+    """The compiler call for the extension; it depends on torch's location and ABI and on the Python headers."""
+    import sysconfig
+
+    import torch
+    inc = Path(torch.__file__).parent / "include"
+    cuda = Path(_nvcc()).resolve().parent.parent / "include"
+    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", sysconfig.get_paths()["include"],
+            "-I", str(cuda), "-isystem", str(inc), "-isystem", str(inc / "torch" / "csrc" / "api" / "include"), str(HOST_SRC),
+            "-L", str(inc.parent / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+
+
+def _host_digest() -> str:
+    import torch
+    return hashlib.sha1(HOST_SRC.read_bytes() + f"{torch.__version__} {sys.version_info[:2]}".encode()).hexdigest()
+
+
 def lib_path() -> Path:
     return OUT_DIR / LIB_NAME
 
@@ -75,12 +98,17 @@ def source_digest() -> str:
     h = hashlib.sha1()
     for src in sources():
         h.update(_digest(src).encode())
+    h.update(HOST_SRC.read_bytes())
     return h.hexdigest()
 
 
+def _host_current() -> bool:
+    return HOST_LIB.exists() and HOST_STAMP.exists() and HOST_STAMP.read_text() == _host_digest()
+
+
 def is_current() -> bool:
-    """True when the library exists and every object's stamp matches its source as it is now."""
-    if not lib_path().exists():
+    """True when the libraries exist and every object's stamp matches its source as it is now."""
+    if not lib_path().exists() or not _host_current():
         return False
     obj_dir = OUT_DIR / OBJ_DIR_NAME
     for src in sources():
@@ -96,8 +124,18 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     everything up to date."""
     nvcc = _nvcc()
     obj_dir = OUT_DIR / OBJ_DIR_NAME
-    obj_dir.mkdir(exist_ok=True)
     import fcntl
+    for d in {obj_dir, HOST_STAMP.parent}:
+        d.mkdir(exist_ok=True)
+    with open(HOST_STAMP.parent / ".host.lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if force or not _host_current():
+            tmp = HOST_LIB.with_suffix(".so.tmp")
+            r = subprocess.run(_host_command() + ["-o", str(tmp)], capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError(f"g++ failed for {HOST_SRC.name}:\n{r.stdout}\n{r.stderr}")
+            os.replace(tmp, HOST_LIB)
+            HOST_STAMP.write_text(_host_digest())
     with open(obj_dir / ".lock", "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:

@@ -125,6 +125,11 @@ def _bf16(*ts):
 def rmsnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6, keep_rstd: bool = True):
     """y = x * rsqrt(mean(x^2) + eps) * gamma over the last dim. Returns (y, rstd[M] fp32; None on CUDA when not
     ``keep_rstd``, which only the backward needs)."""
+    if native.host is not None:
+        r = native.host.rmsnorm_fwd(x, gamma, eps, keep_rstd)
+        if r is not None:
+            native.bump()
+            return r
     H = x.shape[-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, H)
     M = x2.shape[0]
@@ -151,6 +156,11 @@ def _norm_partial_rows(M: int, device: int) -> int:
 def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma: torch.Tensor, rstd: torch.Tensor,
                 add: torch.Tensor | None = None):
     """Returns (dx (+ add), dgamma). ``x`` is the layer INPUT; ``add`` is the residual gradient."""
+    if native.host is not None:
+        r = native.host.rmsnorm_bwd(dy, x, gamma, rstd, add)
+        if r is not None:
+            native.bump(2)
+            return r
     H = x.shape[-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, H)
     dy2 = dy if dy.dim() == 2 and dy.shape[1] == H else dy.reshape(-1, H)
@@ -222,8 +232,9 @@ _rope_cache: dict = {}
 
 def rope_table(T: int, D: int, base: float, device) -> tuple[torch.Tensor, torch.Tensor]:
     """cos/sin [T, D/2] fp32 with freq_j = base^(-2j/D)."""
-    device = torch.device(device)
-    key = (T, D, float(base), device.type, device.index)
+    if not isinstance(device, torch.device):
+        device = torch.device(device)
+    key = (T, D, float(base), device)
     hit = _rope_cache.get(key)
     if hit is not None:
         return hit
@@ -272,6 +283,11 @@ def rope_inplace(buf: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, T: int
 def embedding_fwd(W: torch.Tensor, idx: torch.Tensor, pad_id: int) -> torch.Tensor:
     """out[m] = W[idx[m]], zeros where idx == pad_id. idx is int32 [M]. On CUDA an id >= W.shape[0] reads
     nothing (zeros) and sets native status error 4 (kernel id 401; 402 in the backward)."""
+    if native.host is not None:
+        out = native.host.embedding_fwd(W, idx, pad_id)
+        if out is not None:
+            native.bump()
+            return out
     M = idx.numel()
     H = W.shape[1]
     if not W.is_cuda:
@@ -396,6 +412,20 @@ def dropout_bwd(dout: torch.Tensor, mask: torch.Tensor, p: float) -> torch.Tenso
 
 
 # --------------------------------------------------------------------------- flash attention
+def split_heads(kqv: torch.Tensor, B: int, T: int, QH: int, KVH: int, D: int):
+    """(q, k, v) views [B, T, heads, D] of a packed projection [B * T, (KVH + QH + KVH) * D] = [K | Q | V]."""
+    if native.host is not None:
+        r = native.host.split_heads(kqv, B, T, QH, KVH, D)
+        if r is not None:
+            return r
+    kqv = kqv.view(B, T, -1)
+    sb, st, sc = kqv.stride()
+    o, strides = kqv.storage_offset(), (sb, st, D * sc, sc)
+    return (kqv.as_strided((B, T, QH, D), strides, o + KVH * D * sc),
+            kqv.as_strided((B, T, KVH, D), strides, o),
+            kqv.as_strided((B, T, KVH, D), strides, o + (KVH + QH) * D * sc))
+
+
 def _strides3(t: torch.Tensor) -> list[int]:
     """(batch, token, head) element strides of a [B, T, heads, D] view."""
     s = t.stride()
@@ -486,6 +516,11 @@ def flash_attn_fwd(q, k, v, *, valid_len=None, scale=None, rope=None):
     if scale is None:
         scale = 1.0 / math.sqrt(D)
     cos, sin = rope if rope is not None else (None, None)
+    if native.host is not None and cos is None and flash_tc_forward_dim(D):
+        r = native.host.flash_fwd(q, k, v, valid_len, scale)
+        if r is not None:
+            native.bump()
+            return r
     if not q.is_cuda:
         o, lse, _, _, _ = _attn_reference(q, k, v, valid_len, scale, cos, sin)
         return o.to(q.dtype).contiguous(), lse
@@ -709,13 +744,20 @@ def decode_attn_append(kqv, kcache, vcache, lens, pos: int, QH: int, KVH: int, c
     return out
 
 
+def _few_rows_rule(x, *weights) -> bool:
+    """The few-rows kernels take ``x`` [M, K] with each of ``weights`` by their sizes."""
+    from . import gemm as _g
+    M = x.shape[0]
+    return _g.GEMM_IMPL == "2cta" and M > 0 and all(_g._skinny(M, w.shape[1]) for w in weights)
+
+
 def _few_rows_ok(x, weights, residual, out_cols: int) -> bool:
     """Shapes and layouts of the one-call forms below: few bf16 rows ``x``, contiguous weights, a residual like the output."""
     from . import gemm as _g
     M = x.shape[0]
-    if not (x.is_cuda and _g.GEMM_IMPL == "2cta" and M > 0 and _g._tma_ok(x, *weights)):
+    if not (x.is_cuda and _g._tma_ok(x, *weights) and _few_rows_rule(x, *weights)):
         return False
-    if not all(w.is_contiguous() and _g._skinny(M, w.shape[1]) for w in weights):
+    if not all(w.is_contiguous() for w in weights):
         return False
     return residual is None or (residual.dtype == torch.bfloat16 and residual.shape == (M, out_cols)
                                 and residual.stride(1) == 1)
@@ -726,6 +768,11 @@ def decode_attn_block(x, w_kqv, w_o, kcache, vcache, lens, pos: int, QH: int, KV
     """K|Q|V projection, rotation, cache append, attention and output projection (+ residual) of one token per sequence
     from one native call (the same three kernels as ``gemm``, ``decode_attn_append``, ``gemm``). Returns [B, H], or None
     where one of those forms does not apply."""
+    if native.host is not None and _few_rows_rule(x, w_kqv, w_o):
+        out = native.host.decode_attn_block(x, w_kqv, w_o, kcache, vcache, lens, pos, QH, KVH, cos, sin, scale, residual)
+        if out is not None:
+            native.bump(3)
+            return out
     if not (x.is_cuda and kcache.dim() == 4 and _few_rows_ok(x, (w_kqv, w_o), residual, w_o.shape[1])):
         return None
     B, H = x.shape
@@ -752,6 +799,11 @@ def decode_attn_block(x, w_kqv, w_o, kcache, vcache, lens, pos: int, QH: int, KV
 def mlp_few_rows(x, w_gate_val, w_out, residual=None):
     """SwiGLU MLP of few rows from one native call (``gemm_skinny_swiglu`` and ``gemm``), or None where those forms do not
     apply."""
+    if native.host is not None and _few_rows_rule(x, w_gate_val, w_out):
+        out = native.host.mlp_few_rows(x, w_gate_val, w_out, residual)
+        if out is not None:
+            native.bump(2)
+            return out
     if not _few_rows_ok(x, (w_gate_val, w_out), residual, w_out.shape[1]):
         return None
     M, H = x.shape

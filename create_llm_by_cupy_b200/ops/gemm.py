@@ -40,6 +40,7 @@ def _skinny(M: int, N: int) -> bool:
 
 
 GEMM_WHOLE_TILES = 8      # CTA-pair kernel: do not split the tiles of a part-filled last round
+_ROUTE_TILES, _ROUTE_SKINNY, _ROUTE_SMALL = range(3)      # kernels of ``native.host.gemm``
 
 # Code-path switches (module attributes; tests and the benchmark's baseline arm set them).
 # "1cta": single-CTA 128x256 tiles; "2cta": CTA pairs (cta_group::2) on 256x256 tiles where the
@@ -195,6 +196,24 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         raise ValueError(f"gemm: inner dims differ ({K} vs {Kb})")
     if out_dtype is None:
         out_dtype = out.dtype if out is not None else (add.dtype if add is not None else a.dtype)
+    if (native.host is not None and (impl or GEMM_IMPL) == "2cta" and bn == 0 and max_ctas == 0 and not force_fallback
+            and out_dtype in (torch.bfloat16, torch.float32)):
+        splits, whole = 1, 0
+        if M <= SKINNY_ROWS and not trans_a and (M <= 8 or K >= SKINNY_K) and _skinny(M, N):
+            route = _ROUTE_SKINNY
+        elif M >= 256 and N >= 256:
+            route = _ROUTE_TILES
+            dev = torch._C._cuda_getDevice()
+            splits = _splits(M, N, K, dev, side)
+            if splits == 1:
+                _apply_dynamic()
+                whole = GEMM_WHOLE_TILES if _wgrad_pending.get(dev, False) else 0
+        else:
+            route = _ROUTE_SMALL
+        res = native.host.gemm(a, b, trans_a, trans_b, out, add, out_dtype is torch.float32, alpha, whole, route, splits)
+        if res is not None:
+            native.bump(2 if splits > 1 else 1)
+            return res
 
     if not a.is_cuda:
         af = a.float().t() if trans_a else a.float()
@@ -306,10 +325,7 @@ def gemm_rope_fusable(a: torch.Tensor, b: torch.Tensor, head_dim: int, rope_cols
     if not (GEMM_ROPE_EPILOGUE and a.is_cuda and GEMM_IMPL == "2cta" and head_dim in (64, 128)):
         return False
     M, N = a.shape[0], b.shape[1]
-    return bool(a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and M >= 256 and N >= 256 and N % 8 == 0
-                and rope_cols % head_dim == 0 and 0 < rope_cols <= N
-                and a.stride(1) == 1 and b.stride(1) == 1 and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0
-                and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0)
+    return bool(M >= 256 and N >= 256 and N % 8 == 0 and rope_cols % head_dim == 0 and 0 < rope_cols <= N and _tma_ok(a, b))
 
 
 def gemm_rope(a: torch.Tensor, b: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, T: int, head_dim: int,
@@ -323,13 +339,18 @@ def gemm_rope(a: torch.Tensor, b: torch.Tensor, cos: torch.Tensor, sin: torch.Te
     assert gemm_rope_fusable(a, b, head_dim, rope_cols)
     assert cos.dtype == torch.float32 and sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
     assert cos.shape[0] >= T and cos.shape[1] == head_dim // 2
-    out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     native.status_tensor()
     _apply_dynamic()
     flags = GEMM_WHOLE_TILES if _wgrad_pending.get(a.device.index, False) else 0
     # the epilogue reads the tables transposed ([head_dim / 2][positions]): a thread owns a row, so a warp
     # then reads consecutive words
     tt = rope_tables_transposed(cos, sin)
+    if native.host is not None:
+        out = native.host.gemm_rope(a, b, tt[0], tt[1], T, head_dim, rope_cols, flags)
+        if out is not None:
+            native.bump()
+            return out
+    out = torch.empty((M, N), dtype=torch.bfloat16, device=a.device)
     rc = native.lib().b200_gemm_bf16_2cta_rope(
         native.ptr(a), native.ptr(b), native.ptr(out), M, N, K, a.stride(0), b.stride(0), N, 0, 1, flags,
         native.ptr(tt[0]), native.ptr(tt[1]), T, tt[0].shape[1], rope_cols, head_dim, native.stream_ptr())
@@ -339,6 +360,10 @@ def gemm_rope(a: torch.Tensor, b: torch.Tensor, cos: torch.Tensor, sin: torch.Te
 
 
 def _tma_ok(*ts) -> bool:
+    if native.host is not None:
+        ok = native.host.tma_ok(*ts)
+        if ok is not None:
+            return ok
     return all(t.is_cuda and t.dtype == torch.bfloat16 and t.dim() == 2 and t.stride(1) == 1 and t.stride(0) % 8 == 0
                and t.data_ptr() % 16 == 0 for t in ts)
 
@@ -370,10 +395,15 @@ def gemm_swiglu(x: torch.Tensor, w_gate_val: torch.Tensor, keep_gv: bool = True)
     I = w_gate_val.shape[1] // 2
     _same_inner("gemm_swiglu", K, w_gate_val.shape[0])
     assert gemm_swiglu_fusable(x, w_gate_val)
-    act = torch.empty((M, I), dtype=torch.bfloat16, device=x.device)
-    gv = torch.empty((M, 2 * I), dtype=torch.bfloat16, device=x.device) if keep_gv else None
     native.status_tensor()
     _apply_dynamic()
+    if native.host is not None:
+        r = native.host.gemm_swiglu(x, w_gate_val, keep_gv, _whole_tiles_flag(x.device))
+        if r is not None:
+            native.bump()
+            return r
+    act = torch.empty((M, I), dtype=torch.bfloat16, device=x.device)
+    gv = torch.empty((M, 2 * I), dtype=torch.bfloat16, device=x.device) if keep_gv else None
     rc = native.lib().b200_gemm_bf16_2cta_swiglu(
         native.ptr(x), native.ptr(w_gate_val), native.ptr(gv), native.ptr(act), M, I, K, x.stride(0),
         w_gate_val.stride(0), 2 * I, I, _whole_tiles_flag(x.device), native.stream_ptr())

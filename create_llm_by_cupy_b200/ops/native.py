@@ -19,6 +19,9 @@ from . import build as _build
 _lock = threading.Lock()
 _lib = None
 _status = {}
+# ``_b200host`` (chost/host_ops.cpp) once a device's status block is registered, so never on a machine without a GPU. Its
+# functions take plain CUDA tensors and return None for anything else; the front ends then go on as without it.
+host = None
 
 c_void_p = ctypes.c_void_p
 c_int = ctypes.c_int
@@ -76,6 +79,18 @@ def lib() -> ctypes.CDLL:
         return _lib
 
 
+def _load_host():
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("_b200host", _build.HOST_LIB)
+    try:
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+    except ImportError as e:
+        raise NativeError(f"cannot load {_build.HOST_LIB}: {e}") from e
+    mod.bind(lib()._handle)
+    return mod
+
+
 def source_digest() -> str:
     """Digest of the sources the loaded library was built from (recorded by the benchmark)."""
     return _build.source_digest()
@@ -90,6 +105,7 @@ def _current_index() -> int:
 
 def status_tensor(device=None) -> torch.Tensor:
     """Per-device 4-int status block that kernels write when a bounded wait runs out."""
+    global host
     if device is None:
         t = _status.get(_current_index())
         if t is not None:
@@ -102,6 +118,9 @@ def status_tensor(device=None) -> torch.Tensor:
         t = torch.zeros(4, dtype=torch.int32, device=dev)
         _status[key] = t
         check(lib().b200_set_status_ptr(c_void_p(t.data_ptr())), "b200_set_status_ptr")
+        mod = host or _load_host()
+        mod.device_ready(key)
+        host = mod
     return _status[key]
 
 
