@@ -13,7 +13,7 @@
 //                 with the leader's barrier address). No cluster multicast is used by any load.
 //   empty[s]      one per CTA; the leader's tcgen05.commit arrives on both (multicast commit).
 //   tmem_full[a]  one per CTA; multicast commit after the last k-block of a tile.
-//   tmem_empty[a] leader only, 8 arrivals: the 4 epilogue warps of each CTA (the follower's
+//   tmem_empty[a] leader only: the 4 or 8 epilogue warps of each CTA arrive (the follower's
 //                 arrive remotely through the cluster shared-memory window).
 //   sched_full[i] one per CTA; sched_empty[i] leader only (see "Tile scheduler").
 // Waits are bounded exactly as in the single-CTA kernel.
@@ -22,8 +22,8 @@
 // out dynamically: the leader's producer thread takes the next tile index from a global counter
 // (one tile ahead of the one it is loading), writes it into a
 // 4-slot ring that exists in both CTAs' shared memory and signals sched_full[slot] in both. The
-// follower's producer, the MMA thread and the eight epilogue warps read the ring and each arrive
-// on the leader's sched_empty[slot] (10 arrivals) before the slot is reused. An index beyond the
+// follower's producer, the MMA thread and the epilogue warps of both read the ring and each arrive
+// on the leader's sched_empty[slot] (10 or 18 arrivals) before the slot is reused. An index beyond the
 // last tile is the stop mark; every pair draws exactly one, and the pair that draws the last one
 // puts the counter back to zero for the launch that reuses it. A pair that starts late (its SMs
 // were still busy with the previous kernel, or with a kernel of another stream) simply draws
@@ -38,7 +38,6 @@ namespace b200 {
 constexpr int G2_BM = 128;          // rows per CTA (256 per pair)
 constexpr int G2_BN = 256;          // columns per pair; each CTA stages 128 of them
 constexpr int G2_BK = 64;
-constexpr int G2_THREADS = 192;
 constexpr int G2_STAGES = 6;
 constexpr int G2_A_BYTES = G2_BM * G2_BK * 2;          // 16 KiB
 constexpr int G2_B_BYTES = (G2_BN / 2) * G2_BK * 2;    // 16 KiB
@@ -65,12 +64,21 @@ enum Gemm2Flags : int { G2_OUT_F32 = 1, G2_ADD_C = 2, G2_TMA_OUT = 4, G2_WHOLE_T
 //                  leaves d(gate), d(value) (the backward of silu(gate) * value), d(activation) is never stored
 //   EPI_DELTA      D = A B^T is d(attention output) [tokens, heads x head_dim]; the epilogue also fetches the forward's
 //                  output tile by TMA and leaves delta[b, head, t] = sum_d dO O, which the attention backward needs
+//   EPI_ADD        plain bf16 output with an addend (residual, accumulated gradient) whose tiles are fetched ahead
 //   EPI_SPLIT      a work item is one of `splits` K ranges of a tile; its fp32 sums go to a workspace
 //                  [splits][rows padded to whole tiles][N] that a second kernel adds up
 enum Gemm2Epi : int {
   EPI_PLAIN = 0, EPI_ROPE = 1, EPI_SWIGLU = 2, EPI_CE_STATS = 3, EPI_CE_DLOGITS = 4, EPI_SWIGLU_BWD = 5, EPI_DELTA = 6,
-  EPI_SPLIT = 7
+  EPI_SPLIT = 7, EPI_ADD = 8
 };
+
+// Warpgroups of the epilogue. The epilogues that fetch tiles or store more than one have two, each with half of a tile's
+// columns and two staging tiles of its own, paid for with one stage of the operand ring (5 x 32 KiB + 4 x 16 KiB in
+// place of 6 + 2).
+constexpr int g2_wgs(int epi) {
+  return epi == EPI_ROPE || epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD || epi == EPI_DELTA || epi == EPI_ADD ? 2 : 1;
+}
+constexpr int g2_threads(int epi) { return 64 + 128 * g2_wgs(epi); }
 
 struct Gemm2Params {
   void* D;
@@ -243,15 +251,14 @@ __device__ __forceinline__ void tile_coords2(int t, int num_m, int num_n, int& m
 }
 
 template <bool A_MN, bool B_MN, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(G2_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(g2_threads(EPI), 1)
 gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmD,
                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmE,
                      const Gemm2Params p) {
-  // The SwiGLU-backward epilogue works on two fetched tiles per group and prefetches the next pair: it trades
-  // one stage of the operand ring for two more staging tiles (5 x 32 KiB + 4 x 16 KiB instead of 6 + 2).
-  constexpr int kStages = EPI == EPI_SWIGLU_BWD ? G2_STAGES - 1 : G2_STAGES;
-  constexpr int kStg = EPI == EPI_SWIGLU_BWD ? 4 : 2;
+  constexpr int kWgs = g2_wgs(EPI);
+  constexpr int kStages = kWgs == 2 ? G2_STAGES - 1 : G2_STAGES;
+  constexpr int kStg = 2 * kWgs;
   constexpr int kStgOff = kStages * G2_STAGE_BYTES;
   static_assert(kStgOff + kStg * G2_STG_BYTES == G2_BAR_OFF2 && 2 * kStages + kStg == 2 * G2_STAGES + 2, "smem layout");
   extern __shared__ uint8_t smem_raw2[];
@@ -290,11 +297,11 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], 8);
+      mbar_init(&tempty[a], 8 * kWgs);
     }
     for (int i = 0; i < G2_SCHED; ++i) {
       mbar_init(&sched_full[i], 1);
-      mbar_init(&sched_empty[i], 10);
+      mbar_init(&sched_empty[i], 2 + 8 * kWgs);
     }
     for (int i = 0; i < kStg; ++i) mbar_init(&stage_ready[i], 1);
     *abort_flag = 0;
@@ -421,12 +428,13 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       }
     }
   } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5, both CTAs)
-    const int q = warp & 3;
+    // ------------------------------------------------------------ epilogue (warps 2..5 or 2..9, both CTAs)
+    const int q = warp & 3;                              // tensor-memory lane quarter
+    const int wg = kWgs == 2 ? (warp - 2) >> 2 : 0;
     int acc = 0;
     uint32_t acc_phase = 0;
-    const bool out_f32 = (p.flags & G2_OUT_F32) != 0;
-    const bool add_c = (p.flags & G2_ADD_C) != 0;
+    const bool out_f32 = kWgs == 1 && (p.flags & G2_OUT_F32) != 0;       // the two-warpgroup forms store bf16 through TMA
+    const bool add_c = kWgs == 1 && (p.flags & G2_ADD_C) != 0;
     const bool vec_ok = out_f32 ? ((p.ldd & 3) == 0 && (reinterpret_cast<uintptr_t>(p.D) & 15) == 0 &&
                                    (!add_c || ((p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0)))
                                 : ((p.ldd & 7) == 0 && (reinterpret_cast<uintptr_t>(p.D) & 15) == 0 &&
@@ -493,18 +501,19 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       }
     } else if constexpr (EPI == EPI_SWIGLU) {
       // 256 rows x 128 activation columns per item: accumulator columns [0, 128) are the gate, [128, 256)
-      // the value. Per 64-column group the thread's row leaves as up to three 128-byte staging rows (raw
-      // gate, raw value, activation), each stored by TMA; two staging tiles alternate as in the plain path.
-      uint8_t* stg = smem + kStgOff;
+      // the value. Per 64-column group (one per warpgroup) the thread's row leaves as up to three 128-byte staging rows
+      // (raw gate, raw value, activation), each stored by TMA; two staging tiles alternate as in the plain path.
+      uint8_t* stg = smem + kStgOff + wg * 2 * G2_STG_BYTES;
+      uint64_t* ready = stage_ready + wg * 2;
       const int r = q * 32 + lane;
       const uint32_t swz = uint32_t(r & 7);
-      const bool elected = (warp == 2 && lane == 0);
+      const bool elected = (((warp - 2) & 3) == 0 && lane == 0);
       uint32_t gcount = 0;
       // One group: this thread's 64 fp32 values -> bf16 -> staging row; one thread stores the tile. `more`: another
       // group of the same item follows (its staging tile is released here; an item's first one at the item's start).
       auto put = [&](const uint32_t (&v)[64], const CUtensorMap* map, int x, int y, bool more) -> bool {
         const uint32_t b = gcount & 1;
-        if (!mbar_wait(&stage_ready[b], (gcount >> 1) & 1, abort_flag)) return false;
+        if (!mbar_wait(&ready[b], (gcount >> 1) & 1, abort_flag)) return false;
         uint8_t* rowp = stg + b * G2_STG_BYTES + r * 128;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -516,13 +525,13 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           *reinterpret_cast<uint4*>(rowp + ((uint32_t(c) ^ swz) << 4)) = o;
         }
         fence_proxy_async_smem();
-        named_bar_sync_128(1);
+        named_bar_sync_128(1 + wg);
         if (elected) {
           if (x < p.sw_I) tma_store_2d(map, stg + b * G2_STG_BYTES, x, y);      // a group wholly past the edge is dropped
           tma_store_commit();
           if (more) {
             tma_store_wait_read<1>();
-            mbar_arrive(&stage_ready[(gcount + 1) & 1]);
+            mbar_arrive(&ready[(gcount + 1) & 1]);
           }
         }
         ++gcount;
@@ -536,24 +545,22 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int g0 = wi.nb * (G2_BN / 2);
         if (elected) {
           tma_store_wait_read<1>();                      // the store that last used this staging tile has read it
-          mbar_arrive(&stage_ready[gcount & 1]);
+          mbar_arrive(&ready[gcount & 1]);
         }
         if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN;
-#pragma unroll 1
-        for (int g = 0; g < 2 && ok; ++g) {
+        {
+          const int g = wg;                              // warpgroup w: activation columns [64 w, 64 w + 64) of the tile
           uint32_t ga[64], va[64];
           tmem_ld_32x32b_x32(taddr + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&ga[0]));
           tmem_ld_32x32b_x32(taddr + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&ga[32]));
           tmem_ld_32x32b_x32(taddr + G2_BN / 2 + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&va[0]));
           tmem_ld_32x32b_x32(taddr + G2_BN / 2 + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&va[32]));
           tmem_ld_wait();
-          if (g == 1) {                                  // accumulator fully read: hand it back to the MMA warp
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
-          }
+          tc_fence_before();                             // this warp's columns are read: hand them back to the MMA warp
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
           const int x = g0 + g * 64;
           if (p.sw_store_gv) {
             if (!put(ga, &tmD, x, row0, true)) { ok = false; break; }
@@ -564,31 +571,32 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             const float gt = __uint_as_float(ga[j]);
             ga[j] = __float_as_uint(gt / (1.f + __expf(-gt)) * __uint_as_float(va[j]));
           }
-          if (!put(ga, &tmBh, x, row0, g == 0)) { ok = false; break; }
+          if (!put(ga, &tmBh, x, row0, false)) { ok = false; break; }
         }
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
       if (elected) tma_store_wait<0>();
     } else if constexpr (EPI == EPI_SWIGLU_BWD) {
-      // The accumulator is d(act) for 256 rows x 256 columns. Per 64-column group the stored gate and value tiles
-      // (bf16, the two halves of the forward projection; maps tmBh / tmE) are fetched by TMA into a pair of staging
-      // tiles, turned in place into d(gate) and d(value) and stored (maps tmD / tmC). Two pairs alternate: the next
-      // group's pair is fetched while this one is computed.
-      uint8_t* stg = smem + kStgOff;
+      // The accumulator is d(act) for 256 rows x 256 columns, columns [128 w, 128 w + 128) for warpgroup w. Per 64-column
+      // group the stored gate and value tiles (bf16, the two halves of the forward projection; maps tmBh / tmE) are
+      // fetched by TMA into the warpgroup's pair of staging tiles, turned in place into d(gate) and d(value) and stored
+      // (maps tmD / tmC). One warpgroup fetches and stores while the other computes.
+      uint8_t* stg = smem + kStgOff + wg * 2 * G2_STG_BYTES;
+      uint64_t* ready = stage_ready + wg * 2;
       const int r = q * 32 + lane;
       const uint32_t swz = uint32_t(r & 7);
-      const bool elected = (warp == 2 && lane == 0);
-      uint32_t ucount = 0;                               // groups handled so far; pair = ucount & 1
-      auto fetch = [&](uint32_t uc, int x, int y) {      // by the elected thread: fill pair uc & 1 for a group
-        const uint32_t b = (uc & 1) * 2;
+      const bool elected = (((warp - 2) & 3) == 0 && lane == 0);
+      uint32_t ucount = 0;                               // groups handled so far
+      auto fetch = [&](int x, int y) {                   // by the elected thread: fill the pair for a group
+        tma_store_wait_read<0>();                        // the stores that last used it have read it
         if (x < p.sw_I) {
-          mbar_expect_tx(&stage_ready[b], G2_STG_BYTES);
-          tma_load_2d(stg + b * G2_STG_BYTES, &tmBh, &stage_ready[b], x, y);
-          mbar_expect_tx(&stage_ready[b + 1], G2_STG_BYTES);
-          tma_load_2d(stg + (b + 1) * G2_STG_BYTES, &tmE, &stage_ready[b + 1], x, y);
+          mbar_expect_tx(&ready[0], G2_STG_BYTES);
+          tma_load_2d(stg, &tmBh, &ready[0], x, y);
+          mbar_expect_tx(&ready[1], G2_STG_BYTES);
+          tma_load_2d(stg + G2_STG_BYTES, &tmE, &ready[1], x, y);
         } else {                                         // wholly past the edge: nothing to fetch, nothing is stored
-          mbar_arrive(&stage_ready[b]);
-          mbar_arrive(&stage_ready[b + 1]);
+          mbar_arrive(&ready[0]);
+          mbar_arrive(&ready[1]);
         }
       };
       for (int t = pair; ok && t >= 0 && t < num_tiles;
@@ -596,37 +604,28 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                    : t + num_pairs) {
         const G2Item wi = g2_item(t, p.t_full, num_m, num_n);
         const int row0 = wi.mb * 2 * G2_BM + int(rank) * G2_BM;
-        const int n0 = wi.n0;
-        const int ngroups = wi.bn / 64;
-        if (elected) {
-          tma_store_wait_read<1>();                      // the stores that last used this pair have read it
-          fetch(ucount, n0, row0);
-        }
+        const int n0 = wi.n0 + wg * (G2_BN / 2);
+        if (elected) fetch(n0, row0);
         if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN;
+        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN + wg * (G2_BN / 2);
 #pragma unroll 1
-        for (int g = 0; g < ngroups; ++g) {
-          const uint32_t b = (ucount & 1) * 2;
-          if (elected && g + 1 < ngroups) {              // prefetch the next group's pair
-            tma_store_wait_read<0>();                    // the other pair's stores (previous group) have read it
-            fetch(ucount + 1, n0 + (g + 1) * 64, row0);
-          }
+        for (int g = 0; g < 2; ++g) {
           uint32_t v[64];
           tmem_ld_32x32b_x32(taddr + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
           tmem_ld_32x32b_x32(taddr + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
           tmem_ld_wait();
-          if (g == ngroups - 1) {                        // accumulator fully read: hand it back to the MMA warp
+          if (g == 1) {                                  // this warp's columns are read: hand them back to the MMA warp
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
           }
-          const uint32_t ph = (ucount >> 1) & 1;
-          if (!mbar_wait(&stage_ready[b], ph, abort_flag) || !mbar_wait(&stage_ready[b + 1], ph, abort_flag)) {
+          const uint32_t ph = ucount & 1;
+          if (!mbar_wait(&ready[0], ph, abort_flag) || !mbar_wait(&ready[1], ph, abort_flag)) {
             ok = false;
             break;
           }
-          uint8_t* grow = stg + b * G2_STG_BYTES + r * 128;
+          uint8_t* grow = stg + r * 128;
           uint8_t* vrow = grow + G2_STG_BYTES;
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -648,14 +647,15 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             *vp = vq;
           }
           fence_proxy_async_smem();
-          named_bar_sync_128(1);
+          named_bar_sync_128(1 + wg);
           if (elected) {
             const int x = n0 + g * 64;
             if (x < p.sw_I) {
-              tma_store_2d(&tmD, stg + b * G2_STG_BYTES, x, row0);
-              tma_store_2d(&tmC, stg + (b + 1) * G2_STG_BYTES, x, row0);
+              tma_store_2d(&tmD, stg, x, row0);
+              tma_store_2d(&tmC, stg + G2_STG_BYTES, x, row0);
             }
             tma_store_commit();
+            if (g == 0) fetch(n0 + 64, row0);
           }
           ++ucount;
         }
@@ -663,26 +663,29 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       }
       if (elected) tma_store_wait<0>();
     } else
-    if (p.flags & G2_TMA_OUT) {
+    if (kWgs == 2 || (p.flags & G2_TMA_OUT)) {
       // Output through shared memory and TMA. A tile leaves in groups of 128 bytes per row (64 bf16
       // or 32 fp32 columns): every thread converts its accumulator row and writes it into a
       // 128-row staging tile in the 128-byte swizzle, one thread stores the tile with
       // cp.async.bulk.tensor (full 128-byte lines to L2, clipped at the matrix edge). With `add`
-      // the same staging tile is first filled with the C tile by a TMA load. Two staging tiles
-      // alternate, so the store of one group overlaps the conversion of the next.
+      // the same staging tile is first filled with the C tile by a TMA load. Two staging tiles per warpgroup
+      // alternate, so the store of one group overlaps the conversion of the next; EPI_ADD and EPI_DELTA fetch the tiles of
+      // both groups of a warpgroup before they wait for the accumulator.
+      constexpr bool kAhead = EPI == EPI_ADD || EPI == EPI_DELTA;
       const int gcols = out_f32 ? 32 : 64;
-      uint8_t* stg = smem + kStgOff;
+      uint8_t* stg = smem + kStgOff + wg * 2 * G2_STG_BYTES;
+      uint64_t* ready = stage_ready + wg * 2;
       const int r = q * 32 + lane;
       const uint32_t swz = uint32_t(r & 7);
-      const bool elected = (warp == 2 && lane == 0);
+      const bool elected = (((warp - 2) & 3) == 0 && lane == 0);
       uint32_t gcount = 0;
       auto arm = [&](uint32_t gc, int x, int y) {       // make staging tile gc & 1 ready for group gc
         const uint32_t b = gc & 1;
-        if (add_c || EPI == EPI_DELTA) {
-          mbar_expect_tx(&stage_ready[b], G2_STG_BYTES);
-          tma_load_2d(stg + b * G2_STG_BYTES, &tmC, &stage_ready[b], x, y);
+        if (kAhead || add_c) {
+          mbar_expect_tx(&ready[b], G2_STG_BYTES);
+          tma_load_2d(stg + b * G2_STG_BYTES, &tmC, &ready[b], x, y);
         } else {
-          mbar_arrive(&stage_ready[b]);
+          mbar_arrive(&ready[b]);
         }
       };
       for (int t = pair; ok && t >= 0 && t < num_tiles;
@@ -692,6 +695,9 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int row0 = wi.mb * 2 * G2_BM + int(rank) * G2_BM + (kSplit ? t % p.splits * num_m * 2 * G2_BM : 0);
         const int n0 = wi.n0;
         const int ngroups = wi.bn / gcols;
+        // this warpgroup's groups; a head of 128 columns stays with one (its row sum is one thread's)
+        const int per = kWgs == 1 ? ngroups : max(ngroups / 2, EPI == EPI_DELTA ? p.dl_dim / 64 : 1);
+        const int g_lo = wg * per, g_hi = min(ngroups, g_lo + per);
         const bool rope_on = kRope && !out_f32 && n0 < p.rope_cols;
         const float* cs_row = nullptr;      // element j of this row's tables is at [j * rope_ld]
         const float* sn_row = nullptr;
@@ -709,23 +715,31 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           ce_t = __ldg(p.ce_targets + row) - p.ce_col0;
         }
         float dl_sum = 0.f;                     // EPI_DELTA: dO . O over the head's columns seen so far
-        if (elected) {
+        if (elected && g_lo < g_hi) {
           tma_store_wait_read<1>();                      // the store that last used this staging tile has read it
-          arm(gcount, n0, row0);
+          arm(gcount, n0 + g_lo * gcols, row0);
+          if (kAhead && g_lo + 1 < g_hi) {
+            tma_store_wait_read<0>();
+            arm(gcount + 1, n0 + (g_lo + 1) * gcols, row0);
+          }
         }
         if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN;
+        if (kWgs == 2 && g_lo >= g_hi) {                 // no columns of this tile
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
+        }
 #pragma unroll 1
-        for (int g = 0; g < ngroups; ++g) {
+        for (int g = g_lo; g < g_hi; ++g) {
           const uint32_t b = gcount & 1;
-          if (!mbar_wait(&stage_ready[b], (gcount >> 1) & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait(&ready[b], (gcount >> 1) & 1, abort_flag)) { ok = false; break; }
           uint8_t* rowp = stg + b * G2_STG_BYTES + r * 128;
           if (out_f32) {
             uint32_t v[32];
             tmem_ld_32x32b_x32(taddr + g * 32, v);
             tmem_ld_wait();
-            if (g == ngroups - 1) {                      // accumulator fully read: hand it back to the MMA warp
+            if (g == g_hi - 1) {                         // accumulator fully read: hand it back to the MMA warp
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
@@ -780,7 +794,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 }
               }
             }
-            if (g == ngroups - 1) {
+            if (g == g_hi - 1) {
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
@@ -791,7 +805,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
               float f[8];
 #pragma unroll
               for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(v[8 * c + e]) * p.alpha;
-              if (add_c) {
+              if (EPI == EPI_ADD || add_c) {
                 const uint4 cc = *dst;
                 const bf162* c2 = reinterpret_cast<const bf162*>(&cc);
 #pragma unroll
@@ -831,11 +845,11 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             }
           }
           fence_proxy_async_smem();
-          named_bar_sync_128(1);
+          named_bar_sync_128(1 + wg);
           if (elected) {
             tma_store_2d(&tmD, stg + b * G2_STG_BYTES, n0 + g * gcols, row0);
             tma_store_commit();
-            if (g + 1 < ngroups) {
+            if (!kAhead && g + 1 < g_hi) {
               tma_store_wait_read<1>();
               arm(gcount + 1, n0 + (g + 1) * gcols, row0);
             }
@@ -968,7 +982,7 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
   const int all_pairs = num_sms() / 2;
   // a last round that fills less than half of the pairs is run on half tiles (plain and rotary epilogues only)
   int halved = 0;
-  if (g_half_tiles && (EPI <= EPI_ROPE || EPI == EPI_DELTA) && !(p.flags & G2_WHOLE_TILES) && whole > all_pairs) {
+  if (g_half_tiles && (EPI <= EPI_ROPE || EPI == EPI_DELTA || EPI == EPI_ADD) && !(p.flags & G2_WHOLE_TILES) && whole > all_pairs) {
     const int rem = whole % all_pairs;
     if (rem > 0 && 2 * rem <= all_pairs) halved = rem;
   }
@@ -983,7 +997,7 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     q.sched = next_sched_slot();
     if (q.sched == nullptr) return static_cast<int>(cudaErrorInvalidValue);
   }
-  return static_cast<int>(launch_pdl(kern, dim3(2 * pairs), dim3(G2_THREADS), G2_SMEM, stream, 0, *tA, *tB, *tBh, *tD, *tC,
+  return static_cast<int>(launch_pdl(kern, dim3(2 * pairs), dim3(g2_threads(EPI)), G2_SMEM, stream, 0, *tA, *tB, *tBh, *tD, *tC,
                                      tE ? *tE : *tA, q));
 }
 
@@ -1129,6 +1143,10 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
     if (!(p.flags & G2_TMA_OUT) || a_mn_major) return static_cast<int>(cudaErrorInvalidValue);
     if (b_mn_major) return launch_tc2<false, true, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
     return launch_tc2<false, false, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
+  }
+  if (add && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & G2_OUT_F32)) {
+    if (b_mn_major) return launch_tc2<false, true, EPI_ADD>(tA, tB, tBh, tD, tC, p, stream);
+    return launch_tc2<false, false, EPI_ADD>(tA, tB, tBh, tD, tC, p, stream);
   }
   if (a_mn_major && b_mn_major) return launch_tc2<true, true>(tA, tB, tBh, tD, tC, p, stream);
   if (a_mn_major) return launch_tc2<true, false>(tA, tB, tBh, tD, tC, p, stream);
