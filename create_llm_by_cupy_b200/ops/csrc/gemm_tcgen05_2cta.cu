@@ -72,12 +72,13 @@ enum Gemm2Epi : int {
   EPI_SPLIT = 7, EPI_ADD = 8
 };
 
-// Warpgroups of the epilogue. The epilogues that fetch tiles or store more than one have two, each with half of a tile's
-// columns and two staging tiles of its own, paid for with one stage of the operand ring (5 x 32 KiB + 4 x 16 KiB in
-// place of 6 + 2).
-constexpr int g2_wgs(int epi) {
-  return epi == EPI_ROPE || epi == EPI_SWIGLU || epi == EPI_SWIGLU_BWD || epi == EPI_DELTA || epi == EPI_ADD ? 2 : 1;
-}
+// Warpgroups of the epilogue. Those that fetch the tiles of an addend or rotate have two, each with half of a tile's
+// columns and two staging tiles of its own, so that no group waits for a round trip of the one before: EPI_TIMES
+// The SwiGLU forms stay with one: beside their 90 to 360 MB of tiles the operands' way through L2 is what bounds them
+// (backward 8192 x 5504 x 2048 165 us, 176 with two).
+constexpr int g2_wgs(int epi) { return epi == EPI_ROPE || epi == EPI_DELTA || epi == EPI_ADD ? 2 : 1; }
+// Four staging tiles in place of two cost a stage of the operand ring (5 x 32 KiB + 4 x 16 KiB in place of 6 + 2).
+constexpr int g2_staging(int epi) { return g2_wgs(epi) == 2 || epi == EPI_SWIGLU_BWD ? 4 : 2; }
 constexpr int g2_threads(int epi) { return 64 + 128 * g2_wgs(epi); }
 
 struct Gemm2Params {
@@ -257,8 +258,8 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmE,
                      const Gemm2Params p) {
   constexpr int kWgs = g2_wgs(EPI);
-  constexpr int kStages = kWgs == 2 ? G2_STAGES - 1 : G2_STAGES;
-  constexpr int kStg = 2 * kWgs;
+  constexpr int kStg = g2_staging(EPI);
+  constexpr int kStages = kStg == 4 ? G2_STAGES - 1 : G2_STAGES;
   constexpr int kStgOff = kStages * G2_STAGE_BYTES;
   static_assert(kStgOff + kStg * G2_STG_BYTES == G2_BAR_OFF2 && 2 * kStages + kStg == 2 * G2_STAGES + 2, "smem layout");
   extern __shared__ uint8_t smem_raw2[];
@@ -501,19 +502,18 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       }
     } else if constexpr (EPI == EPI_SWIGLU) {
       // 256 rows x 128 activation columns per item: accumulator columns [0, 128) are the gate, [128, 256)
-      // the value. Per 64-column group (one per warpgroup) the thread's row leaves as up to three 128-byte staging rows
-      // (raw gate, raw value, activation), each stored by TMA; two staging tiles alternate as in the plain path.
-      uint8_t* stg = smem + kStgOff + wg * 2 * G2_STG_BYTES;
-      uint64_t* ready = stage_ready + wg * 2;
+      // the value. Per 64-column group the thread's row leaves as up to three 128-byte staging rows (raw
+      // gate, raw value, activation), each stored by TMA; two staging tiles alternate as in the plain path.
+      uint8_t* stg = smem + kStgOff;
       const int r = q * 32 + lane;
       const uint32_t swz = uint32_t(r & 7);
-      const bool elected = (((warp - 2) & 3) == 0 && lane == 0);
+      const bool elected = (warp == 2 && lane == 0);
       uint32_t gcount = 0;
       // One group: this thread's 64 fp32 values -> bf16 -> staging row; one thread stores the tile. `more`: another
       // group of the same item follows (its staging tile is released here; an item's first one at the item's start).
       auto put = [&](const uint32_t (&v)[64], const CUtensorMap* map, int x, int y, bool more) -> bool {
         const uint32_t b = gcount & 1;
-        if (!mbar_wait(&ready[b], (gcount >> 1) & 1, abort_flag)) return false;
+        if (!mbar_wait(&stage_ready[b], (gcount >> 1) & 1, abort_flag)) return false;
         uint8_t* rowp = stg + b * G2_STG_BYTES + r * 128;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
@@ -525,13 +525,13 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           *reinterpret_cast<uint4*>(rowp + ((uint32_t(c) ^ swz) << 4)) = o;
         }
         fence_proxy_async_smem();
-        named_bar_sync_128(1 + wg);
+        named_bar_sync_128(1);
         if (elected) {
           if (x < p.sw_I) tma_store_2d(map, stg + b * G2_STG_BYTES, x, y);      // a group wholly past the edge is dropped
           tma_store_commit();
           if (more) {
             tma_store_wait_read<1>();
-            mbar_arrive(&ready[(gcount + 1) & 1]);
+            mbar_arrive(&stage_ready[(gcount + 1) & 1]);
           }
         }
         ++gcount;
@@ -545,22 +545,24 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         const int g0 = wi.nb * (G2_BN / 2);
         if (elected) {
           tma_store_wait_read<1>();                      // the store that last used this staging tile has read it
-          mbar_arrive(&ready[gcount & 1]);
+          mbar_arrive(&stage_ready[gcount & 1]);
         }
         if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN;
-        {
-          const int g = wg;                              // warpgroup w: activation columns [64 w, 64 w + 64) of the tile
+#pragma unroll 1
+        for (int g = 0; g < 2 && ok; ++g) {
           uint32_t ga[64], va[64];
           tmem_ld_32x32b_x32(taddr + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&ga[0]));
           tmem_ld_32x32b_x32(taddr + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&ga[32]));
           tmem_ld_32x32b_x32(taddr + G2_BN / 2 + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&va[0]));
           tmem_ld_32x32b_x32(taddr + G2_BN / 2 + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&va[32]));
           tmem_ld_wait();
-          tc_fence_before();                             // this warp's columns are read: hand them back to the MMA warp
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
+          if (g == 1) {                                  // accumulator fully read: hand it back to the MMA warp
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
+          }
           const int x = g0 + g * 64;
           if (p.sw_store_gv) {
             if (!put(ga, &tmD, x, row0, true)) { ok = false; break; }
@@ -571,32 +573,31 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             const float gt = __uint_as_float(ga[j]);
             ga[j] = __float_as_uint(gt / (1.f + __expf(-gt)) * __uint_as_float(va[j]));
           }
-          if (!put(ga, &tmBh, x, row0, false)) { ok = false; break; }
+          if (!put(ga, &tmBh, x, row0, g == 0)) { ok = false; break; }
         }
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
       if (elected) tma_store_wait<0>();
     } else if constexpr (EPI == EPI_SWIGLU_BWD) {
-      // The accumulator is d(act) for 256 rows x 256 columns, columns [128 w, 128 w + 128) for warpgroup w. Per 64-column
-      // group the stored gate and value tiles (bf16, the two halves of the forward projection; maps tmBh / tmE) are
-      // fetched by TMA into the warpgroup's pair of staging tiles, turned in place into d(gate) and d(value) and stored
-      // (maps tmD / tmC). One warpgroup fetches and stores while the other computes.
-      uint8_t* stg = smem + kStgOff + wg * 2 * G2_STG_BYTES;
-      uint64_t* ready = stage_ready + wg * 2;
+      // The accumulator is d(act) for 256 rows x 256 columns. Per 64-column group the stored gate and value tiles
+      // (bf16, the two halves of the forward projection; maps tmBh / tmE) are fetched by TMA into a pair of staging
+      // tiles, turned in place into d(gate) and d(value) and stored (maps tmD / tmC). Two pairs alternate: the next
+      // group's pair is fetched while this one is computed.
+      uint8_t* stg = smem + kStgOff;
       const int r = q * 32 + lane;
       const uint32_t swz = uint32_t(r & 7);
-      const bool elected = (((warp - 2) & 3) == 0 && lane == 0);
-      uint32_t ucount = 0;                               // groups handled so far
-      auto fetch = [&](int x, int y) {                   // by the elected thread: fill the pair for a group
-        tma_store_wait_read<0>();                        // the stores that last used it have read it
+      const bool elected = (warp == 2 && lane == 0);
+      uint32_t ucount = 0;                               // groups handled so far; pair = ucount & 1
+      auto fetch = [&](uint32_t uc, int x, int y) {      // by the elected thread: fill pair uc & 1 for a group
+        const uint32_t b = (uc & 1) * 2;
         if (x < p.sw_I) {
-          mbar_expect_tx(&ready[0], G2_STG_BYTES);
-          tma_load_2d(stg, &tmBh, &ready[0], x, y);
-          mbar_expect_tx(&ready[1], G2_STG_BYTES);
-          tma_load_2d(stg + G2_STG_BYTES, &tmE, &ready[1], x, y);
+          mbar_expect_tx(&stage_ready[b], G2_STG_BYTES);
+          tma_load_2d(stg + b * G2_STG_BYTES, &tmBh, &stage_ready[b], x, y);
+          mbar_expect_tx(&stage_ready[b + 1], G2_STG_BYTES);
+          tma_load_2d(stg + (b + 1) * G2_STG_BYTES, &tmE, &stage_ready[b + 1], x, y);
         } else {                                         // wholly past the edge: nothing to fetch, nothing is stored
-          mbar_arrive(&ready[0]);
-          mbar_arrive(&ready[1]);
+          mbar_arrive(&stage_ready[b]);
+          mbar_arrive(&stage_ready[b + 1]);
         }
       };
       for (int t = pair; ok && t >= 0 && t < num_tiles;
@@ -604,28 +605,37 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                    : t + num_pairs) {
         const G2Item wi = g2_item(t, p.t_full, num_m, num_n);
         const int row0 = wi.mb * 2 * G2_BM + int(rank) * G2_BM;
-        const int n0 = wi.n0 + wg * (G2_BN / 2);
-        if (elected) fetch(n0, row0);
+        const int n0 = wi.n0;
+        const int ngroups = wi.bn / 64;
+        if (elected) {
+          tma_store_wait_read<1>();                      // the stores that last used this pair have read it
+          fetch(ucount, n0, row0);
+        }
         if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN + wg * (G2_BN / 2);
+        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN;
 #pragma unroll 1
-        for (int g = 0; g < 2; ++g) {
+        for (int g = 0; g < ngroups; ++g) {
+          const uint32_t b = (ucount & 1) * 2;
+          if (elected && g + 1 < ngroups) {              // prefetch the next group's pair
+            tma_store_wait_read<0>();                    // the other pair's stores (previous group) have read it
+            fetch(ucount + 1, n0 + (g + 1) * 64, row0);
+          }
           uint32_t v[64];
           tmem_ld_32x32b_x32(taddr + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
           tmem_ld_32x32b_x32(taddr + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
           tmem_ld_wait();
-          if (g == 1) {                                  // this warp's columns are read: hand them back to the MMA warp
+          if (g == ngroups - 1) {                        // accumulator fully read: hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
           }
-          const uint32_t ph = ucount & 1;
-          if (!mbar_wait(&ready[0], ph, abort_flag) || !mbar_wait(&ready[1], ph, abort_flag)) {
+          const uint32_t ph = (ucount >> 1) & 1;
+          if (!mbar_wait(&stage_ready[b], ph, abort_flag) || !mbar_wait(&stage_ready[b + 1], ph, abort_flag)) {
             ok = false;
             break;
           }
-          uint8_t* grow = stg + r * 128;
+          uint8_t* grow = stg + b * G2_STG_BYTES + r * 128;
           uint8_t* vrow = grow + G2_STG_BYTES;
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -647,15 +657,14 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             *vp = vq;
           }
           fence_proxy_async_smem();
-          named_bar_sync_128(1 + wg);
+          named_bar_sync_128(1);
           if (elected) {
             const int x = n0 + g * 64;
             if (x < p.sw_I) {
-              tma_store_2d(&tmD, stg, x, row0);
-              tma_store_2d(&tmC, stg + G2_STG_BYTES, x, row0);
+              tma_store_2d(&tmD, stg + b * G2_STG_BYTES, x, row0);
+              tma_store_2d(&tmC, stg + (b + 1) * G2_STG_BYTES, x, row0);
             }
             tma_store_commit();
-            if (g == 0) fetch(n0 + 64, row0);
           }
           ++ucount;
         }
