@@ -73,7 +73,9 @@ enum Gemm2Epi : int {
 };
 
 // Warpgroups of the epilogue. Those that fetch the tiles of an addend or rotate have two, each with half of a tile's
-// columns and two staging tiles of its own, so that no group waits for a round trip of the one before: EPI_TIMES
+// columns and two staging tiles of its own, so that no group waits for a round trip of the one before (us, before / now): residual added 8192 x 768 x 768
+// 19.5 / 17.1, 777 x 768 x 768 11.4 / 10.0, delta 8192 x 768 x 768 20.9 / 16.8, 2048 x 1024 x 1024 14.3 / 12.3 (8192 x 2048
+// x 2048 55.7 / 56.9, the ring's missing stage), rotation 8192 x 1280 x 768 24.4 / 21.1, 777 rows 12.4 / 10.6.
 // The SwiGLU forms stay with one: beside their 90 to 360 MB of tiles the operands' way through L2 is what bounds them
 // (backward 8192 x 5504 x 2048 165 us, 176 with two).
 constexpr int g2_wgs(int epi) { return epi == EPI_ROPE || epi == EPI_DELTA || epi == EPI_ADD ? 2 : 1; }
@@ -1153,7 +1155,12 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
     if (b_mn_major) return launch_tc2<false, true, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
     return launch_tc2<false, false, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
   }
-  if (add && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & G2_OUT_F32)) {
+  // The addend's tiles fetched ahead (one operand stage less) where the epilogue is a large part of a tile's life: one
+  // round of tiles, or a short K. us, fetched group by group / ahead: 8192 x 2048 over K = 512 34.4 / 26.7, 1024 38.4 / 34.1,
+  // 1536 43.5 / 45.0, 5504 133.9 / 135.2; 8192 x 768 over 1024 21.0 / 19.1, 1536 24.5 / 24.5; one round: 1000 x 4096 over
+  // 256 10.0 / 8.4, 4096 32.3 / 30.4, 2048 x 1024 over 2736 23.2 / 20.6.
+  const int tiles = ((M + 2 * G2_BM - 1) / (2 * G2_BM)) * ((N + G2_BN - 1) / G2_BN);
+  if (add && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & G2_OUT_F32) && (K <= 1280 || tiles <= num_sms() / 2)) {
     if (b_mn_major) return launch_tc2<false, true, EPI_ADD>(tA, tB, tBh, tD, tC, p, stream);
     return launch_tc2<false, false, EPI_ADD>(tA, tB, tBh, tD, tC, p, stream);
   }
