@@ -991,11 +991,14 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
   const int tile_cols = EPI == EPI_SWIGLU ? (p.sw_I + G2_BN / 2 - 1) / (G2_BN / 2) : (p.N + G2_BN - 1) / G2_BN;
   const int whole = ((p.M + 2 * G2_BM - 1) / (2 * G2_BM)) * tile_cols;
   const int all_pairs = num_sms() / 2;
-  // a last round that fills less than half of the pairs is run on half tiles (plain and rotary epilogues only)
+  // a last round that fills less than half of the pairs is run on half tiles (plain, addend, delta and rotary epilogues)
   int halved = 0;
-  if (g_half_tiles && (EPI <= EPI_ROPE || EPI == EPI_DELTA || EPI == EPI_ADD) && !(p.flags & G2_WHOLE_TILES) && whole > all_pairs) {
+  if (g_half_tiles && (EPI <= EPI_ROPE || EPI == EPI_DELTA || EPI == EPI_ADD) && !(p.flags & G2_WHOLE_TILES)) {
     const int rem = whole % all_pairs;
-    if (rem > 0 && 2 * rem <= all_pairs) halved = rem;
+    // The only round counts too, unless it is a weight gradient (A_MN), whose idle pairs the main stream's kernels use (125M
+    // training pass 7810 us, 8014 with halves there). 777 rows, us whole / halves: 768 x 768 10.0 / 8.8, 768 x 2048 15.9 /
+    // 14.9, 1280 x 768 10.1 / 9.0; 2048 x 1024 x 2736 20.7 / 20.0.
+    if (2 * rem <= all_pairs && (whole > all_pairs || !A_MN)) halved = rem;
   }
   const int num_tiles = EPI == EPI_SPLIT ? whole * p.splits : whole + halved;
   int pairs = all_pairs;
