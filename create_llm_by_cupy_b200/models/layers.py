@@ -393,17 +393,25 @@ class ChunkedCrossEntropy_Share:
     """LM head + mean cross-entropy over non-pad targets without an ``[M, V]`` tensor
     (reference: model/fast_layers.py:1280-1488, which makes two chunked passes forward and one backward).
 
-    On CUDA the logits never reach memory. Forward: ONE GEMM over the whole vocabulary whose epilogue folds
-    each 256-column tile of the fp32 accumulator into per-row (max, sum-exp, target logit); a small merge gives
-    the row's log-sum-exp. Backward walks the vocabulary in chunks of ``chunk_size``: the logits of a chunk are
-    recomputed by a GEMM whose epilogue turns them into ``(softmax - onehot) * GradScale / n_valid`` in bf16 (the
-    only [M, chunk] tensor that exists), which feeds the two gradient GEMMs; ``dW`` rows go to
-    ``grad_writer(row_start, row_end)`` -> destination view, so they land directly in the gradient bucket.
+    On CUDA, forward: ONE GEMM over the whole vocabulary whose epilogue folds each 256-column tile of the fp32
+    accumulator into per-row (max, sum-exp, target logit); a small merge gives the row's log-sum-exp. A training
+    forward also stores the fp32 logits of as many leading chunks as ``KEEP_LOGITS_BYTES`` holds (given back by the
+    backward). Backward walks the vocabulary in chunks of ``chunk_size``: the logits of a chunk - the stored ones,
+    else recomputed by a GEMM with the same in its epilogue - become ``(softmax - onehot) * GradScale / n_valid`` in
+    bf16, which feeds the two gradient GEMMs; ``dW`` rows go to ``grad_writer(row_start, row_end)`` -> destination
+    view, so they land directly in the gradient bucket.
 
     Where the fused GEMMs do not apply (CPU tensors, tiny shapes, ``cache_logits`` asked for explicitly) the
     chunked form with fp32 logits per chunk is used: one pass forward, logits kept for the backward only when
     ``cache_logits``.
     """
+
+    # Storing and reading them costs the same whatever the width of x, recomputing them a product that grows with it. 8192
+    # tokens, 32000 columns (1.05 GB from the forward to the backward), forward + backward of the layer with recomputed /
+    # stored logits in us: width 512 1021 / 1061, 768 1396 / 1402, 1024 1626 / 1536, 2048 3060 / 2650, 4096 6040 / 4700; 1000
+    # tokens: 1024 342 / 312, 2048 512 / 431.
+    KEEP_LOGITS_BYTES = 2 << 30
+    KEEP_LOGITS_WIDTH = 1024
 
     def __init__(self, padding_id: int, chunk_size: int = 8192, dtype=torch.bfloat16, cache_logits: bool = False):
         self.padding_id = padding_id
@@ -418,6 +426,17 @@ class ChunkedCrossEntropy_Share:
     def _fused(self, x: torch.Tensor, W: torch.Tensor) -> bool:
         return bool(F.CE_EPILOGUE and not self.cache_logits and F.gemm_ce_fusable(x, W))
 
+    def _logits_buffer(self, x: torch.Tensor, V: int):
+        """[M, keep] fp32 for the leading whole chunks that fit, or None (also when the device has no memory left for it)."""
+        M, ends = x.shape[0], [e for _, e in self._chunks(V)]
+        keep = max([e for e in ends if M * e * 4 <= self.KEEP_LOGITS_BYTES and (e % 32 == 0 or e == V)], default=0)
+        if keep == 0 or x.shape[1] < self.KEEP_LOGITS_WIDTH:
+            return None
+        try:
+            return torch.empty((M, (keep + 3) // 4 * 4), dtype=torch.float32, device=x.device)[:, :keep]
+        except torch.OutOfMemoryError:
+            return None
+
     def forward(self, x: torch.Tensor, t: torch.Tensor, W: torch.Tensor, train_flg: bool = True) -> torch.Tensor:
         """x [M, H], t [M] int32 targets, W [V, H]. Returns the scalar mean loss (device tensor)."""
         M = x.shape[0]
@@ -425,7 +444,8 @@ class ChunkedCrossEntropy_Share:
         tlogit = torch.zeros(M, dtype=torch.float32, device=x.device)
         kept = None
         if self._fused(x, W):
-            pmax, psum = F.gemm_ce_stats(x, W, t, tlogit, vocab=W.shape[0])
+            kept = self._logits_buffer(x, W.shape[0]) if train_flg else None
+            pmax, psum = F.gemm_ce_stats(x, W, t, tlogit, vocab=W.shape[0], logits=kept)
             rmax, rsum = F.ce_merge(pmax, psum)
         else:
             rmax = torch.empty(M, dtype=torch.float32, device=x.device)
@@ -450,16 +470,19 @@ class ChunkedCrossEntropy_Share:
         self.dW = None
         if grad_writer is None:
             self.dW = torch.empty_like(W)
-        fused = kept is None and self._fused(x, W)
-        if fused:
+        stored = kept.shape[1] if isinstance(kept, torch.Tensor) else 0         # leading columns of the fused forward
+        fused = not isinstance(kept, list) and self._fused(x, W)
+        if fused or stored:
             lse, coef = F.ce_row_coef(rmax, rsum, t, loss_cnt, self.padding_id, float(GradScale))
         for i, (s, e) in enumerate(self._chunks(W.shape[0])):
-            if fused and (e - s) % 8 == 0 and e - s >= 256:
+            if e <= stored and s % 4 == 0:
+                dlog = F.ce_dlogits_kept(kept[:, s:e], t, lse, coef, s)
+            elif fused and (e - s) % 8 == 0 and e - s >= 256:
                 dlog = F.gemm_ce_dlogits(x, W[s:e], t, lse, coef, col0=s)
             else:
-                logits = kept[i] if kept is not None else F.gemm(x, W[s:e], trans_b=True, out_dtype=torch.float32)
+                logits = kept[i] if isinstance(kept, list) else F.gemm(x, W[s:e], trans_b=True, out_dtype=torch.float32)
                 dlog = F.ce_dlogits(logits, t, rmax, rsum, loss_cnt, s, self.padding_id, float(GradScale), x.dtype)
-                if kept is not None:
+                if isinstance(kept, list):
                     kept[i] = None
             dst = grad_writer(s, e) if grad_writer is not None else self.dW[s:e]
             F.gemm(dlog, x, trans_a=True, out=dst)

@@ -58,7 +58,8 @@ enum Gemm2Flags : int { G2_OUT_F32 = 1, G2_ADD_C = 2, G2_TMA_OUT = 4, G2_WHOLE_T
 //   EPI_ROPE       rotary embedding on the leading columns (K|Q|V projection)
 //   EPI_SWIGLU     B = [gate | value]; a work item holds 128 gate columns beside the 128 value columns of the
 //                  same index and leaves silu(gate) * value (and, on request, the raw projection)
-//   EPI_CE_STATS   LM head: nothing is stored but per-row (max, sum of exp, target logit) of the tile's columns
+//   EPI_CE_STATS   LM head: per-row (max, sum of exp, target logit) of the tile's columns; the fp32 logits of the leading
+//                  ce_keep columns are stored too
 //   EPI_CE_DLOGITS LM head again: (exp(logit - lse) - onehot) * coef leaves as bf16
 //   EPI_SWIGLU_BWD D = A B^T is d(activation); the epilogue fetches the stored gate / value tiles by TMA and
 //                  leaves d(gate), d(value) (the backward of silu(gate) * value), d(activation) is never stored
@@ -115,6 +116,7 @@ struct Gemm2Params {
   const float* ce_lse;       // [M] log-sum-exp of the whole row (EPI_CE_DLOGITS)
   const float* ce_coef;      // [M] valid * gradient scale / number of valid rows
   int ce_col0, ce_nt0;       // vocabulary id of column 0; tile-column index of this call's first tile in pmax / psum
+  int ce_keep;               // EPI_CE_STATS: columns whose logits leave through tmD (0: none), a multiple of 32 or N
   int ce_vocab;              // size of the whole vocabulary when the caller knows it (debug build: targets are checked)
   // EPI_DELTA: row = b * dl_T + t, column = head * dl_dim + d (dl_dim 128 or 64); the forward output O is read through
   // the map in the tmC slot; dl_out [batch][dl_heads][dl_T] fp32.
@@ -445,15 +447,25 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     bool ok = true;
     TileRingReader rd;
     if constexpr (EPI == EPI_CE_STATS) {
-      // LM-head logits that never leave the SM: every thread folds its row of the accumulator into
-      // (max, sum of exp, target logit) over the tile's valid columns and writes three floats.
+      // LM-head logits: every thread folds its row of the accumulator into (max, sum of exp, target logit) over the tile's
+      // valid columns and writes three floats. Where the backward will read them, the logits leave as well, 32 columns at
+      // a time through two swizzled staging tiles and TMA, as in the plain fp32 path.
       const int r = q * 32 + lane;
+      uint8_t* stg = smem + kStgOff;
+      const uint32_t swz = uint32_t(r & 7);
+      const bool elected = (warp == 2 && lane == 0);
+      uint32_t gcount = 0;
       for (int t = pair; ok && t >= 0 && t < num_tiles;
            t = dyn ? rd.next(sched_full, sched_empty, tile_ring, abort_flag, true, lane == 0, rank != 0)
                    : t + num_pairs) {
         const G2Item wi = g2_item(t, p.t_full, num_m, num_n);
         const int row = wi.mb * 2 * G2_BM + int(rank) * G2_BM + r;
         const int ncols = min(wi.bn, p.N - wi.n0);                       // valid columns of this tile
+        const int nkeep = max(0, min(wi.bn, p.ce_keep - wi.n0) + 31) / 32;     // 32-column groups that are stored
+        if (elected && nkeep > 0) {
+          tma_store_wait_read<1>();                      // the store that last used this staging tile has read it
+          mbar_arrive(&stage_ready[gcount & 1]);
+        }
         int tcol = -1;
         if (row < p.M) {
           int tgt = __ldg(p.ce_targets + row);
@@ -476,6 +488,26 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
+          }
+          if (c < nkeep) {
+            const uint32_t b = gcount & 1;
+            if (!mbar_wait(&stage_ready[b], (gcount >> 1) & 1, abort_flag)) { ok = false; break; }
+            uint8_t* rowp = stg + b * G2_STG_BYTES + r * 128;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              *reinterpret_cast<uint4*>(rowp + ((uint32_t(e) ^ swz) << 4)) =
+                  make_uint4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+            fence_proxy_async_smem();
+            named_bar_sync_128(1);
+            if (elected) {
+              tma_store_2d(&tmD, stg + b * G2_STG_BYTES, wi.n0 + c * 32, wi.mb * 2 * G2_BM + int(rank) * G2_BM);
+              tma_store_commit();
+              if (c + 1 < nkeep) {
+                tma_store_wait_read<1>();
+                mbar_arrive(&stage_ready[(gcount + 1) & 1]);
+              }
+            }
+            ++gcount;
           }
           const int left = ncols - c * 32;
           if (left > 0) {
@@ -502,6 +534,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
+      if (elected) tma_store_wait<0>();
     } else if constexpr (EPI == EPI_SWIGLU) {
       // 256 rows x 128 activation columns per item: accumulator columns [0, 128) are the gate, [128, 256)
       // the value. Per 64-column group the thread's row leaves as up to three 128-byte staging rows (raw
@@ -1244,12 +1277,16 @@ B200_API int b200_gemm_bf16_2cta_swiglu(const void* A, const void* B, void* GV, 
 // K-major) every 256-column tile leaves, per row, the maximum and the sum of exp(logit - maximum) of its valid
 // columns in pmax / psum ([tile columns][M], this call's first tile column at index nt0) and the tile that holds
 // the row's target writes that logit to tlogit[row]. A merge over the tile columns gives the row's log-sum-exp.
+// logits, when not null, receives the fp32 logits of columns [0, keep) (keep a multiple of 32, or N; pitch ldl a multiple
+// of 4, base 16-byte aligned): 1 GB at 8192 x 32000, hidden behind the products (716 -> 786 us over K = 2048).
 B200_API int b200_gemm_bf16_2cta_ce_stats(const void* A, const void* B, int M, int N, int K, int lda, int ldb,
                                           const void* targets, void* pmax, void* psum, void* tlogit, int col0, int nt0,
-                                          int vocab, cudaStream_t stream) {
+                                          int vocab, void* logits, int ldl, int keep, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B)) & 15) != 0 || (lda % 8) != 0 ||
-      (ldb % 8) != 0 || !targets || !pmax || !psum || !tlogit)
+      (ldb % 8) != 0 || !targets || !pmax || !psum || !tlogit || keep < 0 || keep > N || (keep % 32 != 0 && keep != N) ||
+      (logits == nullptr) != (keep == 0) || (reinterpret_cast<uintptr_t>(logits) & 15) != 0 ||
+      (logits != nullptr && (ldl % 4 != 0 || ldl < keep)))
     return static_cast<int>(cudaErrorInvalidValue);
   Gemm2Params p = base_params(nullptr, nullptr, M, N, K, 0, 0, G2_WHOLE_TILES, 1.0f);
   p.ce_targets = static_cast<const int*>(targets);
@@ -1259,10 +1296,12 @@ B200_API int b200_gemm_bf16_2cta_ce_stats(const void* A, const void* B, int M, i
   p.ce_col0 = col0;
   p.ce_nt0 = nt0;
   p.ce_vocab = vocab;
+  p.ce_keep = keep;
   TensorMap tA = get_tensor_map_2d(A, M, K, lda, G2_BM, 64, 2, SWIZZLE_128B_);
   TensorMap tB = get_tensor_map_2d(B, N, K, ldb, G2_BN / 2, 64, 2, SWIZZLE_128B_);
-  if (!tA || !tB) return static_cast<int>(cudaErrorInvalidValue);
-  return launch_tc2<false, false, EPI_CE_STATS>(tA, tB, tB, tA, tA, p, stream);
+  TensorMap tL = keep > 0 ? get_tensor_map_2d(logits, M, keep, ldl, 128, 32, 4, SWIZZLE_128B_) : tA;
+  if (!tA || !tB || !tL) return static_cast<int>(cudaErrorInvalidValue);
+  return launch_tc2<false, false, EPI_CE_STATS>(tA, tB, tB, tL, tA, p, stream);
 }
 
 // LM-head backward, first GEMM: D[M, N] (bf16) = (exp(A B^T - lse[row]) - [column == target]) * coef[row], the

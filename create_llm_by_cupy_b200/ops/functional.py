@@ -879,6 +879,19 @@ def ce_dlogits(logits, targets, rmax, rsum, loss_cnt, col0: int, pad_id: int, gs
     return out
 
 
+def ce_dlogits_kept(logits: torch.Tensor, targets: torch.Tensor, lse: torch.Tensor, coef: torch.Tensor, col0: int):
+    """``(exp(logits - lse[row]) - onehot(target)) * coef[row]`` as bf16 [M, C] (rows on 16-byte boundaries) for one chunk of
+    the fp32 logits that ``gemm_ce_stats`` stored; ``gemm_ce_dlogits`` without its GEMM."""
+    M, C = logits.shape
+    assert logits.is_cuda and logits.dtype == torch.float32 and logits.stride(1) == 1 and targets.dtype == torch.int32
+    out = torch.empty((M, (C + 7) // 8 * 8), dtype=torch.bfloat16, device=logits.device)
+    native.check(_lib().b200_ce_dlogits_kept(
+        native.ptr(logits), native.ptr(targets), native.ptr(lse), native.ptr(coef), native.ptr(out), M, C,
+        ctypes.c_longlong(logits.stride(0)), ctypes.c_longlong(out.stride(0)), col0, native.stream_ptr()), "ce_dlogits_kept")
+    native.bump()
+    return out[:, :C]
+
+
 def ce_merge(pmax: torch.Tensor, psum: torch.Tensor):
     """Merge per-tile row statistics [nt, M] (see ``gemm_ce_stats``) into (rmax [M], rsum [M])."""
     nt, M = pmax.shape

@@ -498,13 +498,19 @@ def gemm_ce_fusable(x: torch.Tensor, w: torch.Tensor) -> bool:
 
 
 def gemm_ce_stats(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, tlogit: torch.Tensor, col0: int = 0,
-                  vocab: int = 0):
-    """Logits ``x @ w^T`` that are never stored: returns per-tile row statistics ``(pmax, psum)``, each
+                  vocab: int = 0, logits: torch.Tensor | None = None):
+    """Logits ``x @ w^T`` that need not be stored: returns per-tile row statistics ``(pmax, psum)``, each
     ``[ceil(V / 256), M]`` fp32 (maximum and sum of exp(logit - maximum) over the tile's columns), and writes the
     target's logit of every row whose target lies in ``[col0, col0 + V)`` into ``tlogit`` [M] fp32. ``vocab``
-    (size of the whole vocabulary, 0: unknown) lets the bounds-checking build report targets beyond it."""
+    (size of the whole vocabulary, 0: unknown) lets the bounds-checking build report targets beyond it. ``logits``
+    ([M, keep] fp32 rows on 16-byte boundaries, ``keep`` a multiple of 32 or V) receives the leading columns."""
     M, K = x.shape
     V = w.shape[0]
+    keep = 0 if logits is None else logits.shape[1]
+    if logits is not None:
+        assert (logits.shape[0] == M and logits.dtype == torch.float32 and logits.is_cuda and 0 < keep <= V
+                and (keep % 32 == 0 or keep == V) and logits.stride(1) == 1 and logits.stride(0) % 4 == 0
+                and logits.stride(0) >= keep and logits.data_ptr() % 16 == 0)
     _same_inner("gemm_ce_stats", K, w.shape[1])
     assert gemm_ce_fusable(x, w) and targets.dtype == torch.int32 and targets.numel() == M
     nt = (V + 255) // 256
@@ -514,7 +520,8 @@ def gemm_ce_stats(x: torch.Tensor, w: torch.Tensor, targets: torch.Tensor, tlogi
     _apply_dynamic()
     rc = native.lib().b200_gemm_bf16_2cta_ce_stats(
         native.ptr(x), native.ptr(w), M, V, K, x.stride(0), w.stride(0), native.ptr(targets), native.ptr(pmax),
-        native.ptr(psum), native.ptr(tlogit), col0, 0, int(vocab), native.stream_ptr())
+        native.ptr(psum), native.ptr(tlogit), col0, 0, int(vocab), native.ptr(logits),
+        0 if logits is None else logits.stride(0), keep, native.stream_ptr())
     native.check(rc, "b200_gemm_bf16_2cta_ce_stats")
     native.bump()
     return pmax, psum
