@@ -165,7 +165,7 @@ rmsnorm_fwd_cta_kernel(const bf16* x, const bf16* gamma, bf16* __restrict__ y,
   }
 }
 
-// Any H (used when H is not a multiple of 8).
+// Any H and any base (used when H is not a multiple of 8 or a tensor does not start on a 16-byte boundary).
 __global__ void rmsnorm_fwd_scalar_kernel(const bf16* __restrict__ x, const bf16* __restrict__ gamma,
                                           bf16* __restrict__ y, float* __restrict__ rstd, int M, int H, float eps) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -385,7 +385,7 @@ rmsnorm_bwd_cta_kernel(const bf16* dy, const bf16* x, const bf16* gamma,
   }
 }
 
-// Generic-H variant: two passes over the row, atomics for dgamma partial rows.
+// Any H and any base: two passes over the row, atomics for dgamma partial rows.
 __global__ void rmsnorm_bwd_scalar_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x,
                                           const bf16* __restrict__ gamma, const float* __restrict__ rstd,
                                           const bf16* __restrict__ add, bf16* __restrict__ dx,
@@ -621,10 +621,9 @@ __global__ void embedding_bwd_kernel(TW* __restrict__ dW, const int* __restrict_
   }
 }
 
-// out = a + b (bf16, n multiple of 8 handled vectorised; tail scalar)
+// out = a + b (bf16): `chunks` times 8 elements vectorised, the others one by one
 __global__ void add_bf16_kernel(const bf16* __restrict__ a, const bf16* __restrict__ b, bf16* __restrict__ out,
-                                size_t n) {
-  const size_t chunks = n >> 3;
+                                size_t n, size_t chunks) {
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < chunks; i += size_t(gridDim.x) * blockDim.x) {
     float x[8], y[8];
     unpack8(reinterpret_cast<const Pack8*>(a)[i], x);
@@ -633,9 +632,8 @@ __global__ void add_bf16_kernel(const bf16* __restrict__ a, const bf16* __restri
     for (int e = 0; e < 8; ++e) x[e] += y[e];
     reinterpret_cast<Pack8*>(out)[i] = pack8(x);
   }
-  if (blockIdx.x == 0)
-    for (size_t i = (chunks << 3) + threadIdx.x; i < n; i += blockDim.x)
-      out[i] = __float2bfloat16(__bfloat162float(a[i]) + __bfloat162float(b[i]));
+  for (size_t i = (chunks << 3) + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
+    out[i] = __float2bfloat16(__bfloat162float(a[i]) + __bfloat162float(b[i]));
 }
 
 // Row-major matrices whose rows do not start on 16-byte boundaries cannot be read by TMA or by 16-byte loads. This
@@ -689,6 +687,13 @@ static inline int grid_for(size_t work_items, int block) {
   return int(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
+// Every base allows 16-byte accesses (null does). Tensors come here that start anywhere, such as slices of a flat buffer;
+// those that do not go to the kernels that access element by element.
+template <typename... P>
+static inline bool on16(const P*... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0;
+}
+
 }  // namespace b200
 
 using namespace b200;
@@ -701,7 +706,7 @@ B200_API int b200_rmsnorm_fwd(const void* x, const void* gamma, void* y, void* r
   const bf16* gp = static_cast<const bf16*>(gamma);
   bf16* yp = static_cast<bf16*>(y);
   float* rp = static_cast<float*>(rstd);
-  if (H % 8 != 0) {
+  if (H % 8 != 0 || !on16(x, gamma, y)) {
     rmsnorm_fwd_scalar_kernel<<<grid, block, 0, st>>>(xp, gp, yp, rp, M, H, eps);
   } else if (H <= 256) {
     B200_CHECK(launch_pdl(rmsnorm_fwd_kernel<1>, dim3(grid), dim3(block), 0, st, 0, xp, gp, yp, rp, M, H, eps));
@@ -748,7 +753,7 @@ B200_API int b200_rmsnorm_bwd(const void* dy, const void* x, const void* gamma, 
   bf16* dxp = static_cast<bf16*>(dx);
   float* pp = static_cast<float*>(partial);
   const size_t smem = size_t(8) * H * sizeof(float);   // 8 warps per CTA in the vector kernels
-  if (H % 8 != 0 || H > 8192) {
+  if (H % 8 != 0 || H > 8192 || !on16(dy, x, gamma, add, dx, partial)) {
     B200_CHECK(cudaMemsetAsync(pp, 0, size_t(rows) * H * sizeof(float), st));
     rmsnorm_bwd_scalar_kernel<<<rows, 128, 0, st>>>(dyp, xp, gp, rp, ap, dxp, pp, M, H);
   } else if (H <= 256) {
@@ -786,7 +791,7 @@ B200_API int b200_repitch(const void* src, void* dst, int R, int nseg, int C, in
 B200_API int b200_swiglu_fwd(const void* gate_val, void* act, int M, int I, int ld, cudaStream_t st) {
   if (M <= 0 || I <= 0) return 0;
   const bf16* g = static_cast<const bf16*>(gate_val);
-  const bool vec = (I % 8 == 0) && (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(g) & 15) == 0);
+  const bool vec = (I % 8 == 0) && (ld % 8 == 0) && on16(gate_val, act);
   if (vec) swiglu_fwd_kernel<<<grid_for(size_t(M) * (I / 8), 256), 256, 0, st>>>(g, static_cast<bf16*>(act), M, I, ld);
   else swiglu_fwd_scalar_kernel<<<grid_for(size_t(M) * I, 256), 256, 0, st>>>(g, static_cast<bf16*>(act), M, I, ld);
   return static_cast<int>(cudaGetLastError());
@@ -796,8 +801,7 @@ B200_API int b200_swiglu_bwd(const void* dact, const void* gate_val, void* d_gat
                              cudaStream_t st) {
   if (M <= 0 || I <= 0) return 0;
   const bf16* g = static_cast<const bf16*>(gate_val);
-  const bool vec = (I % 8 == 0) && (ld % 8 == 0) && ((reinterpret_cast<uintptr_t>(g) & 15) == 0) &&
-                   ((reinterpret_cast<uintptr_t>(d_gate_val) & 15) == 0);
+  const bool vec = (I % 8 == 0) && (ld % 8 == 0) && on16(dact, gate_val, d_gate_val);
   if (vec)
     swiglu_bwd_kernel<<<grid_for(size_t(M) * (I / 8), 256), 256, 0, st>>>(static_cast<const bf16*>(dact), g,
                                                                            static_cast<bf16*>(d_gate_val), M, I, ld);
@@ -819,8 +823,7 @@ B200_API int b200_rope_inplace(void* buf, const void* cs, const void* sn, int M,
                                int col0, int pos0, int inverse, cudaStream_t st) {
   const size_t total = size_t(M) * nheads * (D / 2);
   if (total == 0) return 0;
-  const bool vec = ((D / 2) % 8 == 0) && (ld % 8 == 0) && (col0 % 8 == 0) &&
-                   ((reinterpret_cast<uintptr_t>(buf) & 15) == 0);
+  const bool vec = ((D / 2) % 8 == 0) && (ld % 8 == 0) && (col0 % 8 == 0) && on16(buf, cs, sn);
   if (vec)
     rope_inplace_vec_kernel<<<grid_for(total / 8, 256), 256, 0, st>>>(
         static_cast<bf16*>(buf), static_cast<const float*>(cs), static_cast<const float*>(sn), M, T, nheads, D, ld,
@@ -836,7 +839,7 @@ B200_API int b200_rope_inplace(void* buf, const void* cs, const void* sn, int M,
 B200_API int b200_embedding_fwd(const void* W, const void* idx, void* out, int M, int H, int pad_id, int V,
                                 cudaStream_t st) {
   if (M <= 0) return 0;
-  if (H % 8 == 0)
+  if (H % 8 == 0 && on16(W, out))
     B200_CHECK(launch_pdl(embedding_fwd_kernel, dim3(grid_for(size_t(M) * (H / 8), 256)), dim3(256), 0, st, 0, 
         static_cast<const bf16*>(W), static_cast<const int*>(idx), static_cast<bf16*>(out), M, H, pad_id, V,
         status_ptr()));
@@ -847,11 +850,12 @@ B200_API int b200_embedding_fwd(const void* W, const void* idx, void* out, int M
   return static_cast<int>(cudaGetLastError());
 }
 
-// H must be even. dw_fp32 selects the dtype of dW.
+// H must be even, dout and a bf16 dW on 4-byte boundaries (pairs are added). dw_fp32 selects the dtype of dW.
 B200_API int b200_embedding_bwd(void* dW, const void* idx, const void* dout, int M, int H, int pad_id, int V,
                                 int dw_fp32, cudaStream_t st) {
   if (M <= 0) return 0;
-  if (H % 2 != 0) return static_cast<int>(cudaErrorInvalidValue);
+  if (H % 2 != 0 || ((reinterpret_cast<uintptr_t>(dW) | reinterpret_cast<uintptr_t>(dout)) & 3) != 0)
+    return static_cast<int>(cudaErrorInvalidValue);
   const int grid = grid_for(size_t(M) * (H / 2), 256);
   if (dw_fp32)
     embedding_bwd_kernel<float><<<grid, 256, 0, st>>>(static_cast<float*>(dW), static_cast<const int*>(idx),
@@ -866,9 +870,9 @@ B200_API int b200_embedding_bwd(void* dW, const void* idx, const void* dout, int
 
 B200_API int b200_add_bf16(const void* a, const void* b, void* out, long long n, cudaStream_t st) {
   if (n <= 0) return 0;
-  add_bf16_kernel<<<grid_for(size_t(n) / 8 + 1, 256), 256, 0, st>>>(static_cast<const bf16*>(a),
-                                                                    static_cast<const bf16*>(b),
-                                                                    static_cast<bf16*>(out), size_t(n));
+  const size_t chunks = on16(a, b, out) ? size_t(n) / 8 : 0;
+  add_bf16_kernel<<<grid_for(chunks > 0 ? chunks : size_t(n), 256), 256, 0, st>>>(
+      static_cast<const bf16*>(a), static_cast<const bf16*>(b), static_cast<bf16*>(out), size_t(n), chunks);
   return static_cast<int>(cudaGetLastError());
 }
 

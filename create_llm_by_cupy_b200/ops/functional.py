@@ -314,6 +314,8 @@ def embedding_bwd(dW: torch.Tensor, idx: torch.Tensor, dout: torch.Tensor, pad_i
     _bf16(dout)
     assert idx.dtype == torch.int32 and dW.is_contiguous()
     dout = dout.contiguous()
+    if dout.data_ptr() % 4:                    # the kernel adds pairs
+        dout = dout.clone()
     native.check(_lib().b200_embedding_bwd(native.ptr(dW), native.ptr(idx), native.ptr(dout), M, H, pad_id,
                                            dW.shape[0], int(dW.dtype == torch.float32), native.stream_ptr()),
                  "embedding_bwd")

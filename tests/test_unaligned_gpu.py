@@ -121,3 +121,58 @@ def test_gemm_with_one_column_in_a_transposed_view(M, K):
     want, bound = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t() * (K * 2.0 ** -23)
     for y in (G.gemm(a, w.t()), G.gemm(w.t(), a.t(), trans_a=True).t()):           # [K, 1] with strides (1, K), as B and as A
         assert ((y.double() - want).abs() <= bound + 2.0 ** -8 * want.abs()).all()
+
+
+def at(t, first):
+    """A contiguous copy of ``t`` that starts ``first`` elements behind a 16-byte boundary."""
+    return torch.cat([t.new_zeros(first), t.reshape(-1)])[first:].view(t.shape)
+
+
+# the smallest vector width, every vector kernel of the norms, and a width that none takes
+@pytest.mark.parametrize("M,H", [(1, 8), (3, 256), (5, 768), (300, 1024), (300, 2048), (33, 4096), (5, 8192), (3, 8200), (7, 771)])
+@pytest.mark.parametrize("first", [(1, 0, 0, 0), (0, 3, 0, 0), (0, 0, 2, 0), (0, 0, 0, 4), (7, 5, 6, 1)])
+def test_norm_of_misaligned_bases(M, H, first):
+    x, g, dy, add = (at(t, f) for t, f in zip((bf(M, H, seed=1), bf(H, seed=2), bf(M, H, seed=3), bf(M, H, seed=4)), first))
+    xd, gd, dyd = x.double(), g.double(), dy.double()
+    r = (xd.pow(2).mean(-1, keepdim=True) + 1e-6).rsqrt()
+    y, rstd = F.rmsnorm_fwd(x, g)
+    assert ((y.double() - xd * r * gd).abs() <= 2.0 ** -8 * (xd * r * gd).abs()).all()
+    xh, w = xd * r, dyd * gd
+    dx, dgamma = F.rmsnorm_bwd(dy, x, g, rstd, add=add)
+    want = r * (w - xh * (w * xh).mean(-1, keepdim=True)) + add.double()
+    sums = r * (w.abs() + xh.abs() * (w * xh).abs().mean(-1, keepdim=True)) + add.double().abs()
+    assert ((dx.double() - want).abs() <= 2.0 ** -8 * want.abs() + (H + 8) * 2.0 ** -23 * sums).all()
+    want, sums = (dyd * xh).sum(0), (dyd * xh).abs().sum(0)
+    assert ((dgamma.double() - want).abs() <= 2.0 ** -8 * want.abs() + (M + H) * 2.0 ** -23 * sums).all()
+
+
+@pytest.mark.parametrize("first", [0, 1, 2, 4, 7])
+def test_elementwise_of_misaligned_bases(first):
+    W, idx = bf(100, 64, seed=1), torch.tensor([0, 5, 99, 7, 5], dtype=torch.int32, device="cuda")
+    want = W[idx.long()]
+    want[0] = 0
+    assert torch.equal(F.embedding_fwd(at(W, first), idx, 0), want)
+    dW, dout = torch.zeros(100, 64, device="cuda"), bf(5, 64, seed=2)
+    F.embedding_bwd(dW, idx, at(dout, first), 0)
+    assert torch.equal(dW[99], dout[2].float()) and torch.equal(dW[5], dout[1].float() + dout[4].float()) and not dW[0].any()
+    gv, dact = bf(300, 528, seed=3), bf(300, 264, seed=4)
+    for a, b in ((first, 0), (0, first), (first, first)):
+        for got, ref in ((F.swiglu_fwd(at(gv, a)), F.swiglu_fwd(gv)), (F.swiglu_bwd(at(dact, b), at(gv, a)), F.swiglu_bwd(dact, gv))):
+            # two roundings of the same fp32 formula
+            assert ((got.double() - ref.double()).abs() <= 2.0 ** -7 * ref.double().abs() + 1e-30).all()
+        for n in (1, 8, 1027, 70000):
+            p, q = bf(n, seed=5), bf(n, seed=6)
+            out = at(torch.full((n,), 9.0, dtype=torch.bfloat16, device="cuda"), b)
+            assert torch.equal(F.add(at(p, a), at(q, b), out=out), (p.float() + q.float()).bfloat16())
+    cos, sin = F.rope_table(32, 64, 10000.0, gv.device)
+    buf = bf(30, 256, seed=7)
+    want = F.rope_inplace(buf.clone(), cos, sin, 30, 2, 64, 64).double()
+    for c, f in (((cos, sin), first), ((at(cos, first), at(sin, first)), 0)):
+        got = F.rope_inplace(at(buf, f), *c, 30, 2, 64, 64).double()
+        assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 2.0 ** -22 * buf.double().abs().max()).all()
+
+
+def test_embedding_gradient_at_an_odd_base_is_refused():
+    idx, dout = torch.tensor([1], dtype=torch.int32, device="cuda"), bf(1, 64, seed=1)
+    with pytest.raises(RuntimeError):
+        F.embedding_bwd(at(bf(4, 64, seed=2), 1), idx, dout, 0)
