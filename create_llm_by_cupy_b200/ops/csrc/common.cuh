@@ -73,8 +73,10 @@ int num_sms();
 // tail (about 2 us of every pair of dependent kernels). The two halves of the rule:
 //   * pdl_wait() returns when every kernel before this one has completed and its stores are visible. Nothing that another
 //     kernel may have written - weights included: the one before may be the optimizer - is read, and nothing is written,
-//     before it; only an L2 prefetch, which cannot go stale, may come earlier. Inputs are plain pointers, not
-//     `const __restrict__`: a load the compiler takes for invariant could be moved above the wait.
+//     before it; only an L2 prefetch, which cannot go stale, may come earlier. Inputs are read through plain
+//     pointers: no `const __restrict__`, no __ldg or __ldcs. A load that the compiler takes for invariant, or an intrinsic that
+//     is not volatile, could be moved above the wait, and the read-only path is only for data that nobody writes while the
+//     kernel is resident.
 //   * pdl_trigger() lets the next kernel start once all CTAs of this one have got there (or have ended; a kernel need not
 //     call it). It never stands before pdl_wait(), so that one kernel at most is waiting while another runs: with the
 //     trigger first, two or three kernels' CTAs piled up on the SMs that happened to be free (777 tokens through the 125M

@@ -114,15 +114,13 @@ decode_attn_kernel(const DecodeParams p) {
   const int R = p.QH / p.KVH;
   const int h0 = kvh * R + g * RT, nh = min(RT, R - g * RT);
   const int kl = lane / LPK, dl = lane % LPK;           // key slot and 8-element column of this lane
-  {
-    // the first tiles of this warp travel to L2 while the projection before this kernel runs (a length that is only
-    // being written by then costs a useless or a missing prefetch, nothing else)
-    const int ahead = min(p.lens[b], p.Tmax);
-    if (lane < 2) {
-      const bf16* rows = (lane == 0 ? p.kc : p.vc) + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
-      for (int i = 0, t = rank + warp * cs; i < DA_PREFETCH && t * DA_TILE < ahead; ++i, t += nw * cs)
-        l2_prefetch(rows + size_t(t) * DA_TILE * D, uint32_t(min(DA_TILE, ahead - t * DA_TILE)) * D * 2);
-    }
+  if (APPEND && lane < 2) {
+    // The first tiles of this warp travel to L2 while the projection before this kernel runs: keys up to the new token's,
+    // which the host knows. The lengths may only be being written, so they are not read here; a shorter one costs a
+    // useless prefetch.
+    const bf16* rows = (lane == 0 ? p.kc : p.vc) + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
+    for (int i = 0, t = rank + warp * cs; i < DA_PREFETCH && t * DA_TILE <= p.pos; ++i, t += nw * cs)
+      l2_prefetch(rows + size_t(t) * DA_TILE * D, uint32_t(min(DA_TILE, p.pos + 1 - t * DA_TILE)) * D * 2);
   }
   pdl_wait();
   const int len = min(p.lens[b], p.Tmax);

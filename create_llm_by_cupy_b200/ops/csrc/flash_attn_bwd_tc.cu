@@ -494,8 +494,8 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         for (int j = 0; j < FKV_BQ / 32; ++j) {
           const int row = m0 + lane + 32 * j;
           const size_t idx = (size_t(b) * p.QH + h) * T + min(row, T - 1);
-          lv[j] = __ldg(p.lse + idx);
-          dv[j] = __ldg(p.delta + idx);
+          lv[j] = p.lse[idx];
+          dv[j] = p.delta[idx];
         }
 #pragma unroll
         for (int j = 0; j < FKV_BQ / 32; ++j) {
@@ -913,8 +913,8 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
         for (int j = 0; j < FKW_BQ / 32; ++j) {
           const int row = m0 + lane + 32 * j;
           const size_t idx = (size_t(b) * p.QH + h) * T + min(row, T - 1);
-          lv[j] = __ldg(p.lse + idx);
-          dv[j] = __ldg(p.delta + idx);
+          lv[j] = p.lse[idx];
+          dv[j] = p.delta[idx];
         }
 #pragma unroll
         for (int j = 0; j < FKW_BQ / 32; ++j) {

@@ -18,8 +18,8 @@ namespace b200 {
 // the global stores.
 template <int kD>
 __device__ __forceinline__ void store_row_unrot_from_tmem(uint32_t taddr, bf16* grow, int j0, int nj,
-                                                          const float* __restrict__ cs_row,
-                                                          const float* __restrict__ sn_row, int ld, bool active) {
+                                                          const float* cs_row, const float* sn_row, int ld,
+                                                          bool active) {
 #pragma unroll 1
   constexpr int kHalf = kD / 2;
   for (int j = j0; j < j0 + nj; j += 16) {
@@ -34,8 +34,8 @@ __device__ __forceinline__ void store_row_unrot_from_tmem(uint32_t taddr, bf16* 
       float cc[4], ss[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        cc[e] = __ldg(cs_row + size_t(j + i + e) * ld);
-        ss[e] = __ldg(sn_row + size_t(j + i + e) * ld);
+        cc[e] = cs_row[size_t(j + i + e) * ld];
+        ss[e] = sn_row[size_t(j + i + e) * ld];
       }
       float o1[4], o2[4];
 #pragma unroll

@@ -468,7 +468,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         }
         int tcol = -1;
         if (row < p.M) {
-          int tgt = __ldg(p.ce_targets + row);
+          int tgt = p.ce_targets[row];
 #ifdef B200_BOUNDS_CHECK
           // a target beyond the vocabulary would silently count as "no target logit": the debug build reports it
           if (p.ce_vocab > 0 && tgt >= 0) tgt = checked_index(tgt, p.ce_vocab - 1, p.status, 304);
@@ -754,9 +754,9 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         int ce_t = -1;                          // target as a column of this call (vocabulary id - ce_col0)
         if constexpr (EPI == EPI_CE_DLOGITS) {
           const int row = min(row0 + r, p.M - 1);
-          ce_lse = __ldg(p.ce_lse + row);
-          ce_coef = __ldg(p.ce_coef + row);
-          ce_t = __ldg(p.ce_targets + row) - p.ce_col0;
+          ce_lse = p.ce_lse[row];
+          ce_coef = p.ce_coef[row];
+          ce_t = p.ce_targets[row] - p.ce_col0;
         }
         float dl_sum = 0.f;                     // EPI_DELTA: dO . O over the head's columns seen so far
         if (elected && g_lo < g_hi) {
@@ -813,7 +813,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
               const float sgn = (g & 1) ? 1.f : -1.f;      // first half: x1 c - x2 s; second half: x2 c + x1 s
 #pragma unroll
               for (int j = 0; j < 64; ++j) {
-                const float c = __ldg(cs_row + size_t(j) * p.rope_ld), sn = __ldg(sn_row + size_t(j) * p.rope_ld);
+                const float c = cs_row[size_t(j) * p.rope_ld], sn = sn_row[size_t(j) * p.rope_ld];
                 v[j] = __float_as_uint(fmaf(__uint_as_float(v[j]), c, sgn * __uint_as_float(w[j]) * sn));
               }
             } else {
@@ -831,7 +831,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
               if (rope_g) {                                  // 64-wide head: both halves are in this group
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
-                  const float c = __ldg(cs_row + size_t(j) * p.rope_ld), sn = __ldg(sn_row + size_t(j) * p.rope_ld);
+                  const float c = cs_row[size_t(j) * p.rope_ld], sn = sn_row[size_t(j) * p.rope_ld];
                   const float x1 = __uint_as_float(v[j]), x2 = __uint_as_float(v[j + 32]);
                   v[j] = __float_as_uint(fmaf(x1, c, -x2 * sn));
                   v[j + 32] = __float_as_uint(fmaf(x2, c, x1 * sn));

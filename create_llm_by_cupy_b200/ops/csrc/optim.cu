@@ -281,6 +281,13 @@ ce_dlogits_kernel(const float* __restrict__ logits, const int* __restrict__ targ
   }
 }
 
+// 16 bytes that are read for the last time. Volatile, unlike __ldcs: it stays behind pdl_wait().
+__device__ __forceinline__ float4 ld_once(const float* p) {
+  float4 v;
+  asm volatile("ld.global.cs.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 // (exp(logit - lse) - onehot(target)) * coef as bf16 for one chunk of kept fp32 logits: what the logit-gradient epilogue of
 // the LM-head GEMM forms from recomputed ones. Bound by memory: 8 columns per thread and step, two steps in flight; the
 // logits are read for the last time (evict first), the result stays in L2 for the two products that follow. 8192 x 8192
@@ -302,8 +309,8 @@ ce_dlogits_kept_kernel(const float* logits, const int* targets, const float* lse
   for (int u = 0; u < U; ++u) {
     const int c = c0 + u * 2048;
     if (c + 8 <= C) {
-      v[u][0] = __ldcs(reinterpret_cast<const float4*>(lr + c));
-      v[u][1] = __ldcs(reinterpret_cast<const float4*>(lr + c + 4));
+      v[u][0] = ld_once(lr + c);
+      v[u][1] = ld_once(lr + c + 4);
     }
   }
 #pragma unroll
