@@ -390,16 +390,16 @@ class TimeEmbedding_shard:
 
 
 class ChunkedCrossEntropy_Share:
-    """LM head + mean cross-entropy over non-pad targets without an ``[M, V]`` tensor
+    """LM head + mean cross-entropy over non-pad targets, chunk by chunk of the vocabulary
     (reference: model/fast_layers.py:1280-1488, which makes two chunked passes forward and one backward).
 
     On CUDA, forward: ONE GEMM over the whole vocabulary whose epilogue folds each 256-column tile of the fp32
     accumulator into per-row (max, sum-exp, target logit); a small merge gives the row's log-sum-exp. A training
-    forward also stores the fp32 logits of as many leading chunks as ``KEEP_LOGITS_BYTES`` holds (given back by the
-    backward). Backward walks the vocabulary in chunks of ``chunk_size``: the logits of a chunk - the stored ones,
-    else recomputed by a GEMM with the same in its epilogue - become ``(softmax - onehot) * GradScale / n_valid`` in
-    bf16, which feeds the two gradient GEMMs; ``dW`` rows go to ``grad_writer(row_start, row_end)`` -> destination
-    view, so they land directly in the gradient bucket.
+    forward also stores the fp32 logits of as many leading chunks as ``keep_logits_bytes`` holds (given back by the
+    backward), if the device has that much to spare. Backward walks the vocabulary in chunks of ``chunk_size``: the
+    logits of a chunk - the stored ones, else recomputed by a GEMM with the same in its epilogue - become
+    ``(softmax - onehot) * GradScale / n_valid`` in bf16, which feeds the two gradient GEMMs; ``dW`` rows go to
+    ``grad_writer(row_start, row_end)`` -> destination view, so they land directly in the gradient bucket.
 
     Where the fused GEMMs do not apply (CPU tensors, tiny shapes, ``cache_logits`` asked for explicitly) the
     chunked form with fp32 logits per chunk is used: one pass forward, logits kept for the backward only when
@@ -409,15 +409,23 @@ class ChunkedCrossEntropy_Share:
     # Storing and reading them costs the same whatever the width of x, recomputing them a product that grows with it. 8192
     # tokens, 32000 columns (1.05 GB from the forward to the backward), forward + backward of the layer with recomputed /
     # stored logits in us: width 512 1021 / 1061, 768 1396 / 1402, 1024 1626 / 1536, 2048 3060 / 2650, 4096 6040 / 4700; 1000
-    # tokens: 1024 342 / 312, 2048 512 / 431.
+    # tokens: 1024 342 / 312, 2048 512 / 431. Below KEEP_LOGITS_WORK multiply-adds a product the host bounds the layer, and
+    # the buffer costs it 10 us: 256 x 1024 x 32000 222 / 229, 500 x 1024 x 16384 152 / 165, 1000 x 1024 x 8192 119 / 130; but
+    # 300 x 1024 x 32000 243 / 228, 2000 x 1024 x 8192 153 / 138.
     KEEP_LOGITS_BYTES = 2 << 30
     KEEP_LOGITS_WIDTH = 1024
+    KEEP_LOGITS_WORK = 1 << 33
 
-    def __init__(self, padding_id: int, chunk_size: int = 8192, dtype=torch.bfloat16, cache_logits: bool = False):
+    def __init__(self, padding_id: int, chunk_size: int = 8192, dtype=torch.bfloat16, cache_logits: bool = False,
+                 keep_logits_bytes: int | None = None):
+        """``keep_logits_bytes``: limit of the stored logits, 0 for none (default: ``KEEP_LOGITS_BYTES``)."""
         self.padding_id = padding_id
         self.chunk_size = int(chunk_size)
         self.cache_logits = cache_logits
+        self.keep_logits_bytes = keep_logits_bytes
         self.cache = None
+        self._refused = None            # size of a buffer that the device had no memory for
+        self._kept_on = 0               # raw stream that the stored logits belong to
 
     def _chunks(self, V: int):
         c = self.chunk_size if self.chunk_size > 0 else V
@@ -426,16 +434,38 @@ class ChunkedCrossEntropy_Share:
     def _fused(self, x: torch.Tensor, W: torch.Tensor) -> bool:
         return bool(F.CE_EPILOGUE and not self.cache_logits and F.gemm_ce_fusable(x, W))
 
-    def _logits_buffer(self, x: torch.Tensor, V: int):
-        """[M, keep] fp32 for the leading whole chunks that fit, or None (also when the device has no memory left for it)."""
-        M, ends = x.shape[0], [e for _, e in self._chunks(V)]
-        keep = max([e for e in ends if M * e * 4 <= self.KEEP_LOGITS_BYTES and (e % 32 == 0 or e == V)], default=0)
-        if keep == 0 or x.shape[1] < self.KEEP_LOGITS_WIDTH:
+    def _logits_buffer(self, x: torch.Tensor, W: torch.Tensor):
+        """[M, keep] fp32 for the leading whole chunks that fit the limit, or None: recomputing needs no memory, so none is
+        taken where a step that ran without it could run out. Twice the buffer has to be to spare, and what the backward
+        allocates beside it (the gradient of W, W itself where it is gathered again). One that cannot be made all the
+        same, or only after the allocator has given back its cache, which waits for the device, is not asked for again.
+        None while a graph is captured: it would hold the memory for as long as it lives."""
+        (M, H), V = x.shape, W.shape[0]
+        if H < self.KEEP_LOGITS_WIDTH or M * H * V < self.KEEP_LOGITS_WORK or torch.cuda.is_current_stream_capturing():
+            return None
+        limit = self.KEEP_LOGITS_BYTES if self.keep_logits_bytes is None else int(self.keep_logits_bytes)
+        if M * V * 4 <= limit:
+            keep = V
+        else:
+            keep = max([e for _, e in self._chunks(V) if M * e * 4 <= limit and e % 32 == 0], default=0)
+        if keep == 0:
+            return None
+        size = M * ((keep + 3) // 4 * 4) * 4
+        if self._refused is not None and size >= self._refused:
+            return None
+        room, retries = F.native.memory_room(x.device)
+        if room < 2 * size + 4 * V * H + (64 << 20):
             return None
         try:
-            return torch.empty((M, (keep + 3) // 4 * 4), dtype=torch.float32, device=x.device)[:, :keep]
+            buf = torch.empty((M, (keep + 3) // 4 * 4), dtype=torch.float32, device=x.device)[:, :keep]
         except torch.OutOfMemoryError:
+            self._refused = size
             return None
+        if F.native.memory_room(x.device)[1] != retries:
+            self._refused = size
+            return None
+        self._kept_on = F.native.raw_stream()
+        return buf
 
     def forward(self, x: torch.Tensor, t: torch.Tensor, W: torch.Tensor, train_flg: bool = True) -> torch.Tensor:
         """x [M, H], t [M] int32 targets, W [V, H]. Returns the scalar mean loss (device tensor)."""
@@ -443,8 +473,10 @@ class ChunkedCrossEntropy_Share:
         t = t.reshape(-1).to(torch.int32)
         tlogit = torch.zeros(M, dtype=torch.float32, device=x.device)
         kept = None
+        if train_flg:
+            self.cache = None                   # of a forward that no backward followed
         if self._fused(x, W):
-            kept = self._logits_buffer(x, W.shape[0]) if train_flg else None
+            kept = self._logits_buffer(x, W) if train_flg else None
             pmax, psum = F.gemm_ce_stats(x, W, t, tlogit, vocab=W.shape[0], logits=kept)
             rmax, rsum = F.ce_merge(pmax, psum)
         else:
@@ -465,12 +497,24 @@ class ChunkedCrossEntropy_Share:
     def backward(self, W: torch.Tensor, GradScale: float = 1.0, grad_writer=None) -> torch.Tensor:
         """Returns dx [M, H]. ``grad_writer(s, e)`` must return the [e-s, H] view that receives
         dW[s:e] (overwritten); without it the chunks are collected in ``self.dW``."""
+        try:
+            return self._backward(W, GradScale, grad_writer)
+        except torch.OutOfMemoryError:
+            if not isinstance(self.cache[-1], torch.Tensor):
+                raise
+        # without the stored logits, from the start: every result is overwritten
+        self.cache = (*self.cache[:-1], None)
+        return self._backward(W, GradScale, grad_writer)
+
+    def _backward(self, W: torch.Tensor, GradScale: float, grad_writer) -> torch.Tensor:
         x, t, rmax, rsum, loss_cnt, kept = self.cache
         dx = None
         self.dW = None
         if grad_writer is None:
             self.dW = torch.empty_like(W)
         stored = kept.shape[1] if isinstance(kept, torch.Tensor) else 0         # leading columns of the fused forward
+        if stored and F.native.raw_stream() != self._kept_on:
+            kept.record_stream(torch.cuda.current_stream())
         fused = not isinstance(kept, list) and self._fused(x, W)
         if fused or stored:
             lse, coef = F.ce_row_coef(rmax, rsum, t, loss_cnt, self.padding_id, float(GradScale))

@@ -12,6 +12,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -438,6 +439,21 @@ PyObject* mlp_few_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END
 }
 
+// memory_room(device index, bytes of the device) -> see ``native.memory_room``
+PyObject* memory_room(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  const auto dev = static_cast<c10::DeviceIndex>(n == 2 ? PyLong_AsLong(a[0]) : -1);
+  const long long total = n == 2 ? PyLong_AsLongLong(a[1]) : 0;
+  if (PyErr_Occurred()) return nullptr;
+  const auto st = c10::cuda::CUDACachingAllocator::getDeviceStats(dev);
+  const auto all = static_cast<size_t>(c10::CachingAllocator::StatType::AGGREGATE);
+  const long long share = std::min(static_cast<long long>(c10::cuda::CUDACachingAllocator::getMemoryFraction(dev) * double(total)),
+                                   total - total / 32);
+  return Py_BuildValue("LL", std::max<long long>(share, st.reserved_bytes[all].current) - st.active_bytes[all].current,
+                       static_cast<long long>(st.num_alloc_retries));
+  END_HANDLE_TH_ERRORS
+}
+
 // bind(handle of libb200llm.so): looks the entry points up; raises when one is missing
 PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -473,9 +489,9 @@ PyObject* device_ready(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {METHOD(bind), METHOD(device_ready), METHOD(rmsnorm_fwd), METHOD(rmsnorm_bwd), METHOD(embedding_fwd),
-                         METHOD(gemm), METHOD(tma_ok), METHOD(gemm_rope), METHOD(gemm_swiglu), METHOD(flash_fwd),
-                         METHOD(split_heads), METHOD(decode_attn_block), METHOD(mlp_few_rows), {nullptr, nullptr, 0, nullptr}};
+PyMethodDef methods[] = {METHOD(bind), METHOD(device_ready), METHOD(memory_room), METHOD(rmsnorm_fwd), METHOD(rmsnorm_bwd),
+                         METHOD(embedding_fwd), METHOD(gemm), METHOD(tma_ok), METHOD(gemm_rope), METHOD(gemm_swiglu),
+                         METHOD(flash_fwd), METHOD(split_heads), METHOD(decode_attn_block), METHOD(mlp_few_rows), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_b200host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

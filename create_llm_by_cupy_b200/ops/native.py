@@ -8,6 +8,7 @@ library is only built, never loaded for execution.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 import threading
 from pathlib import Path
@@ -141,13 +142,35 @@ def raise_on_status() -> None:
                           f"token id >= vocabulary size in the embedding forward / backward)")
 
 
+@functools.lru_cache(maxsize=64)
+def _total_memory(device) -> int:
+    return torch.cuda.get_device_properties(device).total_memory
+
+
+def memory_room(device) -> tuple[int, int]:
+    """(bytes that the caching allocator can still hand out on ``device`` while it stays within the process's share and leaves
+    a thirty-second of the device to contexts and communicators; how often it has given its cache back to find memory).
+    The driver, which knows of other processes, takes 150 us and now and then 10 ms to answer; this takes 1."""
+    total = _total_memory(device)
+    if host is not None:
+        return host.memory_room(device.index, total)
+    st = torch.cuda.memory_stats_as_nested_dict(device)
+    share = min(int(torch.cuda.get_per_process_memory_fraction(device) * total), total - total // 32)
+    room = max(share, st["reserved_bytes"]["all"]["current"]) - st["active_bytes"]["all"]["current"]
+    return room, st["num_alloc_retries"]
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         raise NativeError(f"{what} failed with CUDA error {rc}")
 
 
+def raw_stream() -> int:
+    return torch._C._cuda_getCurrentRawStream(_current_index())
+
+
 def stream_ptr() -> c_void_p:
-    return c_void_p(torch._C._cuda_getCurrentRawStream(_current_index()))
+    return c_void_p(raw_stream())
 
 
 def ptr(t: torch.Tensor | None) -> c_void_p:

@@ -11,6 +11,7 @@ pytestmark = pytest.mark.gpu
 def run(x, t, W, chunk, keep, monkeypatch):
     monkeypatch.setattr(ChunkedCrossEntropy_Share, "KEEP_LOGITS_BYTES", keep)
     monkeypatch.setattr(ChunkedCrossEntropy_Share, "KEEP_LOGITS_WIDTH", 0)
+    monkeypatch.setattr(ChunkedCrossEntropy_Share, "KEEP_LOGITS_WORK", 0)
     layer = ChunkedCrossEntropy_Share(0, chunk_size=chunk)
     loss = layer.forward(x, t, W)
     stored = layer.cache[-1]
@@ -54,3 +55,137 @@ def test_chunk_of_kept_logits():
         got = F.ce_dlogits_kept(L, t, lse, coef, s).double()
         # fp32 subtraction and exponential: 2^-22 of an argument of at most 12, then bf16
         assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + (p.abs() + 2) * coef.double()[:, None] * 12 * 2.0 ** -22).all()
+
+
+M, H, V = 4096, 1024, 32000
+SIZE = M * V * 4
+
+
+@pytest.fixture
+def limited():
+    """Limits what the allocator may hold to ``limited(extra)`` bytes more than what is allocated now."""
+    total = torch.cuda.mem_get_info()[1]
+
+    def limit(extra):
+        torch.cuda.empty_cache()
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_allocated() + extra) / total)
+
+    yield limit
+    torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def retries():
+    return torch.cuda.memory_stats()["num_alloc_retries"]
+
+
+def inputs():
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, W = (torch.randn(n, H, device="cuda", generator=g).bfloat16() for n in (M, V))
+    return x, torch.randint(1, V, (M,), device="cuda", generator=g, dtype=torch.int32), W
+
+
+def step(layer, x, t, W):
+    loss = layer.forward(x, t, W)
+    kept = layer.cache[-1] is not None
+    dx = layer.backward(W)
+    return [kept, *(r.cpu() for r in (loss, dx, layer.dW))]
+
+
+def same(got, want):
+    assert abs(float(got[1] - want[1])) <= M * 2.0 ** -23 * float(want[1])
+    for a, b in zip(got[2:], want[2:]):
+        assert ((a.float() - b.float()).abs() <= 1e-30).all()
+
+
+def test_nothing_is_kept_where_memory_is_short(limited):
+    x, t, W = inputs()
+    want = step(ChunkedCrossEntropy_Share(0, keep_logits_bytes=0), x, t, W)
+    assert not want[0]
+    layer = ChunkedCrossEntropy_Share(0)
+    # enough for the step that recomputes (the gradients of x and W, one chunk of logit gradients twice), not for the logits
+    # beside it; a buffer that fits alone is no reason to take it
+    for extra in (SIZE // 2, SIZE + (100 << 20), 2 * SIZE):
+        limited(extra)
+        before = retries()
+        for _ in range(3):
+            got = step(layer, x, t, W)
+            assert not got[0]
+            same(got, want)
+            del got
+        assert retries() == before
+    limited(4 * SIZE)
+    got = step(layer, x, t, W)
+    assert got[0]
+    same(got, want)
+
+
+def test_backward_gives_the_logits_back_when_memory_runs_out(limited, monkeypatch):
+    x, t, W = inputs()
+    want = step(ChunkedCrossEntropy_Share(0, keep_logits_bytes=0), x, t, W)
+    monkeypatch.setattr(F.native, "memory_room", lambda device: (1 << 60, retries()))
+    used, kernel = [], F.ce_dlogits_kept
+    monkeypatch.setattr(F, "ce_dlogits_kept", lambda *a: (used.append(1), kernel(*a))[1])
+    # MiB beside the logits: not enough for the gradient of W (62), then for that but not for a chunk (64) as well, then for all
+    for extra, chunks in ((32, (0, 0)), (80, (0, 1)), (140, (0, 4)), (170, (0, 4)), (300, (4, 4))):
+        limited(SIZE + (extra << 20))
+        layer = ChunkedCrossEntropy_Share(0)
+        del used[:]
+        got = step(layer, x, t, W)
+        assert got[0] and layer.cache is None and chunks[0] <= len(used) <= chunks[1]
+        same(got, want)
+        del got, layer
+
+
+def test_a_buffer_that_cost_the_cache_is_not_asked_for_again(limited, monkeypatch):
+    x, t, W = inputs()
+    layer = ChunkedCrossEntropy_Share(0)
+    monkeypatch.setattr(F.native, "memory_room", lambda device: (1 << 60, retries()))
+    limited(SIZE + (300 << 20))
+    cached = [torch.empty(n << 20, dtype=torch.uint8, device="cuda") for n in (250, 250)]      # in pieces that are too small
+    del cached
+    assert not step(layer, x, t, W)[0] and layer._refused == SIZE
+    before = retries()
+    assert not step(layer, x, t, W)[0] and retries() == before
+    limited(SIZE // 2)
+    refused = ChunkedCrossEntropy_Share(0)
+    assert not step(refused, x, t, W)[0] and refused._refused == SIZE
+
+
+def test_room_by_either_path(monkeypatch):
+    keep = torch.empty(100 << 20, dtype=torch.uint8, device="cuda")
+    F.native.status_tensor()
+    got = F.native.memory_room(keep.device)
+    monkeypatch.setattr(F.native, "host", None)
+    assert got == F.native.memory_room(keep.device)
+    assert got[0] <= torch.cuda.mem_get_info()[1] - torch.cuda.memory_allocated()
+
+
+def test_two_forwards_hold_one_buffer_and_an_evaluation_none():
+    x, t, W = inputs()
+    layer = ChunkedCrossEntropy_Share(0)
+    layer.forward(x, t, W)
+    one = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    layer.forward(x, t, W)
+    assert torch.cuda.memory_allocated() <= one + (1 << 20) and torch.cuda.max_memory_allocated() <= one + (64 << 20)
+    ChunkedCrossEntropy_Share(0).forward(x, t, W, train_flg=False)
+    assert torch.cuda.memory_allocated() <= one + (1 << 20)
+
+
+def test_nothing_is_kept_in_a_captured_step():
+    x, t, W = inputs()
+    layer = ChunkedCrossEntropy_Share(0)
+    want = step(layer, x, t, W)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step(layer, x, t, W)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        loss = layer.forward(x, t, W)
+        kept = layer.cache[-1]
+        dx = layer.backward(W)
+    assert want[0] and kept is None
+    g.replay()
+    same([False, loss.cpu(), dx.cpu(), layer.dW.cpu()], want)
