@@ -104,13 +104,16 @@ PyObject* wrap2(const OptTensor& a, const OptTensor& b) {
   }
   return r;
 }
+// After an error the general path makes the call again and raises. Of a call of several kernels the first ones may have
+// been launched by then; made again they write the same: scratch, fresh outputs, the cache row of the new token. An output
+// that is also the addend is written by the last kernel only.
 template <class F>
 bool launched(F call) {
   int rc;
   Py_BEGIN_ALLOW_THREADS
   rc = call();
   Py_END_ALLOW_THREADS
-  return rc == 0;                              // an error launched nothing; the general path makes it again and raises
+  return rc == 0;
 }
 // Numbers of another type than int (or float) set an error, which CHECK_NUMBERS turns into the general path.
 int as_int(PyObject* o) {

@@ -90,7 +90,8 @@ __device__ __forceinline__ void l2_prefetch(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(bytes) : "memory");
 }
 
-// cluster_x > 0: thread-block clusters of that many CTAs along x (0: none, or fixed by the kernel).
+// cluster_x > 0: thread-block clusters of that many CTAs along x (0: none, or fixed by the kernel). An error is the caller's
+// alone: it does not stay behind for the next one that asks cudaGetLastError.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster_x,
                               Args&&... args) {
@@ -111,7 +112,9 @@ inline cudaError_t launch_pdl(void (*kern)(Params...), dim3 grid, dim3 block, si
     at[1].val.clusterDim.z = 1;
     cfg.numAttrs = 2;
   }
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 // A length or index that a kernel reads from device memory (valid key lengths, target ids) and then uses to bound
