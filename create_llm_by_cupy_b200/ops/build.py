@@ -4,7 +4,8 @@ The library exposes a plain ``extern "C"`` surface that is loaded with ctypes, s
 neither the torch headers nor a Python ABI: a full rebuild is a few nvcc invocations run in
 parallel. nvcc cross-compiles, so the build also runs on a machine without a GPU. Beside it stands ``_b200host.so``, a
 small CPython extension (``chost/host_ops.cpp``, against torch's headers) that issues the operators of short passes; it
-takes the kernels from whichever variant of the library is loaded.
+takes the kernels from whichever variant of the library is loaded. Where it cannot be built (no Python headers, another
+compiler) the operators are issued from Python, which launches the same kernels.
 
     python -m create_llm_by_cupy_b200.ops.build [--force] [--verbose]
 """
@@ -15,6 +16,7 @@ import os
 import shutil
 import subprocess
 import sys
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -40,6 +42,7 @@ OBJ_DIR_NAME = "build_dbg" if BOUNDS_CHECK else "build"
 HOST_SRC = OUT_DIR / "chost" / "host_ops.cpp"
 HOST_LIB = OUT_DIR / "_b200host.so"
 HOST_STAMP = OUT_DIR / "build" / "host_ops.sha1"
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
 
 
 def flags_for(src: Path) -> list[str]:
@@ -78,15 +81,19 @@ def _host_command() -> list[str]:
     import torch
     inc = Path(torch.__file__).parent / "include"
     cuda = Path(_nvcc()).resolve().parent.parent / "include"
-    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+    return [shutil.which("g++") or "g++", *HOST_FLAGS,
             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", "-I", sysconfig.get_paths()["include"],
             "-I", str(cuda), "-isystem", str(inc), "-isystem", str(inc / "torch" / "csrc" / "api" / "include"), str(HOST_SRC),
             "-L", str(inc.parent / "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
 
 
 def _host_digest() -> str:
+    """What the extension depends on, without what only its build needs."""
+    import sysconfig
+
     import torch
-    return hashlib.sha1(HOST_SRC.read_bytes() + f"{torch.__version__} {sys.version_info[:2]}".encode()).hexdigest()
+    on = [*HOST_FLAGS, torch.__version__, torch.compiled_with_cxx11_abi(), sysconfig.get_config_var("SOABI")]
+    return hashlib.sha1(HOST_SRC.read_bytes() + " ".join(map(str, on)).encode()).hexdigest()
 
 
 def lib_path() -> Path:
@@ -102,13 +109,14 @@ def source_digest() -> str:
     return h.hexdigest()
 
 
-def _host_current() -> bool:
+def host_current() -> bool:
+    """True when the extension exists and was made from its source as it is now, for this Python and torch."""
     return HOST_LIB.exists() and HOST_STAMP.exists() and HOST_STAMP.read_text() == _host_digest()
 
 
 def is_current() -> bool:
-    """True when the libraries exist and every object's stamp matches its source as it is now."""
-    if not lib_path().exists() or not _host_current():
+    """True when the library exists and every object's stamp matches its source as it is now."""
+    if not lib_path().exists():
         return False
     obj_dir = OUT_DIR / OBJ_DIR_NAME
     for src in sources():
@@ -119,29 +127,42 @@ def is_current() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile every source under ``csrc/`` that changed and link ``libb200llm.so``. Processes that
-    build at the same time (one per GPU at start-up) take turns on a lock file; the second one then finds
+    """Compile every source under ``csrc/`` that changed and link ``libb200llm.so``, and the extension beside it. Processes
+    that build at the same time (one per GPU at start-up) take turns on a lock file; the second one then finds
     everything up to date."""
     nvcc = _nvcc()
     obj_dir = OUT_DIR / OBJ_DIR_NAME
     import fcntl
-    for d in {obj_dir, HOST_STAMP.parent}:
-        d.mkdir(exist_ok=True)
-    with open(HOST_STAMP.parent / ".host.lock", "w") as lock:
-        fcntl.flock(lock, fcntl.LOCK_EX)
-        if force or not _host_current():
-            tmp = HOST_LIB.with_suffix(".so.tmp")
-            r = subprocess.run(_host_command() + ["-o", str(tmp)], capture_output=True, text=True)
-            if r.returncode != 0:
-                raise RuntimeError(f"g++ failed for {HOST_SRC.name}:\n{r.stdout}\n{r.stderr}")
-            os.replace(tmp, HOST_LIB)
-            HOST_STAMP.write_text(_host_digest())
+    obj_dir.mkdir(exist_ok=True)
+    _build_host(force)
     with open(obj_dir / ".lock", "w") as lock:
         fcntl.flock(lock, fcntl.LOCK_EX)
         try:
             return _build_locked(nvcc, obj_dir, force, verbose)
         finally:
             fcntl.flock(lock, fcntl.LOCK_UN)
+
+
+def _build_host(force: bool) -> None:
+    import fcntl
+    HOST_STAMP.parent.mkdir(exist_ok=True)
+    with open(HOST_STAMP.parent / ".host.lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if not force and host_current():
+            return
+        tmp = HOST_LIB.with_suffix(".so.tmp")
+        try:
+            r = subprocess.run(_host_command() + ["-o", str(tmp)], capture_output=True, text=True)
+            failed = r.returncode != 0 and (r.stdout + r.stderr)[-2000:]
+        except OSError as e:
+            failed = str(e)
+        if failed is not False:
+            HOST_STAMP.unlink(missing_ok=True)
+            warnings.warn(f"{HOST_LIB.name} was not built; operators are issued from Python instead (slower, the same kernels):\n"
+                          f"{failed}", RuntimeWarning)
+            return
+        os.replace(tmp, HOST_LIB)
+        HOST_STAMP.write_text(_host_digest())
 
 
 def _build_locked(nvcc: str, obj_dir: Path, force: bool, verbose: bool) -> Path:

@@ -11,6 +11,7 @@ import ctypes
 import functools
 import os
 import threading
+import warnings
 from pathlib import Path
 
 import torch
@@ -20,8 +21,8 @@ from . import build as _build
 _lock = threading.Lock()
 _lib = None
 _status = {}
-# ``_b200host`` (chost/host_ops.cpp) once a device's status block is registered, so never on a machine without a GPU. Its
-# functions take plain CUDA tensors and return None for anything else; the front ends then go on as without it.
+# ``_b200host`` (chost/host_ops.cpp) once a device's status block is registered, so never on a machine without a GPU, and
+# None throughout where it could not be built or loaded. Its functions take plain CUDA tensors and return None for anything else; the front ends then go on as without it.
 host = None
 
 c_void_p = ctypes.c_void_p
@@ -69,6 +70,9 @@ def lib() -> ctypes.CDLL:
         except RuntimeError as e:
             if "nvcc not found" not in str(e):
                 raise NativeError(str(e)) from e
+            if not _build.host_current():
+                warnings.warn(f"{_build.HOST_LIB} is missing or older than its source; operators are issued from Python "
+                              f"instead (slower, the same kernels)", RuntimeWarning)
             if not _build.is_current():
                 raise NativeError(f"{path} is missing or older than the sources under csrc/ and nvcc is not "
                                   f"available to rebuild it") from e
@@ -81,13 +85,17 @@ def lib() -> ctypes.CDLL:
 
 
 def _load_host():
+    """The extension, or None with a warning: the front ends then issue every operator from Python."""
     import importlib.util
+    if not _build.host_current():
+        return None                       # the build has said why
     spec = importlib.util.spec_from_file_location("_b200host", _build.HOST_LIB)
     try:
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
     except ImportError as e:
-        raise NativeError(f"cannot load {_build.HOST_LIB}: {e}") from e
+        warnings.warn(f"cannot load {_build.HOST_LIB}, operators are issued from Python instead: {e}", RuntimeWarning)
+        return None
     mod.bind(lib()._handle)
     return mod
 
@@ -120,8 +128,9 @@ def status_tensor(device=None) -> torch.Tensor:
         _status[key] = t
         check(lib().b200_set_status_ptr(c_void_p(t.data_ptr())), "b200_set_status_ptr")
         mod = host or _load_host()
-        mod.device_ready(key)
-        host = mod
+        if mod is not None:
+            mod.device_ready(key)
+            host = mod
     return _status[key]
 
 
