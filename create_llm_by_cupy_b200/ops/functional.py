@@ -139,7 +139,7 @@ def rmsnorm_fwd(x: torch.Tensor, gamma: torch.Tensor, eps: float = 1e-6, keep_rs
         y = (xf * rstd[:, None] * gamma.float()).to(x.dtype)
         return y.view(x.shape), rstd
     _bf16(x, gamma)
-    x2 = x2.contiguous()
+    x2, gamma = x2.contiguous(), gamma.contiguous()
     y = torch.empty_like(x2)
     rstd = torch.empty(M, dtype=torch.float32, device=x.device) if keep_rstd else None
     native.check(_lib().b200_rmsnorm_fwd(native.ptr(x2), native.ptr(gamma), native.ptr(y), native.ptr(rstd),
@@ -175,7 +175,7 @@ def rmsnorm_bwd(dy: torch.Tensor, x: torch.Tensor, gamma: torch.Tensor, rstd: to
         dgamma = (dyf * xh).sum(0)
         return dx.to(x.dtype).view(x.shape), dgamma.to(gamma.dtype)
     _bf16(dy, x, gamma, add)
-    x2 = x2.contiguous()
+    x2, gamma, rstd = x2.contiguous(), gamma.contiguous(), rstd.contiguous()
     dy2 = dy2.contiguous()
     add2 = add.reshape(-1, H).contiguous() if add is not None else None
     dx = torch.empty_like(x2)
@@ -296,6 +296,7 @@ def embedding_fwd(W: torch.Tensor, idx: torch.Tensor, pad_id: int) -> torch.Tens
         return out
     _bf16(W)
     assert idx.dtype == torch.int32 and W.is_contiguous()
+    idx = idx.contiguous()
     out = torch.empty((M, H), dtype=W.dtype, device=W.device)
     native.check(_lib().b200_embedding_fwd(native.ptr(W), native.ptr(idx), native.ptr(out), M, H, pad_id,
                                            W.shape[0], native.stream_ptr()), "embedding_fwd")
@@ -313,7 +314,7 @@ def embedding_bwd(dW: torch.Tensor, idx: torch.Tensor, dout: torch.Tensor, pad_i
         return dW
     _bf16(dout)
     assert idx.dtype == torch.int32 and dW.is_contiguous()
-    dout = dout.contiguous()
+    idx, dout = idx.contiguous(), dout.contiguous()
     if dout.data_ptr() % 4:                    # the kernel adds pairs
         dout = dout.clone()
     native.check(_lib().b200_embedding_bwd(native.ptr(dW), native.ptr(idx), native.ptr(dout), M, H, pad_id,

@@ -172,6 +172,20 @@ def test_elementwise_of_misaligned_bases(first):
         assert ((got - want).abs() <= 2.0 ** -7 * want.abs() + 2.0 ** -22 * buf.double().abs().max()).all()
 
 
+def test_strided_gains_and_ids():
+    x, g2, dy = bf(5, 768, seed=1), bf(1536, seed=2), bf(5, 768, seed=3)
+    g = g2[::2]
+    y, rstd = F.rmsnorm_fwd(x, g.clone(memory_format=torch.contiguous_format))
+    assert torch.equal(F.rmsnorm_fwd(x, g)[0], y)
+    wide = torch.stack([rstd, torch.full_like(rstd, float("nan"))], 1)
+    for a, b in zip(F.rmsnorm_bwd(dy, x, g, wide[:, 0]), F.rmsnorm_bwd(dy, x, g.clone(memory_format=torch.contiguous_format), rstd)):
+        assert torch.equal(a, b)
+    W, ids = bf(100, 64, seed=4), torch.tensor([3, 1, 4, 1, 5, 9], dtype=torch.int32, device="cuda")
+    assert torch.equal(F.embedding_fwd(W, ids[::2], -1), W[ids[::2].long()])
+    dW = F.embedding_bwd(torch.zeros(100, 64, device="cuda"), ids[::2], dy[:3, :64], -1)
+    assert torch.equal(dW[ids[::2].long()], dy[:3, :64].float())
+
+
 def test_embedding_gradient_at_an_odd_base_is_refused():
     idx, dout = torch.tensor([1], dtype=torch.int32, device="cuda"), bf(1, 64, seed=1)
     with pytest.raises(RuntimeError):
