@@ -811,8 +811,8 @@ B200_API int b200_flash_fwd(const void* q, const void* k, const void* v, void* o
                             const void* rcos, const void* rsin, const long long* strides, int B, int T, int QH,
                             int KVH, int D, float scale, cudaStream_t st) {
   if (B <= 0 || T <= 0) return 0;
-  const void* ptrs[4] = {q, k, v, o};
-  if (!strides_ok(strides, 12, ptrs, 4) || QH % KVH != 0) return static_cast<int>(cudaErrorInvalidValue);
+  const void* ptrs[6] = {q, k, v, o, rcos, rsin};
+  if (!strides_ok(strides, 12, ptrs, 6) || QH % KVH != 0) return static_cast<int>(cudaErrorInvalidValue);
   FlashParams p = {};
   p.q = static_cast<const bf16*>(q); p.k = static_cast<const bf16*>(k); p.v = static_cast<const bf16*>(v);
   p.o = static_cast<bf16*>(o); p.lse = static_cast<float*>(lse);
@@ -834,8 +834,8 @@ B200_API int b200_flash_bwd(const void* q, const void* k, const void* v, const v
                             const void* rcos, const void* rsin, const long long* strides, int B, int T, int QH,
                             int KVH, int D, float scale, cudaStream_t st) {
   if (B <= 0 || T <= 0) return 0;
-  const void* ptrs[8] = {q, k, v, o, dout, dq, dk, dv};
-  if (!strides_ok(strides, 24, ptrs, 8) || QH % KVH != 0) return static_cast<int>(cudaErrorInvalidValue);
+  const void* ptrs[10] = {q, k, v, o, dout, dq, dk, dv, rcos, rsin};
+  if (!strides_ok(strides, 24, ptrs, 10) || QH % KVH != 0) return static_cast<int>(cudaErrorInvalidValue);
   FlashParams p = {};
   p.q = static_cast<const bf16*>(q); p.k = static_cast<const bf16*>(k); p.v = static_cast<const bf16*>(v);
   p.o = const_cast<bf16*>(static_cast<const bf16*>(o)); p.dout = static_cast<const bf16*>(dout);

@@ -1227,6 +1227,9 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   if (D == 64 && ds_ws == nullptr) return static_cast<int>(cudaErrorInvalidValue);
   for (int i = 0; i < 21; ++i)
     if (s[i] % 8 != 0) return static_cast<int>(cudaErrorInvalidValue);
+  // the gradients leave in 16-byte stores (the maps below check the inputs)
+  if (((reinterpret_cast<uintptr_t>(dq) | reinterpret_cast<uintptr_t>(dk) | reinterpret_cast<uintptr_t>(dv)) & 15) != 0)
+    return static_cast<int>(cudaErrorInvalidValue);
   TensorMap tq128 = get_tensor_map_bthd(q, B, T, QH, D, s[0], s[1], s[2], 128, 64);
   TensorMap tdo128 = get_tensor_map_bthd(dout, B, T, QH, D, s[9], s[10], s[11], 128, 64);
   TensorMap tq64 = get_tensor_map_bthd(q, B, T, QH, D, s[0], s[1], s[2], 64, 64);

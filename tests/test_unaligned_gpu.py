@@ -190,3 +190,20 @@ def test_embedding_gradient_at_an_odd_base_is_refused():
     idx, dout = torch.tensor([1], dtype=torch.int32, device="cuda"), bf(1, 64, seed=1)
     with pytest.raises(RuntimeError):
         F.embedding_bwd(at(bf(4, 64, seed=2), 1), idx, dout, 0)
+
+
+@pytest.mark.parametrize("D", [32, 64, 128])
+@pytest.mark.parametrize("which", range(3))
+def test_attention_gradients_at_misaligned_bases_are_refused(D, which):
+    B, T, QH, KVH = 1, 130, 4, 2
+    q, k, v = bf(B, T, QH, D, seed=1), bf(B, T, KVH, D, seed=2), bf(B, T, KVH, D, seed=3)
+    tabs = F.rope_table(T, D, 10000.0, q.device) if D == 32 else None
+    o, lse = F.flash_attn_fwd(q, k, v, rope=tabs)
+    out = [torch.empty_like(t) for t in (q, k, v)]
+    F.flash_attn_bwd(o, q, k, v, o, lse, rope=tabs, out=out)
+    out[which] = at(out[which], 4)
+    with pytest.raises(RuntimeError):
+        F.flash_attn_bwd(o, q, k, v, o, lse, rope=tabs, out=out)
+    if D == 32:
+        with pytest.raises(RuntimeError):
+            F.flash_attn_fwd(q, k, v, rope=[at(t, int(i == which)) for i, t in enumerate(tabs)] if which < 2 else [at(t, 2) for t in tabs])
