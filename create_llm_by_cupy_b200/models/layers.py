@@ -438,10 +438,9 @@ class ChunkedCrossEntropy_Share:
         """[M, keep] fp32 for the leading whole chunks that fit the limit, or None: recomputing needs no memory, so none is
         taken where a step that ran without it could run out. Twice the buffer has to be to spare, and what the backward
         allocates beside it (the gradient of W, W itself where it is gathered again). One that cannot be made all the
-        same, or only after the allocator has given back its cache, which waits for the device, is not asked for again.
-        None while a graph is captured: it would hold the memory for as long as it lives."""
+        same, or only after the allocator has given back its cache, which waits for the device, is not asked for again."""
         (M, H), V = x.shape, W.shape[0]
-        if H < self.KEEP_LOGITS_WIDTH or M * H * V < self.KEEP_LOGITS_WORK or torch.cuda.is_current_stream_capturing():
+        if H < self.KEEP_LOGITS_WIDTH or M * H * V < self.KEEP_LOGITS_WORK:
             return None
         limit = self.KEEP_LOGITS_BYTES if self.keep_logits_bytes is None else int(self.keep_logits_bytes)
         if M * V * 4 <= limit:

@@ -172,9 +172,10 @@ def test_two_forwards_hold_one_buffer_and_an_evaluation_none():
     assert torch.cuda.memory_allocated() <= one + (1 << 20)
 
 
-def test_nothing_is_kept_in_a_captured_step():
+@pytest.mark.parametrize("limit", [None, 0])
+def test_captured_step(limit):
     x, t, W = inputs()
-    layer = ChunkedCrossEntropy_Share(0)
+    layer = ChunkedCrossEntropy_Share(0, keep_logits_bytes=limit)
     want = step(layer, x, t, W)
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
@@ -184,8 +185,11 @@ def test_nothing_is_kept_in_a_captured_step():
     g = torch.cuda.CUDAGraph()
     with torch.cuda.graph(g):
         loss = layer.forward(x, t, W)
-        kept = layer.cache[-1]
+        kept = layer.cache[-1] is not None
         dx = layer.backward(W)
-    assert want[0] and kept is None
-    g.replay()
-    same([False, loss.cpu(), dx.cpu(), layer.dW.cpu()], want)
+    assert kept == want[0] == (limit is None)
+    for _ in range(2):
+        dx.fill_(float("nan"))
+        layer.dW.fill_(float("nan"))
+        g.replay()
+        same([kept, loss.cpu(), dx.cpu(), layer.dW.cpu()], want)
