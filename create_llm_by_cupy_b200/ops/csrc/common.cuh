@@ -78,7 +78,7 @@ int num_sms();
 //     is not volatile, could be moved above the wait, and the read-only path is only for data that nobody writes while the
 //     kernel is resident.
 //   * pdl_trigger() lets the next kernel start once all CTAs of this one have got there (or have ended; a kernel need not
-//     call it). It never stands before pdl_wait(), so that one kernel at most is waiting while another runs: with the
+//     call it); the first thread of a CTA that gets there counts for the CTA. It never stands before pdl_wait(), so that one kernel at most is waiting while another runs: with the
 //     trigger first, two or three kernels' CTAs piled up on the SMs that happened to be free (777 tokens through the 125M
 //     model: 1152 us without all this, 1049 with the trigger first, 979 like this; one token 520 / 386 / 372).
 // A kernel that waits for another GPU neither triggers nor is launched this way.

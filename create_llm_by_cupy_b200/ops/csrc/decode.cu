@@ -246,7 +246,9 @@ decode_attn_kernel(const DecodeParams p) {
     __syncwarp();                                       // the next tile overwrites s_p
   }
 
-  pdl_trigger();        // here, not at the top: CTAs that arrive while these fill the SMs land unevenly (see gemm_skinny.cu)
+  // Here, not at the top: CTAs that arrive while these fill the SMs land unevenly (see gemm_skinny.cu). The first warp of a
+  // CTA to get here counts, which may be one without a tile.
+  pdl_trigger();
   // over the key slots of the warp, then the warps of the CTA
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);

@@ -74,11 +74,13 @@ enum Gemm2Epi : int {
 };
 
 // Warpgroups of the epilogue. Those that fetch the tiles of an addend or rotate have two, each with half of a tile's
-// columns and two staging tiles of its own, so that no group waits for a round trip of the one before (us, before / now): residual added 8192 x 768 x 768
-// 19.5 / 17.1, 777 x 768 x 768 11.4 / 10.0, delta 8192 x 768 x 768 20.9 / 16.8, 2048 x 1024 x 1024 14.3 / 12.3 (8192 x 2048
-// x 2048 55.7 / 56.9, the ring's missing stage), rotation 8192 x 1280 x 768 24.4 / 21.1, 777 rows 12.4 / 10.6.
-// The SwiGLU forms stay with one: beside their 90 to 360 MB of tiles the operands' way through L2 is what bounds them
-// (backward 8192 x 5504 x 2048 165 us, 176 with two).
+// columns and two staging tiles of its own, so that no group waits for a round trip of the one before. us with one (and the
+// sixth stage of the operand ring) / two: residual added 8192 x 768 x 768 19.5 / 17.1, 777 x 768 x 768 11.4 / 10.0; delta 8192
+// x 768 x 768 18.1 / 15.8, 8192 x 2048 over K = 1024 41.2 / 32.9, 1536 46.9 / 45.4, 2048 56.4 / 56.8, 4096 x 4096 x 4096 103.3 /
+// 103.4; rotation 8192 x 1280 x 768 23.7 / 21.1, 8192 x 3072 x 2048 83.6 / 81.1, 4096 x 6144 x 4096 154.6 / 152.2, but 4096 x
+// 3072 x 2048 45.1 / 46.3 and 1000 x 6144 x 4096 49.5 / 51.3: over a long K the missing stage and the epilogue weigh the same.
+// The SwiGLU forms stay with one (backward 8192 x 5504 x 2048 165 us, 176 with two; forward 256 / 263): their epilogue is not
+// what the tensor pipe waits for.
 constexpr int g2_wgs(int epi) { return epi == EPI_ROPE || epi == EPI_DELTA || epi == EPI_ADD ? 2 : 1; }
 // Four staging tiles in place of two cost a stage of the operand ring (5 x 32 KiB + 4 x 16 KiB in place of 6 + 2).
 constexpr int g2_staging(int epi) { return g2_wgs(epi) == 2 || epi == EPI_SWIGLU_BWD ? 4 : 2; }
@@ -979,7 +981,9 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
   tc_fence_before();
   // Not at the top: waiting CTAs would hold SMs that the weight gradients of the other stream can use (125M training pass
-  // 8050 us with the trigger at the top, 8012 here).
+  // 8050 us with the trigger at the top, 8012 here). Each role gets here by itself and the first one counts: in the leader
+  // the producer, once its last load is issued, in the follower the MMA warp, which has nothing to do there. So the next
+  // kernel is let in when every leader's operands are on their way, not when its stores are.
   pdl_trigger();
   __syncthreads();
   cluster_sync_all();            // the leader's MMAs read the follower's shared memory until here
@@ -1028,8 +1032,9 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
   int halved = 0;
   if (g_half_tiles && (EPI <= EPI_ROPE || EPI == EPI_DELTA || EPI == EPI_ADD) && !(p.flags & G2_WHOLE_TILES)) {
     const int rem = whole % all_pairs;
-    // The only round counts too, unless it is a weight gradient (A_MN), whose idle pairs the main stream's kernels use (125M
-    // training pass 7810 us, 8014 with halves there). 777 rows, us whole / halves: 768 x 768 10.0 / 8.8, 768 x 2048 15.9 /
+    // The only round counts too, unless it is a weight gradient, whose idle pairs the main stream's kernels use (125M
+    // training pass 7810 us, 8014 with halves there). A_MN stands for that: x^T dy is where a transposed A comes from, and one
+    // that is issued alone runs on whole tiles as well. 777 rows, us whole / halves: 768 x 768 10.0 / 8.8, 768 x 2048 15.9 /
     // 14.9, 1280 x 768 10.1 / 9.0; 2048 x 1024 x 2736 20.7 / 20.0.
     if (2 * rem <= all_pairs && (whole > all_pairs || !A_MN)) halved = rem;
   }
