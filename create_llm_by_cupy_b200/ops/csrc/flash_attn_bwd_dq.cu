@@ -114,52 +114,50 @@ flash_bwd_dq_gemm_kernel(const __grid_constant__ CUtensorMap tmDS, const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // A = dS^T [64 keys (k) x 128 queries (m)], B = K [64 keys (k) x 128 d (n)]: both MN-major, 64-element
-      // chunks of the contiguous dimension one box (8 KiB) apart, 16 key rows per k-step (2 KiB)
-      constexpr uint32_t idesc = umma_idesc_bf16(128, kD, 1, 1);
-      bool ok = true;
-      for (int j = 0; j < n_tiles && ok; ++j) {
-        const int s = j % DQG_STAGES;
-        if (!mbar_wait(&full[s], (j / DQG_STAGES) & 1, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t aA = smem_u32(smem + s * DQG_STAGE_BYTES), aK = aA + DQG_TILE;
+    // A = dS^T [64 keys (k) x 128 queries (m)], B = K [64 keys (k) x 128 d (n)]: both MN-major, 64-element
+    // chunks of the contiguous dimension one box (8 KiB) apart, 16 key rows per k-step (2 KiB)
+    constexpr uint32_t idesc = umma_idesc_bf16(128, kD, 1, 1);
+    bool ok = true;
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int s = j % DQG_STAGES;
+      if (!mbar_wait_warp(&full[s], (j / DQG_STAGES) & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      const uint64_t dA = umma_smem_desc(smem_u32(smem + s * DQG_STAGE_BYTES), DQG_BOX, 1024);
+      const uint64_t dK = umma_smem_desc(smem_u32(smem + s * DQG_STAGE_BYTES + DQG_TILE), DQG_BOX, 1024);
 #pragma unroll
-        for (int kk = 0; kk < DQG_KEYS / 16; ++kk)
-          umma_bf16_ss(tmem_base, umma_smem_desc(aA + kk * 2048, DQG_BOX, 1024),
-                       umma_smem_desc(aK + kk * 2048, DQG_BOX, 1024), idesc, (j | kk) != 0);
-        umma_commit(&empty[s]);
-      }
-      if (ok) umma_commit(done);
+      for (int kk = 0; kk < DQG_KEYS / 16; ++kk) umma_bf16_ss_warp(tmem_base, dA + kk * 128, dK + kk * 128, idesc, (j | kk) != 0);
+      umma_commit_warp(&empty[s]);
     }
+    if (ok) umma_commit_warp(done);
   } else {
     const int q = warp & 3;
-    const int row = m0 + q * 32 + lane;
+    const int row0 = m0 + q * 32, live = max(0, min(32, T - row0));
     const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16);
-    if (mbar_wait(done, 0, abort_flag)) {
+    const int pos = min(row0 + lane, T - 1);
+    const float *cs = p.unrot_cos + pos, *sn = p.unrot_sin + pos;
+    // the first 32 pairs' tables come while the products run (rolled loads behind them: 31.5 us where this takes 29)
+    RowTables tab[2];
+    if (p.unrot_cos != nullptr) {
+      load_row_tables(tab[0], cs, sn, p.unrot_ld, 0);
+      load_row_tables(tab[1], cs, sn, p.unrot_ld, 16);
+    }
+    if (mbar_wait_warp(done, 0, abort_flag)) {
       tc_fence_after();
-      const int pos = min(row, T - 1);
-      bf16* grow = p.dq + b * p.dq_bs + (long long)pos * p.dq_ts + h * p.dq_hs;
-      if (p.unrot_cos != nullptr) {
-        store_row_unrot_from_tmem<kD>(taddr, grow, 0, kD / 2, p.unrot_cos + pos, p.unrot_sin + pos, p.unrot_ld, row < T);
-      } else {
-#pragma unroll 1
-      for (int c = 0; c < kD; c += 32) {
-        uint32_t r[32];
-        tmem_ld_32x32b_x32(taddr + c, r);     // warp-collective: every lane takes part, rows past T do not store
-        tmem_ld_wait();
-        if (row < T) {
+      bf16* rows = p.dq + b * p.dq_bs + (long long)min(row0, T - 1) * p.dq_ts + h * p.dq_hs;
+      uint8_t* buf = smem + q * 4096;                 // every product has read its operands: the first stage is free
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 v;
-            bf162* v2 = reinterpret_cast<bf162*>(&v);
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              v2[e] = __floats2bfloat162_rn(__uint_as_float(r[i + 2 * e]), __uint_as_float(r[i + 2 * e + 1]));
-            *reinterpret_cast<uint4*>(grow + c + i) = v;
+      for (int i = 0; i < kD / 64; ++i) {
+        if (p.unrot_cos != nullptr) {
+          if (i > 0) {
+            load_row_tables(tab[0], cs, sn, p.unrot_ld, 32 * i);
+            load_row_tables(tab[1], cs, sn, p.unrot_ld, 32 * i + 16);
           }
+          put_rows_unrot<kD>(taddr, 32 * i, tab[0], buf, lane, 0);
+          put_rows_unrot<kD>(taddr, 32 * i + 16, tab[1], buf, lane, 2);
+          flush_rows(buf, lane, rows, p.dq_ts, 32 * i, kD / 2 + 32 * i, live);
+        } else {
+          store_rows_plain(taddr, 64 * i, buf, lane, rows, p.dq_ts, live);
         }
-      }
       }
     }
   }

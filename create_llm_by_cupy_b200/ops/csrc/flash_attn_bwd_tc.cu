@@ -1,4 +1,4 @@
-// Causal GQA flash-attention BACKWARD on the 5th-generation tensor cores (head_dim 128; dK/dV also 64).
+// Causal GQA flash-attention BACKWARD on the 5th-generation tensor cores (head_dim 128 and 64).
 //
 // Two kernels, both TMA-fed with accumulators in TMEM and the element-wise softmax-gradient math
 // done by two warpgroups that split the columns of each score tile:
@@ -13,14 +13,15 @@
 //        S^T = K Q_i^T (SS)    dP^T = V dO_i^T (SS)   P^T, dS^T -> bf16 into TMEM
 //        dV += P^T dO_i        dK += dS^T Q_i      (A from TMEM, B = the same Q_i / dO_i tiles read
 //                                                   MN-major), accumulated in TMEM over all i
-//   flash_bwd_dkv_wide : the same for head_dim 128 with 128-query iterations: every product is an N = 128 MMA, S^T,
-//        dP^T, dV and dK take all 512 tensor-memory columns, and the products of consecutive iterations are
-//        interleaved instead of double-buffered (see the comment above that kernel). The default for head_dim 128.
+//   flash_bwd_dkv_wide : the same with 128-query iterations: the score products are N = 128 MMAs, S^T, dP^T, dV and dK lie
+//        side by side in tensor memory, and the products of consecutive iterations are interleaved instead of
+//        double-buffered (see the comment above that kernel). What runs for both head dimensions; flash_bwd_dkv_tc is left
+//        for head_dim 128 where the wide kernel's shared memory does not fit.
 // Q and K are expected already rotated; dQ and dK are gradients w.r.t. the rotated tensors unless the
 // caller passes the rotary tables, in which case the epilogues apply the inverse rotation
 // (flash_rope_epilogue.cuh). No atomics and no fp32 scratch. When the caller gives a workspace the
 // dK/dV kernel also stores its dS^T tiles there and dQ is computed from them by a GEMM kernel
-// (flash_attn_bwd_dq.cu) instead of flash_bwd_dq_tc, which recomputes S and dP. The dK/dV kernel and
+// (flash_attn_bwd_dq.cu) instead of flash_bwd_dq_tc, which recomputes S and dP. The wide dK/dV kernel and
 // that GEMM are templates on the head dimension (128 or 64).
 //
 // Reference counterpart: cupy_flash_gqa_backward (model/flash_attention.py:109-176).
@@ -373,13 +374,11 @@ __device__ __forceinline__ DkvPass dkv_pass(int ntile, int T, int R, int vlen) {
   return d;
 }
 
-// kD: head dimension (128, or 64: one 64-column box per K / V / Q / dO tile, four k-steps in the score
-// products, N = 64 in the gradient products, 64 live columns in dV and dK).
-template <int kD>
 __global__ void __launch_bounds__(FBT_THREADS, 1)
 flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                         const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                         const __grid_constant__ CUtensorMap tmDS, const FlashBwdTcParams p) {
+  constexpr int kD = FB_D;
   extern __shared__ uint8_t fb_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fb_smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FdkvSmem::kBar);
@@ -457,9 +456,9 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
         mbar_expect_tx(kv_full, 2 * 128 * kD * 2);
         tma_load_4d(smem + FdkvSmem::kK, &tmK, kv_full, 0, kvh, d.n0, b);
-        if (kD == 128) tma_load_4d(smem + FdkvSmem::kK + 16384, &tmK, kv_full, 64, kvh, d.n0, b);
+        tma_load_4d(smem + FdkvSmem::kK + 16384, &tmK, kv_full, 64, kvh, d.n0, b);
         tma_load_4d(smem + FdkvSmem::kV, &tmV, kv_full, 0, kvh, d.n0, b);
-        if (kD == 128) tma_load_4d(smem + FdkvSmem::kV + 16384, &tmV, kv_full, 64, kvh, d.n0, b);
+        tma_load_4d(smem + FdkvSmem::kV + 16384, &tmV, kv_full, 64, kvh, d.n0, b);
         ++kv_loads;
         for (int it = 0; it < d.iters; ++it, ++g) {
           const int s = g % FKV_ST;
@@ -470,9 +469,9 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           uint8_t* sDO = sQ + FKV_QTILE;
           mbar_expect_tx(&q_full[s], 2 * FKV_BQ * kD * 2);
           tma_load_4d(sQ, &tmQ, &q_full[s], 0, h, m0, b);
-          if (kD == 128) tma_load_4d(sQ + 8192, &tmQ, &q_full[s], 64, h, m0, b);
+          tma_load_4d(sQ + 8192, &tmQ, &q_full[s], 64, h, m0, b);
           tma_load_4d(sDO, &tmDO, &q_full[s], 0, h, m0, b);
-          if (kD == 128) tma_load_4d(sDO + 8192, &tmDO, &q_full[s], 64, h, m0, b);
+          tma_load_4d(sDO + 8192, &tmDO, &q_full[s], 64, h, m0, b);
         }
       }
       (void)kv_loads;
@@ -711,7 +710,7 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 }
 
 // =================================================================== dK, dV with 128-query iterations
-// The same work with a different schedule (head_dim 128). A tcgen05.mma of 64 columns costs about 62 clocks
+// The same work with a different schedule (head_dim 128 and 64). A tcgen05.mma of 64 columns costs about 62 clocks
 // where its arithmetic needs 32, one of 128 columns about 78 for 64 (measured with back-to-back instructions),
 // so the score products want N = 128. S^T and dP^T of a 128-query tile then take 128 tensor-memory columns
 // each, which with the two 128-column accumulators is all there is: nothing is double-buffered. Instead the
@@ -725,21 +724,33 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 // one key row, computes P for its 64 columns, keeps it (packed bf16) in registers and forms dS from it when dP^T
 // is there. Its packed columns go to the first 32 columns of its own 64 (columns [0, 32) and [64, 96) of the
 // tile hold P^T: every k-step of the gradient products names its A address, so the gap does not matter).
+// head_dim 64 keeps P in fp32 between the phases and has 64-column accumulators.
+//
+// What bounds it: the math warps, two to a scheduler (3000 clocks an iteration at head_dim 64: 1400 for P, where the 16
+// exponentials a clock alone need 1024, 1000 for dS, the rest waits and barriers; 3600 at 128, where the products take 2600).
+// What it took to get there, 8 x 1024 tokens with 12 / 4 heads of 64 | 4 x 2048 with 16 / 4 heads of 128, in us: 76.7 (with
+// 64-query iterations) | 182.1 -> 128-query iterations for head_dim 64, 64 columns per tensor-memory load, products issued by
+// the whole warp: 71.8 | 172 -> one copy of the loops for both passes, rows stored through shared memory: 60.7 | 163.8 ->
+// no division in the loops: 58.1 | 161.2. A second S^T tile for head_dim 64 gains nothing and needs barriers of its own
+// for each warpgroup: the one that ran ahead completed a phase for the other.
 constexpr int FKW_BQ = 128;                      // query rows per iteration
-constexpr int FKW_TILE = FKW_BQ * FB_D * 2;      // 32 KiB
+template <int kD>
 struct FdkwSmem {
-  static constexpr int kK = 0, kV = FB_TILE, kQ = 2 * FB_TILE;             // stage s: Q_i (32 KiB), dO_i (32 KiB)
-  static constexpr int kStage = kQ + 2 * 2 * FKW_TILE;                      // [2] dS^T staging tiles (one per warpgroup)
-  static constexpr int kStats = kStage + 2 * FKV_STG;                       // stage s: lse2[128], delta * scale [128]
-  static constexpr int kBar = kStats + 2 * 2 * FKW_BQ * 4;
-  // kv_full, q_full[2], q_empty[2], st_full[2], s_full, dp_full, p_ready, ds_ready, acc_done, acc_free,
-  // stg_full[2], stg_free[2] = 17
-  static constexpr int kUsed = kBar + 17 * 8 + 16;
-  // All the shared memory of an SM: the tiles leave less than the 1 KiB a worst-case alignment of the base would
-  // take, so the kernel checks that what it needs fits behind the aligned base and reports an error otherwise.
-  static constexpr int kTotal = 232448;
+  static constexpr int kTile = 128 * kD * 2;                               // a K, V, Q_i or dO_i tile
+  static constexpr int kStages = kD == 128 ? 2 : 3;                        // ring of Q_i, dO_i and their statistics
+  static constexpr int kK = 0, kV = kTile, kQ = 2 * kTile;                 // stage s: Q_i, dO_i
+  static constexpr int kStage = kQ + kStages * 2 * kTile;                  // [2] dS^T staging tiles (one per warpgroup)
+  static constexpr int kStats = kStage + 2 * FKV_STG;                      // stage s: lse2[128], delta * scale [128]
+  static constexpr int kBar = kStats + kStages * 2 * FKW_BQ * 4;
+  // kv_full, q_full[3], q_empty[3], st_full[3], s_full, dp_full, p_ready, ds_ready, acc_done, acc_free,
+  // stg_full[2], stg_free[2] (head_dim 128: two of the threes)
+  static constexpr int kBars = 11 + 3 * kStages;
+  static constexpr int kUsed = kBar + kBars * 8 + 16;
+  // head_dim 128: all the shared memory of an SM; the tiles leave less than the 1 KiB a worst-case alignment of the base
+  // would take, so the kernel checks that what it needs fits behind the aligned base and reports an error otherwise.
+  static constexpr int kTotal = kD == 128 ? 232448 : kUsed + 1024;
 };
-static_assert(FdkwSmem::kUsed <= FdkwSmem::kTotal, "dK/dV kernel: shared memory");
+static_assert(FdkwSmem<128>::kUsed <= FdkwSmem<128>::kTotal, "dK/dV kernel: shared memory");
 
 struct DkwPass {
   int n0, i_first, n_qt, iters;
@@ -753,9 +764,9 @@ __device__ __forceinline__ DkwPass dkw_pass(int ntile, int T, int R, int vlen) {
   return d;
 }
 
-// P^T for 16 query columns of one key row, packed to bf16 pairs; lse2 points at the 16 per-query values.
+// P^T for 16 query columns of one key row, in place and packed to bf16 pairs; lse2 points at the 16 per-query values.
 template <bool kMask>
-__device__ __forceinline__ void fb_p_chunk(const uint32_t (&rs)[16], uint32_t (&pk)[8], float sl2, const float* lse2,
+__device__ __forceinline__ void fb_p_chunk(uint32_t (&rs)[16], uint32_t (&pk)[8], float sl2, const float* lse2,
                                            int q_base, int key, bool key_dead) {
 #pragma unroll
   for (int e = 0; e < 16; e += 4) {
@@ -769,11 +780,29 @@ __device__ __forceinline__ void fb_p_chunk(const uint32_t (&rs)[16], uint32_t (&
         if (key_dead || key > q_base + e + u) pe = 0.f;
       }
       pv[u] = pe;
+      rs[e + u] = __float_as_uint(pe);
     }
 #pragma unroll
     for (int u = 0; u < 4; u += 2) {
       const bf162 t0 = __floats2bfloat162_rn(pv[u], pv[u + 1]);
       pk[(e + u) >> 1] = *reinterpret_cast<const uint32_t*>(&t0);
+    }
+  }
+}
+
+// dS^T = P^T * (dP^T * scale - delta * scale) for the same 16 columns, from P^T in fp32.
+__device__ __forceinline__ void fb_ds_chunk16(const uint32_t* pv, const uint32_t* rp, uint32_t (&dk)[8], float scale,
+                                              const float* dlt_s) {
+#pragma unroll
+  for (int e = 0; e < 16; e += 4) {
+    const float4 d4 = *reinterpret_cast<const float4*>(dlt_s + e);
+    const float dl[4] = {d4.x, d4.y, d4.z, d4.w};
+#pragma unroll
+    for (int u = 0; u < 4; u += 2) {
+      const bf162 t = __floats2bfloat162_rn(
+          __uint_as_float(pv[e + u]) * fmaf(__uint_as_float(rp[e + u]), scale, -dl[u]),
+          __uint_as_float(pv[e + u + 1]) * fmaf(__uint_as_float(rp[e + u + 1]), scale, -dl[u + 1]));
+      dk[(e + u) >> 1] = *reinterpret_cast<const uint32_t*>(&t);
     }
   }
 }
@@ -796,23 +825,25 @@ __device__ __forceinline__ void fb_ds_from_p_chunk(const uint32_t (&rp)[16], con
   }
 }
 
+template <int kD>
 __global__ void __launch_bounds__(FBT_THREADS, 1)
 flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                           const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                           const __grid_constant__ CUtensorMap tmDS, const FlashBwdTcParams p) {
-  constexpr int kD = FB_D;
+  using Smem = FdkwSmem<kD>;
+  constexpr int kSt = Smem::kStages, kTile = Smem::kTile;
   extern __shared__ uint8_t fb_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fb_smem_raw) + 1023) & ~uintptr_t(1023));
-  if (smem + FdkwSmem::kUsed > fb_smem_raw + FdkwSmem::kTotal) {      // the same for every thread of every CTA
+  if (smem + Smem::kUsed > fb_smem_raw + Smem::kTotal) {      // the same for every thread of every CTA
     if (threadIdx.x == 0 && p.status != nullptr && atomicCAS(p.status, 0, int(ERR_BAD_ARGUMENT)) == 0) p.status[1] = 313;
     return;
   }
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FdkwSmem::kBar);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Smem::kBar);
   uint64_t* kv_full = bars;
-  uint64_t* q_full = bars + 1;                    // [2]
-  uint64_t* q_empty = q_full + 2;                 // [2]
-  uint64_t* st_full = q_empty + 2;                // [2] statistics staged
-  uint64_t* s_full = st_full + 2;                 // S^T of the iteration is in tensor memory
+  uint64_t* q_full = bars + 1;                    // [kSt]
+  uint64_t* q_empty = q_full + kSt;               // [kSt]
+  uint64_t* st_full = q_empty + kSt;              // [kSt] statistics staged
+  uint64_t* s_full = st_full + kSt;               // S^T of the iteration is in tensor memory
   uint64_t* dp_full = s_full + 1;                 // dP^T of the iteration is in tensor memory
   uint64_t* p_ready = dp_full + 1;                // every math thread has written its P^T columns
   uint64_t* ds_ready = p_ready + 1;               // ... its dS^T columns
@@ -837,11 +868,14 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
   const int T = p.T;
   const int R = p.QH / p.KVH;
   const int tile_of_pass[2] = {pair, p.pairing ? p.n_tiles - 1 - pair : pair};
-  const int n_pass = tile_of_pass[0] == tile_of_pass[1] ? 1 : 2;
+  int n_pass = tile_of_pass[0] == tile_of_pass[1] ? 1 : 2;
+  // Known to be 1 or 2, this made a copy of every loop for each pass, and the second pass waited for its instructions to come
+  // from memory: 11000 to 19000 clocks for its first iteration where the others take 3000.
+  asm volatile("" : "+r"(n_pass));
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
-    for (int s = 0; s < 2; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); mbar_init(&st_full[s], 32); }
+    for (int s = 0; s < kSt; ++s) { mbar_init(&q_full[s], 1); mbar_init(&q_empty[s], 1); mbar_init(&st_full[s], 32); }
     mbar_init(s_full, 1);
     mbar_init(dp_full, 1);
     mbar_init(p_ready, 256);
@@ -861,35 +895,36 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
   const uint32_t tmem_base = *tmem_slot;
   pdl_wait();                            // by every role: their bounded waits start counting behind it
   const int vlen = p.valid_len ? checked_index(p.valid_len[b], T, p.status, 302) : T;
-  constexpr uint32_t kColST = 0, kColDPT = 128, kColDV = 256, kColDK = 384;
+  constexpr uint32_t kColST = 0, kColDPT = 128, kColDV = 256, kColDK = 256 + kD;
 
   if (warp == 0) {
     if (lane == 0) {
       int g = 0;
       bool ok = true;
+#pragma unroll 1
       for (int ps = 0; ps < n_pass && ok; ++ps) {
         const DkwPass d = dkw_pass(tile_of_pass[ps], T, R, vlen);
         if (d.iters == 0) continue;
         if (ps > 0) {             // K / V of the previous pass are read by its MMAs until they have all completed
           if (!mbar_wait(acc_done, (ps - 1) & 1, abort_flag)) break;
         }
-        mbar_expect_tx(kv_full, 2 * FB_TILE);
-        tma_load_4d(smem + FdkwSmem::kK, &tmK, kv_full, 0, kvh, d.n0, b);
-        tma_load_4d(smem + FdkwSmem::kK + 16384, &tmK, kv_full, 64, kvh, d.n0, b);
-        tma_load_4d(smem + FdkwSmem::kV, &tmV, kv_full, 0, kvh, d.n0, b);
-        tma_load_4d(smem + FdkwSmem::kV + 16384, &tmV, kv_full, 64, kvh, d.n0, b);
-        for (int it = 0; it < d.iters; ++it, ++g) {
-          const int s = g & 1;
-          const int h = kvh * R + it / d.n_qt;
-          const int m0 = (d.i_first + it % d.n_qt) * FKW_BQ;
-          if (!mbar_wait(&q_empty[s], ((g >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
-          uint8_t* sQ = smem + FdkwSmem::kQ + s * 2 * FKW_TILE;
-          uint8_t* sDO = sQ + FKW_TILE;
-          mbar_expect_tx(&q_full[s], 2 * FKW_TILE);
+        mbar_expect_tx(kv_full, 2 * kTile);
+        tma_load_4d(smem + Smem::kK, &tmK, kv_full, 0, kvh, d.n0, b);
+        if (kD == 128) tma_load_4d(smem + Smem::kK + 16384, &tmK, kv_full, 64, kvh, d.n0, b);
+        tma_load_4d(smem + Smem::kV, &tmV, kv_full, 0, kvh, d.n0, b);
+        if (kD == 128) tma_load_4d(smem + Smem::kV + 16384, &tmV, kv_full, 64, kvh, d.n0, b);
+        for (int it = 0, h = kvh * R, i = d.i_first; it < d.iters; ++it, ++g) {
+          const int s = g % kSt;
+          const int m0 = i * FKW_BQ;
+          if (!mbar_wait(&q_empty[s], ((g / kSt) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          uint8_t* sQ = smem + Smem::kQ + s * 2 * kTile;
+          uint8_t* sDO = sQ + kTile;
+          mbar_expect_tx(&q_full[s], 2 * kTile);
           tma_load_4d(sQ, &tmQ, &q_full[s], 0, h, m0, b);
-          tma_load_4d(sQ + 16384, &tmQ, &q_full[s], 64, h, m0, b);
+          if (kD == 128) tma_load_4d(sQ + 16384, &tmQ, &q_full[s], 64, h, m0, b);
           tma_load_4d(sDO, &tmDO, &q_full[s], 0, h, m0, b);
-          tma_load_4d(sDO + 16384, &tmDO, &q_full[s], 64, h, m0, b);
+          if (kD == 128) tma_load_4d(sDO + 16384, &tmDO, &q_full[s], 64, h, m0, b);
+          if (++i == d.i_first + d.n_qt) { i = d.i_first; ++h; }
         }
       }
     }
@@ -897,14 +932,14 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     // stages the per-query statistics (lse in log2 units, delta * scale) of each query tile in shared memory
     int g = 0;
     bool ok = true;
+#pragma unroll 1
     for (int ps = 0; ps < n_pass && ok; ++ps) {
       const DkwPass d = dkw_pass(tile_of_pass[ps], T, R, vlen);
-      for (int it = 0; it < d.iters; ++it, ++g) {
-        const int s = g & 1;
-        const int h = kvh * R + it / d.n_qt;
-        const int m0 = (d.i_first + it % d.n_qt) * FKW_BQ;
-        if (!mbar_wait(&q_empty[s], ((g >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
-        float* st = reinterpret_cast<float*>(smem + FdkwSmem::kStats + s * 2 * FKW_BQ * 4);
+      for (int it = 0, h = kvh * R, i = d.i_first; it < d.iters; ++it, ++g) {
+        const int s = g % kSt;
+        const int m0 = i * FKW_BQ;
+        if (!mbar_wait(&q_empty[s], ((g / kSt) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        float* st = reinterpret_cast<float*>(smem + Smem::kStats + s * 2 * FKW_BQ * 4);
         // all eight loads in flight before the first store: one after the other (a store to shared memory may not
         // pass a later global load the compiler cannot tell apart from it) they cost four round trips to L2 per
         // iteration, which made this warp the slowest part of the kernel
@@ -923,6 +958,7 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
           st[FKW_BQ + r] = (m0 + r < T) ? dv[j] * p.scale : 0.f;
         }
         mbar_arrive(&st_full[s]);
+        if (++i == d.i_first + d.n_qt) { i = d.i_first; ++h; }
       }
     }
   } else if (warp == 2) {
@@ -931,97 +967,97 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     if (lane == 0 && p.ds != nullptr) {
       uint32_t uses = 0;
       bool ok = true;
+#pragma unroll 1
       for (int ps = 0; ps < n_pass && ok; ++ps) {
         const DkwPass d = dkw_pass(tile_of_pass[ps], T, R, vlen);
-        for (int it = 0; it < d.iters && ok; ++it, ++uses) {
-          const int m0 = (d.i_first + it % d.n_qt) * FKW_BQ;
+        for (int it = 0, h = kvh * R, i = d.i_first; it < d.iters && ok; ++it, ++uses) {
+          const int m0 = i * FKW_BQ;
           for (int w = 0; w < 2; ++w) {
             if (!mbar_wait(&stg_full[w], uses & 1, abort_flag)) { ok = false; break; }
-            tma_store_4d_ds(&tmDS, smem + FdkwSmem::kStage + w * FKV_STG, m0 + w * 64, kvh * R + it / d.n_qt, d.n0, b);
+            tma_store_4d_ds(&tmDS, smem + Smem::kStage + w * FKV_STG, m0 + w * 64, h, d.n0, b);
             tma_store_commit();
           }
           if (!ok) break;
           tma_store_wait_read<0>();
           mbar_arrive(&stg_free[0]);
           mbar_arrive(&stg_free[1]);
+          if (++i == d.i_first + d.n_qt) { i = d.i_first; ++h; }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, FKW_BQ, 0, 0);   // [128 keys x 128 q], K-major operands
       constexpr uint32_t idesc_g = umma_idesc_bf16(128, kD, 0, 1);       // [128 keys x d], B MN-major
-      const uint32_t aK = smem_u32(smem + FdkwSmem::kK), aV = smem_u32(smem + FdkwSmem::kV);
-      auto stage_q = [&](int g) { return smem_u32(smem + FdkwSmem::kQ + (g & 1) * 2 * FKW_TILE); };
+      const uint64_t dsK = umma_smem_desc(smem_u32(smem + Smem::kK), 16, 1024), dsV = umma_smem_desc(smem_u32(smem + Smem::kV), 16, 1024);
+      auto stage_q = [&](int g) { return smem_u32(smem + Smem::kQ + (g % kSt) * 2 * kTile); };
+      auto q_ready = [&](int g) { return mbar_wait_warp(&q_full[g % kSt], (g / kSt) & 1, abort_flag); };
       auto issue_s = [&](int g) {
-        const uint32_t aQ = stage_q(g);
+        const uint64_t dsQ = umma_smem_desc(stage_q(g), 16, 1024);
 #pragma unroll
         for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;       // 128-row tiles, 64-column halves
-          umma_bf16_ss(tmem_base + kColST, umma_smem_desc(aK + off, 16, 1024), umma_smem_desc(aQ + off, 16, 1024),
-                       idesc_s, kk != 0);
+          const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;       // 128-row tiles, 64-column halves; 16-byte units
+          umma_bf16_ss_warp(tmem_base + kColST, dsK + off, dsQ + off, idesc_s, kk != 0);
         }
-        umma_commit(s_full);
+        umma_commit_warp(s_full);
       };
       auto issue_dp = [&](int g) {
-        const uint32_t aDO = stage_q(g) + FKW_TILE;
+        const uint64_t dsDO = umma_smem_desc(stage_q(g) + kTile, 16, 1024);
 #pragma unroll
         for (int kk = 0; kk < kD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_bf16_ss(tmem_base + kColDPT, umma_smem_desc(aV + off, 16, 1024), umma_smem_desc(aDO + off, 16, 1024),
-                       idesc_s, kk != 0);
+          const uint32_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
+          umma_bf16_ss_warp(tmem_base + kColDPT, dsV + off, dsDO + off, idesc_s, kk != 0);
         }
-        umma_commit(dp_full);
+        umma_commit_warp(dp_full);
       };
       bool ok = true;
       int g0 = 0, kv_loads = 0;
+#pragma unroll 1
       for (int ps = 0; ps < n_pass && ok; ++ps) {
         const DkwPass d = dkw_pass(tile_of_pass[ps], T, R, vlen);
         if (d.iters > 0) {
-          if (!mbar_wait(kv_full, kv_loads & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(kv_full, kv_loads & 1, abort_flag)) { ok = false; break; }
           ++kv_loads;
-          if (!mbar_wait(&q_full[g0 & 1], (g0 >> 1) & 1, abort_flag)) { ok = false; break; }
+          if (!q_ready(g0)) { ok = false; break; }
           tc_fence_after();
           issue_s(g0);
           issue_dp(g0);
           if (ps > 0) {           // the accumulators still hold the previous pass until its rows are stored
-            if (!mbar_wait(acc_free, (ps - 1) & 1, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(acc_free, (ps - 1) & 1, abort_flag)) { ok = false; break; }
             tc_fence_after();
           }
         }
         for (int it = 0; it < d.iters && ok; ++it) {
           const int g = g0 + it;
-          const uint32_t aQ = stage_q(g), aDO = aQ + FKW_TILE;
+          const uint64_t mnQ = umma_smem_desc(stage_q(g), 16384, 1024), mnDO = umma_smem_desc(stage_q(g) + kTile, 16384, 1024);
           // dV += P^T dO: A = the packed P^T columns (k-step kk: 16 queries = 8 columns; queries 64.. sit at column
           // 64), B = dO read MN-major (16 query rows per k-step, 64-d halves 16 KiB apart)
-          if (!mbar_wait(p_ready, g & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(p_ready, g & 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < FKW_BQ / 16; ++kk) {
             const uint32_t acol = kk < 4 ? kk * 8 : 64 + (kk - 4) * 8;
-            umma_bf16_ts(tmem_base + kColDV, tmem_base + kColST + acol, umma_smem_desc(aDO + kk * 2048, 16384, 1024),
-                         idesc_g, (it | kk) != 0);
+            umma_bf16_ts_warp(tmem_base + kColDV, tmem_base + kColST + acol, mnDO + kk * 128, idesc_g, (it | kk) != 0);
           }
           if (it + 1 < d.iters) {   // S^T of the next tile may overwrite P^T once dV has read it: issue order
-            if (!mbar_wait(&q_full[(g + 1) & 1], ((g + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+            if (!q_ready(g + 1)) { ok = false; break; }
             tc_fence_after();
             issue_s(g + 1);
           }
-          if (!mbar_wait(ds_ready, g & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(ds_ready, g & 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int kk = 0; kk < FKW_BQ / 16; ++kk) {
             const uint32_t acol = kk < 4 ? kk * 8 : 64 + (kk - 4) * 8;
-            umma_bf16_ts(tmem_base + kColDK, tmem_base + kColDPT + acol, umma_smem_desc(aQ + kk * 2048, 16384, 1024),
-                         idesc_g, (it | kk) != 0);
+            umma_bf16_ts_warp(tmem_base + kColDK, tmem_base + kColDPT + acol, mnQ + kk * 128, idesc_g, (it | kk) != 0);
           }
-          umma_commit(&q_empty[g & 1]);
+          umma_commit_warp(&q_empty[g % kSt]);
           if (it + 1 < d.iters) issue_dp(g + 1);
         }
         if (ok && d.iters == 0 && ps > 0) {
-          if (!mbar_wait(acc_free, (ps - 1) & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(acc_free, (ps - 1) & 1, abort_flag)) { ok = false; break; }
         }
-        if (ok) umma_commit(acc_done);
+        if (ok) umma_commit_warp(acc_done);
         g0 += d.iters;
       }
     }
@@ -1031,46 +1067,43 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
     const int half = wg;                      // dK / dV columns this warpgroup stores at the end of a pass
     const uint32_t lane_sel = uint32_t(q * 32) << 16;
     const float sl2 = p.scale * kFbLog2e;
-    uint8_t* stg_row = smem + FdkwSmem::kStage + wg * FKV_STG + (q * 32 + lane) * 128;
+    uint8_t* stg_row = smem + Smem::kStage + wg * FKV_STG + (q * 32 + lane) * 128;
     const uint32_t swz = uint32_t(lane & 7);
     const bool ds_on = p.ds != nullptr;
     const uint32_t tS = tmem_base + lane_sel + kColST + wg * 64, tP = tmem_base + lane_sel + kColDPT + wg * 64;
     uint32_t stg_uses = 0;
     bool ok = true;
     int g0 = 0;
+#pragma unroll 1
     for (int ps = 0; ps < n_pass && ok; ++ps) {
       const DkwPass d = dkw_pass(tile_of_pass[ps], T, R, vlen);
       const int n0 = d.n0;
       const int key = n0 + q * 32 + lane;
       const bool key_dead = key >= vlen;
-      for (int it = 0; it < d.iters && ok; ++it) {
-        const int g = g0 + it, s2 = g & 1;
-        const int m0 = (d.i_first + it % d.n_qt) * FKW_BQ;
+      for (int it = 0, i = d.i_first; it < d.iters && ok; ++it) {
+        const int g = g0 + it, s2 = g % kSt;
+        const int m0 = i * FKW_BQ;
+        if (++i == d.i_first + d.n_qt) i = d.i_first;
         const int qb = m0 + wg * 64;                                     // first query column of this warpgroup
-        const float* st = reinterpret_cast<const float*>(smem + FdkwSmem::kStats + s2 * 2 * FKW_BQ * 4) + wg * 64;
+        const float* st = reinterpret_cast<const float*>(smem + Smem::kStats + s2 * 2 * FKW_BQ * 4) + wg * 64;
         const bool need_mask = (m0 < n0 + 128) || (n0 + 128 > vlen);     // the diagonal tile or the padded tail
-        uint32_t pk[4][8];                                               // this thread's P^T, 64 columns packed
-        uint32_t ra[16], rb[16];
-        if (!mbar_wait(&st_full[s2], (g >> 1) & 1, abort_flag)) { ok = false; break; }
+        // This thread's P^T between the two phases: packed (head_dim 128), or as it is (64, which has the registers)
+        uint32_t pk[4][8], sc[64];
+        if (!mbar_wait(&st_full[s2], (g / kSt) & 1, abort_flag)) { ok = false; break; }
         if (!mbar_wait(s_full, g & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        auto p_chunk = [&](const uint32_t (&rs)[16], int c) {
+        // all 64 columns in one go: a tensor-memory load queues behind the products that are running, so four loads one
+        // after the other cost that wait four times
+        tmem_ld_32x32b_x32(tS, *reinterpret_cast<uint32_t(*)[32]>(&sc[0]));
+        tmem_ld_32x32b_x32(tS + 32, *reinterpret_cast<uint32_t(*)[32]>(&sc[32]));
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t(&rs)[16] = *reinterpret_cast<uint32_t(*)[16]>(&sc[16 * c]);
           if (need_mask) fb_p_chunk<true>(rs, pk[c], sl2, st + c * 16, qb + c * 16, key, key_dead);
           else fb_p_chunk<false>(rs, pk[c], sl2, st + c * 16, 0, 0, false);
           tmem_st_32x32b_x8(tS + c * 8, pk[c]);
-        };
-        tmem_ld_32x32b_x16(tS, ra);
-        tmem_ld_wait();
-        tmem_ld_32x32b_x16(tS + 16, rb);
-        p_chunk(ra, 0);
-        tmem_ld_wait();
-        tmem_ld_32x32b_x16(tS + 32, ra);
-        p_chunk(rb, 1);
-        tmem_ld_wait();
-        tmem_ld_32x32b_x16(tS + 48, rb);
-        p_chunk(ra, 2);
-        tmem_ld_wait();
-        p_chunk(rb, 3);
+        }
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(p_ready);
@@ -1080,27 +1113,28 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
         if (ds_on) {              // the store of this warpgroup's previous tile must have read the staging tile
           if (!mbar_wait(&stg_free[wg], (stg_uses & 1) ^ 1, abort_flag)) { ok = false; break; }
         }
-        auto ds_chunk = [&](const uint32_t (&rp)[16], int c) {
+        auto ds_chunk = [&](const uint32_t* rp, int c) {
           uint32_t dk_[8];
-          fb_ds_from_p_chunk(rp, pk[c], dk_, p.scale, st + FKW_BQ + c * 16);
+          if (kD == 64) fb_ds_chunk16(&sc[16 * c], rp, dk_, p.scale, st + FKW_BQ + c * 16);
+          else fb_ds_from_p_chunk(*reinterpret_cast<const uint32_t(*)[16]>(rp), pk[c], dk_, p.scale, st + FKW_BQ + c * 16);
           tmem_st_32x32b_x8(tP + c * 8, dk_);
           if (ds_on) {            // 16 queries = two 16-byte chunks of this key's 128-byte staging row
             *reinterpret_cast<uint4*>(stg_row + ((uint32_t(2 * c) ^ swz) << 4)) = make_uint4(dk_[0], dk_[1], dk_[2], dk_[3]);
             *reinterpret_cast<uint4*>(stg_row + ((uint32_t(2 * c + 1) ^ swz) << 4)) = make_uint4(dk_[4], dk_[5], dk_[6], dk_[7]);
           }
         };
-        tmem_ld_32x32b_x16(tP, ra);
+        uint32_t ra[32], rb[32];
+        tmem_ld_32x32b_x32(tP, ra);
+        if (kD == 128) tmem_ld_32x32b_x32(tP + 32, rb);
         tmem_ld_wait();
-        tmem_ld_32x32b_x16(tP + 16, rb);
-        ds_chunk(ra, 0);
-        tmem_ld_wait();
-        tmem_ld_32x32b_x16(tP + 32, ra);
-        ds_chunk(rb, 1);
-        tmem_ld_wait();
-        tmem_ld_32x32b_x16(tP + 48, rb);
-        ds_chunk(ra, 2);
-        tmem_ld_wait();
-        ds_chunk(rb, 3);
+        ds_chunk(&ra[0], 0);
+        ds_chunk(&ra[16], 1);
+        if (kD == 64) {
+          tmem_ld_32x32b_x32(tP + 32, rb);
+          tmem_ld_wait();
+        }
+        ds_chunk(&rb[0], 2);
+        ds_chunk(&rb[16], 3);
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(ds_ready);
@@ -1112,27 +1146,32 @@ flash_bwd_dkv_wide_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_
       }
       if (!ok) break;
       g0 += d.iters;
-      // end of the pass: the accumulators of this key tile are complete once every MMA has run
-      if (!mbar_wait(acc_done, ps & 1, abort_flag)) { ok = false; break; }
+      // End of the pass: the accumulators of this key tile are complete once every MMA has run. Each warp stores 32 rows:
+      // head_dim 64: dK by warpgroup 0, dV by 1; 128: half of the columns of both by each.
+      const int live = max(0, min(32, T - (n0 + q * 32))), pos = min(key, T - 1);
+      if (!mbar_wait_warp(acc_done, ps & 1, abort_flag)) { ok = false; break; }
+      if (ds_on) {                // the rows go through the dS^T staging tile: its last store must have read it
+        if (!mbar_wait_warp(&stg_free[wg], (stg_uses & 1) ^ 1, abort_flag)) { ok = false; break; }
+      }
       tc_fence_after();
-      const bool live = key < T;
-      bf16* krow = p.dk + b * p.dk_bs + (long long)min(key, T - 1) * p.dk_ts + kvh * p.dk_hs;
-      bf16* vrow = p.dv + b * p.dv_bs + (long long)min(key, T - 1) * p.dv_ts + kvh * p.dv_hs;
-      constexpr int kHalfCols = kD / 2;          // dK / dV columns each warpgroup stores
+      uint8_t* buf = smem + Smem::kStage + wg * FKV_STG + q * 4096;
+      bf16* krow = p.dk + b * p.dk_bs + (long long)min(n0 + q * 32, T - 1) * p.dk_ts + kvh * p.dk_hs;
+      bf16* vrow = p.dv + b * p.dv_bs + (long long)min(n0 + q * 32, T - 1) * p.dv_ts + kvh * p.dv_hs;
+      const uint32_t tDK = tmem_base + lane_sel + kColDK, tDV = tmem_base + lane_sel + kColDV;
+      const int c0 = kD == 128 ? half * 64 : 0;
       if (d.iters > 0) {
-        if (p.unrot_cos != nullptr) {
-          const int pos = min(key, T - 1);
-          store_row_unrot_from_tmem<kD>(tmem_base + lane_sel + kColDK, krow, half * (kD / 4), kD / 4,
-                                        p.unrot_cos + pos, p.unrot_sin + pos, p.unrot_ld, live);
-        } else {
-          store_row_from_tmem(tmem_base + lane_sel + kColDK, krow, half * kHalfCols, (half + 1) * kHalfCols, live);
+        if (kD == 128 || wg == 0) {
+          if (p.unrot_cos != nullptr)
+            store_rows_unrot<kD>(tDK, kD == 128 ? half * 32 : 0, p.unrot_cos + pos, p.unrot_sin + pos, p.unrot_ld, buf, lane, krow,
+                                 p.dk_ts, live);
+          else store_rows_plain(tDK, c0, buf, lane, krow, p.dk_ts, live);
         }
-        store_row_from_tmem(tmem_base + lane_sel + kColDV, vrow, half * kHalfCols, (half + 1) * kHalfCols, live);
-      } else if (live) {
+        if (kD == 128 || wg == 1) store_rows_plain(tDV, c0, buf, lane, vrow, p.dv_ts, live);
+      } else if (lane < live) {
         const uint4 z = make_uint4(0, 0, 0, 0);
-        for (int c = half * kHalfCols; c < (half + 1) * kHalfCols; c += 8) {
-          *reinterpret_cast<uint4*>(krow + c) = z;
-          *reinterpret_cast<uint4*>(vrow + c) = z;
+        for (int c = half * (kD / 2); c < (half + 1) * (kD / 2); c += 8) {
+          *reinterpret_cast<uint4*>(krow + lane * p.dk_ts + c) = z;
+          *reinterpret_cast<uint4*>(vrow + lane * p.dv_ts + c) = z;
         }
       }
       tc_fence_before();
@@ -1200,7 +1239,7 @@ static bool dkv_wide_fits() {
       cudaFree(d);
     }
     const int pad = off < 0 ? 1024 : (1024 - off) & 1023;        // bytes lost to the round-up of the base
-    fits[dev] = (FdkwSmem::kUsed + pad <= FdkwSmem::kTotal) ? 1 : -1;
+    fits[dev] = (FdkwSmem<128>::kUsed + pad <= FdkwSmem<128>::kTotal) ? 1 : -1;
   }
   return fits[dev] > 0;
 }
@@ -1249,12 +1288,12 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   if (!configured) {
     B200_CHECK(cudaFuncSetAttribute(flash_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     FdqSmem::kTotal));
-    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     FdkvSmem::kTotal));
-    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    FdkvSmem::kTotal));
-    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    FdkwSmem::kTotal));
+    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_wide_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    FdkwSmem<64>::kTotal));
+    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_wide_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    FdkwSmem<128>::kTotal));
     configured = true;
   }
   const int nt = (T + 127) / 128;
@@ -1287,12 +1326,15 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   const int n_key_tiles = nt * KVH * B;
   p.pairing = g_dkv_pairing >= 0 ? g_dkv_pairing : ((n_key_tiles > num_sms() && n_key_tiles < 3 * num_sms()) ? 1 : 0);
   const int dkv_ctas = (p.pairing ? (nt + 1) / 2 : nt) * KVH * B;
-  if (D == 128 && g_dkv_wide && dkv_wide_fits())
-    B200_CHECK(launch_pdl(flash_bwd_dkv_wide_kernel, dim3(dkv_ctas), dim3(FBT_THREADS), FdkwSmem::kTotal, st, 0, *tq128, *tdo128,
-                          *tk, *tv, *tds, p));
+  if (D == 64)
+    B200_CHECK(launch_pdl(flash_bwd_dkv_wide_kernel<64>, dim3(dkv_ctas), dim3(FBT_THREADS), FdkwSmem<64>::kTotal, st, 0, *tq128,
+                          *tdo128, *tk, *tv, *tds, p));
+  else if (g_dkv_wide && dkv_wide_fits())
+    B200_CHECK(launch_pdl(flash_bwd_dkv_wide_kernel<128>, dim3(dkv_ctas), dim3(FBT_THREADS), FdkwSmem<128>::kTotal, st, 0, *tq128,
+                          *tdo128, *tk, *tv, *tds, p));
   else
-    B200_CHECK(launch_pdl(D == 128 ? flash_bwd_dkv_tc_kernel<128> : flash_bwd_dkv_tc_kernel<64>, dim3(dkv_ctas),
-                          dim3(FBT_THREADS), FdkvSmem::kTotal, st, 0, *tq64, *tdo64, *tk, *tv, *tds, p));
+    B200_CHECK(launch_pdl(flash_bwd_dkv_tc_kernel, dim3(dkv_ctas), dim3(FBT_THREADS), FdkvSmem::kTotal, st, 0, *tq64, *tdo64,
+                          *tk, *tv, *tds, p));
   if (ds_ws != nullptr) return flash_bwd_dq_from_ds(ds_ws, k, dq, valid_len, s + 3, s + 12, B, T, QH, KVH, D, p.bchunk,
                                                       p.unrot_cos, p.unrot_sin, p.unrot_ld, st);
   if (dkv_ctas >= 3 * num_sms()) {
