@@ -23,7 +23,7 @@
 // (one tile ahead of the one it is loading), writes it into a
 // 4-slot ring that exists in both CTAs' shared memory and signals sched_full[slot] in both. The
 // follower's producer, the MMA thread and the epilogue warps of both read the ring and each arrive
-// on the leader's sched_empty[slot] (10 or 18 arrivals) before the slot is reused. An index beyond the
+// on the leader's sched_empty[slot] (10, 18 or, with the mover, 20 arrivals) before the slot is reused. An index beyond the
 // last tile is the stop mark; every pair draws exactly one, and the pair that draws the last one
 // puts the counter back to zero for the launch that reuses it. A pair that starts late (its SMs
 // were still busy with the previous kernel, or with a kernel of another stream) simply draws
@@ -46,7 +46,7 @@ constexpr int G2_SCHED = 4;         // slots of the tile-index ring
 constexpr int G2_STG_BYTES = 128 * 128;                 // epilogue staging tile: 128 rows x 128 bytes
 constexpr int G2_STG_OFF = G2_STAGES * G2_STAGE_BYTES;  // two staging tiles follow the operand ring
 constexpr int G2_BAR_OFF2 = G2_STG_OFF + 2 * G2_STG_BYTES;
-constexpr int G2_SMEM = G2_BAR_OFF2 + (2 * G2_STAGES + 4 + 2 * G2_SCHED + 2) * 8 + 16 + G2_SCHED * 4 + 1024;
+constexpr int G2_SMEM = G2_BAR_OFF2 + (2 * G2_STAGES + 4 + 2 * G2_SCHED + 4) * 8 + 16 + G2_SCHED * 4 + 1024;
 constexpr int G2_SCHED_SLOTS = 1024;   // {next tile, finished pairs} counter pairs, used round-robin by launches
 
 // G2_WHOLE_TILES (caller): never halve tiles - set for GEMMs that run beside a GEMM of another stream,
@@ -79,12 +79,18 @@ enum Gemm2Epi : int {
 // x 768 x 768 18.1 / 15.8, 8192 x 2048 over K = 1024 41.2 / 32.9, 1536 46.9 / 45.4, 2048 56.4 / 56.8, 4096 x 4096 x 4096 103.3 /
 // 103.4; rotation 8192 x 1280 x 768 23.7 / 21.1, 8192 x 3072 x 2048 83.6 / 81.1, 4096 x 6144 x 4096 154.6 / 152.2, but 4096 x
 // 3072 x 2048 45.1 / 46.3 and 1000 x 6144 x 4096 49.5 / 51.3: over a long K the missing stage and the epilogue weigh the same.
-// The SwiGLU forms stay with one (backward 8192 x 5504 x 2048 165 us, 176 with two; forward 256 / 263): their epilogue is not
-// what the tensor pipe waits for.
-constexpr int g2_wgs(int epi) { return epi == EPI_ROPE || epi == EPI_DELTA || epi == EPI_ADD ? 2 : 1; }
+// EPI_SWIGLU stays with one (8192 x 5504 over K = 2048 256 us, 263 with two): a tile of it takes as long as its 480 KiB of
+// operands and results need to and from L2 (57 bytes a clock and SM), whatever its epilogue does.
+// EPI_SWIGLU_BWD has two that share each 64-column group, and a warp of its own for their TMA accesses: with one warpgroup
+// that also fetched and stored, a tile's epilogue took 18000 clocks (each group waited 400 to 1200 for the store before it to
+// be read, each tile 2700 for its first group to arrive) where K = 768 gives the main loop 6100. us before / with both: 8192 x
+// 2048 x 768 52.7 / 44.4, 2048 x 2736 x 1024 27.4 / 22.7, 8192 x 5504 x 2048 165.7 / 167.7 (there the main loop is the longer
+// one either way); two warpgroups without the mover 46.7 / 23.4.
+constexpr bool g2_mover(int epi) { return epi == EPI_SWIGLU_BWD; }
+constexpr int g2_wgs(int epi) { return epi == EPI_ROPE || epi == EPI_DELTA || epi == EPI_ADD || epi == EPI_SWIGLU_BWD ? 2 : 1; }
 // Four staging tiles in place of two cost a stage of the operand ring (5 x 32 KiB + 4 x 16 KiB in place of 6 + 2).
-constexpr int g2_staging(int epi) { return g2_wgs(epi) == 2 || epi == EPI_SWIGLU_BWD ? 4 : 2; }
-constexpr int g2_threads(int epi) { return 64 + 128 * g2_wgs(epi); }
+constexpr int g2_staging(int epi) { return g2_wgs(epi) == 2 ? 4 : 2; }
+constexpr int g2_threads(int epi) { return 64 + 128 * g2_wgs(epi) + (g2_mover(epi) ? 32 : 0); }
 
 struct Gemm2Params {
   void* D;
@@ -264,6 +270,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                      const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmE,
                      const Gemm2Params p) {
   constexpr int kWgs = g2_wgs(EPI);
+  constexpr bool kMover = g2_mover(EPI);
   constexpr int kStg = g2_staging(EPI);
   constexpr int kStages = kStg == 4 ? G2_STAGES - 1 : G2_STAGES;
   constexpr int kStgOff = kStages * G2_STAGE_BYTES;
@@ -277,7 +284,8 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   uint64_t* sched_full = tempty + 2;
   uint64_t* sched_empty = sched_full + G2_SCHED;
   uint64_t* stage_ready = sched_empty + G2_SCHED;      // [kStg]: epilogue staging tile holds its input (or is simply free)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stage_ready + kStg);
+  uint64_t* stage_full = stage_ready + 2;              // EPI_SWIGLU_BWD, [2]: the epilogue has written a pair of tiles
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stage_ready + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* tile_ring = reinterpret_cast<volatile int*>(tmem_slot + 2);
 
@@ -308,9 +316,11 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
     for (int i = 0; i < G2_SCHED; ++i) {
       mbar_init(&sched_full[i], 1);
-      mbar_init(&sched_empty[i], 2 + 8 * kWgs);
+      mbar_init(&sched_empty[i], 2 + 8 * kWgs + (kMover ? 2 : 0));
     }
-    for (int i = 0; i < kStg; ++i) mbar_init(&stage_ready[i], 1);
+    for (int i = 0; i < (kMover ? 2 : kStg); ++i) mbar_init(&stage_ready[i], 1);
+    if (kMover)
+      for (int i = 0; i < 2; ++i) mbar_init(&stage_full[i], 128 * kWgs);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
@@ -433,6 +443,58 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         umma_commit_pair(&tfull[acc]);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
+    }
+  } else if (kMover && warp == 2 + 4 * kWgs) {
+    // ------------------------------------------------------------ mover: every TMA access of the EPI_SWIGLU_BWD epilogue (both CTAs)
+    if (lane == 0) {
+      uint8_t* stg = smem + kStgOff;
+      TileRingReader rd;
+      // Groups of 64 columns, two pairs of staging tiles in turn: fetches the gate and value of a group, stores what the
+      // epilogue has made of them, and fetches the group after next, which may belong to the next item (handed out while the
+      // present one's operands were loaded).
+      int tf = pair, gf = 0;                         // the next group to fetch
+      uint32_t nf = 0;
+      auto fetch = [&]() {
+        const G2Item wi = g2_item(tf, p.t_full, num_m, num_n);
+        const int x = wi.n0 + gf * 64, y = wi.mb * 2 * G2_BM + int(rank) * G2_BM;
+        const uint32_t b = nf & 1;
+        if (x < p.sw_I) {
+          mbar_expect_tx(&stage_ready[b], 2 * G2_STG_BYTES);
+          tma_load_2d(stg + 2 * b * G2_STG_BYTES, &tmBh, &stage_ready[b], x, y);
+          tma_load_2d(stg + (2 * b + 1) * G2_STG_BYTES, &tmE, &stage_ready[b], x, y);
+        } else {                                     // wholly past the edge: nothing to fetch, nothing is stored
+          mbar_arrive(&stage_ready[b]);
+        }
+        ++nf;
+        if (++gf == wi.bn / 64) {
+          gf = 0;
+          tf = dyn ? rd.next(sched_full, sched_empty, tile_ring, abort_flag, false, true, rank != 0) : tf + num_pairs;
+        }
+      };
+      int ts[2], gs[2];                              // the groups that are in the pairs
+      for (int i = 0; i < 2; ++i) {
+        ts[i] = tf;
+        gs[i] = gf;
+        if (tf >= 0 && tf < num_tiles) fetch();
+      }
+      for (uint32_t n = 0;; ++n) {
+        const uint32_t b = n & 1;
+        if (ts[b] < 0 || ts[b] >= num_tiles || !mbar_wait(&stage_full[b], (n >> 1) & 1, abort_flag)) break;
+        const G2Item wi = g2_item(ts[b], p.t_full, num_m, num_n);
+        const int x = wi.n0 + gs[b] * 64, y = wi.mb * 2 * G2_BM + int(rank) * G2_BM;
+        if (x < p.sw_I) {
+          tma_store_2d(&tmD, stg + 2 * b * G2_STG_BYTES, x, y);
+          tma_store_2d(&tmC, stg + (2 * b + 1) * G2_STG_BYTES, x, y);
+        }
+        tma_store_commit();
+        ts[b] = tf;
+        gs[b] = gf;
+        if (tf >= 0 && tf < num_tiles) {
+          tma_store_wait_read<0>();
+          fetch();
+        }
+      }
+      tma_store_wait<0>();
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5 or 2..9, both CTAs)
@@ -617,67 +679,40 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       if (elected) tma_store_wait<0>();
     } else if constexpr (EPI == EPI_SWIGLU_BWD) {
       // The accumulator is d(act) for 256 rows x 256 columns. Per 64-column group the stored gate and value tiles
-      // (bf16, the two halves of the forward projection; maps tmBh / tmE) are fetched by TMA into a pair of staging
-      // tiles, turned in place into d(gate) and d(value) and stored (maps tmD / tmC). Two pairs alternate: the next
-      // group's pair is fetched while this one is computed.
+      // (bf16, the two halves of the forward projection; maps tmBh / tmE) come by TMA into a pair of staging
+      // tiles, are turned in place into d(gate) and d(value), half of the columns by either warpgroup, and leave (maps tmD /
+      // tmC). Two pairs alternate; the mover fetches and stores them.
       uint8_t* stg = smem + kStgOff;
       const int r = q * 32 + lane;
       const uint32_t swz = uint32_t(r & 7);
-      const bool elected = (warp == 2 && lane == 0);
+      constexpr int kCols = 64 / kWgs;                   // this thread's columns of a group
       uint32_t ucount = 0;                               // groups handled so far; pair = ucount & 1
-      auto fetch = [&](uint32_t uc, int x, int y) {      // by the elected thread: fill pair uc & 1 for a group
-        const uint32_t b = (uc & 1) * 2;
-        if (x < p.sw_I) {
-          mbar_expect_tx(&stage_ready[b], G2_STG_BYTES);
-          tma_load_2d(stg + b * G2_STG_BYTES, &tmBh, &stage_ready[b], x, y);
-          mbar_expect_tx(&stage_ready[b + 1], G2_STG_BYTES);
-          tma_load_2d(stg + (b + 1) * G2_STG_BYTES, &tmE, &stage_ready[b + 1], x, y);
-        } else {                                         // wholly past the edge: nothing to fetch, nothing is stored
-          mbar_arrive(&stage_ready[b]);
-          mbar_arrive(&stage_ready[b + 1]);
-        }
-      };
       for (int t = pair; ok && t >= 0 && t < num_tiles;
            t = dyn ? rd.next(sched_full, sched_empty, tile_ring, abort_flag, true, lane == 0, rank != 0)
                    : t + num_pairs) {
-        const G2Item wi = g2_item(t, p.t_full, num_m, num_n);
-        const int row0 = wi.mb * 2 * G2_BM + int(rank) * G2_BM;
-        const int n0 = wi.n0;
-        const int ngroups = wi.bn / 64;
-        if (elected) {
-          tma_store_wait_read<1>();                      // the stores that last used this pair have read it
-          fetch(ucount, n0, row0);
-        }
+        const int ngroups = t < p.t_full ? 4 : 2;
         if (!mbar_wait(&tfull[acc], acc_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN;
+        const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16) + acc * G2_BN + wg * kCols;
 #pragma unroll 1
         for (int g = 0; g < ngroups; ++g) {
-          const uint32_t b = (ucount & 1) * 2;
-          if (elected && g + 1 < ngroups) {              // prefetch the next group's pair
-            tma_store_wait_read<0>();                    // the other pair's stores (previous group) have read it
-            fetch(ucount + 1, n0 + (g + 1) * 64, row0);
-          }
-          uint32_t v[64];
-          tmem_ld_32x32b_x32(taddr + g * 64, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-          tmem_ld_32x32b_x32(taddr + g * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+          const uint32_t b = ucount & 1;
+          uint32_t v[kCols];
+#pragma unroll
+          for (int c = 0; c < kCols; c += 32) tmem_ld_32x32b_x32(taddr + g * 64 + c, *reinterpret_cast<uint32_t(*)[32]>(&v[c]));
           tmem_ld_wait();
           if (g == ngroups - 1) {                        // accumulator fully read: hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty[acc]), 0));
           }
-          const uint32_t ph = (ucount >> 1) & 1;
-          if (!mbar_wait(&stage_ready[b], ph, abort_flag) || !mbar_wait(&stage_ready[b + 1], ph, abort_flag)) {
-            ok = false;
-            break;
-          }
-          uint8_t* grow = stg + b * G2_STG_BYTES + r * 128;
+          if (!mbar_wait(&stage_ready[b], (ucount >> 1) & 1, abort_flag)) { ok = false; break; }
+          uint8_t* grow = stg + 2 * b * G2_STG_BYTES + r * 128;
           uint8_t* vrow = grow + G2_STG_BYTES;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            uint4* gp = reinterpret_cast<uint4*>(grow + ((uint32_t(c) ^ swz) << 4));
-            uint4* vp = reinterpret_cast<uint4*>(vrow + ((uint32_t(c) ^ swz) << 4));
+          for (int c = 0; c < kCols / 8; ++c) {
+            const uint32_t at = (uint32_t(wg * (kCols / 8) + c) ^ swz) << 4;
+            uint4 *gp = reinterpret_cast<uint4*>(grow + at), *vp = reinterpret_cast<uint4*>(vrow + at);
             uint4 gq = *gp, vq = *vp;
             bf162* g2 = reinterpret_cast<bf162*>(&gq);
             bf162* v2 = reinterpret_cast<bf162*>(&vq);
@@ -694,20 +729,11 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             *vp = vq;
           }
           fence_proxy_async_smem();
-          named_bar_sync_128(1);
-          if (elected) {
-            const int x = n0 + g * 64;
-            if (x < p.sw_I) {
-              tma_store_2d(&tmD, stg + b * G2_STG_BYTES, x, row0);
-              tma_store_2d(&tmC, stg + (b + 1) * G2_STG_BYTES, x, row0);
-            }
-            tma_store_commit();
-          }
+          mbar_arrive(&stage_full[b]);
           ++ucount;
         }
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
-      if (elected) tma_store_wait<0>();
     } else
     if (kWgs == 2 || (p.flags & G2_TMA_OUT)) {
       // Output through shared memory and TMA. A tile leaves in groups of 128 bytes per row (64 bf16

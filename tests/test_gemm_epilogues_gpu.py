@@ -1,4 +1,4 @@
-"""Epilogues of the CTA-pair GEMM with two warpgroups (addend fetched ahead, delta, rotation) against fp64: part-filled
+"""Epilogues of the CTA-pair GEMM with two warpgroups (addend fetched ahead, delta, rotation, SwiGLU backward) against fp64: part-filled
 tiles, several rounds, last rounds of half tiles, inner dimensions on both sides of the dispatch."""
 import pytest
 import torch
@@ -73,3 +73,20 @@ def test_rotation(D, B, T, QH, KVH, K):
     lim = torch.cat([e1 + e2, e1 + e2], -1).reshape(M, cols) + (x1.abs() + x2.abs()).repeat(1, 1, 2).reshape(M, cols) * 2.0 ** -22
     assert ((y[:, :cols] - ref).abs() <= lim + BF_ULP * ref.abs() + 1e-30).all()
     assert ((y[:, cols:] - want[:, cols:]).abs() <= bound[:, cols:] + BF_ULP * want[:, cols:].abs() + 1e-30).all()
+
+
+# part-filled groups of 64 columns and groups wholly past the edge (264, 336), one item and several per pair, K of one block
+@pytest.mark.parametrize("M,I", [(256, 256), (300, 264), (513, 336), (2304, 2304), (4100, 2736)])
+@pytest.mark.parametrize("K", [64, 72, 768, 2048])
+def test_swiglu_backward(M, I, K):
+    dout, w, gv = bf(M, K, seed=1, scale=0.1), bf(I, K, seed=2, scale=0.1), bf(M, 2 * I, seed=3, scale=2.0)
+    got = G.gemm_swiglu_bwd(dout, w, gv).double()
+    d, bound = product(dout, w.t())
+    gate, value = gv[:, :I].double(), gv[:, I:].double()
+    s = torch.sigmoid(gate)
+    for out, f in ((got[:, :I], value * s * (1 + gate * (1 - s))), (got[:, I:], gate * s)):
+        # the sums' error times the factor, the factor's own (exp, reciprocal and four products in fp32), the rounding; the
+        # terms of the gate's factor cancel, hence the bound on their size
+        size = (value if out.data_ptr() == got.data_ptr() else torch.ones_like(gate)).abs() * s * (1 + gate.abs())
+        lim = bound * f.abs() + d.abs() * size * 2.0 ** -19 + BF_ULP * (d * f).abs() + 1e-30
+        assert ((out - d * f).abs() <= lim).all()
