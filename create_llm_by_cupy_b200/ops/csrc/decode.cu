@@ -4,8 +4,9 @@
 // many loads are in flight - not bandwidth. So:
 //   * one cluster of CTAs per (sequence, KV head), every CTA and every warp of it taking its own 32-key tiles
 //     (a prefix of n keys is n / 32 independent chains instead of four);
-//   * all query heads of the group share each K / V row that was loaded (up to 4 heads per CTA), with 16-byte
-//     loads, half a tile in flight per lane;
+//   * all query heads of the group share each K / V row that was loaded (up to 4 heads per CTA). A tile is one run of bytes
+//     in the cache: a warp asks for K and V of its first tile with two bulk copies as soon as its inputs are ready and for the
+//     next one when it has read them (through registers a tile was four round trips one after the other);
 //   * the scores of a tile are mma.sync products (rows = heads, columns = keys, fp32 sums): a lane's 16-byte pieces of
 //     q and of the keys are fragments as they stand, because a dot product does not care in which order the head
 //     dimension is walked as long as both sides walk it alike. No exchange between lanes is left before the softmax
@@ -13,20 +14,20 @@
 //     multiply V on the FMA units;
 //   * the partial softmax states (maximum, sum, weighted values) meet in shared memory, first over the warps of
 //     a CTA, then over the CTAs of the cluster through distributed shared memory: no workspace, no second launch.
-// The previous kernel had one CTA of four warps per QUERY head, each warp walking its keys one by one through a
-// five-step shuffle and an exponential. Device time before -> now: B = 1, 16 / 4 heads of 128, 1801 keys 352 -> 11 us;
-// B = 8, 32 / 8 heads of 128, 3001 keys (98 MB of cache, 15 us at the copy rate) 742 -> 28 us (59 with the scores on the
-// FMA units and a second, part-filled round of CTAs at 160 registers); B = 1, 12 / 4 heads of 64, 101 keys 20 -> 7 us.
+// Device time inside a block, us, tiles through registers -> shared memory: B = 8, 32 / 8 heads of 128, 3001 keys (98 MB of
+// cache, 15 us at the copy rate) 35.0 -> 26.2, B = 16, 4001 keys 73.9 -> 51.9, B = 2, 65 keys 21.7 -> 11.4; B = 1, 16 / 4 heads
+// of 128, 1801 keys 11.7 -> 10.0, B = 16, 1001 keys 17.8 -> 16.3; 12 / 4 heads of 64 6.8 to 8.5 before and after.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "ptx.cuh"
 
 namespace b200 {
 namespace cg = cooperative_groups;
 
 constexpr int DA_MAX_WARPS = 16;
 constexpr int DA_TILE = 32;          // keys per warp and step
-constexpr int DA_PREFETCH = 4;       // tiles per warp that are asked for before the kernel's inputs are ready
+constexpr int DA_PREFETCH = 4;       // tiles per warp that are on their way to L2 before the kernel's inputs are ready
 
 struct DecodeParams {
   const bf16* q;        // [B, QH, D]
@@ -44,6 +45,7 @@ struct DecodeParams {
   const float* cosr;            // rotary table rows of `pos`, [D / 2]
   const float* sinr;
   int ld, pos;
+  int* status;
 };
 
 __device__ __forceinline__ void unpack16B(const uint4& u, float (&f)[8]) {
@@ -88,23 +90,30 @@ __device__ __forceinline__ uint4 rotated_chunk(const bf16* x, int dl, const floa
   return pack16B(y);
 }
 
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_u32(dst)), "l"(__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
+
 template <int RT>
 struct alignas(RT * 4) HeadRow {     // one key's scores / weights, one vector load
   float v[RT];
 };
 
-// 128 registers: four CTAs of four warps, or one of sixteen, fit an SM.
-// grid (cluster size, KVH * groups, B), cluster (cluster size, 1, 1), block 32 * warps (any number up to 16).
+// grid (cluster size, KVH * groups, B), cluster (cluster size, 1, 1), block 32 * warps (any number up to 16), dynamic shared
+// memory warps * 2 tiles.
 template <int D, int RT, bool APPEND>
 __global__ void __maxnreg__(128)
 decode_attn_kernel(const DecodeParams p) {
   constexpr int LPK = D / 8;                 // lanes per key, 16 bytes each
   constexpr int KPS = 32 / LPK;              // keys per load step
   constexpr int STEPS = DA_TILE / KPS;       // 16 / 8 / 4 for D = 128 / 64 / 32
-  constexpr int HALF = STEPS >= 16 ? 8 : STEPS;    // loads in flight per lane
+  constexpr int TB = DA_TILE * D * 2;        // bytes of a tile of K or V
+  extern __shared__ __align__(128) uint8_t tiles[];     // [warp]: a tile of K, a tile of V; then the warp's weighted values
+  __shared__ uint64_t full[DA_MAX_WARPS][2];            // K, V of the warp's tile have arrived
+  __shared__ int abort_flag;
   __shared__ HeadRow<RT> s_p[DA_MAX_WARPS][DA_TILE];
   __shared__ float s_m[DA_MAX_WARPS][RT], s_l[DA_MAX_WARPS][RT];
-  __shared__ float s_o[DA_MAX_WARPS][RT][D];
   __shared__ float c_m[RT], c_l[RT], c_o[RT][D];        // this CTA's state, read by the cluster
 
   cg::cluster_group cluster = cg::this_cluster();
@@ -122,8 +131,28 @@ decode_attn_kernel(const DecodeParams p) {
     for (int i = 0, t = rank + warp * cs; i < DA_PREFETCH && t * DA_TILE <= p.pos; ++i, t += nw * cs)
       l2_prefetch(rows + size_t(t) * DA_TILE * D, uint32_t(min(DA_TILE, p.pos + 1 - t * DA_TILE)) * D * 2);
   }
+  if (lane < 2) mbar_init(&full[warp][lane], 1);
+  if (threadIdx.x == 0) abort_flag = 0;
+  mbar_fence_init();
+  __syncthreads();
   pdl_wait();
   const int len = min(p.lens[b], p.Tmax);
+  uint8_t* kt = tiles + size_t(warp) * 2 * TB;
+  uint8_t* vt = kt + TB;
+  const bf16* kb = p.kc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
+  const bf16* vb = p.vc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
+  // A tile of K (which 0) or V (1): its valid keys are one run of bytes. By the first lane; the row of the new token may still
+  // be in writing, nobody uses what arrives for it.
+  auto fetch = [&](int t, int which) {
+    if (t * DA_TILE >= len) return;
+    const uint32_t bytes = uint32_t(min(DA_TILE, len - t * DA_TILE)) * D * 2;
+    mbar_expect_tx(&full[warp][which], bytes);
+    bulk_load(which == 0 ? kt : vt, (which == 0 ? kb : vb) + size_t(t) * DA_TILE * D, bytes, &full[warp][which]);
+  };
+  if (lane == 0) {
+    fetch(rank + warp * cs, 0);
+    fetch(rank + warp * cs, 1);
+  }
 
   __shared__ uint4 s_new[2][LPK];                       // the new token's rotated k and v
   const bf16* new_row = nullptr;
@@ -158,44 +187,32 @@ decode_attn_kernel(const DecodeParams p) {
   for (int r = 0; r < RT; ++r)
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[r][e] = 0.f;
-  const bf16* kb = p.kc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
-  const bf16* vb = p.vc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
-
-  auto piece = [&](const bf16* rows, int which, int key, int chunk) {      // 16 bytes of a key's row
-    uint4 u = make_uint4(0u, 0u, 0u, 0u);
-    if (key < len) {
-      if (APPEND && key == p.pos) u = s_new[which][chunk];
-      else u = reinterpret_cast<const uint4*>(rows + size_t(key) * D)[chunk];
-    }
-    return u;
+  // 16 bytes of a key's row, from the warp's tile or, for the new token, from this launch
+  auto piece = [&](const uint8_t* tile, int which, int key0, int k, int chunk) {
+    const uint4* at = reinterpret_cast<const uint4*>(tile + k * D * 2) + chunk;
+    if (APPEND && key0 + k == p.pos) at = &s_new[which][chunk];
+    return *at;
   };
 
   // tile t goes to CTA t % cs, warp (t / cs) % nw: neighbouring tiles on different SMs
-  for (int t = rank + warp * cs; t * DA_TILE < len; t += nw * cs) {
+  uint32_t phase = 0;
+  for (int t = rank + warp * cs; t * DA_TILE < len; t += nw * cs, phase ^= 1) {
     const int key0 = t * DA_TILE;
     float sc[4][4];                                     // keys 8 nb + 2 tl, + 1 of head hl in [nb][0], [nb][1]
-    uint4 vbuf[HALF];
+    if (!__all_sync(0xffffffffu, mbar_wait(&full[warp][0], phase, &abort_flag))) break;
 #pragma unroll
-    for (int nb0 = 0; nb0 < 4; nb0 += 2) {
-      uint4 kbuf[2][QC];
+    for (int nb = 0; nb < 4; ++nb) {
 #pragma unroll
-      for (int n = 0; n < 2; ++n)
+      for (int e = 0; e < 4; ++e) sc[nb][e] = 0.f;
 #pragma unroll
-        for (int i = 0; i < QC; ++i) kbuf[n][i] = piece(kb, 0, key0 + (nb0 + n) * 8 + hl, tl + 4 * i);
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sc[nb0 + n][e] = 0.f;
-#pragma unroll
-        for (int i = 0; i < QC; ++i) {
-          mma_scores(sc[nb0 + n], qa[i][0], qa[i][1], kbuf[n][i].x, kbuf[n][i].y);
-          mma_scores(sc[nb0 + n], qa[i][2], qa[i][3], kbuf[n][i].z, kbuf[n][i].w);
-        }
+      for (int i = 0; i < QC; ++i) {
+        const uint4 kf = piece(kt, 0, key0, nb * 8 + hl, tl + 4 * i);      // past the length: masked below
+        mma_scores(sc[nb], qa[i][0], qa[i][1], kf.x, kf.y);
+        mma_scores(sc[nb], qa[i][2], qa[i][3], kf.z, kf.w);
       }
     }
-    // the first values travel while the softmax of the tile is formed
-#pragma unroll
-    for (int s = 0; s < HALF; ++s) vbuf[s] = piece(vb, 1, key0 + s * KPS + kl, dl);
+    __syncwarp();                                       // the tile of K has been read
+    if (lane == 0) fetch(t + nw * cs, 0);
     float mx = -INFINITY;
 #pragma unroll
     for (int nb = 0; nb < 4; ++nb)
@@ -226,24 +243,22 @@ decode_attn_kernel(const DecodeParams p) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[r][e] *= cr;
     }
+    if (!__all_sync(0xffffffffu, mbar_wait(&full[warp][1], phase, &abort_flag))) break;
 #pragma unroll
-    for (int half = 0; half < STEPS; half += HALF) {
-      if (half > 0) {
+    for (int st = 0; st < STEPS; ++st) {
+      const int k = st * KPS + kl;
+      uint4 u = piece(vt, 1, key0, k, dl);
+      if (key0 + k >= len) u = make_uint4(0u, 0u, 0u, 0u);     // never written: its weight is 0, but 0 times anything is not
+      float vf[8];
+      unpack16B(u, vf);
+      const HeadRow<RT> w = s_p[warp][k];
 #pragma unroll
-        for (int s = 0; s < HALF; ++s) vbuf[s] = piece(vb, 1, key0 + (half + s) * KPS + kl, dl);
-      }
+      for (int r = 0; r < RT; ++r)
 #pragma unroll
-      for (int s = 0; s < HALF; ++s) {
-        float vf[8];
-        unpack16B(vbuf[s], vf);
-        const HeadRow<RT> w = s_p[warp][(half + s) * KPS + kl];
-#pragma unroll
-        for (int r = 0; r < RT; ++r)
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc[r][e] += w.v[r] * vf[e];
-      }
+        for (int e = 0; e < 8; ++e) acc[r][e] += w.v[r] * vf[e];
     }
-    __syncwarp();                                       // the next tile overwrites s_p
+    __syncwarp();                                       // the next tile overwrites s_p and the tile of V
+    if (lane == 0) fetch(t + nw * cs, 1);
   }
 
   // Here, not at the top: CTAs that arrive while these fill the SMs land unevenly (see gemm_skinny.cu). The first warp of a
@@ -259,7 +274,7 @@ decode_attn_kernel(const DecodeParams p) {
     for (int e = 0; e < 8; ++e) {
 #pragma unroll
       for (int o = LPK; o < 32; o <<= 1) acc[r][e] += __shfl_xor_sync(0xffffffffu, acc[r][e], o);
-      if (kl == 0) s_o[warp][r][dl * 8 + e] = acc[r][e];
+      if (kl == 0) reinterpret_cast<float*>(kt)[r * D + dl * 8 + e] = acc[r][e];      // every copy into it has been waited for
     }
   }
   __syncthreads();
@@ -272,7 +287,7 @@ decode_attn_kernel(const DecodeParams p) {
     for (int w = 0; w < nw; ++w) {
       const float f = __expf(s_m[w][r] - ref);
       ls += s_l[w][r] * f;
-      o += s_o[w][r][d] * f;
+      o += reinterpret_cast<const float*>(tiles + size_t(w) * 2 * TB)[r * D + d] * f;
     }
     c_o[r][d] = o;
     if (d == 0) { c_m[r] = mx; c_l[r] = ls; }
@@ -295,25 +310,36 @@ decode_attn_kernel(const DecodeParams p) {
     p.out[(size_t(b) * p.QH + h0 + r) * D + d] = __float2bfloat16(len <= 0 ? 0.f : o / ls);
   }
   cluster.sync();                                       // peers still read this CTA's state until here
+  if (threadIdx.x == 0 && abort_flag != 0 && p.status != nullptr && atomicCAS(p.status, 0, abort_flag) == 0) p.status[1] = 330;
 }
 
 template <int D, int RT>
 static int launch_decode(DecodeParams p, int B, cudaStream_t st) {
   p.groups = (p.QH / p.KVH + RT - 1) / RT;
   const long pairs = long(B) * p.KVH * p.groups;
-  const int tiles = (p.Tmax + DA_TILE - 1) / DA_TILE;
-  // Up to 8 CTAs per (sequence, KV head): doubled while there are fewer than four per SM in all (as many fit, at four
-  // warps) and the cache has more tiles than CTAs. Up to 16 warps per CTA while at most one CTA per SM exists, else 4 (they
-  // share the SM's registers).
+  const int keys = p.kqv != nullptr ? p.pos + 1 : p.Tmax;       // what the lengths are expected to be, at most; longer ones work too
+  const int tiles = (keys + DA_TILE - 1) / DA_TILE;
+  // Up to 8 CTAs per (sequence, KV head): doubled while there are more tiles than CTAs and one CTA per SM of head_dim 128 (two
+  // of 64, four of 32: the same bytes) is not exceeded yet. At least four warps (they also form the result), up to 128 KiB of
+  // tiles while at most one CTA per SM exists. Swept for the attention alone, us: 8 sequences, 8 KV heads of 128, 3001 keys 34.8
+  // with 256 CTAs of four warps (45.1 with 512, 36.9 with 512 of two); 16 x 4 heads, 1001 keys 21.2 with 256 of four (28.7 with
+  // 512 of four); 4 x 4 heads, 301 keys 14.3 with four warps (22.5 with eight: their 128 KiB have to wait for an empty SM).
+  constexpr int kTiles = 2 * DA_TILE * D * 2;
+  constexpr int kMaxWarps = 131072 / kTiles < DA_MAX_WARPS ? 131072 / kTiles : DA_MAX_WARPS;
   int cs = 1;
-  while (cs < 8 && cs < tiles && pairs * cs < 4L * num_sms()) cs *= 2;
+  while (cs < 8 && cs < tiles && pairs * cs * kTiles <= 16384L * num_sms()) cs *= 2;
   int warps = (tiles + cs - 1) / cs;
-  const int cap = pairs * cs <= num_sms() ? DA_MAX_WARPS : 4;
+  const int cap = pairs * cs <= num_sms() ? kMaxWarps : 4;
   if (warps > cap) warps = cap;
-  if (warps < 1) warps = 1;
+  if (warps < 4) warps = 4;
   if (p.KVH * p.groups > 65535 || B > 65535) return static_cast<int>(cudaErrorInvalidValue);
   const auto kern = p.kqv != nullptr ? decode_attn_kernel<D, RT, true> : decode_attn_kernel<D, RT, false>;
-  return static_cast<int>(launch_pdl(kern, dim3(cs, p.KVH * p.groups, B), dim3(32 * warps), 0, st, cs, p));
+  static const cudaError_t set[2] = {
+      cudaFuncSetAttribute(decode_attn_kernel<D, RT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWarps * kTiles),
+      cudaFuncSetAttribute(decode_attn_kernel<D, RT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWarps * kTiles)};
+  if (set[0] != cudaSuccess || set[1] != cudaSuccess) return static_cast<int>(set[0] != cudaSuccess ? set[0] : set[1]);
+  p.status = status_ptr();
+  return static_cast<int>(launch_pdl(kern, dim3(cs, p.KVH * p.groups, B), dim3(32 * warps), warps * kTiles, st, cs, p));
 }
 
 template <int D>
