@@ -7,7 +7,8 @@
 //     their fp32 sums through distributed shared memory, so a 768 x 768 weight is 48 CTAs and there is no
 //     workspace and no second launch;
 //   * 64 x 64 weight tiles (8 KiB) arrive through a ring of cp.async stages, several CTAs per SM, so that tens of
-//     KiB per SM are in flight;
+//     KiB per SM are in flight; with SwiGLU 32 k x (64 gate + 64 value columns), so that a row is read 128 bytes at a time
+//     there too (64 k x (32 + 32): 4096 x 22016, eight rows, 38.0 us where this takes 35.5; 2048 x 11008, 16 rows, 16.1 / 14.4);
 //   * the product runs as W^T x^T on mma.sync (16 weight columns x 8 tokens x 16 k, fp32 accumulation): one token
 //     costs the same instructions as eight, and both weight layouts feed the same fragments through ldmatrix.
 // One row, weights not in L2 (before: 128-row tiles): 768 x 768 6.8 -> 3.6 us, 2048 x 3072 13.3 -> 5.6, 2048 x 11008
@@ -35,12 +36,14 @@ struct SkinnyParams {
   float alpha;
 };
 
-template <int MT>
+template <int MT, bool GLU>
 struct SkinnySmem {
+  static constexpr int kTk = GLU ? 32 : SK_TK;                     // k per stage
+  static constexpr int kCols = GLU ? 2 * SK_TN : SK_TN;            // weight columns of a CTA
   static constexpr int kStages = MT <= 2 ? 6 : (MT == 4 ? 5 : 4);
   static constexpr int kABytes = MT * 8 * SK_TK * 2;
   static constexpr int kStageBytes = SK_W_BYTES + kABytes;
-  static constexpr int kSum = MT * 8 * SK_TN * 4;                  // fp32 [rows][64] for the cluster's sum
+  static constexpr int kSum = MT * 8 * kCols * 4;                  // fp32 [rows][columns] for the cluster's sum
   static constexpr int kTotal = kStages * kStageBytes > kSum ? kStages * kStageBytes : kSum;
   static constexpr int kPerSm = 228 * 1024 / (kTotal + 1024);      // CTAs that fit an SM: 4 up to 8 rows, then 3
 };
@@ -66,7 +69,8 @@ __device__ __forceinline__ uint32_t sw_addr(uint32_t base, int row, int chunk) {
   return base + uint32_t(row) * 128u + uint32_t((chunk ^ (row & 7)) * 16);
 }
 
-// One stage: the 64 x 64 weight tile and the [8 MT, 64] token tile at k0. Bytes past K, N or M arrive as zeros
+// One stage: 8 KiB of weights (64 k x 64 columns; GLU: 32 k x 64 gate columns, then the 64 value columns of the same index: 128
+// bytes of a row at a time either way) and the tokens' tile at k0. Bytes past K, N or M arrive as zeros
 // (cp.async with a short source size; the address of a skipped chunk is the matrix base).
 template <int MT, bool K_ROWS, bool GLU>
 __device__ __forceinline__ void skinny_load(const SkinnyParams& p, uint32_t stage, int n0, int k0, int k_end) {
@@ -74,13 +78,12 @@ __device__ __forceinline__ void skinny_load(const SkinnyParams& p, uint32_t stag
 #pragma unroll
   for (int i = 0; i < SK_W_BYTES / 16 / SK_THREADS; ++i) {
     const int idx = tid + i * SK_THREADS, row = idx >> 3, chunk = idx & 7;
-    const int k = K_ROWS ? k0 + row : k0 + chunk * 8;
+    const int k = GLU ? k0 + (row & 31) : (K_ROWS ? k0 + row : k0 + chunk * 8);
     int n = K_ROWS ? n0 + chunk * 8 : n0 + row;
     int left;                                             // elements of this chunk inside the matrix
-    if (GLU) {                                            // 32 gate columns beside the 32 value columns of the same index
-      n = n0 + (chunk & 3) * 8;
+    if (GLU) {
       left = k < k_end ? p.I - n : 0;
-      n += chunk < 4 ? 0 : p.I;
+      n += row < 32 ? 0 : p.I;
     } else if (K_ROWS) left = k < k_end ? p.N - n : 0;
     else left = n < p.N ? k_end - k : 0;
     left = left < 0 ? 0 : (left > 8 ? 8 : left);
@@ -88,8 +91,9 @@ __device__ __forceinline__ void skinny_load(const SkinnyParams& p, uint32_t stag
     cp_async16(sw_addr(stage, row, chunk), src, left * 2);
   }
   const uint32_t sa = stage + SK_W_BYTES;
-  for (int idx = tid; idx < MT * 8 * 8; idx += SK_THREADS) {
-    const int row = idx >> 3, chunk = idx & 7, k = k0 + chunk * 8;
+  constexpr int kChunks = SkinnySmem<MT, GLU>::kTk / 8;
+  for (int idx = tid; idx < MT * 8 * kChunks; idx += SK_THREADS) {
+    const int row = idx / kChunks, chunk = idx % kChunks, k = k0 + chunk * 8;
     int left = row < p.M ? k_end - k : 0;
     left = left < 0 ? 0 : (left > 8 ? 8 : left);
     cp_async16(sw_addr(sa, row, chunk), left > 0 ? p.A + size_t(row) * p.lda + k : p.A, left * 2);
@@ -100,31 +104,33 @@ __device__ __forceinline__ void skinny_load(const SkinnyParams& p, uint32_t stag
 template <int MT, bool K_ROWS, bool GLU>
 __global__ void __launch_bounds__(SK_THREADS)
 gemm_skinny_kernel(const SkinnyParams p) {
-  using S = SkinnySmem<MT>;
+  using S = SkinnySmem<MT, GLU>;
   extern __shared__ __align__(128) uint8_t smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int ks = int(gridDim.x), rank = int(blockIdx.x);
-  constexpr int kOut = GLU ? SK_TN / 2 : SK_TN;  // output columns of a CTA
-  const int n0 = int(blockIdx.y) * kOut;
+  const int n0 = int(blockIdx.y) * SK_TN;       // output columns of a CTA: 64
   const int k_begin = rank * p.kslice, k_end = min(p.K, k_begin + p.kslice);
-  const int steps = k_end > k_begin ? (k_end - k_begin + SK_TK - 1) / SK_TK : 0;
+  const int steps = k_end > k_begin ? (k_end - k_begin + S::kTk - 1) / S::kTk : 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t base = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
 
-  float acc[MT][4];
+  constexpr int kHalves = GLU ? 2 : 1;           // gate and value columns
+  float acc[kHalves][MT][4];
 #pragma unroll
-  for (int t = 0; t < MT; ++t)
+  for (int h = 0; h < kHalves; ++h)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) acc[t][e] = 0.f;
+    for (int t = 0; t < MT; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[h][t][e] = 0.f;
 
   pdl_wait();
-  // Short slices: the next kernel's CTAs settle while this one's loads are in flight. Long ones fill the GPU with several
-  // CTAs per SM; CTAs that arrive among them land unevenly and run so (a 7B block 121.5 -> 116 us with the trigger here,
-  // 113 with it behind the loop), so the next kernel is let in at the end.
-  if (steps <= 2 * S::kStages) pdl_trigger();
+  // No pdl_trigger(): the next kernel's CTAs then start as these end. Let in before that, they land unevenly among this one's,
+  // take shared memory and issue slots from what is still running and run unevenly themselves. us with the trigger here for
+  // slices of up to 12 stages and behind the loop for longer ones / without: a 7B block of 8 sequences 113.2 / 104.3, of one
+  // 88.9 / 86.6, a 1.3B block of one 43.4 / 40.8, of 16 54.4 / 52.9, one token through the 125M model 349 / 337 on the device.
 #pragma unroll
   for (int s = 0; s < S::kStages - 1; ++s) {
-    if (s < steps) skinny_load<MT, K_ROWS, GLU>(p, base + s * S::kStageBytes, n0, k_begin + s * SK_TK, k_end);
+    if (s < steps) skinny_load<MT, K_ROWS, GLU>(p, base + s * S::kStageBytes, n0, k_begin + s * S::kTk, k_end);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   const int mi = lane >> 3, mr = lane & 7;       // ldmatrix: matrix and row that this lane addresses
@@ -133,10 +139,10 @@ gemm_skinny_kernel(const SkinnyParams p) {
     __syncthreads();                             // stage s has landed; everyone has left stage s - 1
     const int nx = s + S::kStages - 1;
     if (nx < steps)
-      skinny_load<MT, K_ROWS, GLU>(p, base + (nx % S::kStages) * S::kStageBytes, n0, k_begin + nx * SK_TK, k_end);
+      skinny_load<MT, K_ROWS, GLU>(p, base + (nx % S::kStages) * S::kStageBytes, n0, k_begin + nx * S::kTk, k_end);
     asm volatile("cp.async.commit_group;" ::: "memory");
     const uint32_t sw = base + (s % S::kStages) * S::kStageBytes, sa = sw + SK_W_BYTES;
-    uint32_t w[SK_TK / 16][4];
+    uint32_t w[SK_TK / 16][4];                   // GLU: gate k 0-15, 16-31, then value
 #pragma unroll
     for (int kk = 0; kk < SK_TK / 16; ++kk) {
       // A fragment of 16 weight columns x 16 k: matrices (columns 0-7, k 0-7), (8-15, 0-7), (0-7, 8-15), (8-15, 8-15)
@@ -145,36 +151,43 @@ gemm_skinny_kernel(const SkinnyParams p) {
     }
 #pragma unroll
     for (int t = 0; t < MT; ++t) {
-      uint32_t x0[4], x1[4];                     // tokens 8 t .. 8 t + 7, k 0-31 and 32-63
+      uint32_t x0[4];                            // tokens 8 t .. 8 t + 7, k 0-31
       ldsm4(x0, sw_addr(sa, t * 8 + mr, mi));
-      ldsm4(x1, sw_addr(sa, t * 8 + mr, 4 + mi));
-      mma16816(acc[t], w[0], x0[0], x0[1]);
-      mma16816(acc[t], w[1], x0[2], x0[3]);
-      mma16816(acc[t], w[2], x1[0], x1[1]);
-      mma16816(acc[t], w[3], x1[2], x1[3]);
+      mma16816(acc[0][t], w[0], x0[0], x0[1]);
+      mma16816(acc[0][t], w[1], x0[2], x0[3]);
+      if constexpr (GLU) {
+        mma16816(acc[1][t], w[2], x0[0], x0[1]);
+        mma16816(acc[1][t], w[3], x0[2], x0[3]);
+      } else {
+        uint32_t x1[4];                          // k 32-63
+        ldsm4(x1, sw_addr(sa, t * 8 + mr, 4 + mi));
+        mma16816(acc[0][t], w[2], x1[0], x1[1]);
+        mma16816(acc[0][t], w[3], x1[2], x1[3]);
+      }
     }
   }
-  if (steps > 2 * S::kStages) pdl_trigger();
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
 
-  // fp32 partial sums as [token][64 columns]; the CTAs of the cluster each finish a share of the outputs
+  // fp32 partial sums as [token][columns]; the CTAs of the cluster each finish a share of the outputs
   float* sum = reinterpret_cast<float*>(smem);
 #pragma unroll
-  for (int t = 0; t < MT; ++t)
+  for (int h = 0; h < kHalves; ++h)
 #pragma unroll
-    for (int e = 0; e < 4; ++e)
-      sum[(t * 8 + (lane & 3) * 2 + (e & 1)) * SK_TN + warp * 16 + (lane >> 2) + (e >> 1) * 8] = acc[t][e];
+    for (int t = 0; t < MT; ++t)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        sum[(t * 8 + (lane & 3) * 2 + (e & 1)) * S::kCols + h * SK_TN + warp * 16 + (lane >> 2) + (e >> 1) * 8] = acc[h][t][e];
   cluster.sync();
   const int rows = min(p.M, MT * 8);
-  for (int i = rank * SK_THREADS + int(threadIdx.x); i < rows * kOut; i += ks * SK_THREADS) {
-    const int row = i / kOut, col = n0 + i % kOut, at = row * SK_TN + i % kOut;
+  for (int i = rank * SK_THREADS + int(threadIdx.x); i < rows * SK_TN; i += ks * SK_THREADS) {
+    const int row = i / SK_TN, col = n0 + i % SK_TN, at = row * S::kCols + i % SK_TN;
     if (col >= (GLU ? p.I : p.N)) continue;
     float v = 0.f;
     for (int c = 0; c < ks; ++c) v += cluster.map_shared_rank(sum, c)[at];
     if constexpr (GLU) {
       float u = 0.f;
-      for (int c = 0; c < ks; ++c) u += cluster.map_shared_rank(sum, c)[at + kOut];
+      for (int c = 0; c < ks; ++c) u += cluster.map_shared_rank(sum, c)[at + SK_TN];
       static_cast<bf16*>(p.D)[size_t(row) * p.ldd + col] = __float2bfloat16(v / (1.f + __expf(-v)) * u);
       continue;
     }
@@ -192,15 +205,15 @@ gemm_skinny_kernel(const SkinnyParams p) {
 
 template <int MT, bool K_ROWS, bool GLU>
 static int launch_skinny(SkinnyParams p, cudaStream_t st) {
-  using S = SkinnySmem<MT>;
+  using S = SkinnySmem<MT, GLU>;
   auto kern = gemm_skinny_kernel<MT, K_ROWS, GLU>;
   if (S::kTotal > 48 * 1024) B200_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kTotal));
-  const int tiles = GLU ? (2 * p.I + SK_TN - 1) / SK_TN : (p.N + SK_TN - 1) / SK_TN, ksteps = (p.K + SK_TK - 1) / SK_TK;
+  const int tiles = ((GLU ? p.I : p.N) + SK_TN - 1) / SK_TN, ksteps = (p.K + S::kTk - 1) / S::kTk;
   if (tiles > 65535) return static_cast<int>(cudaErrorInvalidValue);
   // k slices: as many as fill the GPU's resident CTAs once, at most 8 (a portable cluster) and at least 2 stages each
   int ks = 1;
   while (ks < 8 && long(tiles) * ks * 2 <= long(S::kPerSm) * num_sms() && ksteps >= 4 * ks) ks *= 2;
-  p.kslice = (ksteps + ks - 1) / ks * SK_TK;
+  p.kslice = (ksteps + ks - 1) / ks * S::kTk;
   return static_cast<int>(launch_pdl(kern, dim3(ks, tiles), dim3(SK_THREADS), S::kTotal, st, ks, p));
 }
 
