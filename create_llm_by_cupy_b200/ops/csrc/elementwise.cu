@@ -189,13 +189,14 @@ __global__ void rmsnorm_fwd_scalar_kernel(const bf16* __restrict__ x, const bf16
 // residual-stream gradient). dgamma partials: every warp walks rows grid-stride and keeps its
 // column sums in registers; warps of a CTA are combined in shared memory and each CTA writes one
 // row of `partial` [gridDim.x, H] (coalesced), reduced by rmsnorm_dgamma_reduce_kernel.
+// No pdl_trigger() here and in that reduction: 8192 x 2048 forward and backward 47.3 us with it, 46.0 without (the forward
+// keeps it: 777 tokens through the 125M model 804 us, 815 without).
 template <int NV>
 __global__ void __launch_bounds__(256, 2)
 rmsnorm_bwd_kernel(const bf16* dy, const bf16* x, const bf16* gamma,
                    const float* rstd, const bf16* add, bf16* __restrict__ dx,
                    float* __restrict__ partial, int M, int H) {
   pdl_wait();
-  pdl_trigger();
   extern __shared__ float sred[];   // [warps per block][H]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
@@ -287,7 +288,6 @@ rmsnorm_bwd_cta_kernel(const bf16* dy, const bf16* x, const bf16* gamma,
                        const float* rstd, const bf16* add, bf16* __restrict__ dx,
                        float* __restrict__ partial, int M, int H) {
   pdl_wait();
-  pdl_trigger();
   __shared__ float sdot[2][R][8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nchunk = H >> 3;
@@ -415,7 +415,6 @@ __global__ void __launch_bounds__(256)
 rmsnorm_dgamma_reduce_kernel(const float* partial, bf16* __restrict__ dgamma, int nrows, int H,
                              int accumulate) {
   pdl_wait();
-  pdl_trigger();
   // block = 32 columns x 8 row-groups: coalesced 128-byte reads, rows split over the warps
   __shared__ float red[8][33];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
