@@ -1022,6 +1022,202 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   }
 }
 
+// ------------------------------------------------------------------ few tiles: K split over a cluster
+// D = alpha A op(B) (+ C), bf16, where 256 x 128 tiles leave most CTA pairs without one (777 x 768: 24 of 74). What bounds such
+// a GEMM is what an SM can pull: 24 KiB a k-block at 46 bytes a clock, one k-block after the other, 17300 of 24300 clocks over K
+// = 2048. So a tile belongs to a cluster of `splits` pairs, each of which walks its own range of K; then every CTA gets, for
+// its share of the tile's columns, the other pairs' fp32 sums of its 128 rows through distributed shared memory, adds them in
+// the order of the ranges and stores. No workspace, no second launch, deterministic. A CTA has one tile, so nothing here is
+// handed out or double-buffered. us before / now: 777 x 768 x 768 8.7 / 7.3, 777 x 768 x 2048 14.9 / 10.6, 300 x 768 x 768 8.5 /
+// 6.5, 512 x 2048 x 2048 15.2 / 10.7, 1000 x 1024 x 2736 18.7 / 12.5; against K ranges in a workspace 640 x 768 x 4096 15.8 /
+// 12.6, 256 x 2048 x 5504 16.6 / 14.7, but 256 x 4096 x 11008 30.1 / 32.3 (two pairs to a tile here).
+constexpr int GC_STAGES = 5, GC_BN = 128;
+constexpr int GC_STAGE_BYTES = G2_A_BYTES + (GC_BN / 2) * G2_BK * 2;      // 16 KiB of A, 8 KiB of B
+constexpr int GC_CHUNK = 128 * 16 * 4;                                     // 16 fp32 columns of 128 rows
+constexpr int GC_RECV = 6;                                                 // chunks a CTA receives: 1 x 4, 2 x 3 or 3 x 2
+constexpr int GC_BAR = GC_STAGES * GC_STAGE_BYTES + GC_RECV * GC_CHUNK;
+constexpr int GC_SMEM = GC_BAR + (2 * GC_STAGES + 1) * 8 + 16 + 1024;
+constexpr int GC_THREADS = 192;
+
+__device__ __forceinline__ void st_cluster_f4(uint32_t cluster_addr, const uint32_t* v) {
+  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+               : "memory");
+}
+
+template <bool B_MN>
+__global__ void __launch_bounds__(GC_THREADS, 1)
+gemm_bf16_tc2_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Gemm2Params p) {
+  extern __shared__ uint8_t smem_rawc[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_rawc) + 1023) & ~uintptr_t(1023));
+  uint8_t* recv = smem + GC_STAGES * GC_STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + GC_BAR);
+  uint64_t* empty = full + GC_STAGES;
+  uint64_t* tfull = empty + GC_STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tfull + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank(), lead = rank & ~1u;      // pair `rank / 2` of the cluster; `lead` issues its products
+  const int S = p.splits, pr = int(rank >> 1), side = int(rank & 1);
+  const int tile = int(blockIdx.x) / (2 * S), num_m = (p.M + 255) / 256;
+  const int m0 = (tile % num_m) * 256 + side * 128, n0 = (tile / num_m) * GC_BN;
+  const int num_kb = (p.K + G2_BK - 1) / G2_BK, kb0 = pr * num_kb / S, kb1 = (pr + 1) * num_kb / S;
+  // columns [16 lo(q), 16 lo(q + 1)) of the tile are finished by the CTAs of pair q
+  auto lo = [&](int q) { return 8 * q / S; };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < GC_STAGES; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(tfull, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
+  }
+  if (warp == 1) tmem_alloc_pair(tmem_slot, GC_BN);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                  // every CTA's barriers exist before anyone signals them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();                     // by every role: their bounded waits start counting behind it
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int st = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&empty[st], phase ^ 1, abort_flag)) break;
+        uint8_t* sA = smem + st * GC_STAGE_BYTES;
+        uint8_t* sB = sA + G2_A_BYTES;
+        if (rank == lead) mbar_expect_tx(&full[st], 2 * GC_STAGE_BYTES);      // bytes of both CTAs
+        const uint32_t bar = mapa_u32(smem_u32(&full[st]), lead);
+        tma_load_2d_pair(sA, &tmA, bar, kb * G2_BK, m0);
+        if (B_MN) tma_load_2d_pair(sB, &tmB, bar, n0 + side * 64, kb * G2_BK);
+        else tma_load_2d_pair(sB, &tmB, bar, kb * G2_BK, n0 + side * 64);
+        if (++st == GC_STAGES) { st = 0; phase ^= 1; }
+      }
+      pdl_trigger();
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == lead) {
+      constexpr uint32_t idesc = umma_idesc_bf16(2 * G2_BM, GC_BN, 0, B_MN ? 1 : 0);
+      const uint16_t mask = uint16_t(3u << lead);
+      auto commit = [&](uint64_t* bar) {
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(smem_u32(bar)), "h"(mask) : "memory");
+      };
+      int st = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sA = smem_u32(smem + st * GC_STAGE_BYTES), sB = sA + G2_A_BYTES;
+#pragma unroll
+        for (int kk = 0; kk < G2_BK / 16; ++kk)
+          umma_bf16_ss_pair(tmem_base, umma_smem_desc(sA + kk * 32, 16, 1024),
+                            B_MN ? umma_smem_desc(sB + kk * 2048, 8192, 1024) : umma_smem_desc(sB + kk * 32, 16, 1024), idesc,
+                            kb != kb0 || kk != 0 ? 1u : 0u);
+        commit(&empty[st]);
+        if (++st == GC_STAGES) { st = 0; phase ^= 1; }
+      }
+      if (ok) commit(tfull);
+    }
+  }
+  const int q = warp & 3, r = q * 32 + lane, row = m0 + r;
+  const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16);
+  const bool add = (p.flags & G2_ADD_C) != 0;
+  uint4 cc[4][2];                                      // the addend of this thread's columns, asked for before the sums are there
+  if (warp >= 2) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int col = n0 + (lo(pr) + i) * 16 + h * 8;
+        cc[i][h] = make_uint4(0u, 0u, 0u, 0u);
+        if (add && lo(pr) + i < lo(pr + 1) && row < p.M && col < p.N)
+          cc[i][h] = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.C) + size_t(row) * p.ldc + col);
+      }
+    if (mbar_wait_warp(tfull, 0, abort_flag)) {
+      tc_fence_after();
+      for (int o = 1; o < S; ++o) {
+        const int to = (pr + o) % S, slot = pr < to ? pr : pr - 1;      // slot: this pair's place among the receiver's sources
+        const uint32_t dst = mapa_u32(smem_u32(recv), uint32_t(2 * to + side));
+#pragma unroll 1
+        for (int c = lo(to); c < lo(to + 1); ++c) {
+          uint32_t v[16];
+          tmem_ld_32x32b_x16(taddr + c * 16, v);
+          tmem_ld_wait();
+          const int at = slot * (lo(to + 1) - lo(to)) + c - lo(to);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) st_cluster_f4(dst + uint32_t(at * GC_CHUNK + j * 2048 + r * 16), &v[4 * j]);
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();            // the sums are where they belong; every product has read both CTAs' shared memory
+  tc_fence_after();
+  if (warp >= 2 && *abort_flag == 0) {
+    const int nc = lo(pr + 1) - lo(pr);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (i >= nc) break;
+      const int c = lo(pr) + i;
+      uint32_t own[16];
+      tmem_ld_32x32b_x16(taddr + c * 16, own);
+      tmem_ld_wait();
+      float v[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] = 0.f;
+      for (int src = 0; src < S; ++src) {
+        if (src == pr) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) v[e] += __uint_as_float(own[e]);
+        } else {
+          const uint8_t* from = recv + ((src < pr ? src : src - 1) * nc + i) * GC_CHUNK + r * 16;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 f = *reinterpret_cast<const float4*>(from + j * 2048);
+            v[4 * j] += f.x; v[4 * j + 1] += f.y; v[4 * j + 2] += f.z; v[4 * j + 3] += f.w;
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int col = n0 + c * 16 + h * 8;
+        const bf162* c2 = reinterpret_cast<const bf162*>(&cc[i][h]);
+        uint4 o;
+        bf162* o2 = reinterpret_cast<bf162*>(&o);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          float x = v[8 * h + 2 * e] * p.alpha, y = v[8 * h + 2 * e + 1] * p.alpha;
+          if (add) {
+            const float2 f = __bfloat1622float2(c2[e]);
+            x += f.x;
+            y += f.y;
+          }
+          o2[e] = __floats2bfloat162_rn(x, y);
+        }
+        if (row < p.M && col < p.N) *reinterpret_cast<uint4*>(static_cast<bf16*>(p.D) + size_t(row) * p.ldd + col) = o;
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, GC_BN);
+  }
+  if (threadIdx.x == 0 && *abort_flag != 0 && p.status != nullptr) {
+    if (atomicCAS(p.status, 0, int(*abort_flag)) == 0) p.status[1] = 121;
+  }
+}
+
 static int g_dynamic_tiles = 1;
 static int g_half_tiles = 1;
 
@@ -1077,6 +1273,38 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
   }
   return static_cast<int>(launch_pdl(kern, dim3(2 * pairs), dim3(g2_threads(EPI)), G2_SMEM, stream, 0, *tA, *tB, *tBh, *tD, *tC,
                                      tE ? *tE : *tA, q));
+}
+
+// Clusters of 2 * splits CTAs that run at the same time on the current device (0: none, or not known).
+static int cluster_slots(int splits) {
+  static std::mutex mu;
+  static int known[64][5];       // 1 + the number
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  int& n = known[dev][splits];
+  if (n == 0) {
+    const auto a = gemm_bf16_tc2_cluster_kernel<false>, b = gemm_bf16_tc2_cluster_kernel<true>;
+    int got = 0;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2 * splits;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * splits);
+    cfg.blockDim = dim3(GC_THREADS);
+    cfg.dynamicSmemBytes = GC_SMEM;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(a, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(b, cudaFuncAttributeMaxDynamicSharedMemorySize, GC_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&got, a, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      got = 0;
+    }
+    n = 1 + got;
+  }
+  return n - 1;
 }
 
 // out = sum over the splits of ws[split][row][col] (+ C), fixed order. 16-byte accesses where every row allows them.
@@ -1221,6 +1449,20 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
     if (!(p.flags & G2_TMA_OUT) || a_mn_major) return static_cast<int>(cudaErrorInvalidValue);
     if (b_mn_major) return launch_tc2<false, true, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
     return launch_tc2<false, false, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
+  }
+  // Few tiles: two to four pairs to a tile, as many as there are clusters for at once, three k-blocks each at least (four: 300 x
+  // 768 x 768 6.8 us in place of 6.5). Beside weight gradients too (125M training pass of 777 tokens 2811 us, 2686 so). Up to K =
+  // 512 one range, whose sums are those of the GEMM that gathers its weight (257 x 256 x 512 7.2 us, 6.0 with two).
+  if (K > 512 && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & G2_OUT_F32) && N % 8 == 0) {
+    const int halves = ((M + 2 * G2_BM - 1) / (2 * G2_BM)) * ((N + GC_BN - 1) / GC_BN), kbs = (K + G2_BK - 1) / G2_BK;
+    int splits = 4;
+    while (splits > 1 && (halves * splits > num_sms() / 2 || kbs < 3 * splits || halves > cluster_slots(splits))) --splits;
+    if (splits > 1) {
+      p.splits = splits;
+      auto kern = b_mn_major ? gemm_bf16_tc2_cluster_kernel<true> : gemm_bf16_tc2_cluster_kernel<false>;
+      return static_cast<int>(launch_pdl(kern, dim3(2 * splits * halves), dim3(GC_THREADS), GC_SMEM, stream, 2 * splits, *tA,
+                                         b_mn_major ? *tB : *tBh, p));
+    }
   }
   // The addend's tiles fetched ahead (one operand stage less) where the epilogue is a large part of a tile's life: one
   // round of tiles, or a short K. us, fetched group by group / ahead: 8192 x 2048 over K = 512 34.4 / 26.7, 1024 38.4 / 34.1,

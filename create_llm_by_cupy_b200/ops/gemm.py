@@ -134,22 +134,31 @@ GEMM_SPLIT_K = 1
 
 
 @functools.lru_cache(maxsize=4096)
-def split_count(M: int, N: int, K: int, pairs: int) -> int:
+def split_count(M: int, N: int, K: int, pairs: int, cluster: bool = False) -> int:
     """K ranges per 256 x 256 tile (1: no split), by the time each number takes: 0.29 us per 64-deep block of K that one
     pair walks and, for a split, the second kernel with 2 us of launch and the fp32 sums read at about 4 TB/s. A split
     has to win 4 us, what its workspace and second launch cost the host. Measured, one range against the rule's:
     768 x 1280 over K = 8192 44.3 / 22.4 us, 768 x 768 over 8192 44.4 / 17.6, 256 x 4096 over 11008 57.0 / 29.4. Left whole:
-    777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4)."""
+    777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4). ``cluster``: the call can take the
+    kernel that splits K over a cluster (bf16 result, A row-major), which has no second launch and 1 us for its sums; ranges
+    have to be shorter than that then: 640 x 768 over 4096 12.6 us there, 15.8 with 6 ranges; 256 x 4096 over 11008 32.3, 30.1
+    with 4."""
     tiles = -(-M // 256) * -(-N // 256)
     kb = -(-K // 64)
+    whole, gain = 0.29 * kb, 4.0
+    if cluster and K > 512:
+        n = min(4, pairs // (-(-M // 256) * -(-N // 128)), kb // 3)
+        if n > 1:
+            whole, gain = 0.29 * -(-kb // n) + 1.0, 0.0
+
     def cost(n):
-        return 0.29 * kb if n == 1 else 0.29 * -(-kb // n) + 2.0 + 1e-6 * n * M * N
+        return whole if n == 1 else 0.29 * -(-kb // n) + 2.0 + 1e-6 * n * M * N
 
     best = min(range(1, max(1, min(pairs // tiles, kb // 4, 16)) + 1), key=cost)
-    return best if cost(best) < cost(1) - 4.0 else 1
+    return best if cost(best) < whole - gain else 1
 
 
-def _splits(M: int, N: int, K: int, dev: int, side: bool | None) -> int:
+def _splits(M: int, N: int, K: int, dev: int, side: bool | None, cluster: bool) -> int:
     """K ranges per tile for one call. ``split_count`` gives the GEMM the GPU to itself; beside another kernel the idle
     pairs are not idle, and what remains of its gain depends on who waits for the result:
       * while weight gradients are pending (``side`` None) a split pays up to three tenths of the pairs in tiles: 777 x 768
@@ -165,7 +174,7 @@ def _splits(M: int, N: int, K: int, dev: int, side: bool | None) -> int:
     pairs = _cta_pairs(dev)
     if side is None and _wgrad_pending.get(dev, False) and -(-M // 256) * -(-N // 256) * 10 > pairs * 3:
         return 1
-    return split_count(M, N, K, pairs)
+    return split_count(M, N, K, pairs, cluster)
 
 
 _pairs: dict = {}
@@ -204,7 +213,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         elif M >= 256 and N >= 256:
             route = _ROUTE_TILES
             dev = torch._C._cuda_getDevice()
-            splits = _splits(M, N, K, dev, side)
+            splits = _splits(M, N, K, dev, side, not trans_a and N % 8 == 0 and out_dtype is torch.bfloat16)
             if splits == 1:
                 _apply_dynamic()
                 whole = GEMM_WHOLE_TILES if _wgrad_pending.get(dev, False) else 0
@@ -270,7 +279,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                 _copy_rows(tmp, out)
                 return out
             dev = a.get_device()
-            splits = _splits(M, N, K, dev, side)
+            splits = _splits(M, N, K, dev, side, not trans_a and N % 8 == 0 and out_dtype is torch.bfloat16)
             if splits > 1:
                 ws = torch.empty(splits * (-(-M // 256) * 256) * (-(-N // 4) * 4), dtype=torch.float32, device=a.device)
                 rc = lib.b200_gemm_bf16_2cta_split(

@@ -90,3 +90,23 @@ def test_swiglu_backward(M, I, K):
         size = (value if out.data_ptr() == got.data_ptr() else torch.ones_like(gate)).abs() * s * (1 + gate.abs())
         lim = bound * f.abs() + d.abs() * size * 2.0 ** -19 + BF_ULP * (d * f).abs() + 1e-30
         assert ((out - d * f).abs() <= lim).all()
+
+
+# K split over a cluster: 2, 3 and 4 pairs to a tile (37, 24 and 12 tiles of 256 x 128), ranges of unequal length, tiles cut by M
+# and N, one range up to K = 512
+@pytest.mark.parametrize("M,N", [(1100, 896), (777, 768), (256, 256), (300, 264), (300, 1544)])
+@pytest.mark.parametrize("K", [512, 520, 840, 2056])
+@pytest.mark.parametrize("trans_b", [False, True])
+def test_cluster_split(M, N, K, trans_b):
+    a, b, c = bf(M, K, seed=1), bf(K, N, seed=2), bf(M, N, seed=3)
+    w = b.t().contiguous() if trans_b else b
+    want, bound = product(a, b)
+    for add, alpha in ((None, 1.0), (c, 1.0), (c, -0.5)):
+        ref = alpha * want + (c.double() if add is not None else 0)
+        y = G.gemm(a, w, trans_b=trans_b, add=add, alpha=alpha)
+        assert ((y.double() - ref).abs() <= bound + BF_ULP * ref.abs() + 1e-30).all()
+        assert torch.equal(y, G.gemm(a, w, trans_b=trans_b, add=add, alpha=alpha))
+    acc = torch.full((M, N + 16), 7.0, dtype=torch.bfloat16, device="cuda")     # in place, between columns that stay
+    acc[:, 8:8 + N] = c
+    G.gemm(a, w, trans_b=trans_b, add=acc[:, 8:8 + N], out=acc[:, 8:8 + N])
+    assert torch.equal(acc[:, 8:8 + N], G.gemm(a, w, trans_b=trans_b, add=c)) and (acc[:, :8] == 7).all() and (acc[:, 8 + N:] == 7).all()
