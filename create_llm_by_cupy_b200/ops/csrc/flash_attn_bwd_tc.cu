@@ -16,7 +16,7 @@
 //   flash_bwd_dkv_wide : the same with 128-query iterations: the score products are N = 128 MMAs, S^T, dP^T, dV and dK lie
 //        side by side in tensor memory, and the products of consecutive iterations are interleaved instead of
 //        double-buffered (see the comment above that kernel). What runs for both head dimensions; flash_bwd_dkv_tc is left
-//        for head_dim 128 where the wide kernel's shared memory does not fit.
+//        for up to 64 tokens at head_dim 64 and for head_dim 128 where the wide kernel's shared memory does not fit.
 // Q and K are expected already rotated; dQ and dK are gradients w.r.t. the rotated tensors unless the
 // caller passes the rotary tables, in which case the epilogues apply the inverse rotation
 // (flash_rope_epilogue.cuh). No atomics and no fp32 scratch. When the caller gives a workspace the
@@ -374,11 +374,13 @@ __device__ __forceinline__ DkvPass dkv_pass(int ntile, int T, int R, int vlen) {
   return d;
 }
 
+// kD: head dimension (128, or 64: one 64-column box per K / V / Q / dO tile, four k-steps in the score
+// products, N = 64 in the gradient products, 64 live columns in dV and dK).
+template <int kD>
 __global__ void __launch_bounds__(FBT_THREADS, 1)
 flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmDO,
                         const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                         const __grid_constant__ CUtensorMap tmDS, const FlashBwdTcParams p) {
-  constexpr int kD = FB_D;
   extern __shared__ uint8_t fb_smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(fb_smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FdkvSmem::kBar);
@@ -456,9 +458,9 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
         mbar_expect_tx(kv_full, 2 * 128 * kD * 2);
         tma_load_4d(smem + FdkvSmem::kK, &tmK, kv_full, 0, kvh, d.n0, b);
-        tma_load_4d(smem + FdkvSmem::kK + 16384, &tmK, kv_full, 64, kvh, d.n0, b);
+        if (kD == 128) tma_load_4d(smem + FdkvSmem::kK + 16384, &tmK, kv_full, 64, kvh, d.n0, b);
         tma_load_4d(smem + FdkvSmem::kV, &tmV, kv_full, 0, kvh, d.n0, b);
-        tma_load_4d(smem + FdkvSmem::kV + 16384, &tmV, kv_full, 64, kvh, d.n0, b);
+        if (kD == 128) tma_load_4d(smem + FdkvSmem::kV + 16384, &tmV, kv_full, 64, kvh, d.n0, b);
         ++kv_loads;
         for (int it = 0; it < d.iters; ++it, ++g) {
           const int s = g % FKV_ST;
@@ -469,9 +471,9 @@ flash_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           uint8_t* sDO = sQ + FKV_QTILE;
           mbar_expect_tx(&q_full[s], 2 * FKV_BQ * kD * 2);
           tma_load_4d(sQ, &tmQ, &q_full[s], 0, h, m0, b);
-          tma_load_4d(sQ + 8192, &tmQ, &q_full[s], 64, h, m0, b);
+          if (kD == 128) tma_load_4d(sQ + 8192, &tmQ, &q_full[s], 64, h, m0, b);
           tma_load_4d(sDO, &tmDO, &q_full[s], 0, h, m0, b);
-          tma_load_4d(sDO + 8192, &tmDO, &q_full[s], 64, h, m0, b);
+          if (kD == 128) tma_load_4d(sDO + 8192, &tmDO, &q_full[s], 64, h, m0, b);
         }
       }
       (void)kv_loads;
@@ -1288,7 +1290,9 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   if (!configured) {
     B200_CHECK(cudaFuncSetAttribute(flash_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     FdqSmem::kTotal));
-    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    FdkvSmem::kTotal));
+    B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     FdkvSmem::kTotal));
     B200_CHECK(cudaFuncSetAttribute(flash_bwd_dkv_wide_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     FdkwSmem<64>::kTotal));
@@ -1326,14 +1330,16 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
   const int n_key_tiles = nt * KVH * B;
   p.pairing = g_dkv_pairing >= 0 ? g_dkv_pairing : ((n_key_tiles > num_sms() && n_key_tiles < 3 * num_sms()) ? 1 : 0);
   const int dkv_ctas = (p.pairing ? (nt + 1) / 2 : nt) * KVH * B;
-  if (D == 64)
+  // head_dim 64: 128-query iterations from 65 tokens on (100: 11.4 us, 12.1 with 64-query ones; 64: 11.3 / 8.5, half of every
+  // tile would be past the end)
+  if (D == 64 && T > 64)
     B200_CHECK(launch_pdl(flash_bwd_dkv_wide_kernel<64>, dim3(dkv_ctas), dim3(FBT_THREADS), FdkwSmem<64>::kTotal, st, 0, *tq128,
                           *tdo128, *tk, *tv, *tds, p));
-  else if (g_dkv_wide && dkv_wide_fits())
+  else if (D == 128 && g_dkv_wide && dkv_wide_fits())
     B200_CHECK(launch_pdl(flash_bwd_dkv_wide_kernel<128>, dim3(dkv_ctas), dim3(FBT_THREADS), FdkwSmem<128>::kTotal, st, 0, *tq128,
                           *tdo128, *tk, *tv, *tds, p));
   else
-    B200_CHECK(launch_pdl(flash_bwd_dkv_tc_kernel, dim3(dkv_ctas), dim3(FBT_THREADS), FdkvSmem::kTotal, st, 0, *tq64, *tdo64,
+    B200_CHECK(launch_pdl(D == 128 ? flash_bwd_dkv_tc_kernel<128> : flash_bwd_dkv_tc_kernel<64>, dim3(dkv_ctas), dim3(FBT_THREADS), FdkvSmem::kTotal, st, 0, *tq64, *tdo64,
                           *tk, *tv, *tds, p));
   if (ds_ws != nullptr) return flash_bwd_dq_from_ds(ds_ws, k, dq, valid_len, s + 3, s + 12, B, T, QH, KVH, D, p.bchunk,
                                                       p.unrot_cos, p.unrot_sin, p.unrot_ld, st);

@@ -127,7 +127,8 @@ gemm_skinny_kernel(const SkinnyParams p) {
   // No pdl_trigger(): the next kernel's CTAs then start as these end. Let in before that, they land unevenly among this one's,
   // take shared memory and issue slots from what is still running and run unevenly themselves. us with the trigger here for
   // slices of up to 12 stages and behind the loop for longer ones / without: a 7B block of 8 sequences 113.2 / 104.3, of one
-  // 88.9 / 86.6, a 1.3B block of one 43.4 / 40.8, of 16 54.4 / 52.9, one token through the 125M model 349 / 337 on the device.
+  // 88.9 / 86.6, a 1.3B block of one 43.4 / 40.8, of 16 54.4 / 52.9, one token through the 125M model 349 / 337 on the device,
+  // a training pass of 64 tokens 2027 / 2022.
 #pragma unroll
   for (int s = 0; s < S::kStages - 1; ++s) {
     if (s < steps) skinny_load<MT, K_ROWS, GLU>(p, base + s * S::kStageBytes, n0, k_begin + s * S::kTk, k_end);
@@ -151,16 +152,17 @@ gemm_skinny_kernel(const SkinnyParams p) {
     }
 #pragma unroll
     for (int t = 0; t < MT; ++t) {
-      uint32_t x0[4];                            // tokens 8 t .. 8 t + 7, k 0-31
-      ldsm4(x0, sw_addr(sa, t * 8 + mr, mi));
+      uint32_t x0[4], x1[4];                     // tokens 8 t .. 8 t + 7, k 0-31 and 32-63
+      constexpr bool kAhead = MT == 8;           // both before the products (64 x 768 over 768 6.7 us, 7.0 one after the other;
+      ldsm4(x0, sw_addr(sa, t * 8 + mr, mi));    // five rows 3.6, 3.5)
+      if (!GLU && kAhead) ldsm4(x1, sw_addr(sa, t * 8 + mr, 4 + mi));
       mma16816(acc[0][t], w[0], x0[0], x0[1]);
       mma16816(acc[0][t], w[1], x0[2], x0[3]);
-      if constexpr (GLU) {
-        mma16816(acc[1][t], w[2], x0[0], x0[1]);
-        mma16816(acc[1][t], w[3], x0[2], x0[3]);
+      if (GLU) {
+        mma16816(acc[kHalves - 1][t], w[2], x0[0], x0[1]);
+        mma16816(acc[kHalves - 1][t], w[3], x0[2], x0[3]);
       } else {
-        uint32_t x1[4];                          // k 32-63
-        ldsm4(x1, sw_addr(sa, t * 8 + mr, 4 + mi));
+        if (!kAhead) ldsm4(x1, sw_addr(sa, t * 8 + mr, 4 + mi));
         mma16816(acc[0][t], w[2], x1[0], x1[1]);
         mma16816(acc[0][t], w[3], x1[2], x1[3]);
       }
