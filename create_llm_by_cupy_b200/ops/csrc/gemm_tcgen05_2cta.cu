@@ -173,21 +173,28 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_out, uint32_t nco
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
+// By a whole warp in step; one elected lane issues (ptx.cuh says why). Under `if (lane == 0)` a k-block of 256 x 128 took 535
+// clocks where its products take 256, and one of 256 x 256 just its 512. us before / now: 8192 x 768 x 4096 46.5 / 42.2, 8192 x
+// 768 x 2048 27.0 / 25.0, 8192 x 768 x 1280 19.1 / 17.3, 2048 x 1024 x 2736 19.0 / 17.6, 777 x 768 x 2048 (three pairs to a tile)
+// 10.6 / 9.3; 1.3B layers under the power cap: MLP 1383 / 1358, attention 818 / 796.
 __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                                   uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on the barrier at this offset in BOTH CTAs once the MMAs issued so far have completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  const uint16_t mask = 3;
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"(mask)
-               : "memory");
+// Arrive on the barrier at this offset in the CTAs of `mask` once the MMAs issued so far have completed (both of a pair).
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t"
+      "elect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(smem_u32(bar)), "h"(mask)
+      : "memory");
 }
 
 // Write one word into the peer CTA's shared memory and count its 4 bytes on the peer's mbarrier;
@@ -225,7 +232,7 @@ struct TileRingReader {
     // In the leader the index is an ordinary shared-memory store before an arrive; in the follower
     // it arrives as an asynchronous store counted on the barrier. Either way a plain wait sees it.
     (void)remote_writer;
-    if (!mbar_wait(&sched_full[slot], phase, abort_flag)) return -1;
+    if (!(whole_warp ? mbar_wait_warp(&sched_full[slot], phase, abort_flag) : mbar_wait(&sched_full[slot], phase, abort_flag))) return -1;
     const int t = ring[slot];
     if (whole_warp) __syncwarp();
     if (arrive) mbar_arrive_cluster_relaxed_after(mapa_u32(smem_u32(&sched_empty[slot]), 0), t);
@@ -407,7 +414,7 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc_full = umma_idesc_bf16(2 * G2_BM, G2_BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       constexpr uint32_t idesc_half = umma_idesc_bf16(2 * G2_BM, G2_BN / 2, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
@@ -417,30 +424,26 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       bool ok = true;
       TileRingReader rd;
       for (int t = pair; ok && t >= 0 && t < num_tiles;
-           t = dyn ? rd.next(sched_full, sched_empty, tile_ring, abort_flag, false, true, rank != 0) : t + num_pairs) {
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+           t = dyn ? rd.next(sched_full, sched_empty, tile_ring, abort_flag, true, lane == 0, rank != 0) : t + num_pairs) {
+        if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * G2_BN;
         const uint32_t idesc = t < p.t_full ? idesc_full : idesc_half;
         const int kb0 = kb_first(t);
         for (int kb = kb0, kb_end = kb_last(t); kb < kb_end; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sA = smem_u32(smem + stage * G2_STAGE_BYTES);
-          const uint32_t sB = sA + G2_A_BYTES;
+          const uint64_t dA = A_MN ? umma_smem_desc(sA, 8192, 1024) : umma_smem_desc(sA, 16, 1024);
+          const uint64_t dB = B_MN ? umma_smem_desc(sA + G2_A_BYTES, 8192, 1024) : umma_smem_desc(sA + G2_A_BYTES, 16, 1024);
 #pragma unroll
-          for (int kk = 0; kk < G2_BK / 16; ++kk) {
-            const uint64_t adesc = A_MN ? umma_smem_desc(sA + kk * 2048, 8192, 1024)
-                                        : umma_smem_desc(sA + kk * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_smem_desc(sB + kk * 2048, 8192, 1024)
-                                        : umma_smem_desc(sB + kk * 32, 16, 1024);
-            umma_bf16_ss_pair(tmem_d, adesc, bdesc, idesc, kb != kb0 || kk != 0 ? 1u : 0u);
-          }
-          umma_commit_pair(&empty[stage]);
+          for (int kk = 0; kk < G2_BK / 16; ++kk)         // a step of 16: 16 rows of 128 bytes (MN-major) or 32 bytes of each row
+            umma_bf16_ss_pair(tmem_d, dA + kk * (A_MN ? 128 : 2), dB + kk * (B_MN ? 128 : 2), idesc, kb != kb0 || kk != 0 ? 1u : 0u);
+          umma_commit_pair(&empty[stage], 3);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit_pair(&tfull[acc]);
+        umma_commit_pair(&tfull[acc], 3);
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
@@ -1028,9 +1031,9 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 // = 2048. So a tile belongs to a cluster of `splits` pairs, each of which walks its own range of K; then every CTA gets, for
 // its share of the tile's columns, the other pairs' fp32 sums of its 128 rows through distributed shared memory, adds them in
 // the order of the ranges and stores. No workspace, no second launch, deterministic. A CTA has one tile, so nothing here is
-// handed out or double-buffered. us before / now: 777 x 768 x 768 8.7 / 7.3, 777 x 768 x 2048 14.9 / 10.6, 300 x 768 x 768 8.5 /
-// 6.5, 512 x 2048 x 2048 15.2 / 10.7, 1000 x 1024 x 2736 18.7 / 12.5; against K ranges in a workspace 640 x 768 x 4096 15.8 /
-// 12.6, 256 x 2048 x 5504 16.6 / 14.7, but 256 x 4096 x 11008 30.1 / 32.3 (two pairs to a tile here).
+// handed out or double-buffered. us before / now: 777 x 768 x 768 8.7 / 6.9, 777 x 768 x 2048 14.9 / 9.3, 300 x 768 x 768 8.5 / 6.4,
+// 512 x 2048 x 2048 15.2 / 9.5, 1000 x 1024 x 2736 18.7 / 10.8; against K ranges in a workspace 640 x 768 x 4096 15.8 / 11.0,
+// 256 x 2048 x 5504 16.6 / 12.9, 256 x 4096 x 11008 30.1 / 28.9 (two pairs to a tile here).
 constexpr int GC_STAGES = 5, GC_BN = 128;
 constexpr int GC_STAGE_BYTES = G2_A_BYTES + (GC_BN / 2) * G2_BK * 2;      // 16 KiB of A, 8 KiB of B
 constexpr int GC_CHUNK = 128 * 16 * 4;                                     // 16 fp32 columns of 128 rows
@@ -1102,29 +1105,25 @@ gemm_bf16_tc2_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
       pdl_trigger();
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == lead) {
+    if (rank == lead) {
       constexpr uint32_t idesc = umma_idesc_bf16(2 * G2_BM, GC_BN, 0, B_MN ? 1 : 0);
       const uint16_t mask = uint16_t(3u << lead);
-      auto commit = [&](uint64_t* bar) {
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                     ::"r"(smem_u32(bar)), "h"(mask) : "memory");
-      };
       int st = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&full[st], phase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&full[st], phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t sA = smem_u32(smem + st * GC_STAGE_BYTES), sB = sA + G2_A_BYTES;
+        const uint32_t sA = smem_u32(smem + st * GC_STAGE_BYTES);
+        const uint64_t dA = umma_smem_desc(sA, 16, 1024);
+        const uint64_t dB = B_MN ? umma_smem_desc(sA + G2_A_BYTES, 8192, 1024) : umma_smem_desc(sA + G2_A_BYTES, 16, 1024);
 #pragma unroll
         for (int kk = 0; kk < G2_BK / 16; ++kk)
-          umma_bf16_ss_pair(tmem_base, umma_smem_desc(sA + kk * 32, 16, 1024),
-                            B_MN ? umma_smem_desc(sB + kk * 2048, 8192, 1024) : umma_smem_desc(sB + kk * 32, 16, 1024), idesc,
-                            kb != kb0 || kk != 0 ? 1u : 0u);
-        commit(&empty[st]);
+          umma_bf16_ss_pair(tmem_base, dA + kk * 2, dB + kk * (B_MN ? 128 : 2), idesc, kb != kb0 || kk != 0 ? 1u : 0u);
+        umma_commit_pair(&empty[st], mask);
         if (++st == GC_STAGES) { st = 0; phase ^= 1; }
       }
-      if (ok) commit(tfull);
+      if (ok) umma_commit_pair(tfull, mask);
     }
   }
   const int q = warp & 3, r = q * 32 + lane, row = m0 + r;
