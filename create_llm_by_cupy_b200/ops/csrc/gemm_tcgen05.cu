@@ -2,7 +2,7 @@
 //
 // One persistent CTA per SM, warp-specialised:
 //   warp 0      TMA producer   global -> 128B-swizzled shared-memory stages (cp.async.bulk.tensor)
-//   warp 1      MMA issuer     one elected thread issues tcgen05.mma (128 x BN x 16) into TMEM
+//   warp 1      MMA issuer     one elected lane issues tcgen05.mma (128 x BN x 16) into TMEM
 //   warps 2..5  epilogue       tcgen05.ld the fp32 accumulator, scale / add C / convert, store
 // The accumulator is double-buffered in TMEM (2 x BN columns), so the epilogue of tile i overlaps
 // the main loop of tile i+1. Operands may be K-major (row-major [MN, K]) or MN-major (row-major
@@ -341,7 +341,7 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {                                     // the whole warp in step, one elected lane issues (ptx.cuh)
       constexpr uint32_t idesc = umma_idesc_bf16(GEMM_BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
       int stage = 0;
       uint32_t phase = 0;
@@ -349,27 +349,23 @@ gemm_bf16_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int t = int(blockIdx.x) - cta0; t < num_tiles && ok; t += gemm_ctas) {
-        if (!mbar_wait(&tempty[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t tmem_d = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&full[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sA = smem_u32(smem + stage * S::kStageBytes);
-          const uint32_t sB = sA + S::kABytes;
+          const uint64_t dA = A_MN ? umma_smem_desc(sA, 8192, 1024) : umma_smem_desc(sA, 16, 1024);
+          const uint64_t dB = B_MN ? umma_smem_desc(sA + S::kABytes, 8192, 1024) : umma_smem_desc(sA + S::kABytes, 16, 1024);
 #pragma unroll
-          for (int kk = 0; kk < GEMM_BK / 16; ++kk) {
-            const uint64_t adesc = A_MN ? umma_smem_desc(sA + kk * 2048, 8192, 1024)
-                                        : umma_smem_desc(sA + kk * 32, 16, 1024);
-            const uint64_t bdesc = B_MN ? umma_smem_desc(sB + kk * 2048, 8192, 1024)
-                                        : umma_smem_desc(sB + kk * 32, 16, 1024);
-            umma_bf16_ss(tmem_d, adesc, bdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
-          }
-          umma_commit(&empty[stage]);   // frees the smem stage once these MMAs have read it
+          for (int kk = 0; kk < GEMM_BK / 16; ++kk)
+            umma_bf16_ss_warp(tmem_d, dA + kk * (A_MN ? 128 : 2), dB + kk * (B_MN ? 128 : 2), idesc, (kb | kk) != 0 ? 1u : 0u);
+          umma_commit_warp(&empty[stage]);   // frees the smem stage once these MMAs have read it
           if (++stage == S::kStages) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit(&tfull[acc]);       // accumulator complete
+        umma_commit_warp(&tfull[acc]);       // accumulator complete
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
