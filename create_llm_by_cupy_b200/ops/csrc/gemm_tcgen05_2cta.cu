@@ -173,8 +173,9 @@ __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_out, uint32_t nco
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// By a whole warp in step; one elected lane issues (ptx.cuh says why). Under `if (lane == 0)` a k-block of 256 x 128 took 535
-// clocks where its products take 256, and one of 256 x 256 just its 512. us before / now: 8192 x 768 x 4096 46.5 / 42.2, 8192 x
+// By a whole warp in step; one elected lane issues (ptx.cuh says why). Under `if (lane == 0)` the four products of a k-block
+// took the issuing lane longer to set up than half a tile's take to run; a k-block of 256 x 128 then took 310 ns, 280 now (777 x
+// 768, K = 768 to 2048; the products are 135 of it, the rest is operands at 46 bytes a clock and SM). us before / now: 8192 x 768 x 4096 46.5 / 42.2, 8192 x
 // 768 x 2048 27.0 / 25.0, 8192 x 768 x 1280 19.1 / 17.3, 2048 x 1024 x 2736 19.0 / 17.6, 777 x 768 x 2048 (three pairs to a tile)
 // 10.6 / 9.3; 1.3B layers under the power cap: MLP 1383 / 1358, attention 818 / 796.
 __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
@@ -1027,13 +1028,12 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
 // ------------------------------------------------------------------ few tiles: K split over a cluster
 // D = alpha A op(B) (+ C), bf16, where 256 x 128 tiles leave most CTA pairs without one (777 x 768: 24 of 74). What bounds such
-// a GEMM is what an SM can pull: 24 KiB a k-block at 46 bytes a clock, one k-block after the other, 17300 of 24300 clocks over K
-// = 2048. So a tile belongs to a cluster of `splits` pairs, each of which walks its own range of K; then every CTA gets, for
+// a GEMM is what an SM can pull: 24 KiB a k-block at 46 bytes a clock, one k-block after the other. So a tile belongs to a cluster of `splits` pairs, each of which walks its own range of K; then every CTA gets, for
 // its share of the tile's columns, the other pairs' fp32 sums of its 128 rows through distributed shared memory, adds them in
 // the order of the ranges and stores. No workspace, no second launch, deterministic. A CTA has one tile, so nothing here is
-// handed out or double-buffered. us before / now: 777 x 768 x 768 8.7 / 6.9, 777 x 768 x 2048 14.9 / 9.3, 300 x 768 x 768 8.5 / 6.4,
-// 512 x 2048 x 2048 15.2 / 9.5, 1000 x 1024 x 2736 18.7 / 10.8; against K ranges in a workspace 640 x 768 x 4096 15.8 / 11.0,
-// 256 x 2048 x 5504 16.6 / 12.9, 256 x 4096 x 11008 30.1 / 28.9 (two pairs to a tile here).
+// handed out or double-buffered. us on half tiles / so: 777 x 768 x 768 8.7 / 6.9, 777 x 768 x 2048 14.3 / 9.3, 300 x 768 x 768 8.6 / 6.4,
+// 512 x 2048 x 2048 14.6 / 9.4, 1000 x 1024 x 2736 17.7 / 10.7, 640 x 768 x 4096 22.8 / 10.9, 256 x 2048 x 5504 28.6 / 12.7;
+// against K ranges in a workspace 640 x 768 x 4096 15.8 / 11.0, 256 x 4096 x 11008 29.2 / 28.2 (two pairs to a tile).
 constexpr int GC_STAGES = 5, GC_BN = 128;
 constexpr int GC_STAGE_BYTES = G2_A_BYTES + (GC_BN / 2) * G2_BK * 2;      // 16 KiB of A, 8 KiB of B
 constexpr int GC_CHUNK = 128 * 16 * 4;                                     // 16 fp32 columns of 128 rows
@@ -1255,8 +1255,8 @@ static int launch_tc2(const CUtensorMap* tA, const CUtensorMap* tB, const CUtens
     const int rem = whole % all_pairs;
     // The only round counts too, unless it is a weight gradient, whose idle pairs the main stream's kernels use (125M
     // training pass 7810 us, 8014 with halves there). A_MN stands for that: x^T dy is where a transposed A comes from, and one
-    // that is issued alone runs on whole tiles as well. 777 rows, us whole / halves: 768 x 768 10.0 / 8.8, 768 x 2048 15.9 /
-    // 14.9, 1280 x 768 10.1 / 9.0; 2048 x 1024 x 2736 20.7 / 20.0.
+    // that is issued alone runs on whole tiles as well. us whole / halves: 777 x 1280 x 768 10.1 / 9.0, 2048 x 1024 x
+    // 2736 19.7 / 18.8; a last round: 8192 x 768 x 768 15.8 / 14.4, 8192 x 1280 x 768 20.3 / 19.1, 8192 x 2048 x 2048 49.7 / 48.8.
     if (2 * rem <= all_pairs && (whole > all_pairs || !A_MN)) halved = rem;
   }
   const int num_tiles = EPI == EPI_SPLIT ? whole * p.splits : whole + halved;
@@ -1464,9 +1464,9 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
     }
   }
   // The addend's tiles fetched ahead (one operand stage less) where the epilogue is a large part of a tile's life: one
-  // round of tiles, or a short K. us, fetched group by group / ahead: 8192 x 2048 over K = 512 34.4 / 26.7, 1024 38.4 / 34.1,
-  // 1536 43.5 / 45.0, 5504 133.9 / 135.2; 8192 x 768 over 1024 21.0 / 19.1, 1536 24.5 / 24.5; one round: 1000 x 4096 over
-  // 256 10.0 / 8.4, 4096 32.3 / 30.4, 2048 x 1024 over 2736 23.2 / 20.6.
+  // round of tiles, or a short K. us, fetched group by group / ahead: 8192 x 2048 over K = 512 30.2 / 22.0, 1024 36.9 / 30.9,
+  // 1536 43.4 / 43.0, 5504 131.5 / 132.7; 8192 x 768 over 1024 17.8 / 16.5, 1536 21.3 / 20.9; one round: 1000 x 4096 over
+  // 256 9.5 / 8.2, 4096 30.2 / 27.9, 2048 x 1024 over 2736 19.1 / 18.2.
   const int tiles = ((M + 2 * G2_BM - 1) / (2 * G2_BM)) * ((N + G2_BN - 1) / G2_BN);
   if (add && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & G2_OUT_F32) && (K <= 1280 || tiles <= num_sms() / 2)) {
     if (b_mn_major) return launch_tc2<false, true, EPI_ADD>(tA, tB, tBh, tD, tC, p, stream);

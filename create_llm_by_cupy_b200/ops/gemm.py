@@ -141,8 +141,9 @@ def split_count(M: int, N: int, K: int, pairs: int, cluster: bool = False) -> in
     768 x 1280 over K = 8192 44.3 / 22.4 us, 768 x 768 over 8192 44.4 / 17.6, 256 x 4096 over 11008 57.0 / 29.4. Left whole:
     777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4). ``cluster``: the call can take the
     kernel that splits K over a cluster (bf16 result, A row-major), which has no second launch and 1 us for its sums; ranges
-    have to be shorter than that then: 640 x 768 over 4096 11.0 us there, 15.8 with 6 ranges; 256 x 4096 over 11008 28.9, 30.1
-    with 4."""
+    have to be shorter than that then: 640 x 768 over 4096 11.0 us there, 15.8 with 6 ranges; 768 x 1024 over 8192 20.7, 19.1
+    with 6. On the line between them the rule is 1 us off: 256 x 4096 over 11008 28.2 there, 29.2 with the 4 that it takes, 768 x
+    1280 over 8192 20.9, 22.5 with 4."""
     tiles = -(-M // 256) * -(-N // 256)
     kb = -(-K // 64)
     whole, gain = 0.29 * kb, 4.0
