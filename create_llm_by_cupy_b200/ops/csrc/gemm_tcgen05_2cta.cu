@@ -1129,7 +1129,9 @@ gemm_bf16_tc2_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
   const int q = warp & 3, r = q * 32 + lane, row = m0 + r;
   const uint32_t taddr = tmem_base + (uint32_t(q * 32) << 16);
   const bool add = (p.flags & G2_ADD_C) != 0;
+  const int nc = lo(pr + 1) - lo(pr);
   uint4 cc[4][2];                                      // the addend of this thread's columns, asked for before the sums are there
+  uint32_t own[4][16];                                 // its own pair's sums of them
   if (warp >= 2) {
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -1137,11 +1139,15 @@ gemm_bf16_tc2_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
       for (int h = 0; h < 2; ++h) {
         const int col = n0 + (lo(pr) + i) * 16 + h * 8;
         cc[i][h] = make_uint4(0u, 0u, 0u, 0u);
-        if (add && lo(pr) + i < lo(pr + 1) && row < p.M && col < p.N)
+        if (add && i < nc && row < p.M && col < p.N)
           cc[i][h] = *reinterpret_cast<const uint4*>(static_cast<const bf16*>(p.C) + size_t(row) * p.ldc + col);
       }
     if (mbar_wait_warp(tfull, 0, abort_flag)) {
       tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < nc) tmem_ld_32x32b_x16(taddr + (lo(pr) + i) * 16, own[i]);
+      tmem_ld_wait();
       for (int o = 1; o < S; ++o) {
         const int to = (pr + o) % S, slot = pr < to ? pr : pr - 1;      // slot: this pair's place among the receiver's sources
         const uint32_t dst = mapa_u32(smem_u32(recv), uint32_t(2 * to + side));
@@ -1159,24 +1165,25 @@ gemm_bf16_tc2_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
   }
   tc_fence_before();
   __syncthreads();
-  cluster_sync_all();            // the sums are where they belong; every product has read both CTAs' shared memory
-  tc_fence_after();
+  // The sums are where they belong; every product has read both CTAs' shared memory, and both CTAs have read their tensor
+  // memory, which either one's release gives back for the pair.
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, GC_BN);
+  }
   if (warp >= 2 && *abort_flag == 0) {
-    const int nc = lo(pr + 1) - lo(pr);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if (i >= nc) break;
       const int c = lo(pr) + i;
-      uint32_t own[16];
-      tmem_ld_32x32b_x16(taddr + c * 16, own);
-      tmem_ld_wait();
       float v[16];
 #pragma unroll
       for (int e = 0; e < 16; ++e) v[e] = 0.f;
       for (int src = 0; src < S; ++src) {
         if (src == pr) {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) v[e] += __uint_as_float(own[e]);
+          for (int e = 0; e < 16; ++e) v[e] += __uint_as_float(own[i][e]);
         } else {
           const uint8_t* from = recv + ((src < pr ? src : src - 1) * nc + i) * GC_CHUNK + r * 16;
 #pragma unroll
@@ -1205,12 +1212,6 @@ gemm_bf16_tc2_cluster_kernel(const __grid_constant__ CUtensorMap tmA, const __gr
         if (row < p.M && col < p.N) *reinterpret_cast<uint4*>(static_cast<bf16*>(p.D) + size_t(row) * p.ldd + col) = o;
       }
     }
-    tc_fence_before();
-  }
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc_pair(tmem_base, GC_BN);
   }
   if (threadIdx.x == 0 && *abort_flag != 0 && p.status != nullptr) {
     if (atomicCAS(p.status, 0, int(*abort_flag)) == 0) p.status[1] = 121;
