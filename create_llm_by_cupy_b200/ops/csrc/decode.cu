@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "ptx.cuh"
+#include "tile_rows.h"
 
 namespace b200 {
 namespace cg = cooperative_groups;
@@ -141,13 +142,22 @@ decode_attn_kernel(const DecodeParams p) {
   uint8_t* vt = kt + TB;
   const bf16* kb = p.kc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
   const bf16* vb = p.vc + (size_t(b) * p.KVH + kvh) * size_t(p.Tmax) * D;
-  // A tile of K (which 0) or V (1): its valid keys are one run of bytes. By the first lane; the row of the new token may still
-  // be in writing, nobody uses what arrives for it.
+  // A tile of K (which 0) or V (1), by the first lane: its valid keys are one run of bytes, or two with the new token's row
+  // between them. That row is being written by the first CTA and comes from s_new.
   auto fetch = [&](int t, int which) {
     if (t * DA_TILE >= len) return;
-    const uint32_t bytes = uint32_t(min(DA_TILE, len - t * DA_TILE)) * D * 2;
-    mbar_expect_tx(&full[warp][which], bytes);
-    bulk_load(which == 0 ? kt : vt, (which == 0 ? kb : vb) + size_t(t) * DA_TILE * D, bytes, &full[warp][which]);
+    const TileRows rows = tile_rows(t * DA_TILE, DA_TILE, len, APPEND ? p.pos : -1);
+    uint64_t* bar = &full[warp][which];
+    uint8_t* dst = which == 0 ? kt : vt;
+    const bf16* src = (which == 0 ? kb : vb) + size_t(t) * DA_TILE * D;
+    if (rows.first + rows.rest == 0) {                   // the new token's row alone: nothing to wait for
+      mbar_arrive(bar);
+      return;
+    }
+    mbar_expect_tx(bar, uint32_t(rows.first + rows.rest) * D * 2);
+    if (rows.first > 0) bulk_load(dst, src, uint32_t(rows.first) * D * 2, bar);
+    if (APPEND && rows.rest > 0)
+      bulk_load(dst + (rows.first + 1) * D * 2, src + (rows.first + 1) * D, uint32_t(rows.rest) * D * 2, bar);
   };
   if (lane == 0) {
     fetch(rank + warp * cs, 0);
@@ -163,7 +173,7 @@ decode_attn_kernel(const DecodeParams p) {
       const uint4 u = which == 0 ? rotated_chunk<D>(new_row + kvh * D, c, p.cosr, p.sinr)
                                  : reinterpret_cast<const uint4*>(new_row + (p.KVH + p.QH + kvh) * D)[c];
       s_new[which][c] = u;
-      // nobody reads this cache row in this launch: every CTA takes it from its s_new
+      // nobody reads this cache row in this launch: every CTA takes it from its s_new, and no copy covers it
       if (rank == 0 && g == 0)
         reinterpret_cast<uint4*>((which == 0 ? p.kcw : p.vcw) + ((size_t(b) * p.KVH + kvh) * p.Tmax + p.pos) * D)[c] = u;
     }

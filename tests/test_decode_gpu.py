@@ -73,7 +73,8 @@ def attention_bound(out, n):
     return 2.0 ** -8 * out.abs() + 6 * (n * 2.0 ** -23 + 64 * 2.0 ** -22)
 
 
-@pytest.mark.parametrize("B,QH,KVH,D,lens", ROUNDS + [(3, 6, 2, 64, [33, 32, 40]), (2, 8, 2, 128, [1, 300])])
+@pytest.mark.parametrize("B,QH,KVH,D,lens", ROUNDS + [(3, 6, 2, 64, [33, 32, 40]), (2, 8, 2, 128, [1, 300]),
+                                                      (2, 4, 2, 64, [33, 33]), (1, 4, 1, 128, [1]), (2, 2, 2, 32, [97, 65])])
 def test_decode_append_against_fp64(B, QH, KVH, D, lens):
     """Tables of 0, 1 / 2 and 1 make the rotation exact, so that the rotated rows are known to the last bit."""
     Tmax = max(lens)
