@@ -19,6 +19,8 @@
 // of 128, 1801 keys 11.7 -> 10.0, B = 16, 1001 keys 17.8 -> 16.3; 12 / 4 heads of 64 6.8 to 8.5 before and after.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "ptx.cuh"
 #include "tile_rows.h"
@@ -343,10 +345,20 @@ static int launch_decode(DecodeParams p, int B, cudaStream_t st) {
   if (warps < 4) warps = 4;
   if (p.KVH * p.groups > 65535 || B > 65535) return static_cast<int>(cudaErrorInvalidValue);
   const auto kern = p.kqv != nullptr ? decode_attn_kernel<D, RT, true> : decode_attn_kernel<D, RT, false>;
-  static const cudaError_t set[2] = {
-      cudaFuncSetAttribute(decode_attn_kernel<D, RT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWarps * kTiles),
-      cudaFuncSetAttribute(decode_attn_kernel<D, RT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWarps * kTiles)};
-  if (set[0] != cudaSuccess || set[1] != cudaSuccess) return static_cast<int>(set[0] != cudaSuccess ? set[0] : set[1]);
+  // Asked for on each device that the process uses (a failure is not kept). With the 64 KiB that head_dim 128 needs at least
+  // set on the first device alone, a launch on a second one would be refused.
+  static std::atomic<bool> allowed[2][64];
+  int dev = 0;
+  B200_CHECK(cudaGetDevice(&dev));
+  std::atomic<bool>* done = dev >= 0 && dev < 64 ? &allowed[p.kqv != nullptr][dev] : nullptr;
+  if (done == nullptr || !done->load(std::memory_order_acquire)) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWarps * kTiles);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return static_cast<int>(e);
+    }
+    if (done != nullptr) done->store(true, std::memory_order_release);
+  }
   p.status = status_ptr();
   return static_cast<int>(launch_pdl(kern, dim3(cs, p.KVH * p.groups, B), dim3(32 * warps), warps * kTiles, st, cs, p));
 }
