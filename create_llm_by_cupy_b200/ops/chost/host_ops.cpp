@@ -209,7 +209,7 @@ PyObject* embedding_fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 enum Route { TILES = 0, SKINNY = 1, SMALL = 2 };
 
-// gemm(a, b, trans_a, trans_b, out or None, add or None, fp32 output, alpha, whole-tiles flag, route, K splits) -> out.
+// gemm(a, b, trans_a, trans_b, out or None, add or None, fp32 output, alpha, whole-tiles and whole-K flags, route, K splits) -> out.
 // Routes: CTA-pair tiles (splits > 1: over K), the few-rows kernel, single-CTA tiles.
 PyObject* gemm(PyObject*, PyObject* const* a, Py_ssize_t n) {
   ARGS(11)

@@ -50,8 +50,8 @@ constexpr int G2_SMEM = G2_BAR_OFF2 + (2 * G2_STAGES + 4 + 2 * G2_SCHED + 4) * 8
 constexpr int G2_SCHED_SLOTS = 1024;   // {next tile, finished pairs} counter pairs, used round-robin by launches
 
 // G2_WHOLE_TILES (caller): never halve tiles - set for GEMMs that run beside a GEMM of another stream,
-// whose CTAs fill the SMs a part-filled last round leaves idle anyway.
-enum Gemm2Flags : int { G2_OUT_F32 = 1, G2_ADD_C = 2, G2_TMA_OUT = 4, G2_WHOLE_TILES = 8 };
+// whose CTAs fill the SMs a part-filled last round leaves idle anyway. G2_WHOLE_K (caller): never split K over a cluster.
+enum Gemm2Flags : int { G2_OUT_F32 = 1, G2_ADD_C = 2, G2_TMA_OUT = 4, G2_WHOLE_TILES = 8, G2_WHOLE_K = 16 };
 
 // What the epilogue does with the accumulator (a template parameter: the plain instantiations keep their
 // register count).
@@ -1453,7 +1453,7 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
   // Few tiles: two to four pairs to a tile, as many as there are clusters for at once, three k-blocks each at least (four: 300 x
   // 768 x 768 6.8 us in place of 6.5). Beside weight gradients too (125M training pass of 777 tokens 2811 us, 2686 so). Up to K =
   // 512 one range, whose sums are those of the GEMM that gathers its weight (257 x 256 x 512 7.2 us, 6.0 with two).
-  if (K > 512 && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & G2_OUT_F32) && N % 8 == 0) {
+  if (K > 512 && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & (G2_OUT_F32 | G2_WHOLE_K)) && N % 8 == 0) {
     const int halves = ((M + 2 * G2_BM - 1) / (2 * G2_BM)) * ((N + GC_BN - 1) / GC_BN), kbs = (K + G2_BK - 1) / G2_BK;
     int splits = 4;
     while (splits > 1 && (halves * splits > num_sms() / 2 || kbs < 3 * splits || halves > cluster_slots(splits))) --splits;

@@ -40,6 +40,7 @@ def _skinny(M: int, N: int) -> bool:
 
 
 GEMM_WHOLE_TILES = 8      # CTA-pair kernel: do not split the tiles of a part-filled last round
+GEMM_WHOLE_K = 16         # CTA-pair kernel: do not split K over a cluster
 _ROUTE_TILES, _ROUTE_SKINNY, _ROUTE_SMALL = range(3)      # kernels of ``native.host.gemm``
 
 # Code-path switches (module attributes; tests and the benchmark's baseline arm set them).
@@ -129,8 +130,15 @@ def _copy_rows(src: torch.Tensor, dst: torch.Tensor) -> torch.Tensor:
     return dst
 
 
-# 1: GEMMs with too few 256 x 256 tiles for the CTA pairs and a long K run as several K ranges per tile.
+# 1: GEMMs with too few tiles for the CTA pairs run as several K ranges per tile, over a cluster or over a workspace; 0: every
+# tile walks K once, so that the sums are those of the other tile kernels (the one that gathers its weight among them).
 GEMM_SPLIT_K = 1
+
+
+def _whole_flags(dev: int, side: bool | None) -> int:
+    """Flags of a CTA-pair GEMM on device ``dev`` that keep its tiles or its K whole (``side``: see ``_splits``)."""
+    whole = GEMM_WHOLE_TILES if _wgrad_pending.get(dev, False) else 0
+    return whole if GEMM_SPLIT_K and side is not False else whole | GEMM_WHOLE_K
 
 
 @functools.lru_cache(maxsize=4096)
@@ -217,7 +225,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
             splits = _splits(M, N, K, dev, side, not trans_a and N % 8 == 0 and out_dtype is torch.bfloat16)
             if splits == 1:
                 _apply_dynamic()
-                whole = GEMM_WHOLE_TILES if _wgrad_pending.get(dev, False) else 0
+                whole = _whole_flags(dev, side)
         else:
             route = _ROUTE_SMALL
         res = native.host.gemm(a, b, trans_a, trans_b, out, add, out_dtype is torch.float32, alpha, whole, route, splits)
@@ -293,8 +301,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
             # Half tiles shorten the tail of a GEMM that has the GPU to itself. While weight-gradient GEMMs
             # are in flight on the side stream the tail is filled by the other kernel's CTAs, and narrower
             # tiles only cost efficiency (measured on the 1.3 B step: 1.1 ms faster alone, 1.2 ms slower beside).
-            if _wgrad_pending.get(dev, False):
-                flags |= GEMM_WHOLE_TILES
+            flags |= _whole_flags(dev, side)
             rc = lib.b200_gemm_bf16_2cta(
                 c_void_p(pa), c_void_p(pb), c_void_p(po), native.ptr(add), M, N, K, lda, ldb, ldd, ldc, int(trans_a),
                 int(not trans_b), flags, c_float(alpha), native.stream_ptr())

@@ -52,3 +52,18 @@ def test_split_rule():
         s = G.split_count(M, N, K, 74)
         tiles = -(-M // 256) * -(-N // 256)
         assert 1 <= s <= 16 and (s == 1 or (tiles * s <= 74 and s <= -(-K // 64)))
+
+
+@pytest.mark.parametrize("M,N,K", [(777, 768, 768), (300, 264, 2056), (512, 2048, 2048), (256, 256, 16384)])
+def test_switched_off(M, N, K, monkeypatch):
+    """GEMM_SPLIT_K = 0 (and a weight gradient that has to stay whole): one range of K whatever kernel runs, so the sums are those
+    of the single-CTA kernel bit for bit; with the switch on the same shapes are split."""
+    a, b, c = bf(M, K, seed=1), bf(K, N, seed=2), bf(M, N, seed=3)
+    want, plus = G.gemm(a, b, impl="1cta"), G.gemm(a, b, add=c, impl="1cta")
+    assert not torch.equal(G.gemm(a, b), want)
+    monkeypatch.setattr(G, "GEMM_SPLIT_K", 0)
+    assert torch.equal(G.gemm(a, b), want) and torch.equal(G.gemm(a, b, add=c), plus)
+    monkeypatch.setattr(G.native, "host", None)
+    assert torch.equal(G.gemm(a, b), want) and torch.equal(G.gemm(a, b, add=c), plus)
+    monkeypatch.setattr(G, "GEMM_SPLIT_K", 1)
+    assert torch.equal(G.gemm(a, b, side=False), want) and not torch.equal(G.gemm(a, b), want)
