@@ -1307,6 +1307,23 @@ static int cluster_slots(int splits) {
   return n - 1;
 }
 
+static int cluster_tiles(int M, int N) { return ((M + 2 * G2_BM - 1) / (2 * G2_BM)) * ((N + GC_BN - 1) / GC_BN); }
+
+// Pairs to a tile for few tiles (1: the other kernels): two to four, three k-blocks each at least (four: 300 x 768 x 768 6.8 us
+// in place of 6.5), and only as many as run at once: a B200 holds 33 clusters of two pairs, 22 of three and 15 of four, fewer
+// than its 74 pairs make, so 777 x 768 (24 tiles) takes two and 768 x 768 (18) three. Beside weight gradients too (125M
+// training pass of 777 tokens 2811 us, 2686 so). us one range / so: K = 576 257 x 256 7.5 / 5.9, 777 x 768 8.0 / 6.6, 1000 x 1024
+// 8.2 / 6.8; 768 8.3 / 5.8, 8.8 / 7.0, 9.1 / 7.2. Up to K = 512 the sums stay those of one range, which the GEMM that gathers
+// its weight is compared with bit for bit: a line of results, not of time (384 6.9 / 5.5, 7.1 / 6.2, 7.3 / 6.3; 512 7.3 / 5.8, 7.7 /
+// 6.6, 7.9 / 6.6).
+static int cluster_splits(int M, int N, int K) {
+  if (K <= 512) return 1;
+  const int tiles = cluster_tiles(M, N), kbs = (K + G2_BK - 1) / G2_BK;
+  int splits = 4;
+  while (splits > 1 && (tiles * splits > num_sms() / 2 || kbs < 3 * splits || tiles > cluster_slots(splits))) --splits;
+  return splits;
+}
+
 // out = sum over the splits of ws[split][row][col] (+ C), fixed order. 16-byte accesses where every row allows them.
 __global__ void __launch_bounds__(256)
 splitk_sum_kernel(const float* ws, void* D, const void* C, int M, int N, int splits, int ldws, size_t plane,
@@ -1382,6 +1399,12 @@ B200_API int b200_gemm_2cta_half_tiles(int on) {
   return old;
 }
 
+// Ranges of K that b200_gemm_bf16_2cta splits such a product into on the current device (1: none) where its layout and result
+// allow it (row-major A, bf16 result, N a multiple of 8, D and C TMA-addressable).
+B200_API int b200_gemm_2cta_cluster_splits(int M, int N, int K) {
+  return M > 0 && N > 0 && K > 0 ? cluster_splits(M, N, K) : 1;
+}
+
 static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, int M, int N, int K, int lda, int ldb,
                          int ldd, int ldc, int a_mn_major, int b_mn_major, int flags, float alpha,
                          const float* rope_cos, const float* rope_sin, int rope_T, int rope_ld, int rope_cols,
@@ -1450,18 +1473,13 @@ static int gemm_2cta_run(const void* A, const void* B, void* D, const void* C, i
     if (b_mn_major) return launch_tc2<false, true, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
     return launch_tc2<false, false, EPI_ROPE>(tA, tB, tBh, tD, tC, p, stream);
   }
-  // Few tiles: two to four pairs to a tile, as many as there are clusters for at once, three k-blocks each at least (four: 300 x
-  // 768 x 768 6.8 us in place of 6.5). Beside weight gradients too (125M training pass of 777 tokens 2811 us, 2686 so). Up to K =
-  // 512 one range, whose sums are those of the GEMM that gathers its weight (257 x 256 x 512 7.2 us, 6.0 with two).
-  if (K > 512 && !a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & (G2_OUT_F32 | G2_WHOLE_K)) && N % 8 == 0) {
-    const int halves = ((M + 2 * G2_BM - 1) / (2 * G2_BM)) * ((N + GC_BN - 1) / GC_BN), kbs = (K + G2_BK - 1) / G2_BK;
-    int splits = 4;
-    while (splits > 1 && (halves * splits > num_sms() / 2 || kbs < 3 * splits || halves > cluster_slots(splits))) --splits;
+  if (!a_mn_major && (p.flags & G2_TMA_OUT) && !(flags & (G2_OUT_F32 | G2_WHOLE_K)) && N % 8 == 0) {
+    const int splits = cluster_splits(M, N, K);
     if (splits > 1) {
       p.splits = splits;
       auto kern = b_mn_major ? gemm_bf16_tc2_cluster_kernel<true> : gemm_bf16_tc2_cluster_kernel<false>;
-      return static_cast<int>(launch_pdl(kern, dim3(2 * splits * halves), dim3(GC_THREADS), GC_SMEM, stream, 2 * splits, *tA,
-                                         b_mn_major ? *tB : *tBh, p));
+      return static_cast<int>(launch_pdl(kern, dim3(2 * splits * cluster_tiles(M, N)), dim3(GC_THREADS), GC_SMEM, stream, 2 * splits,
+                                         *tA, b_mn_major ? *tB : *tBh, p));
     }
   }
   // The addend's tiles fetched ahead (one operand stage less) where the epilogue is a large part of a tile's life: one

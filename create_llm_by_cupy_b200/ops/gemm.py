@@ -142,29 +142,34 @@ def _whole_flags(dev: int, side: bool | None) -> int:
 
 
 @functools.lru_cache(maxsize=4096)
-def split_count(M: int, N: int, K: int, pairs: int, cluster: bool = False) -> int:
+def split_count(M: int, N: int, K: int, pairs: int, cluster: int = 1) -> int:
     """K ranges per 256 x 256 tile (1: no split), by the time each number takes: 0.29 us per 64-deep block of K that one
     pair walks and, for a split, the second kernel with 2 us of launch and the fp32 sums read at about 4 TB/s. A split
     has to win 4 us, what its workspace and second launch cost the host. Measured, one range against the rule's:
     768 x 1280 over K = 8192 44.3 / 22.4 us, 768 x 768 over 8192 44.4 / 17.6, 256 x 4096 over 11008 57.0 / 29.4. Left whole:
-    777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4). ``cluster``: the call can take the
-    kernel that splits K over a cluster (bf16 result, A row-major), which has no second launch and 1 us for its sums; ranges
+    777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4). ``cluster``: ranges of the kernel
+    that splits K over a cluster, if the call takes it (1: it does not), which has no second launch and 1 us for its sums; ranges
     have to be shorter than that then: 640 x 768 over 4096 11.0 us there, 15.8 with 6 ranges; 768 x 1024 over 8192 20.7, 19.1
     with 6. On the line between them the rule is 1 us off: 256 x 4096 over 11008 28.2 there, 29.2 with the 4 that it takes, 768 x
     1280 over 8192 20.9, 22.5 with 4."""
     tiles = -(-M // 256) * -(-N // 256)
     kb = -(-K // 64)
     whole, gain = 0.29 * kb, 4.0
-    if cluster and K > 512:
-        n = min(4, pairs // (-(-M // 256) * -(-N // 128)), kb // 3)
-        if n > 1:
-            whole, gain = 0.29 * -(-kb // n) + 1.0, 0.0
+    if cluster > 1:
+        whole, gain = 0.29 * -(-kb // cluster) + 1.0, 0.0
 
     def cost(n):
         return whole if n == 1 else 0.29 * -(-kb // n) + 2.0 + 1e-6 * n * M * N
 
     best = min(range(1, max(1, min(pairs // tiles, kb // 4, 16)) + 1), key=cost)
     return best if cost(best) < whole - gain else 1
+
+
+@functools.lru_cache(maxsize=4096)
+def cluster_splits(M: int, N: int, K: int, dev: int) -> int:
+    """Ranges of K that the CTA-pair kernel splits a bf16 product with a row-major ``a`` into by itself (1: none) on the
+    current device ``dev``."""
+    return native.lib().b200_gemm_2cta_cluster_splits(M, N, K)
 
 
 def _splits(M: int, N: int, K: int, dev: int, side: bool | None, cluster: bool) -> int:
@@ -183,7 +188,7 @@ def _splits(M: int, N: int, K: int, dev: int, side: bool | None, cluster: bool) 
     pairs = _cta_pairs(dev)
     if side is None and _wgrad_pending.get(dev, False) and -(-M // 256) * -(-N // 256) * 10 > pairs * 3:
         return 1
-    return split_count(M, N, K, pairs, cluster)
+    return split_count(M, N, K, pairs, cluster_splits(M, N, K, dev) if cluster else 1)
 
 
 _pairs: dict = {}

@@ -92,12 +92,17 @@ def test_swiglu_backward(M, I, K):
         assert ((out - d * f).abs() <= lim).all()
 
 
-# K split over a cluster: 2, 3 and 4 pairs to a tile (37, 24 and 12 tiles of 256 x 128), ranges of unequal length, tiles cut by M
-# and N, one range up to K = 512
-@pytest.mark.parametrize("M,N", [(1100, 896), (777, 768), (256, 256), (300, 264), (300, 1544)])
+# K split over a cluster: 2, 3 (uneven shares of a tile's columns) and 4 pairs to a tile (24 and 26, 18 and 20, 2 and 6 tiles of
+# 256 x 128), ranges of unequal length, three k-blocks each at least, tiles cut by M and N, one range up to K = 512; 35 tiles,
+# for which no B200 holds clusters enough
+CLUSTER_PAIRS = {(1100, 896): 1, (777, 768): 2, (300, 1544): 2, (768, 768): 3, (400, 1200): 3, (256, 256): 4, (300, 264): 4}
+
+
+@pytest.mark.parametrize("M,N", list(CLUSTER_PAIRS))
 @pytest.mark.parametrize("K", [512, 520, 840, 2056])
 @pytest.mark.parametrize("trans_b", [False, True])
 def test_cluster_split(M, N, K, trans_b):
+    assert G.cluster_splits(M, N, K, 0) == (1 if K <= 512 else min(CLUSTER_PAIRS[M, N], -(-K // 64) // 3))
     a, b, c = bf(M, K, seed=1), bf(K, N, seed=2), bf(M, N, seed=3)
     w = b.t().contiguous() if trans_b else b
     want, bound = product(a, b)

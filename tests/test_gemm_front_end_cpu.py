@@ -33,6 +33,7 @@ def lib(monkeypatch):
     empty = torch.empty
     monkeypatch.setattr(torch, "empty", lambda *a, **k: empty(*a, **k).as_subclass(FakeCuda))
     monkeypatch.setattr(G, "_cta_pairs", lambda index: 74)
+    monkeypatch.setattr(G, "cluster_splits", lambda M, N, K, dev: 1)
     monkeypatch.setattr(G, "WGRAD_OVERLAP", False)
     monkeypatch.setattr(native, "lib", lambda: rec)
     monkeypatch.setattr(native, "status_tensor", lambda device=None: None)
