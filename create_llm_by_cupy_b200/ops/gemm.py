@@ -147,16 +147,16 @@ def split_count(M: int, N: int, K: int, pairs: int, cluster: int = 1) -> int:
     pair walks and, for a split, the second kernel with 2 us of launch and the fp32 sums read at about 4 TB/s. A split
     has to win 4 us, what its workspace and second launch cost the host. Measured, one range against the rule's:
     768 x 1280 over K = 8192 44.3 / 22.4 us, 768 x 768 over 8192 44.4 / 17.6, 256 x 4096 over 11008 57.0 / 29.4. Left whole:
-    777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4). ``cluster``: ranges of the kernel
-    that splits K over a cluster, if the call takes it (1: it does not), which has no second launch and 1 us for its sums; ranges
-    have to be shorter than that then: 640 x 768 over 4096 11.0 us there, 15.8 with 6 ranges; 768 x 1024 over 8192 20.7, 19.1
-    with 6. On the line between them the rule is 1 us off: 256 x 4096 over 11008 28.2 there, 29.2 with the 4 that it takes, 768 x
-    1280 over 8192 20.9, 22.5 with 4."""
+    777 x 768 over 2048 (16.6 / 14.2 with 3), 768 x 768 over 1024 (12.0 / 12.4 with 4).
+
+    ``cluster``: ranges of the kernel that splits K over a cluster, if the call takes it (1: it does not). That one has neither
+    cost, so a split has to win the same 4 us against it, and 4 more, by which ``cost`` is short of what a split takes (256 x
+    4096 over 11008: 24 us more than its launch and tail, ``cost`` says 19). us over the cluster / split: 768 x 768 over 8192 16.6 /
+    18.1, 768 x 1280 20.9 / 22.8, 768 x 1024 20.7 / 19.3, 256 x 4096 over 11008 28.4 / 29.5, 512 x 512 over 16384 20.6 / 18.8, all
+    left to the cluster; split are 512 x 512 over 32768 35.2 / 25.7, 777 x 768 66.9 / 41.6, 256 x 4096 over 22016 52.4 / 45.4."""
     tiles = -(-M // 256) * -(-N // 256)
     kb = -(-K // 64)
-    whole, gain = 0.29 * kb, 4.0
-    if cluster > 1:
-        whole, gain = 0.29 * -(-kb // cluster) + 1.0, 0.0
+    whole, gain = (0.29 * kb, 4.0) if cluster <= 1 else (0.23 * -(-kb // cluster) + 0.8, 8.0)
 
     def cost(n):
         return whole if n == 1 else 0.29 * -(-kb // n) + 2.0 + 1e-6 * n * M * N

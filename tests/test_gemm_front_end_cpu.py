@@ -110,6 +110,23 @@ def test_split_k_beside_other_kernels(lib, monkeypatch, tiles, pending, side, sp
     assert lib.names()[-2] == ("b200_gemm_bf16_2cta_split" if split else "b200_gemm_bf16_2cta")
 
 
+# us with K split over a cluster of that many pairs / over ranges in a workspace (the best number of them)
+BOTH_SPLITS = [
+    (256, 256, 2048, 4, 6.8, 11.3), (256, 256, 4096, 4, 8.4, 12.4), (256, 256, 8192, 4, 11.8, 13.8), (256, 256, 16384, 4, 18.5, 16.2),
+    (256, 256, 65536, 4, 59.3, 30.6), (512, 512, 4096, 4, 9.3, 13.2), (512, 512, 8192, 4, 13.1, 15.3), (512, 512, 16384, 4, 20.6, 18.8),
+    (512, 512, 32768, 4, 35.2, 25.7), (640, 768, 4096, 3, 11.3, 15.2), (768, 768, 8192, 3, 16.6, 18.1), (768, 768, 16384, 3, 26.4, 23.9),
+    (768, 1024, 4096, 2, 13.2, 15.6), (768, 1024, 8192, 2, 20.7, 19.3), (768, 1280, 8192, 2, 20.9, 22.8),
+    (256, 4096, 11008, 2, 28.4, 29.5), (256, 4096, 22016, 2, 52.4, 45.4), (512, 2048, 8192, 2, 21.3, 23.1),
+    (256, 2048, 5504, 3, 13.0, 16.4), (256, 2048, 11008, 3, 19.9, 20.3), (300, 1544, 8192, 2, 20.5, 21.8),
+    (777, 768, 32768, 2, 66.9, 41.6), (1024, 1024, 16384, 2, 36.1, 34.4), (400, 2048, 11008, 2, 25.5, 25.9)]
+
+
+@pytest.mark.parametrize("M,N,K,cluster,us_cluster,us_workspace", BOTH_SPLITS)
+def test_a_workspace_has_to_win_its_host_cost_beside_a_cluster_too(M, N, K, cluster, us_cluster, us_workspace):
+    assert G.split_count(M, N, K, 74) > 1                    # without the cluster kernel each of them is split
+    assert (G.split_count(M, N, K, 74, cluster) > 1) == (us_cluster - us_workspace > 4)
+
+
 @pytest.mark.parametrize("M,K,name", [(8, 64, "b200_gemm_skinny"), (9, 504, "b200_gemm_bf16"), (9, 512, "b200_gemm_skinny"),
                                       (64, 511, "b200_gemm_bf16"), (64, 512, "b200_gemm_skinny"), (65, 512, "b200_gemm_bf16")])
 def test_few_rows_over_a_short_inner_dimension(lib, M, K, name):
