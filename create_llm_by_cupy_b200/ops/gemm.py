@@ -172,6 +172,13 @@ def cluster_splits(M: int, N: int, K: int, dev: int) -> int:
     return native.lib().b200_gemm_2cta_cluster_splits(M, N, K)
 
 
+def _cluster_result(N: int, out_dtype: torch.dtype, add: torch.Tensor | None) -> bool:
+    """Whether the kernel that splits K over a cluster takes such a result and addend: bf16 in whole 16-byte pieces (an output
+    that is not goes through one that is)."""
+    return (N % 8 == 0 and out_dtype is torch.bfloat16
+            and (add is None or (add.stride(0) % 8 == 0 and add.data_ptr() % 16 == 0)))
+
+
 def _splits(M: int, N: int, K: int, dev: int, side: bool | None, cluster: bool) -> int:
     """K ranges per tile for one call. ``split_count`` gives the GEMM the GPU to itself; beside another kernel the idle
     pairs are not idle, and what remains of its gain depends on who waits for the result:
@@ -227,7 +234,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         elif M >= 256 and N >= 256:
             route = _ROUTE_TILES
             dev = torch._C._cuda_getDevice()
-            splits = _splits(M, N, K, dev, side, not trans_a and N % 8 == 0 and out_dtype is torch.bfloat16)
+            splits = _splits(M, N, K, dev, side, not trans_a and _cluster_result(N, out_dtype, add))
             if splits == 1:
                 _apply_dynamic()
                 whole = _whole_flags(dev, side)
@@ -293,7 +300,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
                 _copy_rows(tmp, out)
                 return out
             dev = a.get_device()
-            splits = _splits(M, N, K, dev, side, not trans_a and N % 8 == 0 and out_dtype is torch.bfloat16)
+            splits = _splits(M, N, K, dev, side, not trans_a and _cluster_result(N, out_dtype, add))
             if splits > 1:
                 ws = torch.empty(splits * (-(-M // 256) * 256) * (-(-N // 4) * 4), dtype=torch.float32, device=a.device)
                 rc = lib.b200_gemm_bf16_2cta_split(

@@ -127,6 +127,16 @@ def test_a_workspace_has_to_win_its_host_cost_beside_a_cluster_too(M, N, K, clus
     assert (G.split_count(M, N, K, 74, cluster) > 1) == (us_cluster - us_workspace > 4)
 
 
+def test_an_addend_that_the_cluster_kernel_does_not_take_leaves_the_workspace_split(lib, monkeypatch):
+    monkeypatch.setattr(G, "cluster_splits", lambda M, N, K, dev: 4)
+    a, b = fake(256, 4096), fake(4096, 256)
+    buf = fake(256 * 264 + 8)
+    aligned, base = buf[:256 * 264].view(256, 264)[:, :256], buf[1:256 * 264 + 1].view(256, 264)[:, :256]
+    for add, split in ((None, False), (aligned, False), (base, True), (fake(256, 257)[:, :256], True)):
+        G.gemm(a, b, add=add)
+        assert lib.names()[-1] == ("b200_gemm_bf16_2cta_split" if split else "b200_gemm_bf16_2cta"), add
+
+
 @pytest.mark.parametrize("M,K,name", [(8, 64, "b200_gemm_skinny"), (9, 504, "b200_gemm_bf16"), (9, 512, "b200_gemm_skinny"),
                                       (64, 511, "b200_gemm_bf16"), (64, 512, "b200_gemm_skinny"), (65, 512, "b200_gemm_bf16")])
 def test_few_rows_over_a_short_inner_dimension(lib, M, K, name):
