@@ -324,41 +324,92 @@ decode_attn_kernel(const DecodeParams p) {
   if (threadIdx.x == 0 && abort_flag != 0 && p.status != nullptr && atomicCAS(p.status, 0, abort_flag) == 0) p.status[1] = 330;
 }
 
+// What one of the decode attention's kernels may use and how much of it fits, per device of the process (nothing is kept of a
+// request that failed).
+struct DecodeDevice {
+  std::atomic<bool> allowed{false};       // its dynamic shared memory: more than 48 KiB from head_dim 128's 4 warps on
+  std::atomic<int> fit[5] = {};           // 1 + the CTAs of 1 to 4 warps that run at the same time
+  std::atomic<int> clusters[4][DA_MAX_WARPS + 1] = {};      // 1 + the clusters of 1, 2, 4, 8 CTAs of that many warps
+};
+
 template <int D, int RT>
 static int launch_decode(DecodeParams p, int B, cudaStream_t st) {
   p.groups = (p.QH / p.KVH + RT - 1) / RT;
   const long pairs = long(B) * p.KVH * p.groups;
-  const int keys = p.kqv != nullptr ? p.pos + 1 : p.Tmax;       // what the lengths are expected to be, at most; longer ones work too
-  const int tiles = (keys + DA_TILE - 1) / DA_TILE;
-  // Up to 8 CTAs per (sequence, KV head): doubled while there are more tiles than CTAs and one CTA per SM of head_dim 128 (two
-  // of 64, four of 32: the same bytes) is not exceeded yet. At least four warps (they also form the result), up to 128 KiB of
-  // tiles while at most one CTA per SM exists. Swept for the attention alone, us: 8 sequences, 8 KV heads of 128, 3001 keys 34.8
-  // with 256 CTAs of four warps (45.1 with 512, 36.9 with 512 of two); 16 x 4 heads, 1001 keys 21.2 with 256 of four (28.7 with
-  // 512 of four); 4 x 4 heads, 301 keys 14.3 with four warps (22.5 with eight: their 128 KiB have to wait for an empty SM).
+  if (p.KVH * p.groups > 65535 || B > 65535) return static_cast<int>(cudaErrorInvalidValue);
   constexpr int kTiles = 2 * DA_TILE * D * 2;
   constexpr int kMaxWarps = 131072 / kTiles < DA_MAX_WARPS ? 131072 / kTiles : DA_MAX_WARPS;
-  int cs = 1;
-  while (cs < 8 && cs < tiles && pairs * cs * kTiles <= 16384L * num_sms()) cs *= 2;
-  int warps = (tiles + cs - 1) / cs;
-  const int cap = pairs * cs <= num_sms() ? kMaxWarps : 4;
-  if (warps > cap) warps = cap;
-  if (warps < 4) warps = 4;
-  if (p.KVH * p.groups > 65535 || B > 65535) return static_cast<int>(cudaErrorInvalidValue);
   const auto kern = p.kqv != nullptr ? decode_attn_kernel<D, RT, true> : decode_attn_kernel<D, RT, false>;
-  // Asked for on each device that the process uses (a failure is not kept). With the 64 KiB that head_dim 128 needs at least
-  // set on the first device alone, a launch on a second one would be refused.
-  static std::atomic<bool> allowed[2][64];
+  // With the shared memory asked for on the first device alone, a launch on a second one would be refused.
+  static DecodeDevice devices[2][64];
   int dev = 0;
   B200_CHECK(cudaGetDevice(&dev));
-  std::atomic<bool>* done = dev >= 0 && dev < 64 ? &allowed[p.kqv != nullptr][dev] : nullptr;
-  if (done == nullptr || !done->load(std::memory_order_acquire)) {
+  DecodeDevice* known = dev >= 0 && dev < 64 ? &devices[p.kqv != nullptr][dev] : nullptr;
+  if (known == nullptr || !known->allowed.load(std::memory_order_acquire)) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxWarps * kTiles);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return static_cast<int>(e);
     }
-    if (done != nullptr) done->store(true, std::memory_order_release);
+    if (known != nullptr) known->allowed.store(true, std::memory_order_release);
   }
+  auto once = [](std::atomic<int>* kept, auto query) -> long {        // a count that the device is asked for once, 0: not known
+    int n = kept != nullptr ? kept->load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+      if (query(&n) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+      }
+      ++n;
+      if (kept != nullptr) kept->store(n, std::memory_order_relaxed);
+    }
+    return n - 1;
+  };
+  auto fit = [&](int warps) -> long {      // CTAs of that many warps (up to 4) that run at the same time
+    return once(known != nullptr ? &known->fit[warps] : nullptr, [&](int* n) {
+      const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, kern, 32 * warps, warps * kTiles);
+      *n *= num_sms();
+      return e;
+    });
+  };
+  auto fit_clusters = [&](int cs, int warps) -> long {
+    return once(known != nullptr ? &known->clusters[cs == 8 ? 3 : cs >> 1][warps] : nullptr, [&](int* n) {
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = cs;
+      at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(cs);
+      cfg.blockDim = dim3(32 * warps);
+      cfg.dynamicSmemBytes = warps * kTiles;
+      cfg.attrs = at;
+      cfg.numAttrs = 1;
+      return cudaOccupancyMaxActiveClusters(n, kern, &cfg);
+    });
+  };
+  const int keys = p.kqv != nullptr ? p.pos + 1 : p.Tmax;       // what the lengths are expected to be, at most; longer ones work too
+  const int tiles = (keys + DA_TILE - 1) / DA_TILE;
+  // Up to 8 CTAs per (sequence, KV head): doubled while there are more tiles than CTAs, one CTA per SM of head_dim 128 (two
+  // of 64, four of 32: the same bytes) is not exceeded yet and twice as many still run at the same time. At least four warps
+  // (they also form the result), up to 128 KiB of tiles while at most one CTA per SM exists. Swept for the attention alone, us:
+  // 8 sequences, 8 KV heads of 128, 3001 keys 34.8 with 256 CTAs of four warps (45.1 with 512, 36.9 with 512 of two); 16 x 4
+  // heads, 1001 keys 21.2 with 256 of four (28.7 with 512 of four); 4 x 4 heads, 301 keys 14.3 with four warps (22.5 with eight:
+  // their 128 KiB have to wait for an empty SM); 32 x 4 heads of 32, 301 keys 6.4 with 512 of four (11.2 with 1024).
+  int cs = 1;
+  while (cs < 8 && cs < tiles && pairs * cs * kTiles <= 16384L * num_sms() && 2 * pairs * cs <= fit(4)) cs *= 2;
+  int warps = (tiles + cs - 1) / cs;
+  const int cap = pairs * cs <= num_sms() ? kMaxWarps : 4;
+  if (warps > cap) warps = cap;
+  if (warps < 4) warps = 4;
+  // More than four only where all clusters still run at once: CTAs of which an SM holds one leave no room for the last of 16
+  // clusters of eight (a 1.3B block of 4 sequences, 2048 keys 53.4 us with eight warps, 47.3 with four; 125M, 3001 keys 35.1 with
+  // twelve, 29.9 with eight).
+  while (warps > 4 && pairs > fit_clusters(cs, warps)) warps = (warps - 1) / 4 * 4 < 4 ? 4 : (warps - 1) / 4 * 4;
+  // Fewer where only they all run at once, with a twentieth to spare for an uneven spread: 512 CTAs of head_dim 128, 31 keys
+  // 12.4 us with two warps (18.9 with four, of which 296 fit), 3001 keys 131 (142); 1024 16.7 and 252 with one (36 and 283).
+  auto one_round = [&](int w) { return 20 * pairs * cs <= 19 * fit(w); };
+  if (warps == 4 && pairs * cs > num_sms() && one_round(1))
+    while (!one_round(warps)) --warps;
   p.status = status_ptr();
   return static_cast<int>(launch_pdl(kern, dim3(cs, p.KVH * p.groups, B), dim3(32 * warps), warps * kTiles, st, cs, p));
 }
