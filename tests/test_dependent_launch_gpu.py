@@ -54,8 +54,11 @@ def _producers():
     wide_w, small_w = rnd(1024, R * C // 8, seed=5, std=1 / 32), rnd(1024, 8192, seed=6, std=1 / 32)
     yield "gemm_few_rows", lambda: F.gemm(a[:8], wide_w).view(-1, C)
     yield "gemm_small", lambda: F.gemm(a[:200], small_w).view(-1, C)
-    long_a, long_w, gate = rnd(R, 8192, seed=7), rnd(8192, C, seed=8, std=1 / 90), rnd(1024, 2 * C, seed=9, std=1 / 32)
-    yield "gemm_split_k", lambda: F.gemm(long_a, long_w)
+    long_a, long_w, gate = rnd(8192, R, seed=7), rnd(8192, C, seed=8, std=1 / 90), rnd(1024, 2 * C, seed=9, std=1 / 32)
+    assert G._splits(R, C, 8192, 0, None, False) > 1            # ranges in a workspace, then their sum
+    yield "gemm_split_k", lambda: F.gemm(long_a, long_w, trans_a=True)
+    assert G.cluster_splits(R, C, 2048, 0) > 1 and G._splits(R, C, 2048, 0, None, True) == 1
+    yield "gemm_cluster", lambda: F.gemm(x[:R], long_w[:2048])
     yield "gemm_swiglu", lambda: F.gemm_swiglu(a, gate)[1]
     ids = torch.arange(4096, dtype=torch.int32, device=DEV) * 3
     yield "embedding", lambda: F.embedding_fwd(x, ids, -1)
@@ -88,17 +91,28 @@ def _consumers():
     yield "norm_gain", lambda s: F.rmsnorm_fwd(x, s[-1])
     yield "norm_bwd", lambda s: F.rmsnorm_bwd(s, x, g, rstd)
     yield "norm_bwd_x_add", lambda s: F.rmsnorm_bwd(x, s, s[-1], rstd, add=s)
-    yield "gemm", lambda s: F.gemm(s, rnd(C, 768, seed=24))
+    # few tiles: K over a cluster
+    assert all(G.cluster_splits(R, N, C, 0) > 1 and G._splits(R, N, C, 0, None, True) == 1 for N in (256, R, 768, C))
+    yield "gemm_cluster", lambda s: F.gemm(s, rnd(C, 768, seed=24))
+    yield "gemm_cluster_weight_t", lambda s: F.gemm(x, s, trans_b=True)
+    yield "gemm_cluster_add", lambda s: F.gemm(x, sq, add=s)
+    # more of them, or a short K: one range
+    assert G.cluster_splits(R, 3072, C, 0) == G.cluster_splits(4096, R, C, 0) == G.cluster_splits(R, C, 512, 0) == 1
+    wide, tall = rnd(C, 3072, seed=28, std=1 / 45), rnd(4096, C, seed=29)
+    yield "gemm", lambda s: F.gemm(s, wide)
     yield "gemm_weight", lambda s: F.gemm(x[:300, :R], s)
-    yield "gemm_weight_t", lambda s: F.gemm(x, s, trans_b=True)
+    yield "gemm_weight_t", lambda s: F.gemm(tall, s, trans_b=True)
     yield "gemm_weight_grad", lambda s: F.gemm(s, x, trans_a=True)
-    yield "gemm_add", lambda s: F.gemm(x, sq, add=s)
+    yield "gemm_add", lambda s: F.gemm(x[:, :512], sq[:512], add=s)
     yield "gemm_fp32_add", lambda s: F.gemm(x, sq[:, :C // 2], add=s.view(torch.float32))
     yield "gemm_small", lambda s: F.gemm(s[-200:], sq)
     yield "gemm_few_rows", lambda s: F.gemm(s[-7:], sq)
     yield "gemm_few_rows_weight", lambda s: F.gemm(x[:7, :R], s, add=s[:7])
-    yield "gemm_split_k", lambda s: F.gemm(s, sq[:, :256])
-    yield "gemm_split_k_add", lambda s: F.gemm(x, sq[:, :256], add=s[:, :256])
+    yield "gemm_cluster_few", lambda s: F.gemm(s, sq[:, :256])
+    yield "gemm_cluster_few_add", lambda s: F.gemm(x, sq[:, :256], add=s[:, :256])
+    assert G._splits(R, 256, C, 0, None, False) > 1             # an fp32 result: ranges in a workspace, then their sum
+    yield "gemm_split_k", lambda s: F.gemm(s, sq[:, :256], out_dtype=torch.float32)
+    yield "gemm_split_k_add", lambda s: F.gemm(x, sq[:, :256], add=s.view(torch.float32)[:, :256])
     for D in (64, 128):
         cos, sin = F.rope_table(R, D, 10000.0, x.device)
         yield f"gemm_rope_{D}", lambda s, D=D, c=cos, sn=sin: F.gemm_rope(s, sq, c, sn, R, D, C // 2)
@@ -157,7 +171,8 @@ def consumers():
     return made
 
 
-PRODUCERS = ["norm", "norm_bwd", "gemm", "gemm_add", "gemm_few_rows", "gemm_small", "gemm_split_k", "gemm_swiglu", "embedding", "repitch",
+PRODUCERS = ["norm", "norm_bwd", "gemm", "gemm_add", "gemm_few_rows", "gemm_small", "gemm_split_k", "gemm_cluster", "gemm_swiglu",
+             "embedding", "repitch",
              "flash_fwd", "flash_bwd", "ce_stats"]
 
 

@@ -20,11 +20,13 @@ def product(a, b):
     return a @ b, (a.abs() @ b.abs()) * (a.shape[1] * 2.0 ** -23)
 
 
-# 256 x 256 tiles: 1, 4 with remainders, 80 and 100 (a round of 74 pairs and half tiles), 152 (two rounds and half tiles)
-@pytest.mark.parametrize("M,N", [(256, 256), (300, 264), (513, 1000), (2304, 2304), (2048, 3200), (2050, 4104)])
+# 256 x 256 tiles: 1, 4 with remainders (over K > 512 the cluster kernel's), 32 (one round, too many for that one), 80 and 100 (a
+# round of 74 pairs and half tiles), 152 (two rounds and half tiles)
+@pytest.mark.parametrize("M,N", [(256, 256), (300, 264), (513, 1000), (2048, 1024), (2304, 2304), (2048, 3200), (2050, 4104)])
 @pytest.mark.parametrize("K", [64, 72, 768, 1280, 1344, 4096])
 @pytest.mark.parametrize("trans_b", [False, True])
 def test_addend(M, N, K, trans_b):
+    assert (G.cluster_splits(M, N, K, 0) > 1) == (M < 2048 and K > 512) and G._splits(M, N, K, 0, None, True) == 1
     a, b, c = bf(M, K, seed=1), bf(K, N, seed=2), bf(M, N, seed=3)
     w = b.t().contiguous() if trans_b else b
     want, bound = product(a, b)

@@ -199,6 +199,33 @@ def test_virtual_ranks_gemm_with_the_all_gather_fused_in(W, only_b):
     vr.close()
 
 
+@pytest.mark.parametrize("M,H,N2", [(384, 512, 768), (384, 768, 768), (300, 2048, 512), (777, 1360, 1280)])
+def test_virtual_ranks_gemm_with_the_all_gather_against_the_forms_of_the_plain_one(M, H, N2, monkeypatch):
+    """It walks K once: equal to the plain GEMM bit for bit at every K where that one does too (GEMM_SPLIT_K = 0), and within the
+    error of two orders of fp32 sums and two roundings where that one adds ranges of K."""
+    from create_llm_by_cupy_b200.ops import gemm as G
+    from create_llm_by_cupy_b200.parallel.symm import LocalVirtualRanks
+
+    W = 2
+    n_unit = -(-H * N2 // (W * 128)) * (W * 128)
+    vr = LocalVirtualRanks(W, heap_bytes=32 << 20)
+    off, shards = vr.alloc(n_unit // W, torch.bfloat16)
+    full = (torch.randn(n_unit, generator=torch.Generator().manual_seed(H)) * 0.5).to(torch.bfloat16)
+    for r, sh in enumerate(shards):
+        sh.copy_(full[r * (n_unit // W):(r + 1) * (n_unit // W)])
+    a = (torch.randn(M, H, generator=torch.Generator().manual_seed(7)) * 0.5).to(torch.bfloat16).cuda()
+    w = full[:H * N2].view(H, N2).cuda()
+    out = vr.gemm_allgather(a, off, n_unit // W, torch.zeros(n_unit, dtype=torch.bfloat16, device="cuda"), 0, (H, N2), trans_b=False)
+    split = G.gemm(a, w)
+    monkeypatch.setattr(G, "GEMM_SPLIT_K", 0)
+    assert torch.equal(out, G.gemm(a, w))
+    assert torch.equal(out, split) == (G.cluster_splits(M, N2, H, 0) == 1)
+    lim = a.double().abs() @ w.double().abs() * (H * 2.0 ** -22) + 2.0 ** -7 * out.double().abs()
+    assert ((out.double() - split.double()).abs() <= lim).all()
+    assert native.read_status() == (0, 0)
+    vr.close()
+
+
 def test_heap_guard_blocks_report_a_write_past_the_end_of_an_allocation():
     from create_llm_by_cupy_b200.parallel.comm import SingleProcessComm
     from create_llm_by_cupy_b200.parallel.symm import SymmetricHeap
