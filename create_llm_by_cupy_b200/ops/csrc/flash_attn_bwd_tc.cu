@@ -1339,8 +1339,8 @@ B200_API int b200_flash_bwd_tc(const void* q, const void* k, const void* v, cons
     B200_CHECK(launch_pdl(flash_bwd_dkv_wide_kernel<128>, dim3(dkv_ctas), dim3(FBT_THREADS), FdkwSmem<128>::kTotal, st, 0, *tq128,
                           *tdo128, *tk, *tv, *tds, p));
   else
-    B200_CHECK(launch_pdl(D == 128 ? flash_bwd_dkv_tc_kernel<128> : flash_bwd_dkv_tc_kernel<64>, dim3(dkv_ctas), dim3(FBT_THREADS), FdkvSmem::kTotal, st, 0, *tq64, *tdo64,
-                          *tk, *tv, *tds, p));
+    B200_CHECK(launch_pdl(D == 128 ? flash_bwd_dkv_tc_kernel<128> : flash_bwd_dkv_tc_kernel<64>, dim3(dkv_ctas),
+                          dim3(FBT_THREADS), FdkvSmem::kTotal, st, 0, *tq64, *tdo64, *tk, *tv, *tds, p));
   if (ds_ws != nullptr) return flash_bwd_dq_from_ds(ds_ws, k, dq, valid_len, s + 3, s + 12, B, T, QH, KVH, D, p.bchunk,
                                                       p.unrot_cos, p.unrot_sin, p.unrot_ld, st);
   if (dkv_ctas >= 3 * num_sms()) {

@@ -484,6 +484,8 @@ B200_API int b200_flash_fwd_tc3(const void* q, const void* k, const void* v, voi
   if (ctas > 0x7fffffffLL) return static_cast<int>(cudaErrorInvalidValue);
   const dim3 grid(static_cast<unsigned>(ctas));
   if (D == 128)
-    return static_cast<int>(launch_pdl(flash_fwd_tc3_kernel<128>, grid, dim3(F3<128>::kThreads), F3<128>::kSmem, st, 0, *tq, *tk, *tv, *to, p));
-  return static_cast<int>(launch_pdl(flash_fwd_tc3_kernel<64>, grid, dim3(F3<64>::kThreads), F3<64>::kSmem, st, 0, *tq, *tk, *tv, *to, p));
+    return static_cast<int>(launch_pdl(flash_fwd_tc3_kernel<128>, grid, dim3(F3<128>::kThreads), F3<128>::kSmem, st, 0, *tq, *tk,
+                                       *tv, *to, p));
+  return static_cast<int>(launch_pdl(flash_fwd_tc3_kernel<64>, grid, dim3(F3<64>::kThreads), F3<64>::kSmem, st, 0, *tq, *tk,
+                                     *tv, *to, p));
 }

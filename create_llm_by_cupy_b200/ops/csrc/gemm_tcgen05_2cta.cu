@@ -174,10 +174,10 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // By a whole warp in step; one elected lane issues (ptx.cuh says why). Under `if (lane == 0)` the four products of a k-block
-// took the issuing lane longer to set up than half a tile's take to run; a k-block of 256 x 128 then took 310 ns, 280 now (777 x
-// 768, K = 768 to 2048; the products are 135 of it, the rest is operands at 46 bytes a clock and SM). us before / now: 8192 x 768 x 4096 46.5 / 42.2, 8192 x
-// 768 x 2048 27.0 / 25.0, 8192 x 768 x 1280 19.1 / 17.3, 2048 x 1024 x 2736 19.0 / 17.6, 777 x 768 x 2048 (three pairs to a tile)
-// 10.6 / 9.3; 1.3B layers under the power cap: MLP 1383 / 1358, attention 818 / 796.
+// took the issuing lane longer to set up than half a tile's take to run; a k-block of 256 x 128 then took 310 ns, 280 now (777
+// x 768, one range of K = 768 to 2048; the products are 135 of it, the rest is operands at 46 bytes a clock and SM). us before /
+// now: 8192 x 768 x 4096 46.5 / 42.2, 8192 x 768 x 2048 27.0 / 25.0, 8192 x 768 x 1280 19.1 / 17.3, 2048 x 1024 x 2736 19.0 / 17.6,
+// 777 x 768 x 2048 (two pairs to a tile) 10.6 / 9.3; 1.3B layers under the power cap: MLP 1383 / 1358, attention 818 / 796.
 __device__ __forceinline__ void umma_bf16_ss_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                                   uint32_t accumulate) {
   asm volatile(
@@ -1028,12 +1028,14 @@ gemm_bf16_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
 
 // ------------------------------------------------------------------ few tiles: K split over a cluster
 // D = alpha A op(B) (+ C), bf16, where 256 x 128 tiles leave most CTA pairs without one (777 x 768: 24 of 74). What bounds such
-// a GEMM is what an SM can pull: 24 KiB a k-block at 46 bytes a clock, one k-block after the other. So a tile belongs to a cluster of `splits` pairs, each of which walks its own range of K; then every CTA gets, for
-// its share of the tile's columns, the other pairs' fp32 sums of its 128 rows through distributed shared memory, adds them in
-// the order of the ranges and stores. No workspace, no second launch, deterministic. A CTA has one tile, so nothing here is
-// handed out or double-buffered. us on half tiles / so: 777 x 768 x 768 8.7 / 6.9, 777 x 768 x 2048 14.3 / 9.3, 300 x 768 x 768 8.6 / 6.4,
-// 512 x 2048 x 2048 14.6 / 9.4, 1000 x 1024 x 2736 17.7 / 10.7, 640 x 768 x 4096 22.8 / 10.9, 256 x 2048 x 5504 28.6 / 12.7;
-// against K ranges in a workspace 640 x 768 x 4096 15.8 / 11.0, 256 x 4096 x 11008 29.2 / 28.2 (two pairs to a tile).
+// a GEMM is what an SM can pull: 24 KiB a k-block at 46 bytes a clock, one k-block after the other. So a tile belongs to a
+// cluster of `splits` pairs, each of which walks its own range of K; then every CTA gets, for its share of the tile's columns,
+// the other pairs' fp32 sums of its 128 rows through distributed shared memory, adds them in the order of the ranges and
+// stores. No workspace, no second launch; the sums are the same from run to run, and on any device that holds as many
+// clusters. A CTA has one tile, so nothing here is handed out or double-buffered. us on half tiles / so (cluster_splits says
+// how many pairs): 777 x 768 x 768 8.8 / 7.0, 777 x 768 x 2048 14.3 / 9.4, 300 x 768 x 768 8.6 / 6.3, 512 x 2048 x 2048 14.6 / 9.4, 1000 x
+// 1024 x 2736 17.7 / 10.8, 640 x 768 x 4096 22.9 / 11.3, 256 x 2048 x 5504 28.6 / 13.0; against K ranges in a workspace 640 x 768 x
+// 4096 15.2 / 11.3, 256 x 4096 x 11008 29.5 / 28.4.
 constexpr int GC_STAGES = 5, GC_BN = 128;
 constexpr int GC_STAGE_BYTES = G2_A_BYTES + (GC_BN / 2) * G2_BK * 2;      // 16 KiB of A, 8 KiB of B
 constexpr int GC_CHUNK = 128 * 16 * 4;                                     // 16 fp32 columns of 128 rows

@@ -550,7 +550,7 @@ def flash_attn_fwd(q, k, v, *, valid_len=None, scale=None, rope=None):
 def set_flash_bwd_wide(on: bool) -> bool:
     """head_dim 128: run the dK/dV kernel with 128-query iterations and interleaved products (default), or
     (``on`` False) the kernel with double-buffered 64-query iterations. Returns the previous setting. For A/B runs and
-    tests; head_dim 64 always runs the former."""
+    tests; head_dim 64 goes by its length: the former from 65 tokens on, the latter below."""
     return bool(_lib().b200_flash_bwd_wide(1 if on else 0))
 
 
