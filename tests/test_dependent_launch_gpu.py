@@ -57,7 +57,7 @@ def _producers():
     long_a, long_w, gate = rnd(8192, R, seed=7), rnd(8192, C, seed=8, std=1 / 90), rnd(1024, 2 * C, seed=9, std=1 / 32)
     assert G._splits(R, C, 8192, 0, None, False) > 1            # ranges in a workspace, then their sum
     yield "gemm_split_k", lambda: F.gemm(long_a, long_w, trans_a=True)
-    assert G.cluster_splits(R, C, 2048, 0) > 1 and G._splits(R, C, 2048, 0, None, True) == 1
+    assert G._splits(R, C, 2048, 0, None, True) == 1            # 32 tiles: two ranges each over the 33 clusters of a B200
     yield "gemm_cluster", lambda: F.gemm(x[:R], long_w[:2048])
     yield "gemm_swiglu", lambda: F.gemm_swiglu(a, gate)[1]
     ids = torch.arange(4096, dtype=torch.int32, device=DEV) * 3
@@ -92,10 +92,10 @@ def _consumers():
     yield "norm_bwd", lambda s: F.rmsnorm_bwd(s, x, g, rstd)
     yield "norm_bwd_x_add", lambda s: F.rmsnorm_bwd(x, s, s[-1], rstd, add=s)
     # few tiles: K over a cluster
-    assert all(G.cluster_splits(R, N, C, 0) > 1 and G._splits(R, N, C, 0, None, True) == 1 for N in (256, R, 768, C))
+    assert all(G.cluster_splits(R, N, C, 0) > 1 and G._splits(R, N, C, 0, None, True) == 1 for N in (256, R, 768, 1024))
     yield "gemm_cluster", lambda s: F.gemm(s, rnd(C, 768, seed=24))
     yield "gemm_cluster_weight_t", lambda s: F.gemm(x, s, trans_b=True)
-    yield "gemm_cluster_add", lambda s: F.gemm(x, sq, add=s)
+    yield "gemm_cluster_add", lambda s: F.gemm(x, sq[:, :1024], add=s[:, :1024])
     # more of them, or a short K: one range
     assert G.cluster_splits(R, 3072, C, 0) == G.cluster_splits(4096, R, C, 0) == G.cluster_splits(R, C, 512, 0) == 1
     wide, tall = rnd(C, 3072, seed=28, std=1 / 45), rnd(4096, C, seed=29)
